@@ -800,9 +800,13 @@ __global__ void k_to_storage(const float *__restrict__ a, T *__restrict__ b, Ite
   HFM_END_ITEMS
 }
 
-// Chunks per slot for the vector kernels (about 4096 elements each) and their grid.
-int item_chunks(int64_t n) {
-  int64_t c = (n + 4095) / 4096;
+// Chunks per slot for the vector kernels and their grid: about 4096 elements each, and down to
+// 1024 (one 16-byte access per thread) while all slots together make fewer than two chunks
+// per SM - one 64^3 slot is 64 chunks of 4096, which left more than half of the SMs idle
+// (k_cg_xr 4.4 -> 3.6 us, k_cg_p, whose chunks were four times longer, 6.7 -> 3.5 us).
+int item_chunks(int64_t n, int B) {
+  const int64_t fill = (2 * (int64_t)sm_count() + B - 1) / B;
+  const int64_t c = std::max((n + 4095) / 4096, std::min((n + 1023) / 1024, fill));
   return (int)std::max<int64_t>(1, std::min<int64_t>(c, 4096));
 }
 int item_blocks(int B, int CH) {
@@ -1295,7 +1299,7 @@ class Engine : public EngineBase {
   int outer_step(cudaStream_t s) {
     const int B = m_->slots;
     const int64_t nf = n(0);
-    const Items it{B, item_chunks(nf), nf};
+    const Items it{B, item_chunks(nf, B), nf};
     const int vb = it.CH, ib = item_blocks(B, it.CH);
     k_ir_update<<<ib, 256, 0, s>>>(m_->x64, m_->cg[0], it, m_->state, m_->outer);
     HFM_CHECK_LAUNCH("k_ir_update");
@@ -1331,7 +1335,7 @@ class Engine : public EngineBase {
     const int B = m_->slots;
     const int64_t nf = n(0);
     float *x = m_->cg[0], *r = m_->cg[1], *p = m_->cg[2], *q = m_->cg[3];
-    const Items it{B, item_chunks(nf), nf};
+    const Items it{B, item_chunks(nf, B), nf};
     const int vb = it.CH, ib = item_blocks(B, it.CH);
     const int scaled = std::is_same<T, __half>::value ? 2 : 0;
     int st;
@@ -1359,10 +1363,11 @@ class Engine : public EngineBase {
       HFM_CHECK_LAUNCH("k_dot_partials");
       nblk_rz = vb;
     }
-    // k_cg_p writes no per-chunk partials, so it takes chunks four times longer: every chunk
-    // re-sums the slot's r . z partials (three block barriers), which at 4096 elements held
-    // it near 0.7 of the copy bandwidth
-    const Items itp{B, std::max(1, it.CH / 4), nf};
+    // k_cg_p writes no per-chunk partials, so it takes chunks four times longer where those
+    // still fill the GPU: every chunk re-sums the slot's r . z partials (three block barriers),
+    // which at 4096 elements held it near 0.7 of the copy bandwidth
+    const bool fills = (int64_t)B * (it.CH / 4) >= 2 * (int64_t)sm_count();
+    const Items itp{B, fills ? it.CH / 4 : it.CH, nf};
     k_cg_p<T><<<item_blocks(B, itp.CH), 256, 0, s>>>(z, p, itp, m_->state, rz_part, nblk_rz,
                                                      m_->scal, m_->active, scaled, m_->gscale);
     HFM_CHECK_LAUNCH("k_cg_p");
@@ -1916,7 +1921,7 @@ int hfm_mg_create(const hfm_mg_config *cfg, int Z, int Y, int X, int slots, hfm_
     m->saw[1] = dalloc(m.get(), nf * es, &st);
   }
   m->partials_per_slot = std::max<int64_t>(std::max<int64_t>(4096, max_partial_blocks(lv[0], slots)),
-                                          item_chunks(lv[0].n()));
+                                          item_chunks(lv[0].n(), slots));
   m->partials = (double *)dalloc(m.get(), (size_t)slots * m->partials_per_slot * 8, &st);
   if (cfg->accel != HFM_ACCEL_NONE)
     m->partials2 = (double *)dalloc(m.get(), (size_t)slots * m->partials_per_slot * 8, &st);

@@ -501,8 +501,12 @@ int resident_blocks(const void *kernel) {
 
 // Grid shape: (plane tiles, z chunks, instances); z chunks sized so that the launch fills the
 // GPU's resident blocks once (a second, partly filled wave doubled the time of the small
-// levels: 64 instances of 32^3 made 512 blocks against 444 resident), at least 4 planes each
-// (even for the restriction).
+// levels: 64 instances of 32^3 made 512 blocks against 444 resident).  Where chunks of 4 planes
+// leave resident blocks idle, a plane more per block is a step more in a chain of dependent
+// loads and nothing else runs meanwhile, so the chunks go down to one plane (two for the
+// restriction): one instance, float32 SIGMA7, 32^3 .. 8^3, a sweep takes 6.7 us with 4-plane
+// chunks and 3.2 us with one-plane chunks.  Chunks of fewer than 4 planes are taken only while
+// the whole launch is resident, which also bounds the partial sums per instance.
 template <class T>
 dim3 fast_grid(FastArgs<T> &a, int B, int rows, bool even_chunks, int per_sm) {
   const int nvx = a.X >> 2;
@@ -511,7 +515,7 @@ dim3 fast_grid(FastArgs<T> &a, int B, int rows, bool even_chunks, int per_sm) {
   const int64_t target = (int64_t)sm_count() * per_sm;
   int64_t chunks = std::max<int64_t>(1, target / ((int64_t)tiles * B));
   int zc = (int)((a.Z + chunks - 1) / chunks);
-  if (zc < 4) zc = 4;
+  if (zc < 4 && (int64_t)tiles * B * ((a.Z + zc - 1) / zc) > target) zc = 4;
   if (even_chunks && (zc & 1)) ++zc;
   if (zc > a.Z) zc = a.Z;
   a.zc = zc;

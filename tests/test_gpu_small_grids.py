@@ -1,0 +1,49 @@
+"""Kernels and launch rules for grids that leave most of the GPU idle (one instance, small or
+ragged extents)."""
+import numpy as np
+import pytest
+
+from oracle import mg, weights as W
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def T(hfm):
+    import torch
+    return torch
+
+
+def dev(T, a):
+    return T.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).cuda()
+
+
+# one instance marches one plane per block (two for the restriction), 700 instances the
+# whole column: the same cells, the same bits
+@pytest.mark.parametrize("shape", [(2, 2, 4), (6, 4, 8), (10, 6, 12), (16, 16, 16), (34, 8, 44)])
+@pytest.mark.parametrize("form", ["const7", "k27", "sigma7"])
+def test_result_does_not_depend_on_the_chunk_length(hfm, T, shape, form):
+    B = 700
+    rng = np.random.default_rng(3)
+    x = rng.standard_normal((4,) + shape)
+    f = rng.standard_normal((4,) + shape)
+    sig = np.exp(rng.standard_normal((3, 4) + shape))
+    ops = hfm.ops
+
+    def op(rep):
+        if form == "const7":
+            return ops.Const7(0.5, 1.0, 2.0)
+        if form == "k27":
+            return ops.Stencil27(W.w5_pressure27())
+        return ops.Sigma7(*(rep(dev(T, sig[k])) for k in range(3)))
+
+    def run(rep):
+        o, xd, fd = op(rep), rep(dev(T, x)), rep(dev(T, f))
+        y = ops.jacobi(o, xd, fd, 2.0 / 3.0, sweeps=2)
+        return y, ops.residual(o, y, fd), ops.residual_restrict(o, y, fd)
+
+    one = run(lambda t: t[:1].contiguous())
+    many = run(lambda t: t.repeat(B // 4, 1, 1, 1))
+    for a, b in zip(one, many):
+        np.testing.assert_array_equal(a[0].cpu().numpy(), b[0].cpu().numpy())
+        np.testing.assert_array_equal(a[0].cpu().numpy(), b[B - 4].cpu().numpy())
