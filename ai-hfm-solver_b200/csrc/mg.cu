@@ -1191,8 +1191,8 @@ class Engine : public EngineBase {
     PhiSrc<T> p = src(still_zero ? nullptr : buf(l, cur_[l]), n(l));
     if (restricted) {
       // done by the two-sweep pass
-    } else if (xend) {
-      // residual of the iterate with its x = X-1 plane read as zero, zero there, restricted
+    } else if (xend && ((g(l).Z | g(l).Y | g(l).X) & 1)) {
+      // odd extents: the residual as a field, then the flooring restriction
       T *rf = (T *)m_->saw[0];
       p.zero_xend = 1;
       if ((st = launch_residual<T>(lk(l), lo(l), p, rhs(l), n(l), rf, n(l), m_->slots,
@@ -1201,10 +1201,14 @@ class Engine : public EngineBase {
         return st;
       if ((st = launch_restrict<T>(rf, n(l), rhs(l + 1), n(l + 1), m_->slots, g(l), m_->active, s)))
         return st;
-    } else if ((st = launch_residual_restrict<T>(lk(l), lo(l), p, rhs(l), n(l), nullptr, 0,
-                                                 rhs(l + 1), n(l + 1), m_->slots, g(l), 0u,
-                                                 m_->active, chk ? m_->partials : nullptr, &nblk, s)))
-      return st;
+    } else {
+      // x-end rule: residual of the iterate with its x = X-1 plane read as zero, zero there
+      p.zero_xend = xend;
+      if ((st = launch_residual_restrict<T>(lk(l), lo(l), p, rhs(l), n(l), nullptr, 0, rhs(l + 1),
+                                            n(l + 1), m_->slots, g(l), xend ? HFM_FLAG_ZERO_XEND : 0u,
+                                            m_->active, chk ? m_->partials : nullptr, &nblk, s)))
+        return st;
+    }
     if (chk && (st = check(nblk, cur_[0], s))) return st;
     if (fcycle) {
       if ((st = vcycle(l + 1, true, true, 0, s))) return st;

@@ -176,6 +176,27 @@ __device__ __forceinline__ double block_reduce(double v) {
   return t;
 }
 
+// RESTRICT: the two coarse cells of a thread's vector gain plane z of its residuals (x pairs
+// within the vector, y pairs across the two rows); an odd plane completes and stores them.
+template <class T, int R>
+__device__ __forceinline__ void coarse_cells(const FastArgs<T> &a, int64_t inst, int z, int g, int x0,
+                                             bool valid, const F4 (&res)[R], float (&cpart)[2]) {
+  cpart[0] += 0.125f * ((res[0].v[0] + res[0].v[1]) + (res[R - 1].v[0] + res[R - 1].v[1]));
+  cpart[1] += 0.125f * ((res[0].v[2] + res[0].v[3]) + (res[R - 1].v[2] + res[R - 1].v[3]));
+  if (!(z & 1)) return;
+  if (valid) {
+    const int Yc = a.Y >> 1, Xc = a.X >> 1;
+    T *cp = a.coarse + inst * a.coarse_stride + ((int64_t)(z >> 1) * Yc + g) * Xc + (x0 >> 1);
+    if (sizeof(T) == 4) {
+      *reinterpret_cast<float2 *>(cp) = make_float2(cpart[0], cpart[1]);
+    } else {
+      cp[0] = St<T>::from(cpart[0]);
+      cp[1] = St<T>::from(cpart[1]);
+    }
+  }
+  cpart[0] = cpart[1] = 0.f;
+}
+
 // ---------------------------------------------------------------------------------------
 // 7-point forms (CONST7, SIGMA7).  R rows per thread.
 // ---------------------------------------------------------------------------------------
@@ -355,24 +376,7 @@ __global__ void __launch_bounds__(kFastThreads, R == 1 ? 4 : 2)
       pm[r] = pc[r];
       pc[r] = pp[r];
     }
-    if (MODE == M_RESTRICT) {
-      // x-pairs within the vector, y-pairs across the thread's two rows, z-pairs over planes
-      cpart[0] += 0.125f * ((res[0].v[0] + res[0].v[1]) + (res[R - 1].v[0] + res[R - 1].v[1]));
-      cpart[1] += 0.125f * ((res[0].v[2] + res[0].v[3]) + (res[R - 1].v[2] + res[R - 1].v[3]));
-      if (z & 1) {
-        if (valid) {
-          const int Yc = Y >> 1, Xc = X >> 1;
-          T *cp = a.coarse + inst * a.coarse_stride + ((int64_t)(z >> 1) * Yc + g) * Xc + (x0 >> 1);
-          if (sizeof(T) == 4) {
-            *reinterpret_cast<float2 *>(cp) = make_float2(cpart[0], cpart[1]);
-          } else {
-            cp[0] = St<T>::from(cpart[0]);
-            cp[1] = St<T>::from(cpart[1]);
-          }
-        }
-        cpart[0] = cpart[1] = 0.f;
-      }
-    }
+    if (MODE == M_RESTRICT) coarse_cells<T, R>(a, inst, z, g, x0, valid, res, cpart);
   }
   if ((MODE != M_SMOOTH || a.dot_rhs) && a.partials) {
     double t = block_reduce(acc);
@@ -381,9 +385,13 @@ __global__ void __launch_bounds__(kFastThreads, R == 1 ? 4 : 2)
 }
 
 // ---------------------------------------------------------------------------------------
-// 27-point form (K27): per-plane partial sums into three pending outputs.
+// 27-point form (K27): per-plane partial sums into three pending outputs.  R rows per thread:
+// one for sweeps and residuals, two for the residual + restriction, whose four input rows per
+// plane serve both.  On one instance of 16 x 32 x 32 the latter takes 7.8 us, bound by its
+// chain of dependent loads; a thread per coarse cell with 216 bounds-checked loads took 21 us
+// (and 82 us on 64 x 128 x 128, where the plane-marching TMA kernel takes 8 us).
 // ---------------------------------------------------------------------------------------
-template <class T, int MODE, int CORR>
+template <class T, int MODE, int CORR, int R>
 __global__ void __launch_bounds__(kFastThreads)
     k_fast27(FastArgs<T> a) {
   const int64_t inst = blockIdx.z;
@@ -391,92 +399,109 @@ __global__ void __launch_bounds__(kFastThreads)
   const int X = a.X, Y = a.Y, Z = a.Z;
   const int nvx = X >> 2;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = i < Y * nvx;
-  const int y = valid ? i / nvx : 0;
-  const int x0 = valid ? (i - y * nvx) * 4 : 0;
+  const int ngroups = (Y + R - 1) / R;
+  const bool valid = i < ngroups * nvx;
+  const int g = valid ? i / nvx : 0;
+  const int y0 = g * R;  // RESTRICT: Y is even, so both rows are inside
+  const int x0 = valid ? (i - g * nvx) * 4 : 0;
   const int64_t ib = inst * a.stride, ic = inst * a.corr_stride;
   const int64_t plane = (int64_t)Y * X;
   const int z0 = blockIdx.y * a.zc;
   const int z1 = min(Z, z0 + a.zc);
   const float *K = a.op.k;
 
-  // s[a] of plane p = sum_{b,c} K[a][b][c] phi'(p, y+b-1, x+c-1)
-  auto plane_sums = [&](int p, F4 &s0, F4 &s1, F4 &s2, F4 &centre) {
-    F4 rows[3];
-    float ls[3], rs[3];
+  // s[a][r] of plane p = sum_{b,c} K[a][b][c] phi'(p, y0+r+b-1, x+c-1)
+  auto plane_sums = [&](int p, F4 (&s0)[R], F4 (&s1)[R], F4 (&s2)[R], F4 (&centre)[R]) {
+    F4 rows[R + 2];
+    float ls[R + 2], rs[R + 2];
 #pragma unroll
-    for (int b = 0; b < 3; ++b) {
-      const int yy = y + b - 1;
+    for (int b = 0; b < R + 2; ++b) {
+      const int yy = y0 + b - 1;
       const bool in = valid && p >= 0 && p < Z && yy >= 0 && yy < Y;
       rows[b] = phi_vec<T, CORR>(a, ib, ic, p, yy, x0, in);
       halo_x<T, CORR>(a, ib, ic, p, yy, x0, in, rows[b], ls[b], rs[b]);
     }
-    centre = rows[1];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float t0 = 0.f, t1 = 0.f, t2 = 0.f;
+    for (int r = 0; r < R; ++r) {
+      centre[r] = rows[r + 1];
 #pragma unroll
-      for (int b = 0; b < 3; ++b) {
-        const float xm = e == 0 ? ls[b] : rows[b].v[e - 1];
-        const float xc = rows[b].v[e];
-        const float xp = e == 3 ? rs[b] : rows[b].v[e + 1];
-        t0 += K[3 * b + 0] * xm + K[3 * b + 1] * xc + K[3 * b + 2] * xp;
-        t1 += K[9 + 3 * b + 0] * xm + K[9 + 3 * b + 1] * xc + K[9 + 3 * b + 2] * xp;
-        t2 += K[18 + 3 * b + 0] * xm + K[18 + 3 * b + 1] * xc + K[18 + 3 * b + 2] * xp;
+      for (int e = 0; e < 4; ++e) {
+        float t0 = 0.f, t1 = 0.f, t2 = 0.f;
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+          const float xm = e == 0 ? ls[r + b] : rows[r + b].v[e - 1];
+          const float xc = rows[r + b].v[e];
+          const float xp = e == 3 ? rs[r + b] : rows[r + b].v[e + 1];
+          t0 += K[3 * b + 0] * xm + K[3 * b + 1] * xc + K[3 * b + 2] * xp;
+          t1 += K[9 + 3 * b + 0] * xm + K[9 + 3 * b + 1] * xc + K[9 + 3 * b + 2] * xp;
+          t2 += K[18 + 3 * b + 0] * xm + K[18 + 3 * b + 1] * xc + K[18 + 3 * b + 2] * xp;
+        }
+        s0[r].v[e] = t0;
+        s1[r].v[e] = t1;
+        s2[r].v[e] = t2;
       }
-      s0.v[e] = t0;
-      s1.v[e] = t1;
-      s2.v[e] = t2;
     }
   };
 
   // pending: out(z) = s0(z-1) + s1(z) + s2(z+1)
-  F4 acc_cur, acc_next, cen_cur, cen_next, d0, d1, d2, dc;
-  plane_sums(z0 - 1, d0, d1, d2, dc);
-  F4 s0, s1, s2;
-  plane_sums(z0, s0, s1, s2, cen_cur);
+  F4 acc_cur[R], acc_next[R], cen_cur[R], cen_next[R];
+  {
+    F4 d0[R], d1[R], d2[R], dc[R], s0[R], s1[R], s2[R];
+    plane_sums(z0 - 1, d0, d1, d2, dc);
+    plane_sums(z0, s0, s1, s2, cen_cur);
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    acc_cur.v[e] = d0.v[e] + s1.v[e];
-    acc_next.v[e] = s0.v[e];
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        acc_cur[r].v[e] = d0[r].v[e] + s1[r].v[e];
+        acc_next[r].v[e] = s0[r].v[e];
+      }
   }
   const float diag = K[13];
   double acc2 = 0.0;
+  float cpart[2] = {0.f, 0.f};  // RESTRICT: the two coarse cells of this vector, summed over planes
   for (int z = z0; z < z1; ++z) {
-    F4 n0, n1, n2;
+    F4 n0[R], n1[R], n2[R], res[R];
     plane_sums(z + 1, n0, n1, n2, cen_next);
-    F4 Ax, res;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) Ax.v[e] = acc_cur.v[e] + n2.v[e];
-    const int64_t off = (int64_t)z * plane + (int64_t)y * X + x0;
-    F4 f{{0.f, 0.f, 0.f, 0.f}};
-    if (a.rhs && valid) f = ld4<T>(a.rhs + ib + off);
-    if (MODE == M_SMOOTH) {
+    for (int r = 0; r < R; ++r) {
+      const int y = y0 + r;
+      const bool in = valid && y < Y;
+      F4 Ax;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) res.v[e] = cen_cur.v[e] + a.omega * __fdividef(f.v[e] - Ax.v[e], diag);
-      if (a.dot_rhs && valid) {
+      for (int e = 0; e < 4; ++e) Ax.v[e] = acc_cur[r].v[e] + n2[r].v[e];
+      const int64_t off = (int64_t)z * plane + (int64_t)y * X + x0;
+      F4 f{{0.f, 0.f, 0.f, 0.f}};
+      if (a.rhs && in) f = ld4<T>(a.rhs + ib + off);
+      if (MODE == M_SMOOTH) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc2 += (double)res.v[e] * f.v[e];
+        for (int e = 0; e < 4; ++e) res[r].v[e] = cen_cur[r].v[e] + a.omega * __fdividef(f.v[e] - Ax.v[e], diag);
+        if (a.dot_rhs && in) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc2 += (double)res[r].v[e] * f.v[e];
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) res[r].v[e] = Ax.v[e] - f.v[e];
+        if (a.zero_xend_out && x0 + 4 == X) res[r].v[3] = 0.f;
+        if (in) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            acc2 += (double)res[r].v[e] * (a.dot_phi ? cen_cur[r].v[e] : res[r].v[e]);
+        }
       }
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) res.v[e] = Ax.v[e] - f.v[e];
-      if (a.zero_xend_out && x0 + 4 == X) res.v[3] = 0.f;
-      if (valid) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc2 += (double)res.v[e] * (a.dot_phi ? cen_cur.v[e] : res.v[e]);
+      if (in && a.out) {
+        if (MODE == M_SMOOTH && a.top_copy && z == 1) st4<T>(a.out + ib + y * X + x0, res[r]);
+        if (!(MODE == M_SMOOTH && a.top_copy && z == 0 && Z > 1)) st4<T>(a.out + ib + off, res[r]);
       }
-    }
-    if (valid && a.out) {
-      if (MODE == M_SMOOTH && a.top_copy && z == 1) st4<T>(a.out + ib + y * X + x0, res);
-      if (!(MODE == M_SMOOTH && a.top_copy && z == 0 && Z > 1)) st4<T>(a.out + ib + off, res);
-    }
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      acc_cur.v[e] = acc_next.v[e] + n1.v[e];
-      acc_next.v[e] = n0.v[e];
+      for (int e = 0; e < 4; ++e) {
+        acc_cur[r].v[e] = acc_next[r].v[e] + n1[r].v[e];
+        acc_next[r].v[e] = n0[r].v[e];
+      }
+      cen_cur[r] = cen_next[r];
     }
-    cen_cur = cen_next;
+    if (MODE == M_RESTRICT) coarse_cells<T, R>(a, inst, z, g, x0, valid, res, cpart);
   }
   if ((MODE != M_SMOOTH || a.dot_rhs) && a.partials) {
     double t = block_reduce(acc2);
@@ -529,7 +554,6 @@ bool fast_eligible(int kind, Grid3 g, bool restrict_mode) {
     return false;
   if ((g.X & 3) || g.X < 4) return false;
   if (restrict_mode) {
-    if (kind == HFM_OP_K27) return false;
     if ((g.Y & 1) || (g.Z & 1)) return false;
   }
   return true;
@@ -576,12 +600,13 @@ int fast_launch(int kind, int mode, const DevOp &op, const PhiSrc<T> &phi, const
   // dispatch
   if (kind == HFM_OP_K27) {
     if (mode == M_SMOOTH) {
-      if (corr == C_NONE) HFM_FAST_GO((k_fast27<T, M_SMOOTH, C_NONE>));
-      else if (corr == C_COARSE) HFM_FAST_GO((k_fast27<T, M_SMOOTH, C_COARSE>));
-      else HFM_FAST_GO((k_fast27<T, M_SMOOTH, C_SAME>));
+      if (corr == C_NONE) HFM_FAST_GO((k_fast27<T, M_SMOOTH, C_NONE, 1>));
+      else if (corr == C_COARSE) HFM_FAST_GO((k_fast27<T, M_SMOOTH, C_COARSE, 1>));
+      else HFM_FAST_GO((k_fast27<T, M_SMOOTH, C_SAME, 1>));
     } else {
       if (corr != C_NONE) return fail(HFM_ERR_UNSUPPORTED, "fast path: corrected residual");
-      HFM_FAST_GO((k_fast27<T, M_RESID, C_NONE>));
+      if (mode == M_RESID) HFM_FAST_GO((k_fast27<T, M_RESID, C_NONE, 1>));
+      else HFM_FAST_GO((k_fast27<T, M_RESTRICT, C_NONE, 2>));
     }
   } else {
 #define HFM_FAST7(KIND)                                                                        \

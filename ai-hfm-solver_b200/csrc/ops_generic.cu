@@ -398,13 +398,13 @@ template <class T>
 int launch_residual(int kind, const DevOp &op, const PhiSrc<T> &phi, const T *b,
                     int64_t b_stride, T *r, int64_t r_stride, int B, Grid3 g, unsigned flags,
                     const int *active, double *partials, int *nblk_out, cudaStream_t s) {
-  if (phi.base && !phi.corr && !phi.zero_xend && r && phi.base_stride == r_stride &&
+  if (phi.base && !phi.corr && r && phi.base_stride == r_stride &&
       (!b || b_stride == r_stride) && tma_eligible(kind, g, FAST_RESID, nullptr, 0, (int)sizeof(T)) &&
       face_tma_ok<T>(kind, phi, flags) &&
       vec_aligned<T>(kind, op, phi, b, r, nullptr, r_stride, 16))
     return tma_launch<T>(kind, FAST_RESID, op, phi, b, r, nullptr, r_stride, 0, B, g, 0.f,
                          flags, active, partials, nblk_out, s);
-  if (fast_eligible(kind, g, false) && !phi.corr && !phi.zero_xend && r &&
+  if (fast_eligible(kind, g, false) && !phi.corr && r &&
       (!b || b_stride == r_stride) && (!phi.base || phi.base_stride == r_stride) &&
       vec_aligned<T>(kind, op, phi, b, r, nullptr, r_stride, 4 * (int64_t)sizeof(T)))
     return fast_launch<T>(kind, FAST_RESID, op, phi, b, r, nullptr, r_stride, 0, B, g, 0.f,
@@ -433,14 +433,14 @@ int launch_residual_restrict(int kind, const DevOp &op, const PhiSrc<T> &phi, co
                              const int *active, double *partials, int *nblk_out,
                              cudaStream_t s) {
   if ((g.Z | g.Y | g.X) & 1) return fail(HFM_ERR_BAD_ARG, "residual_restrict needs even extents");
-  if (phi.base && !phi.corr && !phi.zero_xend && b && phi.base_stride == b_stride &&
+  if (phi.base && !phi.corr && b && phi.base_stride == b_stride &&
       (!r_fine || rf_stride == b_stride) && rc_stride == b_stride / 8 &&
       tma_eligible(kind, g, FAST_RESTRICT, nullptr, 0, (int)sizeof(T)) &&
       face_tma_ok<T>(kind, phi, flags) &&
       vec_aligned<T>(kind, op, phi, b, r_fine, nullptr, b_stride, 16))
     return tma_launch<T>(kind, FAST_RESTRICT, op, phi, b, r_fine, r_coarse, b_stride, rc_stride,
                          B, g, 0.f, flags, active, partials, nblk_out, s);
-  if (fast_eligible(kind, g, true) && !phi.corr && !phi.zero_xend && b &&
+  if (fast_eligible(kind, g, true) && !phi.corr && b &&
       (!r_fine || rf_stride == b_stride) && (!phi.base || phi.base_stride == b_stride) &&
       rc_stride == b_stride / 8 &&
       vec_aligned<T>(kind, op, phi, b, r_fine, r_coarse, b_stride, 4 * (int64_t)sizeof(T)))

@@ -637,7 +637,7 @@ bool tma_eligible(int kind, Grid3 g, int mode, const void *corr, int corr_coarse
   if (corr && !corr_coarse) return false;
   if (corr && ((g.X / 2) * es) % 16) return false;
   if (corr && ((g.Y | g.Z) & 1)) return false;
-  if (mode == M_RESTRICT && (kind == HFM_OP_K27 || (g.Y & 1) || (g.Z & 1))) return false;
+  if (mode == M_RESTRICT && ((g.Y & 1) || (g.Z & 1))) return false;
   if (mode != M_SMOOTH && corr) return false;
   return true;
 }
@@ -904,6 +904,7 @@ int tma_launch(int kind, int mode, const DevOp &op, const PhiSrc<T> &phi, const 
     HFM_TMA_GO(HFM_OP_CONST7, M_RESTRICT, 0);
   } else {
     HFM_TMA_MODES(HFM_OP_K27)
+    HFM_TMA_GO(HFM_OP_K27, M_RESTRICT, 0);
   }
 #undef HFM_TMA_MODES
 #undef HFM_TMA_GO

@@ -47,3 +47,26 @@ def test_result_does_not_depend_on_the_chunk_length(hfm, T, shape, form):
     for a, b in zip(one, many):
         np.testing.assert_array_equal(a[0].cpu().numpy(), b[0].cpu().numpy())
         np.testing.assert_array_equal(a[0].cpu().numpy(), b[B - 4].cpu().numpy())
+
+
+# the 27-point residual + restriction: plane-marching (X >= 48), register-queue and generic
+# kernels; the x-end rule comes with the handle's outflow rule
+@pytest.mark.parametrize("shape", [(2, 2, 4), (4, 6, 8), (6, 34, 20), (10, 8, 48), (12, 18, 64), (6, 16, 68), (4, 4, 6)])
+@pytest.mark.parametrize("xend", [False, True])
+def test_pressure_residual_restriction(hfm, T, shape, xend):
+    rng = np.random.default_rng(5)
+    B = 3
+    x = rng.standard_normal((B,) + shape).astype(np.float32)
+    f = rng.standard_normal((B,) + shape).astype(np.float32)
+    K = rng.standard_normal((3, 3, 3))
+    rc, rf = hfm.ops.residual_restrict(hfm.ops.Stencil27(K), dev(T, x), dev(T, f),
+                                       flags=hfm._lib.FLAG_ZERO_XEND if xend else 0, want_fine=True)
+    op = mg.Stencil27(np.asarray(K, np.float32), dtype=np.float64)
+    for b in range(B):
+        ref = mg.residual(op, x[b], f[b])
+        if xend:
+            ref[..., -1] = 0
+        scale = np.abs(ref).max()  # 27 products of O(1): 28 roundings of 6e-8 of it
+        assert np.abs(rf[b].cpu().numpy() - ref).max() <= 1e-5 * scale
+        c = ref.reshape(shape[0] // 2, 2, shape[1] // 2, 2, shape[2] // 2, 2).mean(axis=(1, 3, 5))
+        assert np.abs(rc[b].cpu().numpy() - c).max() <= 1e-5 * scale
