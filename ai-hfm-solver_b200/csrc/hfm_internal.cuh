@@ -297,8 +297,31 @@ template <class T> struct SubArgs {
   float omega, coarse_omega;
   int nu_pre, nu_post, coarse_sweeps;
 };
+// The steps of the fused coarse levels: operation, level (0 = l0) and repetitions, in order.
+enum SubOp : unsigned char {
+  SO_SWEEP0,        // `count` sweeps, the first from a zero iterate
+  SO_SWEEP,         // `count` sweeps of the current iterate
+  SO_RESTRICT0,     // right-hand side of the next level = R(-f) (zero iterate)
+  SO_RESTRICT,      // right-hand side of the next level = R(A phi - f)
+  SO_RESTRICT_RHS,  // right-hand side of the next level = R f
+  SO_CORRECT0,      // phi = -P (next level's iterate)
+  SO_CORRECT,       // phi -= P (next level's iterate)
+  SO_PROLONG,       // phi = P (next level's iterate)
+  SO_COARSE         // the coarsest level: `count` sweeps from zero with coarse_omega
+};
+constexpr int kMaxSubSteps = 160;
+template <class T> struct SubProgram {
+  SubArgs<T> a;
+  int nsteps;
+  unsigned char op[kMaxSubSteps], lev[kMaxSubSteps], cnt[kMaxSubSteps];
+  const T *phi0;  // initial iterate of level l0 (nullable: zero), instance stride lv[0].n
+  // with store_all, where the right-hand sides and iterates of the levels below l0 are written
+  int store_all;
+  T *g_rhs[kMaxSubLevels], *g_phi[kMaxSubLevels];
+  int o_top;      // float offset of the pair sums of level l0 (quad form)
+};
 size_t subcycle_smem_bytes(const Grid3 *g, int nlev, bool sigma);
-template <class T> int launch_subcycle(int kind, SubArgs<T> a, int B, cudaStream_t s);
+template <class T> int launch_subprogram(int kind, SubProgram<T> &p, int B, cudaStream_t s);
 
 // The small end of a V-cycle as one persistent kernel (subcycle.cu): a level l1 that the
 // plane-marching TMA kernels do not take, with the fused coarse cycle directly below it.

@@ -1002,9 +1002,6 @@ class Engine : public EngineBase {
     if ((k != HFM_OP_SIGMA7 && k != HFM_OP_CONST7 && k != HFM_OP_K27) ||
         (c.options & HFM_OPT_NO_FUSED_COARSE))
       return -1;
-    // one block per instance: with few instances the separate kernels, which spread a level
-    // over many SMs, are as fast (measured: a single 64 x 128 x 128 pressure solve)
-    if (m_->slots < 8) return -1;
     if (n(m_->L - 1) > coarse_smem_limit()) return -1;
     int l0 = m_->L - 1;
     while (l0 - 1 >= 1 && n(l0 - 1) <= 4096 && m_->L - (l0 - 1) <= kMaxSubLevels) --l0;
@@ -1012,13 +1009,48 @@ class Engine : public EngineBase {
     Grid3 gs[kMaxSubLevels];
     for (int l = l0; l < m_->L; ++l) gs[l - l0] = g(l);
     if (subcycle_smem_bytes(gs, m_->L - l0, k == HFM_OP_SIGMA7) > kSubcycleMaxSmem) return -1;
-    return l0;
+    SubProgram<T> p;  // the longest list of the cycle form fits
+    return fused_program(l0, c.cycle == HFM_CYCLE_F ? SUB_FV : SUB_V, p) ? l0 : -1;
   }
 
-  int fused_vcycle(int l0, cudaStream_t s) {
-    SubArgs<T> a = make_sub(l0);
+  // Steps of the cycles vcycle() runs from level l down (l relative to l0): V from a zero or the
+  // current iterate, F from zero.  Returns false when the list is full.
+  static bool add_step(SubProgram<T> &p, SubOp op, int l, int cnt) {
+    if (p.nsteps >= kMaxSubSteps || cnt > 255) return false;
+    p.op[p.nsteps] = op;
+    p.lev[p.nsteps] = (unsigned char)l;
+    p.cnt[p.nsteps++] = (unsigned char)cnt;
+    return true;
+  }
+  bool add_cycle(SubProgram<T> &p, int l, bool zero, bool fcycle) {
+    const hfm_mg_config &c = m_->cfg;
+    if (l == p.a.nlev - 1) return add_step(p, SO_COARSE, l, c.coarse_sweeps);
+    if (c.nu_pre && !add_step(p, zero ? SO_SWEEP0 : SO_SWEEP, l, c.nu_pre)) return false;
+    const bool still_zero = zero && c.nu_pre == 0;
+    if (!add_step(p, still_zero ? SO_RESTRICT0 : SO_RESTRICT, l, 1)) return false;
+    if (!add_cycle(p, l + 1, true, fcycle)) return false;
+    // the coarsest level is solved from zero: a second visit would repeat the first
+    if (fcycle && l + 1 < p.a.nlev - 1 && !add_cycle(p, l + 1, false, false)) return false;
+    if (!add_step(p, still_zero ? SO_CORRECT0 : SO_CORRECT, l, 1)) return false;
+    return !c.nu_post || add_step(p, SO_SWEEP, l, c.nu_post);
+  }
+
+  // The levels from l0 down in one launch: a V-cycle from the zero or the current iterate, an
+  // F-cycle from zero, or that F-cycle followed by a V-cycle (the two coarse visits of an
+  // F-cycle).
+  enum { SUB_V0, SUB_V, SUB_F, SUB_FV };
+  int fused_cycle(int l0, int what, cudaStream_t s) {
+    SubProgram<T> p;
+    if (!fused_program(l0, what, p)) return fail(HFM_ERR_BAD_ARG, "fused coarse levels: too many steps");
+    if (what == SUB_V) p.phi0 = buf(l0, cur_[l0]);
     cur_[l0] = 0;
-    return launch_subcycle<T>(kind(), a, m_->slots, s);
+    return launch_subprogram<T>(kind(), p, m_->slots, s);
+  }
+  bool fused_program(int l0, int what, SubProgram<T> &p) {
+    memset(&p, 0, sizeof(p));
+    p.a = make_sub(l0);
+    if (!add_cycle(p, 0, what != SUB_V, what == SUB_F || what == SUB_FV)) return false;
+    return what != SUB_FV || add_cycle(p, 0, false, false);
   }
 
   // Arguments of the fused coarse cycle from level l0 down (right-hand side rhs(l0), result
@@ -1153,7 +1185,7 @@ class Engine : public EngineBase {
     int st;
     if (l == m_->L - 1) return coarse_solve(l, s);
     if (zero && !fcycle && !(l == 0 && check_level0) && small_ok(l)) return small_vcycle(l, s);
-    if (zero && !fcycle && l > 0 && l == fused_l0_) return fused_vcycle(l, s);
+    if (l > 0 && l == fused_l0_) return fused_cycle(l, fcycle ? SUB_F : zero ? SUB_V0 : SUB_V, s);
     if (zero) cur_[l] = 0;
     // NS outflow rule on the fine level (as the reference cycle applies it): the iterate is
     // read as zero on x = X-1 and the residual is zero there
@@ -1211,8 +1243,13 @@ class Engine : public EngineBase {
     }
     if (chk && (st = check(nblk, cur_[0], s))) return st;
     if (fcycle) {
-      if ((st = vcycle(l + 1, true, true, 0, s))) return st;
-      if ((st = vcycle(l + 1, false, false, 0, s))) return st;
+      if (l + 1 == fused_l0_) {
+        if ((st = fused_cycle(l + 1, SUB_FV, s))) return st;
+      } else {
+        if ((st = vcycle(l + 1, true, true, 0, s))) return st;
+        // the coarsest level is solved from zero: a second visit would repeat the first
+        if (l + 1 < m_->L - 1 && (st = vcycle(l + 1, false, false, 0, s))) return st;
+      }
     } else {
       if ((st = vcycle(l + 1, true, false, 0, s))) return st;
     }

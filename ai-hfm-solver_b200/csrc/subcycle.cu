@@ -322,12 +322,432 @@ __device__ void subcycle_body(const SubArgs<T> &a, int64_t inst, unsigned char *
     a.out[inst * (int64_t)L0.n + i] = St<T>::from(res[pix(w.z, w.y, w.x, L0.Y, L0.X)]);
 }
 
+// ------------------------------------------------------------------ the program kernel
+// One block of 1024 threads per instance interprets a list of steps (V or F cycles from a
+// zero or a given iterate, or the reference's sawtooth leg) over the levels from l0 down.  It
+// is bound by the chain of barrier-separated passes on one SM, so each pass is made short:
+//   * level l0 (TOP: rows of a multiple of 4 cells) belongs to the threads quad by quad: a
+//     thread keeps its quad's right-hand side, face coefficients, 1 / diagonal and iterate in
+//     registers for the whole launch, x neighbours come by shuffle, and a sweep reads four
+//     16-byte rows (y and z neighbours) of unpadded-in-x fields, free of bank conflicts;
+//   * the levels below run one cell per thread from shared memory; the restricted residual
+//     forms every fine residual in its own thread and then sums eight;
+//   * the coarsest level's sweeps keep each cell's coefficients in registers and synchronise
+//     only the warps that hold cells.
+// One instance of 16^3 .. 4^3 (SIGMA7 float32, V(2,2), 32 coarsest sweeps): 24 us a launch
+// against 47 us for the eleven launches it replaces; in a served bf16 stream, beside other
+// kernels, 34 us against 55 us for 512 threads with all fields and faces in padded shared
+// arrays.  8 x 16 x 16 and 4 x 8 x 8 of the 27-point operator, the F-cycle's F and V visits
+// in one launch: 35 us against 160 us launch by launch.
+constexpr int kProgThreads = 1024;
+
+// fc = R(A phi - f), in two phases: every fine residual by its own thread into `res` (padded,
+// interior), then the eight of each coarse cell in the order z, y, x.
 template <int KIND, class T>
-__global__ void __launch_bounds__(kSubThreads) k_subcycle(const __grid_constant__ SubArgs<T> a) {
+__device__ void prog_restrict(const SubLevel<T> &L, const float *ph, const float *Fc, const float *f,
+                              float *res, const SubLevel<T> &Lc, float *fc) {
+  Walk w(threadIdx.x, blockDim.x, L.Y, L.X);
+  for (int i = threadIdx.x; i < L.n; i += blockDim.x, w.step(L.Y, L.X)) {
+    const int ip = pix(w.z, w.y, w.x, L.Y, L.X);
+    float dg;
+    const float ax = ph ? sub_apply<KIND, T>(L, ph, Fc, w.z, w.y, w.x, ip, i, &dg) : 0.f;
+    res[ip] = ax - f[i];
+  }
+  __syncthreads();
+  const int PX = L.X + 2, PXY = PX * (L.Y + 2);
+  Walk v(threadIdx.x, blockDim.x, Lc.Y, Lc.X);
+  for (int j = threadIdx.x; j < Lc.n; j += blockDim.x, v.step(Lc.Y, Lc.X)) {
+    const float *q = res + pix(2 * v.z, 2 * v.y, 2 * v.x, L.Y, L.X);
+    float sum = 0.f;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) sum += q[(c >> 2) * PXY + ((c >> 1) & 1) * PX + (c & 1)];
+    fc[j] = 0.125f * sum;
+  }
+  __syncthreads();
+}
+
+// fc = R f (f unpadded)
+template <class T>
+__device__ void prog_restrict_rhs(const SubLevel<T> &L, const float *f, const SubLevel<T> &Lc, float *fc) {
+  Walk v(threadIdx.x, blockDim.x, Lc.Y, Lc.X);
+  for (int j = threadIdx.x; j < Lc.n; j += blockDim.x, v.step(Lc.Y, Lc.X)) {
+    const float *q = f + (2 * v.z * L.Y + 2 * v.y) * L.X + 2 * v.x;
+    float sum = 0.f;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) sum += 0.125f * q[((c >> 2) * L.Y + ((c >> 1) & 1)) * L.X + (c & 1)];
+    fc[j] = sum;
+  }
+  __syncthreads();
+}
+
+// phi = [phi] + sign * P(coarse) on the level's interior (both padded)
+template <class T>
+__device__ void prog_correct(const SubLevel<T> &L, float *ph, const SubLevel<T> &Lc, const float *coarse,
+                             float sign, bool zero) {
+  Walk w(threadIdx.x, blockDim.x, L.Y, L.X);
+  for (int i = threadIdx.x; i < L.n; i += blockDim.x, w.step(L.Y, L.X)) {
+    const int ip = pix(w.z, w.y, w.x, L.Y, L.X);
+    const float c = sign * coarse[pix(w.z >> 1, w.y >> 1, w.x >> 1, Lc.Y, Lc.X)];
+    ph[ip] = zero ? c : ph[ip] + c;
+  }
+  __syncthreads();
+}
+
+// `sweeps` sweeps from zero on the coarsest level; returns the buffer holding the result.
+// Up to 1024 cells: one per thread, its coefficients in registers, a barrier among the warps
+// that hold cells (a warp barrier when one does).
+template <int KIND, class T>
+__device__ int prog_coarse(const SubLevel<T> &L, float *F, float om, int sweeps) {
+  float *buf[2] = {F + L.o_phi, F + L.o_tmp};
+  const float *f = F + L.o_rhs, *Fc = F + L.o_face;
+  const int n = L.n;
+  if (n > (int)blockDim.x) {
+    for (int k = 0; k < sweeps; ++k)
+      sub_sweep<KIND, T>(L, k == 0 ? nullptr : buf[k & 1], Fc, f, buf[(k & 1) ^ 1], om, buf[k & 1]);
+    return sweeps & 1;
+  }
+  const int nthr = (n + 31) & ~31;
+  if ((int)threadIdx.x < nthr) {
+    const int X = L.X, Y = L.Y, Z = L.Z, PX = X + 2, PXY = PX * (Y + 2);
+    const int i = min((int)threadIdx.x, n - 1);
+    const bool in = (int)threadIdx.x < n;
+    const int x = i % X, t = i / X, y = t % Y, z = t / Y;
+    const int ip = pix(z, y, x, Y, X);
+    constexpr int NK = KIND == HFM_OP_K27 ? 27 : 6;
+    float c[NK], rd;
+    if (KIND == HFM_OP_K27) {
+#pragma unroll
+      for (int j = 0; j < NK; ++j) c[j] = L.k[j];
+      rd = __fdividef(1.f, L.k[13]);
+    } else if (KIND == HFM_OP_CONST7) {
+      c[0] = c[1] = L.k[2];
+      c[2] = c[3] = L.k[1];
+      c[4] = c[5] = L.k[0];
+      rd = __fdividef(1.f, 2.f * (L.k[0] + L.k[1] + L.k[2]));
+    } else {
+      const float *fx = Fc, *fy = fx + Z * Y * (X + 1), *fz = fy + Z * (Y + 1) * X, *dg = fz + (Z + 1) * Y * X;
+      const int ixf = (z * Y + y) * (X + 1) + x, iyf = (z * (Y + 1) + y) * X + x;
+      c[0] = fx[ixf];
+      c[1] = fx[ixf + 1];
+      c[2] = fy[iyf];
+      c[3] = fy[iyf + X];
+      c[4] = fz[i];
+      c[5] = fz[i + X * Y];
+      rd = __fdividef(1.f, dg[i]);
+    }
+    const float fv = f[i];
+    float v = om * (fv * rd);
+    if (in) buf[1][ip] = v;
+    for (int k = 1; k < sweeps; ++k) {
+      if (nthr == 32) __syncwarp();
+      else asm volatile("bar.sync 1, %0;" ::"r"(nthr) : "memory");
+      const float *p = buf[k & 1] + ip;
+      float ax;
+      if (KIND == HFM_OP_K27) {
+        ax = 0.f;
+#pragma unroll
+        for (int j = 0; j < 27; ++j)
+          if (c[j] != 0.f) ax += c[j] * p[(j / 9 - 1) * PXY + ((j / 3) % 3 - 1) * PX + (j % 3 - 1)];
+      } else if (KIND == HFM_OP_CONST7) {
+        ax = 2.f * (c[4] + c[2] + c[0]) * v - c[4] * (p[-PXY] + p[PXY]) - c[2] * (p[-PX] + p[PX]) -
+             c[0] * (p[-1] + p[1]);
+      } else {
+        ax = c[0] * (v - p[-1]) + c[1] * (v - p[1]) + c[2] * (v - p[-PX]) + c[3] * (v - p[PX]) +
+             c[4] * (v - p[-PXY]) + c[5] * (v - p[PXY]);
+      }
+      v += om * ((fv - ax) * rd);
+      if (in) buf[(k & 1) ^ 1][ip] = v;
+    }
+  }
+  __syncthreads();
+  return sweeps & 1;
+}
+
+// Four consecutive values of T as float and back (16 or 8 bytes).
+template <class T> __device__ __forceinline__ void ldq4(const T *p, float (&v)[4]) {
+  if constexpr (sizeof(T) == 4) {
+    const float4 m = *reinterpret_cast<const float4 *>(p);
+    v[0] = m.x; v[1] = m.y; v[2] = m.z; v[3] = m.w;
+  } else {
+    const uint2 u = *reinterpret_cast<const uint2 *>(p);
+    const T *h = reinterpret_cast<const T *>(&u);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = St<T>::to(h[e]);
+  }
+}
+template <class T> __device__ __forceinline__ void stq4(T *p, const float (&v)[4]) {
+  if constexpr (sizeof(T) == 4) {
+    *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  } else {
+    T h[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) h[e] = St<T>::from(v[e]);
+    *reinterpret_cast<uint2 *>(p) = *reinterpret_cast<const uint2 *>(h);
+  }
+}
+
+// A thread's quad of level l0 (quad form).  Fields are [Z + 2][Y + 2][X], the ghost rows and
+// planes zero; `ip` is the quad's first cell in them.
+template <int KIND> struct TopQuad {
+  int x0, y, z, ip, X, Y, PZ;
+  bool valid, work;  // holds cells; its warp does (the shuffles need whole warps)
+  float f[4], p[4];
+  // SIGMA7: x faces of the four cells, y and z faces below and above, 1 / diagonal
+  float ax[KIND == HFM_OP_SIGMA7 ? 5 : 1], ay[2][KIND == HFM_OP_SIGMA7 ? 4 : 1],
+      az[2][KIND == HFM_OP_SIGMA7 ? 4 : 1], rd[KIND == HFM_OP_SIGMA7 ? 4 : 1];
+
+  // neighbours across the quad's ends of row values v (row base pointer r, in the grid)
+  __device__ __forceinline__ void ends(const float *r, const float (&v)[4], float &l, float &h) const {
+    l = __shfl_up_sync(0xffffffffu, v[3], 1);
+    h = __shfl_down_sync(0xffffffffu, v[0], 1);
+    const int lane = threadIdx.x & 31;
+    if (lane == 0 && x0 > 0) l = r[-1];
+    if (lane == 31 && x0 + 4 < X) h = r[4];
+    if (x0 == 0) l = 0.f;
+    if (x0 + 4 == X) h = 0.f;
+  }
+  template <class T>
+  __device__ __forceinline__ void apply(const SubLevel<T> &L, const float *ph, float (&A)[4]) const {
+    const float *c = ph + ip;
+    if (KIND == HFM_OP_K27) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) A[e] = 0.f;
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+          const float *r = c + (a - 1) * PZ + (b - 1) * X;
+          float m[4], l, h;
+          if (a == 1 && b == 1) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) m[e] = p[e];
+          } else {
+            ldq4<float>(r, m);
+          }
+          ends(r, m, l, h);
+          const float k0 = L.k[9 * a + 3 * b], k1 = L.k[9 * a + 3 * b + 1], k2 = L.k[9 * a + 3 * b + 2];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            A[e] += k0 * (e == 0 ? l : m[e - 1]);
+            A[e] += k1 * m[e];
+            A[e] += k2 * (e == 3 ? h : m[e + 1]);
+          }
+        }
+      return;
+    }
+    float l, h, ym[4], yp[4], zm[4], zp[4];
+    ldq4<float>(c - X, ym);
+    ldq4<float>(c + X, yp);
+    ldq4<float>(c - PZ, zm);
+    ldq4<float>(c + PZ, zp);
+    ends(c, p, l, h);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float xm = e == 0 ? l : p[e - 1], xp = e == 3 ? h : p[e + 1];
+      if (KIND == HFM_OP_CONST7) {
+        const float kz = L.k[0], ky = L.k[1], kx = L.k[2], d = 2.f * (kz + ky + kx);
+        A[e] = d * p[e] - kz * (zm[e] + zp[e]) - ky * (ym[e] + yp[e]) - kx * (xm + xp);
+      } else {
+        A[e] = ax[e] * (p[e] - xm) + ax[e + 1] * (p[e] - xp) + ay[0][e] * (p[e] - ym[e]) +
+               ay[1][e] * (p[e] - yp[e]) + az[0][e] * (p[e] - zm[e]) + az[1][e] * (p[e] - zp[e]);
+      }
+    }
+  }
+  template <class T> __device__ __forceinline__ float rdiag(const SubLevel<T> &L, int e) const {
+    if (KIND == HFM_OP_SIGMA7) return rd[e];
+    return __fdividef(1.f, KIND == HFM_OP_K27 ? L.k[13] : 2.f * (L.k[0] + L.k[1] + L.k[2]));
+  }
+  __device__ __forceinline__ void store(float *ph) const {
+    if (valid) *reinterpret_cast<float4 *>(ph + ip) = make_float4(p[0], p[1], p[2], p[3]);
+  }
+  template <class T> __device__ void init(const SubLevel<T> &L, int64_t inst, const T *rhs) {
+    X = L.X;
+    Y = L.Y;
+    PZ = (Y + 2) * X;
+    const int nvx = X >> 2, nq = L.n >> 2, q = threadIdx.x;
+    valid = q < nq;
+    work = (q & ~31) < nq;
+    const int qq = valid ? q : 0;
+    const int t = qq / nvx;
+    x0 = 4 * (qq - t * nvx);
+    y = t % Y;
+    z = t / Y;
+    ip = (z + 1) * PZ + (y + 1) * X + x0;
+    if (!valid) x0 = 0;
+    const int64_t i = inst * (int64_t)L.n + 4 * qq;
+    ldq4<T>(rhs + i, f);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) p[e] = 0.f;
+    if (KIND == HFM_OP_SIGMA7) {
+      const T *sx = L.sx + i, *sy = L.sy + i, *sz = L.sz + i;
+      const int P = X * Y;
+      float c[4], lo[4], hi[4];
+      ldq4<T>(sx, c);
+      ax[0] = L.cx * (x0 > 0 ? 0.5f * (c[0] + St<T>::to(sx[-1])) : c[0]);
+      ax[4] = L.cx * (x0 + 4 < X ? 0.5f * (c[3] + St<T>::to(sx[4])) : c[3]);
+#pragma unroll
+      for (int e = 1; e < 4; ++e) ax[e] = L.cx * (0.5f * (c[e] + c[e - 1]));
+      ldq4<T>(sy, c);
+      ldq4<T>(y > 0 ? sy - X : sy, lo);
+      ldq4<T>(y + 1 < Y ? sy + X : sy, hi);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        ay[0][e] = L.cy * (0.5f * (c[e] + lo[e]));  // at a wall (s + s) / 2 = s
+        ay[1][e] = L.cy * (0.5f * (c[e] + hi[e]));
+      }
+      ldq4<T>(sz, c);
+      ldq4<T>(z > 0 ? sz - P : sz, lo);
+      ldq4<T>(z + 1 < L.Z ? sz + P : sz, hi);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        az[0][e] = L.cz * (0.5f * (c[e] + lo[e]));
+        az[1][e] = L.cz * (0.5f * (c[e] + hi[e]));
+        rd[e] = __fdividef(1.f, ax[e] + ax[e + 1] + ay[0][e] + ay[1][e] + az[0][e] + az[1][e]);
+      }
+    }
+  }
+};
+
+template <int KIND, class T, bool TOP>
+__global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant__ SubProgram<T> P) {
+  const SubArgs<T> &a = P.a;
   const int64_t inst = blockIdx.x;
   if (a.active && !a.active[inst]) return;
   extern __shared__ __align__(16) unsigned char sub_smem[];
-  subcycle_body<KIND, T, false>(a, inst, sub_smem);
+  float *F = reinterpret_cast<float *>(sub_smem);
+  const int nl = a.nlev;
+  const SubLevel<T> &L0 = a.lv[0];
+  TopQuad<KIND> tq;
+  // both fields of every level zero (the ghosts stay so), face arrays, right-hand side of l0
+  for (int l = 0; l < nl; ++l) {
+    const SubLevel<T> &L = a.lv[l];
+    for (int i = threadIdx.x; i < L.o_rhs - L.o_phi; i += kProgThreads) F[L.o_phi + i] = 0.f;
+    if (KIND == HFM_OP_SIGMA7 && !(TOP && l == 0)) sub_faces_init<T>(L, inst, F + L.o_face);
+  }
+  if (TOP) {
+    tq.template init<T>(L0, inst, a.rhs);
+  } else {
+    for (int i = threadIdx.x; i < L0.n; i += kProgThreads) F[L0.o_rhs + i] = St<T>::to(a.rhs[inst * (int64_t)L0.n + i]);
+  }
+  __syncthreads();
+  if (P.phi0) {  // the given iterate of l0, in its first field
+    const T *src = P.phi0 + inst * (int64_t)L0.n;
+    if (TOP) {
+      if (tq.valid) ldq4<T>(src + 4 * threadIdx.x, tq.p);
+      tq.store(F + L0.o_phi);
+    } else {
+      Walk w(threadIdx.x, kProgThreads, L0.Y, L0.X);
+      for (int i = threadIdx.x; i < L0.n; i += kProgThreads, w.step(L0.Y, L0.X))
+        F[L0.o_phi + pix(w.z, w.y, w.x, L0.Y, L0.X)] = St<T>::to(src[i]);
+    }
+    __syncthreads();
+  }
+  unsigned cur = 0;  // bit l: level l's iterate is in tmp
+  for (int s = 0; s < P.nsteps; ++s) {
+    const int op = P.op[s], l = P.lev[s], cnt = P.cnt[s];
+    const SubLevel<T> &L = a.lv[l];
+    const SubLevel<T> &Lc = a.lv[l + 1 < nl ? l + 1 : l];
+    const int c = (cur >> l) & 1;
+    float *ph = F + (c ? L.o_tmp : L.o_phi);    // the iterate
+    float *other = F + (c ? L.o_phi : L.o_tmp);
+    float *coarse = F + (((cur >> (l + 1)) & 1) ? Lc.o_tmp : Lc.o_phi);
+    if (op == SO_COARSE) {
+      const int r = prog_coarse<KIND, T>(L, F, a.coarse_omega, cnt);
+      cur = (cur & ~(1u << l)) | ((unsigned)r << l);
+    } else if (TOP && l == 0) {
+      if (op == SO_SWEEP0 || op == SO_SWEEP) {
+        for (int k = 0; k < cnt; ++k) {
+          if (tq.work) {
+            if (op == SO_SWEEP0 && k == 0) {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) tq.p[e] = a.omega * (tq.f[e] * tq.rdiag(L, e));
+            } else {
+              float A[4];
+              tq.apply(L0, ph, A);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) tq.p[e] += a.omega * ((tq.f[e] - A[e]) * tq.rdiag(L, e));
+            }
+            tq.store(other);
+          }
+          __syncthreads();
+          float *t = ph;
+          ph = other;
+          other = t;
+        }
+        if (cnt & 1) cur ^= 1u;
+      } else if (op == SO_RESTRICT || op == SO_RESTRICT0 || op == SO_RESTRICT_RHS) {
+        // x pairs of the quad's residuals, then the four rows of each coarse cell
+        float *pairs = F + P.o_top;
+        const float scale = op == SO_RESTRICT_RHS ? -1.f : 1.f;  // r = A phi - f, or f itself
+        if (tq.work) {
+          float A[4] = {0.f, 0.f, 0.f, 0.f};
+          if (op == SO_RESTRICT) tq.apply(L0, ph, A);
+          if (tq.valid)
+            *reinterpret_cast<float2 *>(pairs + 2 * threadIdx.x) =
+                make_float2(scale * ((A[0] - tq.f[0]) + (A[1] - tq.f[1])),
+                            scale * ((A[2] - tq.f[2]) + (A[3] - tq.f[3])));
+        }
+        __syncthreads();
+        const int Xh = L.X >> 1;
+        Walk v(threadIdx.x, kProgThreads, Lc.Y, Lc.X);
+        for (int j = threadIdx.x; j < Lc.n; j += kProgThreads, v.step(Lc.Y, Lc.X)) {
+          const float *q = pairs + (2 * v.z * L.Y + 2 * v.y) * Xh + v.x;
+          const float *q1 = q + L.Y * Xh;
+          F[Lc.o_rhs + j] = 0.125f * ((q[0] + q[Xh]) + (q1[0] + q1[Xh]));
+        }
+        __syncthreads();
+      } else {  // SO_CORRECT0, SO_CORRECT, SO_PROLONG
+        if (tq.valid) {
+          const float sign = op == SO_PROLONG ? 1.f : -1.f;
+          const int ic = pix(tq.z >> 1, tq.y >> 1, tq.x0 >> 1, Lc.Y, Lc.X);
+          const float c0 = sign * coarse[ic], c1 = sign * coarse[ic + 1];
+          const bool z0 = op != SO_CORRECT;
+          tq.p[0] = z0 ? c0 : tq.p[0] + c0;
+          tq.p[1] = z0 ? c0 : tq.p[1] + c0;
+          tq.p[2] = z0 ? c1 : tq.p[2] + c1;
+          tq.p[3] = z0 ? c1 : tq.p[3] + c1;
+          tq.store(ph);
+        }
+        __syncthreads();
+      }
+    } else {
+      const float *f = F + L.o_rhs, *Fc = F + L.o_face;
+      if (op == SO_SWEEP0 || op == SO_SWEEP) {
+        for (int k = 0; k < cnt; ++k) {
+          sub_sweep<KIND, T>(L, op == SO_SWEEP0 && k == 0 ? nullptr : ph, Fc, f, other, a.omega, ph);
+          float *t = ph;
+          ph = other;
+          other = t;
+        }
+        if (cnt & 1) cur ^= 1u << l;
+      } else if (op == SO_RESTRICT || op == SO_RESTRICT0) {
+        prog_restrict<KIND, T>(L, op == SO_RESTRICT0 ? nullptr : ph, Fc, f, other, Lc, F + Lc.o_rhs);
+      } else if (op == SO_RESTRICT_RHS) {
+        prog_restrict_rhs<T>(L, f, Lc, F + Lc.o_rhs);
+      } else {
+        prog_correct<T>(L, ph, Lc, coarse, op == SO_PROLONG ? 1.f : -1.f, op != SO_CORRECT);
+      }
+    }
+  }
+  T *out = a.out + inst * (int64_t)L0.n;
+  if (TOP) {
+    if (tq.valid) stq4<T>(out + 4 * threadIdx.x, tq.p);
+  } else {
+    const float *res = F + ((cur & 1) ? L0.o_tmp : L0.o_phi);
+    Walk w(threadIdx.x, kProgThreads, L0.Y, L0.X);
+    for (int i = threadIdx.x; i < L0.n; i += kProgThreads, w.step(L0.Y, L0.X))
+      out[i] = St<T>::from(res[pix(w.z, w.y, w.x, L0.Y, L0.X)]);
+  }
+  if (P.store_all)
+    for (int l = 1; l < nl; ++l) {
+      const SubLevel<T> &L = a.lv[l];
+      const float *res = F + (((cur >> l) & 1) ? L.o_tmp : L.o_phi);
+      Walk w(threadIdx.x, kProgThreads, L.Y, L.X);
+      for (int i = threadIdx.x; i < L.n; i += kProgThreads, w.step(L.Y, L.X)) {
+        P.g_rhs[l][inst * (int64_t)L.n + i] = St<T>::from(F[L.o_rhs + i]);
+        P.g_phi[l][inst * (int64_t)L.n + i] = St<T>::from(res[pix(w.z, w.y, w.x, L.Y, L.X)]);
+      }
+    }
 }
 
 }  // namespace
@@ -340,16 +760,6 @@ size_t subcycle_smem_bytes(const Grid3 *g, int nlev, bool sigma) {
     if (sigma) f += (size_t)sub_faces(Z, Y, X) + n;
   }
   return ((f * 4 + 15) / 16) * 16;
-}
-
-template <int KIND, class T>
-int go_subcycle(const SubArgs<T> &a, int B, size_t smem, cudaStream_t s) {
-  int st = set_max_dynamic_smem((const void *)k_subcycle<KIND, T>, (int)kSubcycleMaxSmem,
-                                "cudaFuncSetAttribute(k_subcycle)");
-  if (st) return st;
-  k_subcycle<KIND, T><<<B, kSubThreads, smem, s>>>(a);
-  HFM_CHECK_LAUNCH("k_subcycle");
-  return HFM_OK;
 }
 
 // Shared-memory layout of the coarse-end cycle, level after level: phi and tmp (padded), rhs,
@@ -565,20 +975,57 @@ template int launch_small<float>(int, SmallArgs<float>, int, cudaStream_t);
 template int launch_small<__nv_bfloat16>(int, SmallArgs<__nv_bfloat16>, int, cudaStream_t);
 template int launch_small<__half>(int, SmallArgs<__half>, int, cudaStream_t);
 
+template <int KIND, class T, bool TOP>
+int go_subprog(const SubProgram<T> &p, int B, size_t smem, cudaStream_t s) {
+  int st = set_max_dynamic_smem((const void *)k_subprog<KIND, T, TOP>, (int)kSubcycleMaxSmem,
+                                "cudaFuncSetAttribute(k_subprog)");
+  if (st) return st;
+  k_subprog<KIND, T, TOP><<<B, kProgThreads, smem, s>>>(p);
+  HFM_CHECK_LAUNCH("k_subprog");
+  return HFM_OK;
+}
+
 template <class T>
-int launch_subcycle(int kind, SubArgs<T> a, int B, cudaStream_t s) {
-  const size_t smem = layout_sub<T>(kind, a);
+int launch_subprogram(int kind, SubProgram<T> &p, int B, cudaStream_t s) {
+  const SubLevel<T> &L0 = p.a.lv[0];
+  // the quad form: whole quads per row, and at most one quad per thread
+  const bool top = (L0.X & 3) == 0 && L0.n <= 4 * kProgThreads;
+  size_t smem = layout_sub<T>(kind, p.a);
   if (!smem) return fail(HFM_ERR_BAD_ARG, "subcycle: levels exceed shared memory");
+  if (top) {  // level l0 keeps two fields without x ghosts and the pair sums; no faces
+    SubLevel<T> &L = p.a.lv[0];
+    const int np = (L.Z + 2) * (L.Y + 2) * L.X;
+    L.o_phi = 0;
+    L.o_tmp = np;
+    L.o_rhs = L.o_face = 2 * np;
+    p.o_top = 2 * np;
+    int off = 2 * np + L.n / 2;
+    for (int l = 1; l < p.a.nlev; ++l) {
+      SubLevel<T> &q = p.a.lv[l];
+      const int shift = off - q.o_phi;
+      const int size = (l + 1 < p.a.nlev ? p.a.lv[l + 1].o_phi : (int)(smem / 4)) - q.o_phi;
+      q.o_phi += shift;
+      q.o_tmp += shift;
+      q.o_rhs += shift;
+      q.o_face += shift;
+      off += size;
+    }
+    smem = (size_t)off * 4;
+    if (smem > kSubcycleMaxSmem) return fail(HFM_ERR_BAD_ARG, "subcycle: levels exceed shared memory");
+  }
   switch (kind) {
-    case HFM_OP_SIGMA7: return go_subcycle<HFM_OP_SIGMA7, T>(a, B, smem, s);
-    case HFM_OP_CONST7: return go_subcycle<HFM_OP_CONST7, T>(a, B, smem, s);
-    case HFM_OP_K27: return go_subcycle<HFM_OP_K27, T>(a, B, smem, s);
+    case HFM_OP_SIGMA7:
+      return top ? go_subprog<HFM_OP_SIGMA7, T, true>(p, B, smem, s) : go_subprog<HFM_OP_SIGMA7, T, false>(p, B, smem, s);
+    case HFM_OP_CONST7:
+      return top ? go_subprog<HFM_OP_CONST7, T, true>(p, B, smem, s) : go_subprog<HFM_OP_CONST7, T, false>(p, B, smem, s);
+    case HFM_OP_K27:
+      return top ? go_subprog<HFM_OP_K27, T, true>(p, B, smem, s) : go_subprog<HFM_OP_K27, T, false>(p, B, smem, s);
     default: return fail(HFM_ERR_UNSUPPORTED, "subcycle: operator kind");
   }
 }
 
-template int launch_subcycle<float>(int, SubArgs<float>, int, cudaStream_t);
-template int launch_subcycle<__nv_bfloat16>(int, SubArgs<__nv_bfloat16>, int, cudaStream_t);
-template int launch_subcycle<__half>(int, SubArgs<__half>, int, cudaStream_t);
+template int launch_subprogram<float>(int, SubProgram<float> &, int, cudaStream_t);
+template int launch_subprogram<__nv_bfloat16>(int, SubProgram<__nv_bfloat16> &, int, cudaStream_t);
+template int launch_subprogram<__half>(int, SubProgram<__half> &, int, cudaStream_t);
 
 }  // namespace hfm

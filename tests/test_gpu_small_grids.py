@@ -70,3 +70,31 @@ def test_pressure_residual_restriction(hfm, T, shape, xend):
         assert np.abs(rf[b].cpu().numpy() - ref).max() <= 1e-5 * scale
         c = ref.reshape(shape[0] // 2, 2, shape[1] // 2, 2, shape[2] // 2, 2).mean(axis=(1, 3, 5))
         assert np.abs(rc[b].cpu().numpy() - c).max() <= 1e-5 * scale
+
+
+# the fused coarse levels against one launch per level step: first fused level in quads
+# (X % 4 == 0) and cell by cell (X % 4 != 0), one level and several below it, every operator,
+# V and F cycles (the F-cycle's second visit starts from a non-zero iterate)
+@pytest.mark.parametrize("shape", [(16, 16, 16), (32, 24, 40), (20, 20, 20), (12, 36, 28), (8, 64, 24)])
+@pytest.mark.parametrize("form", ["const7", "k27", "sigma7"])
+@pytest.mark.parametrize("cycle,nu", [("V", (2, 2)), ("V", (0, 1)), ("V", (1, 0)), ("F", (2, 2)), ("F", (1, 2))])
+def test_fused_coarse_levels_few_slots(hfm, T, shape, form, cycle, nu):
+    M, ops = hfm.multigrid, hfm.ops
+    rng = np.random.default_rng(17)
+    B = 2
+    f = dev(T, rng.standard_normal((B,) + shape))
+    sig = np.exp(rng.standard_normal((3, B) + shape))
+    op = {"const7": lambda: ops.Const7(0.5, 1.0, 2.0), "k27": lambda: ops.Stencil27(W.w5_pressure27()),
+          "sigma7": lambda: ops.Sigma7(*(dev(T, sig[k]) for k in range(3)))}[form]()
+    outs = []
+    for fused in (True, False):
+        cfg = M.SolverConfig(cycle=cycle, nu_pre=nu[0], nu_post=nu[1], tol=1e-300, max_cycles=10,
+                             coarse_sweeps=5, min_coarse_edge=3, fused_coarse=fused)
+        with M.Multigrid(shape, op.kind, cfg, slots=B) as h:
+            h.set_operator(op)
+            for s in range(B):
+                h.load(s, f[s].contiguous())
+            h.run(3)
+            outs.append(np.stack([h.fetch(s).cpu().numpy() for s in range(B)]))
+    # three cycles of a few dozen float32 roundings per value, damped by the smoothing
+    assert np.abs(outs[0] - outs[1]).max() <= 1e-5 * np.abs(outs[1]).max()
