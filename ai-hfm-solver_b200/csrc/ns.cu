@@ -60,34 +60,47 @@ __device__ __forceinline__ Quad my_quad(int64_t nq, int Y, int nvx) {
   return c;
 }
 
-// Values x0 - 1 .. x0 + 4 of row (z, y) of f, zero outside the grid.  VEC: X a multiple of 4
-// and f 16-byte aligned; every lane of the warp calls it (shuffles).
-template <bool VEC>
-__device__ __forceinline__ void row6(const float *f, int z, int y, const Quad &c, int Z, int Y, int X,
-                                     float (&v)[6]) {
-  const bool in = c.valid && z >= 0 && z < Z && y >= 0 && y < Y;
-  const float *r = f + ((int64_t)z * Y + y) * X + c.x0;
-  if (VEC) {
-    float4 m = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (in) m = __ldg(reinterpret_cast<const float4 *>(r));
-    const int lane = threadIdx.x & 31;
-    float l = __shfl_up_sync(0xffffffffu, m.w, 1), h = __shfl_down_sync(0xffffffffu, m.x, 1);
-    if (lane == 0 && in && c.x0 > 0) l = __ldg(r - 1);
-    if (lane == 31 && in && c.x0 + 4 < X) h = __ldg(r + 4);
-    v[0] = in && c.x0 > 0 ? l : 0.f;
-    v[1] = m.x;
-    v[2] = m.y;
-    v[3] = m.z;
-    v[4] = m.w;
-    v[5] = in && c.x0 + 4 < X ? h : 0.f;
-  } else {
+// A row of one field around a thread's quad, loaded (the loads of several rows are issued
+// before the first is used) and then completed to the values x0 - 1 .. x0 + 4, zero outside
+// the grid.  VEC: X a multiple of 4 and f 16-byte aligned - one 16-byte load, the two edge
+// values from the neighbouring lanes (lanes 0 and 31 load theirs); every lane of the warp
+// calls both.
+template <bool VEC> struct Row {
+  float m[VEC ? 5 : 6];  // VEC: the quad and the edge that lanes 0 / 31 load
+  bool in;
+  __device__ __forceinline__ void load(const float *f, int z, int y, const Quad &c, int Z, int Y, int X) {
+    in = c.valid && z >= 0 && z < Z && y >= 0 && y < Y;
+    const float *r = f + ((int64_t)z * Y + y) * X + c.x0;
+    if (VEC) {
+      float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (in) q = __ldg(reinterpret_cast<const float4 *>(r));
+      m[0] = q.x; m[1] = q.y; m[2] = q.z; m[3] = q.w;
+      const int lane = threadIdx.x & 31;
+      m[4] = 0.f;
+      if (in && lane == 0 && c.x0 > 0) m[4] = __ldg(r - 1);
+      if (in && lane == 31 && c.x0 + 4 < X) m[4] = __ldg(r + 4);
+    } else {
 #pragma unroll
-    for (int e = 0; e < 6; ++e) {
-      const int x = c.x0 + e - 1;
-      v[e] = in && x >= 0 && x < X ? __ldg(r + e - 1) : 0.f;
+      for (int e = 0; e < 6; ++e) {
+        const int x = c.x0 + e - 1;
+        m[e % (VEC ? 5 : 6)] = in && x >= 0 && x < X ? __ldg(r + e - 1) : 0.f;
+      }
     }
   }
-}
+  __device__ __forceinline__ void values(const Quad &c, int X, float (&v)[6]) const {
+    if (VEC) {
+      const int lane = threadIdx.x & 31;
+      const float l = __shfl_up_sync(0xffffffffu, m[3], 1), h = __shfl_down_sync(0xffffffffu, m[0], 1);
+      v[0] = in && c.x0 > 0 ? (lane == 0 ? m[4] : l) : 0.f;
+      v[5] = in && c.x0 + 4 < X ? (lane == 31 ? m[4] : h) : 0.f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e + 1] = m[e];
+    } else {
+#pragma unroll
+      for (int e = 0; e < 6; ++e) v[e] = m[e % (VEC ? 5 : 6)];
+    }
+  }
+};
 
 template <bool VEC>
 __device__ __forceinline__ void ldq(const float *p, const Quad &c, int X, float (&v)[4]) {
@@ -132,13 +145,18 @@ __global__ void __launch_bounds__(kRowThreads) k_momentum(const __grid_constant_
     for (int q = 0; q < 4; ++q) d[f][q][0] = d[f][q][1] = make_float2(0.f, 0.f);
   float cen[3][4];
 #pragma unroll
-  for (int a = 0; a < 3; ++a)
+  for (int a = 0; a < 3; ++a) {
+    Row<VEC> rows[3][3];  // a plane's nine rows in flight together
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+#pragma unroll
+      for (int f = 0; f < 3; ++f) rows[b][f].load(m.a[f], c.z + a - 1, c.y + b - 1, c, Z, Y, X);
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
       float v[3][6];
 #pragma unroll
       for (int f = 0; f < 3; ++f) {
-        row6<VEC>(m.a[f], c.z + a - 1, c.y + b - 1, c, Z, Y, X, v[f]);
+        rows[b][f].values(c, X, v[f]);
         if (a == 1 && b == 1) {
 #pragma unroll
           for (int e = 0; e < 4; ++e) cen[f][e] = v[f][e + 1];
@@ -156,6 +174,7 @@ __global__ void __launch_bounds__(kRowThreads) k_momentum(const __grid_constant_
           }
         }
     }
+  }
   if (!c.valid) return;
   const int64_t i = ((int64_t)c.z * Y + c.y) * X + c.x0;
 #pragma unroll
@@ -273,12 +292,15 @@ __global__ void __launch_bounds__(kRowThreads) k_pgrad(const __grid_constant__ G
   float2 d[3][2];
 #pragma unroll
   for (int q = 0; q < 3; ++q) d[q][0] = d[q][1] = make_float2(0.f, 0.f);
+  Row<VEC> rows[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) rows[k].load(m.p, c.z + k / 3 - 1, c.y + k % 3 - 1, c, Z, Y, X);
 #pragma unroll
   for (int a = 0; a < 3; ++a)
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
       float v[6];
-      row6<VEC>(m.p, c.z + a - 1, c.y + b - 1, c, Z, Y, X, v);
+      rows[3 * a + b].values(c, X, v);
 #pragma unroll
       for (int t = 0; t < 3; ++t)
 #pragma unroll
@@ -315,13 +337,18 @@ __global__ void __launch_bounds__(kRowThreads) k_divergence(const __grid_constan
 #pragma unroll
   for (int q = 0; q < 3; ++q) d[q][0] = d[q][1] = make_float2(0.f, 0.f);
 #pragma unroll
-  for (int a = 0; a < 3; ++a)
+  for (int a = 0; a < 3; ++a) {
+    Row<VEC> rows[3][3];
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) rows[b][q].load(m.a[q], c.z + a - 1, c.y + b - 1, c, Z, Y, X);
 #pragma unroll
     for (int b = 0; b < 3; ++b)
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
         float v[6];
-        row6<VEC>(m.a[q], c.z + a - 1, c.y + b - 1, c, Z, Y, X, v);
+        rows[b][q].values(c, X, v);
 #pragma unroll
         for (int t = 0; t < 3; ++t) {
           const float2 w = m.K.k[9 * a + 3 * b + t][q];
@@ -329,6 +356,7 @@ __global__ void __launch_bounds__(kRowThreads) k_divergence(const __grid_constan
           d[q][1] = __ffma2_rn(w, make_float2(v[t + 2], v[t + 3]), d[q][1]);
         }
       }
+  }
   if (!c.valid) return;
   float o[4];
   o[0] = -((d[0][0].x + d[1][0].x) + d[2][0].x);
