@@ -287,6 +287,7 @@ template <class T> struct SubLevel {
   const T *sx, *sy, *sz;     // the level's conductivities, instance stride n
   int o_phi, o_tmp, o_rhs;   // float offsets of the level's fields in shared memory
   int o_face;                // float offset of its face arrays and diagonal (SIGMA7)
+  int o_idx;                 // float offset of its cell table (8 bytes per cell)
 };
 template <class T> struct SubArgs {
   SubLevel<T> lv[kMaxSubLevels];
@@ -319,8 +320,10 @@ template <class T> struct SubProgram {
   int store_all;
   T *g_rhs[kMaxSubLevels], *g_phi[kMaxSubLevels];
   int o_top;      // float offset of the pair sums of level l0 (quad form)
+  int clear;      // 16-byte words of shared memory in use
 };
 size_t subcycle_smem_bytes(const Grid3 *g, int nlev, bool sigma);
+template <class T> bool subprogram_fits(int kind, SubProgram<T> &p);
 template <class T> int launch_subprogram(int kind, SubProgram<T> &p, int B, cudaStream_t s);
 
 // The small end of a V-cycle as one persistent kernel (subcycle.cu): a level l1 that the

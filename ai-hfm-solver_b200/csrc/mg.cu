@@ -1006,11 +1006,8 @@ class Engine : public EngineBase {
     int l0 = m_->L - 1;
     while (l0 - 1 >= 1 && n(l0 - 1) <= 4096 && m_->L - (l0 - 1) <= kMaxSubLevels) --l0;
     if (l0 >= m_->L - 1) return -1;
-    Grid3 gs[kMaxSubLevels];
-    for (int l = l0; l < m_->L; ++l) gs[l - l0] = g(l);
-    if (subcycle_smem_bytes(gs, m_->L - l0, k == HFM_OP_SIGMA7) > kSubcycleMaxSmem) return -1;
-    SubProgram<T> p;  // the longest list of the cycle form fits
-    return fused_program(l0, c.cycle == HFM_CYCLE_F ? SUB_FV : SUB_V, p) ? l0 : -1;
+    SubProgram<T> p;  // the longest list of the cycle form and the levels' fields fit
+    return fused_program(l0, c.cycle == HFM_CYCLE_F ? SUB_FV : SUB_V, p) && subprogram_fits<T>(k, p) ? l0 : -1;
   }
 
   // Steps of the cycles vcycle() runs from level l down (l relative to l0): V from a zero or the
@@ -1091,6 +1088,10 @@ class Engine : public EngineBase {
   bool small_ok(int l) {
     const hfm_mg_config &c = m_->cfg;
     if (!(c.options & HFM_OPT_PERSISTENT) || fused_l0_ < 0 || l + 1 != fused_l0_) return false;
+    if (m_->slots < 8) return false;  // one block holds a slot's coarse end
+    Grid3 gs[kMaxSubLevels];
+    for (int k = l + 1; k < m_->L; ++k) gs[k - l - 1] = g(k);
+    if (subcycle_smem_bytes(gs, m_->L - l - 1, kind() == HFM_OP_SIGMA7) > kSubcycleMaxSmem) return false;
     if (lk(l) == HFM_OP_FACE7) return false;
     if (tma_eligible(lk(l), g(l), FAST_SMOOTH, nullptr, 0, (int)sizeof(T))) return false;
     if ((g(l).Z | g(l).Y | g(l).X) & 1) return false;

@@ -323,140 +323,360 @@ __device__ void subcycle_body(const SubArgs<T> &a, int64_t inst, unsigned char *
 }
 
 // ------------------------------------------------------------------ the program kernel
-// One block of 1024 threads per instance interprets a list of steps (V or F cycles from a
-// zero or a given iterate, or the reference's sawtooth leg) over the levels from l0 down.  It
-// is bound by the chain of barrier-separated passes on one SM, so each pass is made short:
-//   * level l0 (TOP: rows of a multiple of 4 cells) belongs to the threads quad by quad: a
-//     thread keeps its quad's right-hand side, face coefficients, 1 / diagonal and iterate in
-//     registers for the whole launch, x neighbours come by shuffle, and a sweep reads four
-//     16-byte rows (y and z neighbours) of unpadded-in-x fields, free of bank conflicts;
-//   * the levels below run one cell per thread from shared memory; the restricted residual
-//     forms every fine residual in its own thread and then sums eight;
-//   * the coarsest level's sweeps keep each cell's coefficients in registers and synchronise
-//     only the warps that hold cells.
-// One instance of 16^3 .. 4^3 (SIGMA7 float32, V(2,2), 32 coarsest sweeps): 24 us a launch
-// against 47 us for the eleven launches it replaces; in a served bf16 stream, beside other
-// kernels, 34 us against 55 us for 512 threads with all fields and faces in padded shared
-// arrays.  8 x 16 x 16 and 4 x 8 x 8 of the 27-point operator, the F-cycle's F and V visits
-// in one launch: 35 us against 160 us launch by launch.
-constexpr int kProgThreads = 1024;
+// One block of 512 threads per instance interprets a list of steps (V or F cycles from a zero
+// or a given iterate, or the reference's sawtooth leg) over the levels from l0 down.  It is
+// bound by the chain of barrier-separated passes on one SM - each pass by its shared-memory
+// wavefronts - so each pass reads as little as it can:
+//   * level l0 (TOP: rows of a multiple of 4 cells) belongs to the threads in pairs of quads,
+//     4 cells of x in two planes: a thread keeps its right-hand side, face coefficients,
+//     1 / diagonal and iterate in registers for the whole launch, x neighbours come by
+//     shuffle, and a sweep reads six 16-byte rows of fields without x padding, free of bank
+//     conflicts;
+//   * the next level (MID, not the coarsest) has a pair of cells in z per thread, their
+//     coefficients in registers; the levels below run from shared memory;
+//   * the coarsest level's sweeps keep the pairs' coefficients in registers too and synchronise
+//     only the warps that hold cells;
+//   * the face coefficients of all shared-memory levels are formed cell by cell in one pass
+//     whose global loads are all in flight together.
+// One instance of 16^3 .. 4^3 (SIGMA7 float32, V(2,2), 32 coarsest sweeps): 14.3 us a launch,
+// against 47 us for the eleven launches it replaces and 24 us with 1024 threads, one quad per
+// thread and the levels below walked cell by cell with integer divisions.  8 x 16 x 16 and
+// 4 x 8 x 8 of the 27-point operator, the F-cycle's F and V visits in one launch: 20 us
+// (35 us before, 160 us launch by launch).  In a served bf16 stream, beside other kernels: 22 us
+// (34 us before).  Left over: 3.7 us of set-up (global loads), 0.11 us per coarsest sweep, 0.6 us
+// per sweep of 16^3.
+constexpr int kProgThreads = 512;
 
-// fc = R(A phi - f), in two phases: every fine residual by its own thread into `res` (padded,
-// interior), then the eight of each coarse cell in the order z, y, x.
-template <int KIND, class T>
-__device__ void prog_restrict(const SubLevel<T> &L, const float *ph, const float *Fc, const float *f,
-                              float *res, const SubLevel<T> &Lc, float *fc) {
-  Walk w(threadIdx.x, blockDim.x, L.Y, L.X);
-  for (int i = threadIdx.x; i < L.n; i += blockDim.x, w.step(L.Y, L.X)) {
-    const int ip = pix(w.z, w.y, w.x, L.Y, L.X);
-    float dg;
-    const float ax = ph ? sub_apply<KIND, T>(L, ph, Fc, w.z, w.y, w.x, ip, i, &dg) : 0.f;
-    res[ip] = ax - f[i];
+// Cell i of a level: padded index and coordinates, from a table formed once per launch.
+struct Cell {
+  int ip, z, y, x;
+};
+__device__ __forceinline__ Cell cell_of(const uint2 *tab, int i) {
+  const uint2 u = tab[i];
+  return Cell{(int)(u.x & 0xffffu), (int)(u.x >> 16), (int)(u.y >> 16), (int)(u.y & 0xffffu)};
+}
+
+// A thread-strided pass over the cells of level L.
+#define HFM_FOR_CELLS(L, F)                                                              \
+  for (int i = threadIdx.x; i < (L).n; i += kProgThreads) {                              \
+    const Cell q = cell_of(reinterpret_cast<const uint2 *>((F) + (L).o_idx), i);
+
+// Cell i of level L: its table entry and, for SIGMA7, its face coefficients (the low ones,
+// and the high ones at the walls) and 1 / diagonal.  The global loads and the shared-memory
+// stores are apart, so that the loads can be in flight while the block clears its fields.
+template <int KIND, class T> struct CellInit {
+  int x, y, z, t, i;
+  float vx, vy, vz, xl, xh, yl, yh, zl, zh;
+  __device__ __forceinline__ void load(const SubLevel<T> &L, int64_t inst, int cell) {
+    const int X = L.X, Y = L.Y, P = X * Y;
+    i = cell;
+    x = i % X;
+    t = i / X;
+    y = t % Y;
+    z = t / Y;
+    if (KIND == HFM_OP_SIGMA7) {
+      const int64_t g = inst * (int64_t)L.n + i;
+      const T *sx = L.sx + g, *sy = L.sy + g, *sz = L.sz + g;
+      // at a wall the neighbour's conductivity is the cell's own: (s + s) / 2 = s
+      vx = St<T>::ld(sx);
+      vy = St<T>::ld(sy);
+      vz = St<T>::ld(sz);
+      xl = St<T>::ld(sx - (x > 0 ? 1 : 0));
+      xh = St<T>::ld(sx + (x + 1 < X ? 1 : 0));
+      yl = St<T>::ld(sy - (y > 0 ? X : 0));
+      yh = St<T>::ld(sy + (y + 1 < Y ? X : 0));
+      zl = St<T>::ld(sz - (z > 0 ? P : 0));
+      zh = St<T>::ld(sz + (z + 1 < L.Z ? P : 0));
+    }
   }
-  __syncthreads();
-  const int PX = L.X + 2, PXY = PX * (L.Y + 2);
-  Walk v(threadIdx.x, blockDim.x, Lc.Y, Lc.X);
-  for (int j = threadIdx.x; j < Lc.n; j += blockDim.x, v.step(Lc.Y, Lc.X)) {
-    const float *q = res + pix(2 * v.z, 2 * v.y, 2 * v.x, L.Y, L.X);
-    float sum = 0.f;
+  __device__ __forceinline__ void store(const SubLevel<T> &L, float *F) const {
+    const int X = L.X, Y = L.Y, Z = L.Z, P = X * Y;
+    reinterpret_cast<uint2 *>(F + L.o_idx)[i] =
+        make_uint2((unsigned)pix(z, y, x, Y, X) | ((unsigned)z << 16), ((unsigned)y << 16) | (unsigned)x);
+    if (KIND == HFM_OP_SIGMA7) {
+      const float axm = L.cx * (0.5f * (vx + xl)), axp = L.cx * (0.5f * (vx + xh));
+      const float aym = L.cy * (0.5f * (vy + yl)), ayp = L.cy * (0.5f * (vy + yh));
+      const float azm = L.cz * (0.5f * (vz + zl)), azp = L.cz * (0.5f * (vz + zh));
+      float *fx = F + L.o_face, *fy = fx + Z * Y * (X + 1), *fz = fy + Z * (Y + 1) * X;
+      const int ixf = i + t, iyf = i + z * X;
+      fx[ixf] = axm;
+      if (x + 1 == X) fx[ixf + 1] = axp;
+      fy[iyf] = aym;
+      if (y + 1 == Y) fy[iyf + X] = ayp;
+      fz[i] = azm;
+      if (z + 1 == Z) fz[i + P] = azp;
+      (fz + (Z + 1) * P)[i] = __fdividef(1.f, axm + axp + aym + ayp + azm + azp);
+    }
+  }
+};
+
+// Two cells, (z, y, x) and (z + 1, y, x) with z even, and their coefficients in registers (MID
+// and the coarsest level): a neighbour row read from shared memory serves both.
+__host__ __device__ __forceinline__ int cell_pairs(int Z, int Y, int X) { return ((Z + 1) >> 1) * Y * X; }
+template <int KIND> struct CellPair {
+  static constexpr bool SIG = KIND == HFM_OP_SIGMA7;
+  float w[KIND == HFM_OP_K27 ? 27 : 3];              // K27 weights / CONST7 kz, ky, kx
+  float xy[2][SIG ? 4 : 1], zf[SIG ? 3 : 1], rd[2];  // SIGMA7 faces; 1 / diagonal
+  float v[2];                                        // the iterate
+  int ip, i;  // padded and unpadded index of the first cell
+  bool valid, two;
+  template <class T> __device__ __forceinline__ void load(const SubLevel<T> &L, const float *F, int t) {
+    const int X = L.X, Y = L.Y, Z = L.Z;
+    valid = t < cell_pairs(Z, Y, X);
+    if (!valid) t = 0;
+    const int x = t % X, r = t / X, y = r % Y, z = 2 * (r / Y), P = X * Y;
+    two = valid && z + 1 < Z;
+    i = (z * Y + y) * X + x;
+    ip = pix(z, y, x, Y, X);
+    v[0] = v[1] = 0.f;
+    if constexpr (KIND == HFM_OP_K27) {
 #pragma unroll
-    for (int c = 0; c < 8; ++c) sum += q[(c >> 2) * PXY + ((c >> 1) & 1) * PX + (c & 1)];
-    fc[j] = 0.125f * sum;
+      for (int j = 0; j < 27; ++j) w[j] = L.k[j];
+      rd[0] = rd[1] = __fdividef(1.f, L.k[13]);
+    } else if constexpr (KIND == HFM_OP_CONST7) {
+#pragma unroll
+      for (int j = 0; j < 3; ++j) w[j] = L.k[j];
+      rd[0] = rd[1] = __fdividef(1.f, 2.f * (L.k[0] + L.k[1] + L.k[2]));
+    } else {
+      const float *fx = F + L.o_face, *fy = fx + Z * Y * (X + 1), *fz = fy + Z * (Y + 1) * X;
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        const int zg = g == 0 || two ? z + g : z, ig = i + (zg - z) * P;
+        const int ixf = ig + zg * Y + y, iyf = ig + zg * X;
+        xy[g][0] = fx[ixf];
+        xy[g][1] = fx[ixf + 1];
+        xy[g][2] = fy[iyf];
+        xy[g][3] = fy[iyf + X];
+        rd[g] = (fz + (Z + 1) * P)[ig];
+      }
+      zf[0] = fz[i];
+      zf[1] = fz[i + P];
+      zf[2] = fz[i + (two ? 2 * P : P)];
+    }
+  }
+  template <class T> __device__ __forceinline__ void rhs(const SubLevel<T> &L, const float *f, float (&r)[2]) const {
+    r[0] = f[i];
+    r[1] = f[i + (two ? L.X * L.Y : 0)];
+  }
+  template <class T> __device__ __forceinline__ void store(const SubLevel<T> &L, float *ph, const float (&u)[2]) const {
+    if (valid) ph[ip] = u[0];
+    if (two) ph[ip + (L.X + 2) * (L.Y + 2)] = u[1];
+  }
+  // s += the neighbours times their coefficients (K27: minus the weights); SIGMA7 / CONST7 with
+  // `diff`: s += the sum of coefficient (neighbour - own)
+  template <class T>
+  __device__ __forceinline__ void around(const SubLevel<T> &L, const float *ph, float (&s)[2], bool diff) const {
+    const float *p = ph + ip;
+    const int PX = L.X + 2, PXY = PX * (L.Y + 2);
+    if constexpr (KIND == HFM_OP_K27) {
+      float t[2][3] = {{s[0], 0.f, 0.f}, {s[1], 0.f, 0.f}};
+      const int top = two ? 2 * PXY : PXY;  // plane z + 2
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 9; ++b) {
+          const float n = p[(a == 3 ? top : (a - 1) * PXY) + (b / 3 - 1) * PX + (b % 3 - 1)];
+#pragma unroll
+          for (int g = 0; g < 2; ++g) {
+            const int k = a - g;
+            if (k < 0 || k > 2 || (k == 1 && b == 4)) continue;
+            t[g][b / 3] -= w[9 * k + b] * n;
+          }
+        }
+      s[0] = (t[0][0] + t[0][1]) + t[0][2];
+      s[1] = (t[1][0] + t[1][1]) + t[1][2];
+    } else {
+      const float zm = p[-PXY], zp = p[two ? 2 * PXY : PXY];
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        const float *q = p + g * PXY;
+        const float o = diff ? v[g] : 0.f, zl = g == 0 ? zm : v[0], zh = g == 0 ? v[1] : zp;
+        float a, b;
+        if constexpr (SIG) {
+          a = xy[g][0] * (q[-1] - o) + xy[g][1] * (q[1] - o);
+          b = xy[g][2] * (q[-PX] - o) + xy[g][3] * (q[PX] - o);
+          s[g] = (s[g] + a) + (b + (zf[g] * (zl - o) + zf[g + 1] * (zh - o)));
+        } else {
+          a = w[2] * ((q[-1] - o) + (q[1] - o));
+          b = w[1] * ((q[-PX] - o) + (q[PX] - o));
+          s[g] = (s[g] + a) + (b + w[0] * ((zl - o) + (zh - o)));
+        }
+      }
+    }
+  }
+  // v + om (f - A phi) / D, as (1 - om) v + (om / D) (f + neighbours)
+  template <class T>
+  __device__ __forceinline__ void sweep(const SubLevel<T> &L, const float *ph, const float (&f)[2], float om) {
+    float s[2] = {f[0], f[1]};
+    around(L, ph, s, false);
+    v[0] = (1.f - om) * v[0] + (om * rd[0]) * s[0];
+    v[1] = two ? (1.f - om) * v[1] + (om * rd[1]) * s[1] : 0.f;
+  }
+  __device__ __forceinline__ void sweep0(const float (&f)[2], float om) {
+    v[0] = (om * rd[0]) * f[0];
+    v[1] = two ? (om * rd[1]) * f[1] : 0.f;
+  }
+  // A phi - f, the 7-point forms difference by difference
+  template <class T>
+  __device__ __forceinline__ void residual(const SubLevel<T> &L, const float *ph, const float (&f)[2], float (&r)[2]) const {
+    float s[2] = {0.f, 0.f};
+    if constexpr (KIND == HFM_OP_K27) {
+      s[0] = -(w[13] * v[0]);
+      s[1] = -(w[13] * v[1]);
+    }
+    around(L, ph, s, true);
+    r[0] = -s[0] - f[0];
+    r[1] = -s[1] - f[1];
+  }
+};
+
+// One sweep of a level's iterate `in` (null: zero) into `out`.
+template <int KIND, class T>
+__device__ void prog_sweep(const SubLevel<T> &L, float *F, const float *in, float *out, float om) {
+  const float *f = F + L.o_rhs, *Fc = F + L.o_face;
+  const float *rd = Fc + sub_faces(L.Z, L.Y, L.X);
+  const float rc = KIND == HFM_OP_SIGMA7 ? 0.f
+                   : __fdividef(1.f, KIND == HFM_OP_K27 ? L.k[13] : 2.f * (L.k[0] + L.k[1] + L.k[2]));
+  HFM_FOR_CELLS(L, F)
+    const float r = KIND == HFM_OP_SIGMA7 ? rd[i] : rc;
+    if (in) {
+      float dg;
+      const float ax = sub_apply<KIND, T>(L, in, Fc, q.z, q.y, q.x, q.ip, i, &dg);
+      out[q.ip] = in[q.ip] + om * ((f[i] - ax) * r);
+    } else {
+      out[q.ip] = om * (f[i] * r);
+    }
   }
   __syncthreads();
 }
 
-// fc = R f (f unpadded)
+// The second phase of a restriction: each coarse cell's eight fine residuals (padded field,
+// ordered z, y, x), averaged into the coarse level's right-hand side.
 template <class T>
-__device__ void prog_restrict_rhs(const SubLevel<T> &L, const float *f, const SubLevel<T> &Lc, float *fc) {
-  Walk v(threadIdx.x, blockDim.x, Lc.Y, Lc.X);
-  for (int j = threadIdx.x; j < Lc.n; j += blockDim.x, v.step(Lc.Y, Lc.X)) {
-    const float *q = f + (2 * v.z * L.Y + 2 * v.y) * L.X + 2 * v.x;
+__device__ void prog_sum8(const SubLevel<T> &L, float *F, const float *res, const SubLevel<T> &Lc) {
+  __syncthreads();
+  const int PX = L.X + 2, PXY = PX * (L.Y + 2);
+  HFM_FOR_CELLS(Lc, F)
+    const float *r = res + pix(2 * q.z, 2 * q.y, 2 * q.x, L.Y, L.X);
     float sum = 0.f;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) sum += 0.125f * q[((c >> 2) * L.Y + ((c >> 1) & 1)) * L.X + (c & 1)];
-    fc[j] = sum;
+    for (int c = 0; c < 8; ++c) sum += r[(c >> 2) * PXY + ((c >> 1) & 1) * PX + (c & 1)];
+    F[Lc.o_rhs + i] = 0.125f * sum;
+  }
+  __syncthreads();
+}
+
+// Next level's right-hand side = R(A phi - f) (phi null: zero): every fine residual by its own
+// thread into `res`, then the sums.
+template <int KIND, class T>
+__device__ void prog_restrict(const SubLevel<T> &L, float *F, const float *ph, float *res,
+                              const SubLevel<T> &Lc) {
+  const float *f = F + L.o_rhs, *Fc = F + L.o_face;
+  HFM_FOR_CELLS(L, F)
+    float dg;
+    const float ax = ph ? sub_apply<KIND, T>(L, ph, Fc, q.z, q.y, q.x, q.ip, i, &dg) : 0.f;
+    res[q.ip] = ax - f[i];
+  }
+  prog_sum8<T>(L, F, res, Lc);
+}
+
+// Next level's right-hand side = R f
+template <class T>
+__device__ void prog_restrict_rhs(const SubLevel<T> &L, float *F, const SubLevel<T> &Lc) {
+  const float *f = F + L.o_rhs;
+  HFM_FOR_CELLS(Lc, F)
+    const float *r = f + (2 * q.z * L.Y + 2 * q.y) * L.X + 2 * q.x;
+    float sum = 0.f;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) sum += 0.125f * r[((c >> 2) * L.Y + ((c >> 1) & 1)) * L.X + (c & 1)];
+    F[Lc.o_rhs + i] = sum;
   }
   __syncthreads();
 }
 
 // phi = [phi] + sign * P(coarse) on the level's interior (both padded)
 template <class T>
-__device__ void prog_correct(const SubLevel<T> &L, float *ph, const SubLevel<T> &Lc, const float *coarse,
-                             float sign, bool zero) {
-  Walk w(threadIdx.x, blockDim.x, L.Y, L.X);
-  for (int i = threadIdx.x; i < L.n; i += blockDim.x, w.step(L.Y, L.X)) {
-    const int ip = pix(w.z, w.y, w.x, L.Y, L.X);
-    const float c = sign * coarse[pix(w.z >> 1, w.y >> 1, w.x >> 1, Lc.Y, Lc.X)];
-    ph[ip] = zero ? c : ph[ip] + c;
+__device__ void prog_correct(const SubLevel<T> &L, float *F, float *ph, const SubLevel<T> &Lc,
+                             const float *coarse, float sign, bool zero) {
+  HFM_FOR_CELLS(L, F)
+    const float c = sign * coarse[pix(q.z >> 1, q.y >> 1, q.x >> 1, Lc.Y, Lc.X)];
+    ph[q.ip] = zero ? c : ph[q.ip] + c;
   }
   __syncthreads();
 }
 
+// The coarsest level's sweeps of a 7-point operator, one cell per thread (a warp's chain of
+// dependent instructions sets the time of these sweeps: 218 cycles for 64 cells on two warps,
+// 456 in pairs on one warp).  Unrolled by two, so that each field's addresses are formed once.
+template <int KIND, class T>
+__device__ __forceinline__ void coarse_cells7(const SubLevel<T> &L, float *F, float om, int sweeps, int nthr) {
+  const int X = L.X, Y = L.Y, Z = L.Z, PX = X + 2, PXY = PX * (Y + 2), P = X * Y;
+  const bool in = (int)threadIdx.x < L.n;
+  const int i = in ? threadIdx.x : L.n - 1;
+  const Cell q = cell_of(reinterpret_cast<const uint2 *>(F + L.o_idx), i);
+  float c[6], od;
+  if (KIND == HFM_OP_CONST7) {
+    c[0] = c[1] = L.k[2];
+    c[2] = c[3] = L.k[1];
+    c[4] = c[5] = L.k[0];
+    od = om * __fdividef(1.f, 2.f * (L.k[0] + L.k[1] + L.k[2]));
+  } else {
+    const float *fx = F + L.o_face, *fy = fx + Z * Y * (X + 1), *fz = fy + Z * (Y + 1) * X;
+    const int ixf = i + q.z * Y + q.y, iyf = i + q.z * X;
+    c[0] = fx[ixf];
+    c[1] = fx[ixf + 1];
+    c[2] = fy[iyf];
+    c[3] = fy[iyf + X];
+    c[4] = fz[i];
+    c[5] = fz[i + P];
+    od = om * (fz + (Z + 1) * P)[i];
+  }
+  const float f = F[L.o_rhs + i], keep = 1.f - om;
+  float *p0 = F + L.o_phi + q.ip, *p1 = F + L.o_tmp + q.ip;
+  float v = od * f;
+  auto sweep = [&](const float *p, float *out) {
+    if (nthr == 32) __syncwarp();
+    else asm volatile("bar.sync 1, %0;" ::"r"(nthr) : "memory");
+    const float a = f + c[0] * p[-1] + c[1] * p[1], b = c[2] * p[-PX] + c[3] * p[PX];
+    v = keep * v + od * ((a + b) + (c[4] * p[-PXY] + c[5] * p[PXY]));
+    if (in) *out = v;
+  };
+  if (in) *p1 = v;
+  for (int k = 1; k < sweeps; k += 2) {
+    sweep(p1, p0);
+    if (k + 1 < sweeps) sweep(p0, p1);
+  }
+}
+
 // `sweeps` sweeps from zero on the coarsest level; returns the buffer holding the result.
-// Up to 1024 cells: one per thread, its coefficients in registers, a barrier among the warps
-// that hold cells (a warp barrier when one does).
+// Where the block has a thread for each cell (K27: for each pair of cells, whose 27 neighbours
+// mostly coincide), coefficients stay in registers and a barrier among the warps that hold
+// cells (a warp barrier when one does) parts the sweeps.
 template <int KIND, class T>
 __device__ int prog_coarse(const SubLevel<T> &L, float *F, float om, int sweeps) {
-  float *buf[2] = {F + L.o_phi, F + L.o_tmp};
-  const float *f = F + L.o_rhs, *Fc = F + L.o_face;
-  const int n = L.n;
-  if (n > (int)blockDim.x) {
+  const int np = KIND == HFM_OP_K27 ? cell_pairs(L.Z, L.Y, L.X) : L.n;
+  if (np > kProgThreads) {
     for (int k = 0; k < sweeps; ++k)
-      sub_sweep<KIND, T>(L, k == 0 ? nullptr : buf[k & 1], Fc, f, buf[(k & 1) ^ 1], om, buf[k & 1]);
+      prog_sweep<KIND, T>(L, F, k == 0 ? nullptr : F + (k & 1 ? L.o_tmp : L.o_phi), F + (k & 1 ? L.o_phi : L.o_tmp), om);
     return sweeps & 1;
   }
-  const int nthr = (n + 31) & ~31;
+  const int nthr = (np + 31) & ~31;
   if ((int)threadIdx.x < nthr) {
-    const int X = L.X, Y = L.Y, Z = L.Z, PX = X + 2, PXY = PX * (Y + 2);
-    const int i = min((int)threadIdx.x, n - 1);
-    const bool in = (int)threadIdx.x < n;
-    const int x = i % X, t = i / X, y = t % Y, z = t / Y;
-    const int ip = pix(z, y, x, Y, X);
-    constexpr int NK = KIND == HFM_OP_K27 ? 27 : 6;
-    float c[NK], rd;
-    if (KIND == HFM_OP_K27) {
-#pragma unroll
-      for (int j = 0; j < NK; ++j) c[j] = L.k[j];
-      rd = __fdividef(1.f, L.k[13]);
-    } else if (KIND == HFM_OP_CONST7) {
-      c[0] = c[1] = L.k[2];
-      c[2] = c[3] = L.k[1];
-      c[4] = c[5] = L.k[0];
-      rd = __fdividef(1.f, 2.f * (L.k[0] + L.k[1] + L.k[2]));
+    if constexpr (KIND != HFM_OP_K27) {
+      coarse_cells7<KIND, T>(L, F, om, sweeps, nthr);
     } else {
-      const float *fx = Fc, *fy = fx + Z * Y * (X + 1), *fz = fy + Z * (Y + 1) * X, *dg = fz + (Z + 1) * Y * X;
-      const int ixf = (z * Y + y) * (X + 1) + x, iyf = (z * (Y + 1) + y) * X + x;
-      c[0] = fx[ixf];
-      c[1] = fx[ixf + 1];
-      c[2] = fy[iyf];
-      c[3] = fy[iyf + X];
-      c[4] = fz[i];
-      c[5] = fz[i + X * Y];
-      rd = __fdividef(1.f, dg[i]);
-    }
-    const float fv = f[i];
-    float v = om * (fv * rd);
-    if (in) buf[1][ip] = v;
-    for (int k = 1; k < sweeps; ++k) {
-      if (nthr == 32) __syncwarp();
-      else asm volatile("bar.sync 1, %0;" ::"r"(nthr) : "memory");
-      const float *p = buf[k & 1] + ip;
-      float ax;
-      if (KIND == HFM_OP_K27) {
-        ax = 0.f;
-#pragma unroll
-        for (int j = 0; j < 27; ++j)
-          if (c[j] != 0.f) ax += c[j] * p[(j / 9 - 1) * PXY + ((j / 3) % 3 - 1) * PX + (j % 3 - 1)];
-      } else if (KIND == HFM_OP_CONST7) {
-        ax = 2.f * (c[4] + c[2] + c[0]) * v - c[4] * (p[-PXY] + p[PXY]) - c[2] * (p[-PX] + p[PX]) -
-             c[0] * (p[-1] + p[1]);
-      } else {
-        ax = c[0] * (v - p[-1]) + c[1] * (v - p[1]) + c[2] * (v - p[-PX]) + c[3] * (v - p[PX]) +
-             c[4] * (v - p[-PXY]) + c[5] * (v - p[PXY]);
+      CellPair<KIND> c;
+      c.load(L, F, threadIdx.x);
+      float f[2];
+      c.rhs(L, F + L.o_rhs, f);
+      c.sweep0(f, om);
+      c.store(L, F + L.o_tmp, c.v);
+      for (int k = 1; k < sweeps; ++k) {
+        if (nthr == 32) __syncwarp();
+        else asm volatile("bar.sync 1, %0;" ::"r"(nthr) : "memory");
+        c.sweep(L, F + (k & 1 ? L.o_tmp : L.o_phi), f, om);
+        c.store(L, F + (k & 1 ? L.o_phi : L.o_tmp), c.v);
       }
-      v += om * ((fv - ax) * rd);
-      if (in) buf[(k & 1) ^ 1][ip] = v;
     }
   }
   __syncthreads();
@@ -486,123 +706,239 @@ template <class T> __device__ __forceinline__ void stq4(T *p, const float (&v)[4
   }
 }
 
-// A thread's quad of level l0 (quad form).  Fields are [Z + 2][Y + 2][X], the ghost rows and
-// planes zero; `ip` is the quad's first cell in them.
-template <int KIND> struct TopQuad {
-  int x0, y, z, ip, X, Y, PZ;
-  bool valid, work;  // holds cells; its warp does (the shuffles need whole warps)
-  float f[4], p[4];
-  // SIGMA7: x faces of the four cells, y and z faces below and above, 1 / diagonal
-  float ax[KIND == HFM_OP_SIGMA7 ? 5 : 1], ay[2][KIND == HFM_OP_SIGMA7 ? 4 : 1],
-      az[2][KIND == HFM_OP_SIGMA7 ? 4 : 1], rd[KIND == HFM_OP_SIGMA7 ? 4 : 1];
+// A thread's pair of quads of level l0: cells x0 .. x0 + 3 of row y in planes z and z + 1 (z
+// even; the second one outside the grid when Z is odd and z the last plane).  Fields are
+// [Z + 2][Y + 2][X], the ghost rows and planes zero; `ip` is the first quad's first cell.
+// A sweep is evaluated as p = (1 - om) p + (om / D) (f + S) with S the neighbours times their
+// coefficients (8 operations a cell; forming f - A p difference by difference takes 15, and
+// a sweep was bound by the issue of those); the residuals that are restricted keep the
+// differences.
+template <int KIND> struct TopPair {
+  static constexpr bool SIG = KIND == HFM_OP_SIGMA7;
+  int ip, ic;       // the first cell in the fields, its parent in the next level's padded field
+  bool valid, two;  // holds cells; in both planes
+  bool first, last;  // the quad starts / ends its row
+  float f[2][4], p[2][4];
+  // SIGMA7: x faces of each quad, y faces below / above, z faces below, between and above,
+  // omega / diagonal
+  float ax[2][SIG ? 5 : 1], ay[2][2][SIG ? 4 : 1], az[3][SIG ? 4 : 1], od[2][SIG ? 4 : 1];
 
-  // neighbours across the quad's ends of row values v (row base pointer r, in the grid)
-  __device__ __forceinline__ void ends(const float *r, const float (&v)[4], float &l, float &h) const {
+  // neighbours across the ends of a quad's row values v (r: the row in the field)
+  template <class T>
+  __device__ __forceinline__ void ends(const SubLevel<T> &L, const float *r, const float (&v)[4], float &l, float &h) const {
     l = __shfl_up_sync(0xffffffffu, v[3], 1);
     h = __shfl_down_sync(0xffffffffu, v[0], 1);
-    const int lane = threadIdx.x & 31;
-    if (lane == 0 && x0 > 0) l = r[-1];
-    if (lane == 31 && x0 + 4 < X) h = r[4];
-    if (x0 == 0) l = 0.f;
-    if (x0 + 4 == X) h = 0.f;
+    if (128 % L.X) {  // rows continue in the next warp
+      const int lane = threadIdx.x & 31;
+      if (lane == 0 && !first) l = r[-1];
+      if (lane == 31 && !last) h = r[4];
+    }
+    l = first ? 0.f : l;
+    h = last ? 0.f : h;
   }
-  template <class T>
-  __device__ __forceinline__ void apply(const SubLevel<T> &L, const float *ph, float (&A)[4]) const {
+  struct Around {  // the rows around the pair
+    float zm[4], zp[4], ym[2][4], yp[2][4], l[2], h[2];
+  };
+  template <class T> __device__ __forceinline__ void gather(const SubLevel<T> &L, const float *ph, Around &n) const {
     const float *c = ph + ip;
-    if (KIND == HFM_OP_K27) {
+    const int X = L.X, PZ = (L.Y + 2) * X;
+    ldq4<float>(c - PZ, n.zm);
+    ldq4<float>(two ? c + 2 * PZ : c + PZ, n.zp);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) A[e] = 0.f;
+    for (int g = 0; g < 2; ++g) {
+      ldq4<float>(c + g * PZ - X, n.ym[g]);
+      ldq4<float>(c + g * PZ + X, n.yp[g]);
+      ends(L, c + g * PZ, p[g], n.l[g], n.h[g]);
+    }
+  }
+  // K27: s -= the 26 neighbours times their weights
+  template <class T>
+  __device__ __forceinline__ void around27(const SubLevel<T> &L, const float *ph, float (&s)[2][4]) const {
+    const float *c = ph + ip;
+    const int X = L.X, PZ = (L.Y + 2) * X;
 #pragma unroll
-      for (int a = 0; a < 3; ++a)
+    for (int a = 0; a < 4; ++a)  // planes z - 1 .. z + 2
 #pragma unroll
-        for (int b = 0; b < 3; ++b) {
-          const float *r = c + (a - 1) * PZ + (b - 1) * X;
-          float m[4], l, h;
-          if (a == 1 && b == 1) {
+      for (int b = 0; b < 3; ++b) {
+        // past the ghost plane (second quad outside): its sums are never used
+        const float *r = c + ((a == 3 && !two ? 2 : a) - 1) * PZ + (b - 1) * X;
+        float m[4], l, h;
+        ldq4<float>(r, m);
+        ends(L, r, m, l, h);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) m[e] = p[e];
-          } else {
-            ldq4<float>(r, m);
-          }
-          ends(r, m, l, h);
-          const float k0 = L.k[9 * a + 3 * b], k1 = L.k[9 * a + 3 * b + 1], k2 = L.k[9 * a + 3 * b + 2];
+        for (int g = 0; g < 2; ++g) {
+          const int k = a - g;  // plane k of quad g's stencil
+          if (k < 0 || k > 2) continue;
+          const float k0 = L.k[9 * k + 3 * b], k1 = L.k[9 * k + 3 * b + 1], k2 = L.k[9 * k + 3 * b + 2];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            A[e] += k0 * (e == 0 ? l : m[e - 1]);
-            A[e] += k1 * m[e];
-            A[e] += k2 * (e == 3 ? h : m[e + 1]);
+            s[g][e] -= k0 * (e == 0 ? l : m[e - 1]);
+            if (k != 1 || b != 1) s[g][e] -= k1 * m[e];
+            s[g][e] -= k2 * (e == 3 ? h : m[e + 1]);
           }
         }
-      return;
-    }
-    float l, h, ym[4], yp[4], zm[4], zp[4];
-    ldq4<float>(c - X, ym);
-    ldq4<float>(c + X, yp);
-    ldq4<float>(c - PZ, zm);
-    ldq4<float>(c + PZ, zp);
-    ends(c, p, l, h);
+      }
+  }
+  template <class T>
+  __device__ __forceinline__ void sweep(const SubLevel<T> &L, const float *ph, float om) {
+    float s[2][4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float xm = e == 0 ? l : p[e - 1], xp = e == 3 ? h : p[e + 1];
-      if (KIND == HFM_OP_CONST7) {
-        const float kz = L.k[0], ky = L.k[1], kx = L.k[2], d = 2.f * (kz + ky + kx);
-        A[e] = d * p[e] - kz * (zm[e] + zp[e]) - ky * (ym[e] + yp[e]) - kx * (xm + xp);
+    for (int g = 0; g < 2; ++g)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[g][e] = f[g][e];
+    if constexpr (KIND == HFM_OP_K27) {
+      around27(L, ph, s);
+    } else {
+      Around n;
+      gather(L, ph, n);
+#pragma unroll
+      for (int g = 0; g < 2; ++g)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float xm = e == 0 ? n.l[g] : p[g][e - 1], xp = e == 3 ? n.h[g] : p[g][e + 1];
+          const float zl = g == 0 ? n.zm[e] : p[0][e], zh = g == 0 ? p[1][e] : n.zp[e];
+          if constexpr (KIND == HFM_OP_CONST7) {
+            const float kz = L.k[0], ky = L.k[1], kx = L.k[2];
+            s[g][e] += kz * (zl + zh);
+            s[g][e] += ky * (n.ym[g][e] + n.yp[g][e]);
+            s[g][e] += kx * (xm + xp);
+          } else {
+            s[g][e] += az[g][e] * zl;
+            s[g][e] += az[g + 1][e] * zh;
+            s[g][e] += ay[g][0][e] * n.ym[g][e];
+            s[g][e] += ay[g][1][e] * n.yp[g][e];
+            s[g][e] += ax[g][e] * xm;
+            s[g][e] += ax[g][e + 1] * xp;
+          }
+        }
+    }
+    const float keep = 1.f - om;
+#pragma unroll
+    for (int g = 0; g < 2; ++g)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) p[g][e] = keep * p[g][e] + odiag(L, g, e, om) * s[g][e];
+  }
+  template <class T> __device__ __forceinline__ float odiag(const SubLevel<T> &L, int g, int e, float om) const {
+    if constexpr (SIG) return od[g][e];
+    return om * __fdividef(1.f, KIND == HFM_OP_K27 ? L.k[13] : 2.f * (L.k[0] + L.k[1] + L.k[2]));
+  }
+  // r = A phi - f
+  template <class T>
+  __device__ __forceinline__ void residual(const SubLevel<T> &L, const float *ph, float (&r)[2][4]) const {
+    if constexpr (KIND == HFM_OP_K27) {
+#pragma unroll
+      for (int g = 0; g < 2; ++g)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) r[g][e] = -(L.k[13] * p[g][e]);
+      around27(L, ph, r);
+#pragma unroll
+      for (int g = 0; g < 2; ++g)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) r[g][e] = -r[g][e] - f[g][e];
+    } else {
+      Around n;
+      gather(L, ph, n);
+#pragma unroll
+      for (int g = 0; g < 2; ++g)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float xm = e == 0 ? n.l[g] : p[g][e - 1], xp = e == 3 ? n.h[g] : p[g][e + 1];
+          const float zl = g == 0 ? n.zm[e] : p[0][e], zh = g == 0 ? p[1][e] : n.zp[e], q = p[g][e];
+          if constexpr (KIND == HFM_OP_CONST7) {
+            const float kz = L.k[0], ky = L.k[1], kx = L.k[2], d = 2.f * (kz + ky + kx);
+            r[g][e] = d * q - kz * (zl + zh) - ky * (n.ym[g][e] + n.yp[g][e]) - kx * (xm + xp) - f[g][e];
+          } else {
+            r[g][e] = ax[g][e] * (q - xm) + ax[g][e + 1] * (q - xp) + ay[g][0][e] * (q - n.ym[g][e]) +
+                      ay[g][1][e] * (q - n.yp[g][e]) + az[g][e] * (q - zl) + az[g + 1][e] * (q - zh) - f[g][e];
+          }
+        }
+    }
+  }
+  // x pairs of both planes' values: what the restriction adds up of this pair
+  __device__ __forceinline__ void pairs(const float (&r)[2][4], float *out) const {
+    if (two)
+      *reinterpret_cast<float2 *>(out + 2 * threadIdx.x) =
+          make_float2((r[0][0] + r[0][1]) + (r[1][0] + r[1][1]), (r[0][2] + r[0][3]) + (r[1][2] + r[1][3]));
+  }
+  template <class T> __device__ __forceinline__ void store(const SubLevel<T> &L, float *ph) const {
+    if (valid) *reinterpret_cast<float4 *>(ph + ip) = make_float4(p[0][0], p[0][1], p[0][2], p[0][3]);
+    if (two) *reinterpret_cast<float4 *>(ph + ip + (L.Y + 2) * L.X) = make_float4(p[1][0], p[1][1], p[1][2], p[1][3]);
+  }
+  // Index in an unpadded field of the level (plane z + 1: X Y further); 0 without cells.
+  template <class T> static __device__ __forceinline__ int place(const SubLevel<T> &L, int &x0, int &y, int &z) {
+    const int nvx = L.X >> 2, np = ((L.Z + 1) >> 1) * L.Y * nvx;
+    const int q = (int)threadIdx.x < np ? threadIdx.x : 0, t = q / nvx;
+    x0 = 4 * (q - t * nvx);
+    y = t % L.Y;
+    z = 2 * (t / L.Y);
+    return (z * L.Y + y) * L.X + x0;
+  }
+  // Threads of warps without cells stay out (the shuffles need whole warps of the others).
+  template <class T> static __device__ __forceinline__ bool working(const SubLevel<T> &L) {
+    return (int)(threadIdx.x & ~31u) < ((L.Z + 1) >> 1) * L.Y * (L.X >> 2);
+  }
+  template <class T> __device__ __forceinline__ void load(const SubLevel<T> &L, const T *src, float (&v)[2][4]) const {
+    int x0, y, z;
+    const int i = place(L, x0, y, z);
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      if (g == 0 ? valid : two) {
+        ldq4<T>(src + i + g * L.X * L.Y, v[g]);
       } else {
-        A[e] = ax[e] * (p[e] - xm) + ax[e + 1] * (p[e] - xp) + ay[0][e] * (p[e] - ym[e]) +
-               ay[1][e] * (p[e] - yp[e]) + az[0][e] * (p[e] - zm[e]) + az[1][e] * (p[e] - zp[e]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[g][e] = 0.f;
       }
     }
   }
-  template <class T> __device__ __forceinline__ float rdiag(const SubLevel<T> &L, int e) const {
-    if (KIND == HFM_OP_SIGMA7) return rd[e];
-    return __fdividef(1.f, KIND == HFM_OP_K27 ? L.k[13] : 2.f * (L.k[0] + L.k[1] + L.k[2]));
-  }
-  __device__ __forceinline__ void store(float *ph) const {
-    if (valid) *reinterpret_cast<float4 *>(ph + ip) = make_float4(p[0], p[1], p[2], p[3]);
-  }
-  template <class T> __device__ void init(const SubLevel<T> &L, int64_t inst, const T *rhs) {
-    X = L.X;
-    Y = L.Y;
-    PZ = (Y + 2) * X;
-    const int nvx = X >> 2, nq = L.n >> 2, q = threadIdx.x;
-    valid = q < nq;
-    work = (q & ~31) < nq;
-    const int qq = valid ? q : 0;
-    const int t = qq / nvx;
-    x0 = 4 * (qq - t * nvx);
-    y = t % Y;
-    z = t / Y;
-    ip = (z + 1) * PZ + (y + 1) * X + x0;
-    if (!valid) x0 = 0;
-    const int64_t i = inst * (int64_t)L.n + 4 * qq;
-    ldq4<T>(rhs + i, f);
+  template <class T>
+  __device__ __forceinline__ void init(const SubLevel<T> &L, const SubLevel<T> &Lc, int64_t inst, const T *rhs, float om) {
+    const int X = L.X, Y = L.Y, Z = L.Z, P = X * Y;
+    int x0, y, z;
+    const int i = place(L, x0, y, z);
+    valid = (int)threadIdx.x < ((Z + 1) >> 1) * Y * (X >> 2);
+    two = valid && z + 1 < Z;
+    first = x0 == 0;
+    last = x0 + 4 == X;
+    ip = ((z + 1) * (Y + 2) + (y + 1)) * X + x0;
+    ic = pix(z >> 1, y >> 1, x0 >> 1, Lc.Y, Lc.X);
+    const int64_t i0 = inst * (int64_t)L.n + i;
+    load<T>(L, rhs + inst * (int64_t)L.n, f);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) p[e] = 0.f;
-    if (KIND == HFM_OP_SIGMA7) {
-      const T *sx = L.sx + i, *sy = L.sy + i, *sz = L.sz + i;
-      const int P = X * Y;
+    for (int g = 0; g < 2; ++g)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) p[g][e] = 0.f;
+    if constexpr (SIG) {
       float c[4], lo[4], hi[4];
-      ldq4<T>(sx, c);
-      ax[0] = L.cx * (x0 > 0 ? 0.5f * (c[0] + St<T>::to(sx[-1])) : c[0]);
-      ax[4] = L.cx * (x0 + 4 < X ? 0.5f * (c[3] + St<T>::to(sx[4])) : c[3]);
-#pragma unroll
-      for (int e = 1; e < 4; ++e) ax[e] = L.cx * (0.5f * (c[e] + c[e - 1]));
-      ldq4<T>(sy, c);
-      ldq4<T>(y > 0 ? sy - X : sy, lo);
-      ldq4<T>(y + 1 < Y ? sy + X : sy, hi);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        ay[0][e] = L.cy * (0.5f * (c[e] + lo[e]));  // at a wall (s + s) / 2 = s
-        ay[1][e] = L.cy * (0.5f * (c[e] + hi[e]));
-      }
+      const T *sz = L.sz + i0;
       ldq4<T>(sz, c);
       ldq4<T>(z > 0 ? sz - P : sz, lo);
-      ldq4<T>(z + 1 < L.Z ? sz + P : sz, hi);
+      ldq4<T>(z + 1 < Z ? sz + P : sz, hi);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
+      for (int e = 0; e < 4; ++e) {  // at a wall the cell's own conductivity: (s + s) / 2 = s
         az[0][e] = L.cz * (0.5f * (c[e] + lo[e]));
         az[1][e] = L.cz * (0.5f * (c[e] + hi[e]));
-        rd[e] = __fdividef(1.f, ax[e] + ax[e + 1] + ay[0][e] + ay[1][e] + az[0][e] + az[1][e]);
+      }
+      ldq4<T>(z + 2 < Z ? sz + 2 * P : (z + 1 < Z ? sz + P : sz), c);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) az[2][e] = L.cz * (0.5f * (hi[e] + c[e]));
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        const int64_t k = i0 + (z + g < Z ? g * P : 0);
+        const T *sx = L.sx + k, *sy = L.sy + k;
+        ldq4<T>(sx, c);
+        ax[g][0] = L.cx * (0.5f * (c[0] + St<T>::to(sx[first ? 0 : -1])));
+        ax[g][4] = L.cx * (0.5f * (c[3] + St<T>::to(sx[last ? 3 : 4])));
+#pragma unroll
+        for (int e = 1; e < 4; ++e) ax[g][e] = L.cx * (0.5f * (c[e] + c[e - 1]));
+        ldq4<T>(sy, c);
+        ldq4<T>(y > 0 ? sy - X : sy, lo);
+        ldq4<T>(y + 1 < Y ? sy + X : sy, hi);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          ay[g][0][e] = L.cy * (0.5f * (c[e] + lo[e]));
+          ay[g][1][e] = L.cy * (0.5f * (c[e] + hi[e]));
+          od[g][e] = om * __fdividef(1.f, ax[g][e] + ax[g][e + 1] + ay[g][0][e] + ay[g][1][e] + az[g][e] + az[g + 1][e]);
+        }
       }
     }
   }
@@ -617,34 +953,52 @@ __global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant_
   float *F = reinterpret_cast<float *>(sub_smem);
   const int nl = a.nlev;
   const SubLevel<T> &L0 = a.lv[0];
-  TopQuad<KIND> tq;
-  // both fields of every level zero (the ghosts stay so), face arrays, right-hand side of l0
-  for (int l = 0; l < nl; ++l) {
-    const SubLevel<T> &L = a.lv[l];
-    for (int i = threadIdx.x; i < L.o_rhs - L.o_phi; i += kProgThreads) F[L.o_phi + i] = 0.f;
-    if (KIND == HFM_OP_SIGMA7 && !(TOP && l == 0)) sub_faces_init<T>(L, inst, F + L.o_face);
-  }
-  if (TOP) {
-    tq.template init<T>(L0, inst, a.rhs);
-  } else {
-    for (int i = threadIdx.x; i < L0.n; i += kProgThreads) F[L0.o_rhs + i] = St<T>::to(a.rhs[inst * (int64_t)L0.n + i]);
-  }
+  // the cells of the shared-memory levels as one list, the coarsest first: a thread's first
+  // cell is loaded, then its quads; meanwhile the block clears its shared memory (the ghosts
+  // of the fields stay zero)
+  constexpr int LB = TOP ? 1 : 0;
+  CellInit<KIND, T> ci;
+  int l = nl - 1, first = 0;
+  int k = threadIdx.x;
+  auto find = [&]() {
+    while (l >= LB && k >= first + a.lv[l].n) first += a.lv[l--].n;
+    return l >= LB;
+  };
+  bool more = find();
+  if (more) ci.load(a.lv[l], inst, k - first);
+  for (int i = threadIdx.x; i < P.clear; i += kProgThreads) reinterpret_cast<float4 *>(F)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  TopPair<KIND> tp;
+  if (TOP) tp.template init<T>(L0, a.lv[1], inst, a.rhs, a.omega);
   __syncthreads();
+  while (more) {
+    ci.store(a.lv[l], F);
+    k += kProgThreads;
+    more = find();
+    if (more) ci.load(a.lv[l], inst, k - first);
+  }
+  if (!TOP)
+    for (int i = threadIdx.x; i < L0.n; i += kProgThreads) F[L0.o_rhs + i] = St<T>::to(a.rhs[inst * (int64_t)L0.n + i]);
+  __syncthreads();
+  const SubLevel<T> &L1 = a.lv[1];
+  const bool mid = nl > 2 && cell_pairs(L1.Z, L1.Y, L1.X) <= kProgThreads;  // level 1 in registers
+  CellPair<KIND> mc;
+  if (mid) mc.load(L1, F, threadIdx.x);
   if (P.phi0) {  // the given iterate of l0, in its first field
     const T *src = P.phi0 + inst * (int64_t)L0.n;
     if (TOP) {
-      if (tq.valid) ldq4<T>(src + 4 * threadIdx.x, tq.p);
-      tq.store(F + L0.o_phi);
+      tp.template load<T>(L0, src, tp.p);
+      tp.store(L0, F + L0.o_phi);
     } else {
-      Walk w(threadIdx.x, kProgThreads, L0.Y, L0.X);
-      for (int i = threadIdx.x; i < L0.n; i += kProgThreads, w.step(L0.Y, L0.X))
-        F[L0.o_phi + pix(w.z, w.y, w.x, L0.Y, L0.X)] = St<T>::to(src[i]);
+      HFM_FOR_CELLS(L0, F)
+        F[L0.o_phi + q.ip] = St<T>::to(src[i]);
+      }
     }
     __syncthreads();
   }
   unsigned cur = 0;  // bit l: level l's iterate is in tmp
   for (int s = 0; s < P.nsteps; ++s) {
-    const int op = P.op[s], l = P.lev[s], cnt = P.cnt[s];
+    const int op = P.op[s], cnt = P.cnt[s];
+    l = P.lev[s];
     const SubLevel<T> &L = a.lv[l];
     const SubLevel<T> &Lc = a.lv[l + 1 < nl ? l + 1 : l];
     const int c = (cur >> l) & 1;
@@ -654,98 +1008,145 @@ __global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant_
     if (op == SO_COARSE) {
       const int r = prog_coarse<KIND, T>(L, F, a.coarse_omega, cnt);
       cur = (cur & ~(1u << l)) | ((unsigned)r << l);
-    } else if (TOP && l == 0) {
-      if (op == SO_SWEEP0 || op == SO_SWEEP) {
-        for (int k = 0; k < cnt; ++k) {
-          if (tq.work) {
-            if (op == SO_SWEEP0 && k == 0) {
+    } else if (op == SO_SWEEP0 || op == SO_SWEEP) {
+      for (int n = 0; n < cnt; ++n) {
+        const bool zero = op == SO_SWEEP0 && n == 0;
+        if (TOP && l == 0) {
+          if (tp.working(L0)) {
+            if (zero) {
 #pragma unroll
-              for (int e = 0; e < 4; ++e) tq.p[e] = a.omega * (tq.f[e] * tq.rdiag(L, e));
+              for (int g = 0; g < 2; ++g)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) tp.p[g][e] = tp.odiag(L0, g, e, a.omega) * tp.f[g][e];
             } else {
-              float A[4];
-              tq.apply(L0, ph, A);
-#pragma unroll
-              for (int e = 0; e < 4; ++e) tq.p[e] += a.omega * ((tq.f[e] - A[e]) * tq.rdiag(L, e));
+              tp.sweep(L0, ph, a.omega);
             }
-            tq.store(other);
+            if (!tp.two) {  // the second quad is outside the grid
+#pragma unroll
+              for (int e = 0; e < 4; ++e) tp.p[1][e] = 0.f;
+            }
+            tp.store(L0, other);
           }
           __syncthreads();
-          float *t = ph;
-          ph = other;
-          other = t;
+        } else if (mid && l == 1) {
+          if (mc.valid) {
+            float f[2];
+            mc.rhs(L1, F + L1.o_rhs, f);
+            if (zero) mc.sweep0(f, a.omega);
+            else mc.sweep(L1, ph, f, a.omega);
+            mc.store(L1, other, mc.v);
+          }
+          __syncthreads();
+        } else {
+          prog_sweep<KIND, T>(L, F, zero ? nullptr : ph, other, a.omega);
         }
-        if (cnt & 1) cur ^= 1u;
-      } else if (op == SO_RESTRICT || op == SO_RESTRICT0 || op == SO_RESTRICT_RHS) {
-        // x pairs of the quad's residuals, then the four rows of each coarse cell
+        float *t = ph;
+        ph = other;
+        other = t;
+      }
+      if (cnt & 1) cur ^= 1u << l;
+    } else if (op == SO_RESTRICT || op == SO_RESTRICT0) {
+      const bool zero = op == SO_RESTRICT0;
+      if (TOP && l == 0) {
         float *pairs = F + P.o_top;
-        const float scale = op == SO_RESTRICT_RHS ? -1.f : 1.f;  // r = A phi - f, or f itself
-        if (tq.work) {
-          float A[4] = {0.f, 0.f, 0.f, 0.f};
-          if (op == SO_RESTRICT) tq.apply(L0, ph, A);
-          if (tq.valid)
-            *reinterpret_cast<float2 *>(pairs + 2 * threadIdx.x) =
-                make_float2(scale * ((A[0] - tq.f[0]) + (A[1] - tq.f[1])),
-                            scale * ((A[2] - tq.f[2]) + (A[3] - tq.f[3])));
+        if (tp.working(L0)) {
+          float r[2][4];
+          if (zero) {
+#pragma unroll
+            for (int g = 0; g < 2; ++g)
+#pragma unroll
+              for (int e = 0; e < 4; ++e) r[g][e] = -tp.f[g][e];
+          } else {
+            tp.residual(L0, ph, r);
+          }
+          tp.pairs(r, pairs);
         }
         __syncthreads();
         const int Xh = L.X >> 1;
-        Walk v(threadIdx.x, kProgThreads, Lc.Y, Lc.X);
-        for (int j = threadIdx.x; j < Lc.n; j += kProgThreads, v.step(Lc.Y, Lc.X)) {
-          const float *q = pairs + (2 * v.z * L.Y + 2 * v.y) * Xh + v.x;
-          const float *q1 = q + L.Y * Xh;
-          F[Lc.o_rhs + j] = 0.125f * ((q[0] + q[Xh]) + (q1[0] + q1[Xh]));
+        HFM_FOR_CELLS(Lc, F)
+          const float *r = pairs + (q.z * L.Y + 2 * q.y) * Xh + q.x;
+          F[Lc.o_rhs + i] = 0.125f * (r[0] + r[Xh]);
         }
         __syncthreads();
-      } else {  // SO_CORRECT0, SO_CORRECT, SO_PROLONG
-        if (tq.valid) {
-          const float sign = op == SO_PROLONG ? 1.f : -1.f;
-          const int ic = pix(tq.z >> 1, tq.y >> 1, tq.x0 >> 1, Lc.Y, Lc.X);
-          const float c0 = sign * coarse[ic], c1 = sign * coarse[ic + 1];
-          const bool z0 = op != SO_CORRECT;
-          tq.p[0] = z0 ? c0 : tq.p[0] + c0;
-          tq.p[1] = z0 ? c0 : tq.p[1] + c0;
-          tq.p[2] = z0 ? c1 : tq.p[2] + c1;
-          tq.p[3] = z0 ? c1 : tq.p[3] + c1;
-          tq.store(ph);
+      } else if (mid && l == 1) {
+        if (mc.valid) {
+          float f[2], r[2];
+          mc.rhs(L1, F + L1.o_rhs, f);
+          if (zero) {
+            r[0] = -f[0];
+            r[1] = -f[1];
+          } else {
+            mc.residual(L1, ph, f, r);
+          }
+          mc.store(L1, other, r);
         }
-        __syncthreads();
-      }
-    } else {
-      const float *f = F + L.o_rhs, *Fc = F + L.o_face;
-      if (op == SO_SWEEP0 || op == SO_SWEEP) {
-        for (int k = 0; k < cnt; ++k) {
-          sub_sweep<KIND, T>(L, op == SO_SWEEP0 && k == 0 ? nullptr : ph, Fc, f, other, a.omega, ph);
-          float *t = ph;
-          ph = other;
-          other = t;
-        }
-        if (cnt & 1) cur ^= 1u << l;
-      } else if (op == SO_RESTRICT || op == SO_RESTRICT0) {
-        prog_restrict<KIND, T>(L, op == SO_RESTRICT0 ? nullptr : ph, Fc, f, other, Lc, F + Lc.o_rhs);
-      } else if (op == SO_RESTRICT_RHS) {
-        prog_restrict_rhs<T>(L, f, Lc, F + Lc.o_rhs);
+        prog_sum8<T>(L1, F, other, Lc);
       } else {
-        prog_correct<T>(L, ph, Lc, coarse, op == SO_PROLONG ? 1.f : -1.f, op != SO_CORRECT);
+        prog_restrict<KIND, T>(L, F, zero ? nullptr : ph, other, Lc);
+      }
+    } else if (op == SO_RESTRICT_RHS) {
+      if (TOP && l == 0) {
+        float *pairs = F + P.o_top;
+        tp.pairs(tp.f, pairs);
+        __syncthreads();
+        const int Xh = L.X >> 1;
+        HFM_FOR_CELLS(Lc, F)
+          const float *r = pairs + (q.z * L.Y + 2 * q.y) * Xh + q.x;
+          F[Lc.o_rhs + i] = 0.125f * (r[0] + r[Xh]);
+        }
+        __syncthreads();
+      } else {
+        prog_restrict_rhs<T>(L, F, Lc);
+      }
+    } else {  // SO_CORRECT0, SO_CORRECT, SO_PROLONG
+      const float sign = op == SO_PROLONG ? 1.f : -1.f;
+      const bool zero = op != SO_CORRECT;
+      if (TOP && l == 0) {
+        if (tp.valid) {
+          const float c0 = sign * coarse[tp.ic], c1 = sign * coarse[tp.ic + 1];
+#pragma unroll
+          for (int g = 0; g < 2; ++g)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float d = e < 2 ? c0 : c1;
+              tp.p[g][e] = (g == 0 || tp.two) ? (zero ? d : tp.p[g][e] + d) : 0.f;
+            }
+          tp.store(L0, ph);
+        }
+        __syncthreads();
+      } else if (mid && l == 1) {
+        if (mc.valid) {
+          const Cell q = cell_of(reinterpret_cast<const uint2 *>(F + L1.o_idx), mc.i);
+          const float d = sign * coarse[pix(q.z >> 1, q.y >> 1, q.x >> 1, Lc.Y, Lc.X)];
+          mc.v[0] = zero ? d : mc.v[0] + d;
+          mc.v[1] = !mc.two ? 0.f : zero ? d : mc.v[1] + d;
+          mc.store(L1, ph, mc.v);
+        }
+        __syncthreads();
+      } else {
+        prog_correct<T>(L, F, ph, Lc, coarse, sign, zero);
       }
     }
   }
   T *out = a.out + inst * (int64_t)L0.n;
   if (TOP) {
-    if (tq.valid) stq4<T>(out + 4 * threadIdx.x, tq.p);
+    int x0, y, z;
+    const int i = tp.place(L0, x0, y, z);
+    if (tp.valid) stq4<T>(out + i, tp.p[0]);
+    if (tp.two) stq4<T>(out + i + L0.X * L0.Y, tp.p[1]);
   } else {
     const float *res = F + ((cur & 1) ? L0.o_tmp : L0.o_phi);
-    Walk w(threadIdx.x, kProgThreads, L0.Y, L0.X);
-    for (int i = threadIdx.x; i < L0.n; i += kProgThreads, w.step(L0.Y, L0.X))
-      out[i] = St<T>::from(res[pix(w.z, w.y, w.x, L0.Y, L0.X)]);
+    HFM_FOR_CELLS(L0, F)
+      out[i] = St<T>::from(res[q.ip]);
+    }
   }
   if (P.store_all)
-    for (int l = 1; l < nl; ++l) {
+    for (l = 1; l < nl; ++l) {
       const SubLevel<T> &L = a.lv[l];
       const float *res = F + (((cur >> l) & 1) ? L.o_tmp : L.o_phi);
-      Walk w(threadIdx.x, kProgThreads, L.Y, L.X);
-      for (int i = threadIdx.x; i < L.n; i += kProgThreads, w.step(L.Y, L.X)) {
+      HFM_FOR_CELLS(L, F)
         P.g_rhs[l][inst * (int64_t)L.n + i] = St<T>::from(F[L.o_rhs + i]);
-        P.g_phi[l][inst * (int64_t)L.n + i] = St<T>::from(res[pix(w.z, w.y, w.x, L.Y, L.X)]);
+        P.g_phi[l][inst * (int64_t)L.n + i] = St<T>::from(res[q.ip]);
       }
     }
 }
@@ -985,34 +1386,51 @@ int go_subprog(const SubProgram<T> &p, int B, size_t smem, cudaStream_t s) {
   return HFM_OK;
 }
 
+// The quad form of level l0: whole quads per row, and at most one pair of quads per thread.
+template <class T> bool program_top(const SubProgram<T> &p) {
+  const SubLevel<T> &L = p.a.lv[0];
+  return (L.X & 3) == 0 && ((L.Z + 1) >> 1) * L.Y * (L.X >> 2) <= kProgThreads;
+}
+
+// Shared-memory layout of a program: per level the fields, right-hand side and faces as
+// layout_sub places them, then the cell table; the quad form of level l0 keeps two fields
+// without x ghosts and the pair sums only.  Returns the bytes.
+template <class T> size_t layout_program(int kind, SubProgram<T> &p) {
+  const bool top = program_top(p);
+  int64_t off = 0;
+  for (int l = 0; l < p.a.nlev; ++l) {
+    SubLevel<T> &q = p.a.lv[l];
+    const int np = sub_padded(q.Z, q.Y, q.X);
+    q.o_phi = (int)off;
+    if (top && l == 0) {
+      const int nt = (q.Z + 2) * (q.Y + 2) * q.X;
+      q.o_tmp = nt;
+      q.o_rhs = q.o_face = q.o_idx = p.o_top = 2 * nt;
+      off = 2 * nt + ((q.Z + 1) >> 1) * q.Y * (q.X >> 1);
+      continue;
+    }
+    q.o_tmp = (int)off + np;
+    q.o_rhs = (int)off + 2 * np;
+    q.o_face = q.o_rhs + q.n;
+    off = q.o_face + (kind == HFM_OP_SIGMA7 ? sub_faces(q.Z, q.Y, q.X) + q.n : 0);
+    off = (off + 1) & ~1;
+    q.o_idx = (int)off;
+    off = (off + 2 * q.n + 3) & ~3;
+  }
+  off = (off + 3) & ~3;
+  p.clear = (int)(off / 4);
+  return (size_t)off * 4;
+}
+
+template <class T> bool subprogram_fits(int kind, SubProgram<T> &p) {
+  return layout_program<T>(kind, p) <= kSubcycleMaxSmem;
+}
+
 template <class T>
 int launch_subprogram(int kind, SubProgram<T> &p, int B, cudaStream_t s) {
-  const SubLevel<T> &L0 = p.a.lv[0];
-  // the quad form: whole quads per row, and at most one quad per thread
-  const bool top = (L0.X & 3) == 0 && L0.n <= 4 * kProgThreads;
-  size_t smem = layout_sub<T>(kind, p.a);
-  if (!smem) return fail(HFM_ERR_BAD_ARG, "subcycle: levels exceed shared memory");
-  if (top) {  // level l0 keeps two fields without x ghosts and the pair sums; no faces
-    SubLevel<T> &L = p.a.lv[0];
-    const int np = (L.Z + 2) * (L.Y + 2) * L.X;
-    L.o_phi = 0;
-    L.o_tmp = np;
-    L.o_rhs = L.o_face = 2 * np;
-    p.o_top = 2 * np;
-    int off = 2 * np + L.n / 2;
-    for (int l = 1; l < p.a.nlev; ++l) {
-      SubLevel<T> &q = p.a.lv[l];
-      const int shift = off - q.o_phi;
-      const int size = (l + 1 < p.a.nlev ? p.a.lv[l + 1].o_phi : (int)(smem / 4)) - q.o_phi;
-      q.o_phi += shift;
-      q.o_tmp += shift;
-      q.o_rhs += shift;
-      q.o_face += shift;
-      off += size;
-    }
-    smem = (size_t)off * 4;
-    if (smem > kSubcycleMaxSmem) return fail(HFM_ERR_BAD_ARG, "subcycle: levels exceed shared memory");
-  }
+  const bool top = program_top(p);
+  const size_t smem = layout_program<T>(kind, p);
+  if (smem > kSubcycleMaxSmem) return fail(HFM_ERR_BAD_ARG, "subcycle: levels exceed shared memory");
   switch (kind) {
     case HFM_OP_SIGMA7:
       return top ? go_subprog<HFM_OP_SIGMA7, T, true>(p, B, smem, s) : go_subprog<HFM_OP_SIGMA7, T, false>(p, B, smem, s);
@@ -1024,6 +1442,9 @@ int launch_subprogram(int kind, SubProgram<T> &p, int B, cudaStream_t s) {
   }
 }
 
+template bool subprogram_fits<float>(int, SubProgram<float> &);
+template bool subprogram_fits<__nv_bfloat16>(int, SubProgram<__nv_bfloat16> &);
+template bool subprogram_fits<__half>(int, SubProgram<__half> &);
 template int launch_subprogram<float>(int, SubProgram<float> &, int, cudaStream_t);
 template int launch_subprogram<__nv_bfloat16>(int, SubProgram<__nv_bfloat16> &, int, cudaStream_t);
 template int launch_subprogram<__half>(int, SubProgram<__half> &, int, cudaStream_t);
