@@ -1007,7 +1007,38 @@ class Engine : public EngineBase {
     while (l0 - 1 >= 1 && n(l0 - 1) <= 4096 && m_->L - (l0 - 1) <= kMaxSubLevels) --l0;
     if (l0 >= m_->L - 1) return -1;
     SubProgram<T> p;  // the longest list of the cycle form and the levels' fields fit
-    return fused_program(l0, c.cycle == HFM_CYCLE_F ? SUB_FV : SUB_V, p) && subprogram_fits<T>(k, p) ? l0 : -1;
+    const bool listed = c.cycle == HFM_CYCLE_SAWTOOTH
+                            ? sawtooth_program(l0, p)
+                            : fused_program(l0, c.cycle == HFM_CYCLE_F ? SUB_FV : SUB_V, p);
+    return listed && subprogram_fits<T>(k, p) ? l0 : -1;
+  }
+
+  // The sawtooth's leg over the levels from l0 down: restricted residuals to the coarsest, its
+  // sweeps from zero, then prolongation + one sweep per level.  False where the levels do not
+  // halve evenly (the separate kernels floor odd extents and stop at extents of 1) and for the
+  // x-end and top rules' levels, which are above l0.
+  bool sawtooth_program(int l0, SubProgram<T> &p) {
+    const hfm_mg_config &c = m_->cfg;
+    for (int l = l0; l + 1 < m_->L; ++l)
+      if (((g(l).Z | g(l).Y | g(l).X) & 1)) return false;
+    memset(&p, 0, sizeof(p));
+    p.a = make_sub(l0);
+    p.a.coarse_omega = c.omega;
+    const int last = p.a.nlev - 1;
+    for (int l = 0; l < last; ++l)
+      if (!add_step(p, SO_RESTRICT_RHS, l, 1)) return false;
+    if (!add_step(p, SO_COARSE, last, sawtooth_coarse_sweeps())) return false;
+    for (int l = last - 1; l >= 0; --l)
+      if (!add_step(p, SO_PROLONG, l, 1) || !add_step(p, SO_SWEEP, l, 1)) return false;
+    p.store_all = 1;
+    for (int l = 1; l <= last; ++l) {
+      p.g_rhs[l] = rhs(l0 + l);
+      p.g_phi[l] = buf(l0 + l, 0);
+    }
+    return true;
+  }
+  int sawtooth_coarse_sweeps() const {
+    return (m_->cfg.options & HFM_OPT_SAWTOOTH_COARSE_SWEEPS) ? m_->cfg.coarse_sweeps : 1;
   }
 
   // Steps of the cycles vcycle() runs from level l down (l relative to l0): V from a zero or the
@@ -1290,28 +1321,44 @@ class Engine : public EngineBase {
     T *r0 = (T *)m_->saw[0], *w0 = (T *)m_->saw[1];
     int st, nblk = 0;
     const unsigned xend = c.flags & HFM_FLAG_ZERO_XEND;
-    // 1. r = A phi - b (NS: r[..., X-1] = 0), residual norm for the stopping test
-    if ((st = launch_residual<T>(lk(0), lo(0), src(buf(0, cur_[0]), n(0)), rhs(0), n(0),
-                                 r0, n(0), m_->slots, g(0), xend, m_->active, m_->partials,
-                                 &nblk, s)))
-      return st;
+    // 1. r = A phi - b (NS: r[..., X-1] = 0), residual norm for the stopping test, and its
+    //    restriction in the same pass where the fine extents are even
+    const bool even = L > 1 && !((g(0).Z | g(0).Y | g(0).X) & 1);
+    if (even)
+      st = launch_residual_restrict<T>(lk(0), lo(0), src(buf(0, cur_[0]), n(0)), rhs(0), n(0), r0, n(0),
+                                       rhs(1), n(1), m_->slots, g(0), xend, m_->active, m_->partials,
+                                       &nblk, s);
+    else
+      st = launch_residual<T>(lk(0), lo(0), src(buf(0, cur_[0]), n(0)), rhs(0), n(0), r0, n(0), m_->slots,
+                              g(0), xend, m_->active, m_->partials, &nblk, s);
+    if (st) return st;
     if ((st = check(nblk, cur_[0], s))) return st;
-    // 2. restriction chain r -> r_1 -> ... -> r_{L-1} (coarse rhs buffers)
-    for (int l = 1; l < L; ++l) {
+    // 2. restriction chain r -> r_1 -> ... -> r_{L-1} (coarse rhs buffers), down to the fused levels
+    const int lf = fused_l0_ >= 1 ? fused_l0_ : L - 1;
+    for (int l = even ? 2 : 1; l <= lf; ++l) {
       const T *f = l == 1 ? r0 : rhs(l - 1);
       if ((st = launch_restrict<T>(f, n(l - 1), rhs(l), n(l), m_->slots, g(l - 1), m_->active, s)))
         return st;
     }
-    // 3. coarsest: one Jacobi sweep from w = 0 (coarse_sweeps of them with
-    //    HFM_OPT_SAWTOOTH_COARSE_SWEEPS), the last one landing in buffer 0
-    const int ncs = (c.options & HFM_OPT_SAWTOOTH_COARSE_SWEEPS) ? c.coarse_sweeps : 1;
-    for (int k = 0; k < ncs; ++k) {
-      const int dst = (ncs - 1 - k) & 1;
-      PhiSrc<T> p = src(k == 0 ? nullptr : buf(L - 1, dst ^ 1), n(L - 1));
-      if ((st = smooth(L - 1, p, rhs(L - 1), buf(L - 1, dst), c.omega, 0u, s))) return st;
+    int up = L - 2;  // next level of the way up
+    if (fused_l0_ >= 1) {
+      // 2.-4. of the levels of at most 4096 cells in one launch
+      SubProgram<T> p;
+      sawtooth_program(fused_l0_, p);
+      if ((st = launch_subprogram<T>(kind(), p, m_->slots, s))) return st;
+      up = fused_l0_ - 1;
+    } else {
+      // 3. coarsest: one Jacobi sweep from w = 0 (coarse_sweeps of them with
+      //    HFM_OPT_SAWTOOTH_COARSE_SWEEPS), the last one landing in buffer 0
+      const int ncs = sawtooth_coarse_sweeps();
+      for (int k = 0; k < ncs; ++k) {
+        const int dst = (ncs - 1 - k) & 1;
+        PhiSrc<T> p = src(k == 0 ? nullptr : buf(L - 1, dst ^ 1), n(L - 1));
+        if ((st = smooth(L - 1, p, rhs(L - 1), buf(L - 1, dst), c.omega, 0u, s))) return st;
+      }
     }
     // 4. coarse levels: w = P w; one Jacobi
-    for (int l = L - 2; l >= 1; --l) {
+    for (int l = up; l >= 1; --l) {
       PhiSrc<T> p = with_coarse(src(nullptr, n(l)), l + 1, buf(l + 1, 0), 1.f);
       if ((st = smooth(l, p, rhs(l), buf(l, 0), c.omega, 0u, s))) return st;
     }

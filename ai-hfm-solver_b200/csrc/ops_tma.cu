@@ -200,7 +200,7 @@ template <class T, int N> __device__ __forceinline__ void vst(T *p, const float 
 template <class T, int CORR, bool SIG, bool DS = false>
 __device__ __forceinline__ void issue_plane(const TmaArgs<T> &a, char *stage, uint32_t bar, int p,
                                             int x0, int y0, int b) {
-  using G = Geo<T, SIG, CORR != 0, DS>;
+  using G = Geo<T, SIG, CORR == 1, DS>;
   constexpr int TY = G::TY;
   (void)TY;
   mbar_expect(bar, a.stage_bytes);
@@ -211,7 +211,7 @@ __device__ __forceinline__ void issue_plane(const TmaArgs<T> &a, char *stage, ui
     tma_load(smem_u32(stage + G::O_SZ), &a.m_sz, x0, y0, p, b, bar);
   }
   if (a.has_f) tma_load(smem_u32(stage + G::O_F), &a.m_f, x0, y0, p, b, bar);
-  if (CORR) tma_load(smem_u32(stage + G::O_CC), &a.m_cc, (x0 >> 1) - G::HX, (y0 >> 1) - 1, p >> 1, b, bar);
+  if (CORR == 1) tma_load(smem_u32(stage + G::O_CC), &a.m_cc, (x0 >> 1) - G::HX, (y0 >> 1) - 1, p >> 1, b, bar);
   if (DS) tma_load(smem_u32(stage + G::O_DS), &a.m_ds, x0 - G::HX, y0 - 1, p, b, bar);
 }
 
@@ -230,7 +230,8 @@ template <int KIND, class T, int MODE, int CORR>
 __global__ void __launch_bounds__(Geo<T>::THREADS, Geo<T>::MINB) k_tma(const __grid_constant__ TmaArgs<T> a) {
   constexpr bool SIG = KIND == HFM_OP_SIGMA7;
   constexpr bool PRE2 = MODE == M_PRE2;
-  using G = Geo<T, SIG, CORR != 0, PRE2>;
+  constexpr bool DS = PRE2 || CORR == 2;  // a second tile with the phi halos
+  using G = Geo<T, SIG, CORR == 1, DS>;
   constexpr int TY = G::TY, V = G::VEC, NS = G::NS;
   extern __shared__ __align__(128) char smem[];
   __shared__ __align__(8) uint64_t bars[NS];
@@ -260,7 +261,7 @@ __global__ void __launch_bounds__(Geo<T>::THREADS, Geo<T>::MINB) k_tma(const __g
   if (tid == 0) {
     for (; p_next <= p_last && p_next < p_first + NS; ++p_next) {
       const int q = p_next - p_first;
-      issue_plane<T, CORR, SIG, PRE2>(a, smem + (q % NS) * G::STAGE, smem_u32(&bars[q % NS]), p_next, x0, y0, b);
+      issue_plane<T, CORR, SIG, DS>(a, smem + (q % NS) * G::STAGE, smem_u32(&bars[q % NS]), p_next, x0, y0, b);
     }
   }
   int p_waited = p_first - 1;  // last plane whose loads completed
@@ -289,7 +290,9 @@ __global__ void __launch_bounds__(Geo<T>::THREADS, Geo<T>::MINB) k_tma(const __g
       return a.omega * sld<T>(ph + ry * G::PW + rx) *
              sld<T>(reinterpret_cast<const T *>(st + G::O_DS) + ry * G::PW + rx);
     float v = a.has_phi ? sld<T>(ph + ry * G::PW + rx) : 0.f;
-    if (CORR) {
+    if (CORR == 2) {
+      v += a.corr_sign * sld<T>(reinterpret_cast<const T *>(st + G::O_DS) + ry * G::PW + rx);
+    } else if (CORR) {
       const int yy = y0 - 1 + ry, xx = x0 - G::HX + rx;
       const int cyy = (yy >> 1) - ((y0 >> 1) - 1), cxx = (xx >> 1) - ((x0 >> 1) - G::HX);
       const T *cc = reinterpret_cast<const T *>(st + G::O_CC);
@@ -315,7 +318,12 @@ __global__ void __launch_bounds__(Geo<T>::THREADS, Geo<T>::MINB) k_tma(const __g
 #pragma unroll
       for (int e = 0; e < V; ++e) v[e] = 0.f;
     }
-    if (CORR) {
+    if (CORR == 2) {
+      float cv[V];
+      vld<T, V>(reinterpret_cast<const T *>(st + G::O_DS) + ry * G::PW + rx, cv);
+#pragma unroll
+      for (int e = 0; e < V; ++e) v[e] += a.corr_sign * cv[e];
+    } else if (CORR) {
       // coarse cells of x pairs: tile column (gx >> 1) - ((x0 >> 1) - HX) = V/2 c + HX
       const int cyy = ((y0 - 1 + ry) >> 1) - ((y0 >> 1) - 1);
       float cv[V / 2];
@@ -355,7 +363,7 @@ __global__ void __launch_bounds__(Geo<T>::THREADS, Geo<T>::MINB) k_tma(const __g
     if (tid == 0 && z > z0 && p_next <= p_last) {
       const int q = p_next - p_first;
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      issue_plane<T, CORR, SIG, PRE2>(a, smem + (q % NS) * G::STAGE, smem_u32(&bars[q % NS]), p_next, x0, y0, b);
+      issue_plane<T, CORR, SIG, DS>(a, smem + (q % NS) * G::STAGE, smem_u32(&bars[q % NS]), p_next, x0, y0, b);
       ++p_next;
     }
     mine = wait_plane(z + 1, a.wait_budget);
@@ -572,7 +580,7 @@ int make_map(CUtensorMap *m, const void *ptr, int X, int Y, int Z, int B, int64_
 
 template <int KIND, class T, int MODE, int CORR>
 int go(const TmaArgs<T> &a, dim3 grid, cudaStream_t s) {
-  using G = Geo<T, KIND == HFM_OP_SIGMA7, CORR != 0, MODE == M_PRE2>;
+  using G = Geo<T, KIND == HFM_OP_SIGMA7, CORR == 1, MODE == M_PRE2 || CORR == 2>;
   const int smem = G::NS * G::STAGE;
   int st = set_max_dynamic_smem((const void *)k_tma<KIND, T, MODE, CORR>, smem,
                                 "cudaFuncSetAttribute(k_tma)");
@@ -634,9 +642,8 @@ bool tma_eligible(int kind, Grid3 g, int mode, const void *corr, int corr_coarse
   // (measured: 32^3 and 24^3 levels of 64 instances).
   if (g.X < 48 || g.Y < (es == 4 ? 8 : 16)) return false;
   if ((g.X * es) % 16) return false;  // tensor-map strides are multiples of 16 bytes
-  if (corr && !corr_coarse) return false;
-  if (corr && ((g.X / 2) * es) % 16) return false;
-  if (corr && ((g.Y | g.Z) & 1)) return false;
+  if (corr && corr_coarse && (((g.X / 2) * es) % 16 || ((g.Y | g.Z) & 1))) return false;
+  if (corr && !corr_coarse && kind == HFM_OP_FACE7) return false;
   if (mode == M_RESTRICT && ((g.Y & 1) || (g.Z & 1))) return false;
   if (mode != M_SMOOTH && corr) return false;
   return true;
@@ -859,14 +866,17 @@ int tma_launch(int kind, int mode, const DevOp &op, const PhiSrc<T> &phi, const 
   }
   a.has_f = rhs != nullptr;
   if (a.has_f && (st = make_map<T>(&a.m_f, rhs, g.X, g.Y, g.Z, B, stride, TX, TY))) return st;
-  const int corr = phi.corr ? 1 : 0;
-  if (corr && (st = make_map<T>(&a.m_cc, phi.corr, g.X / 2, g.Y / 2, g.Z / 2, B, phi.corr_stride,
-                                G::CW, TY / 2 + 2)))
+  // a correction on the coarse grid, or (the reference cycle's phi - w) on this one
+  const int corr = phi.corr ? (phi.corr_coarse ? 1 : 2) : 0;
+  if (corr == 1 && (st = make_map<T>(&a.m_cc, phi.corr, g.X / 2, g.Y / 2, g.Z / 2, B, phi.corr_stride,
+                                     G::CW, TY / 2 + 2)))
+    return st;
+  if (corr == 2 && (st = make_map<T>(&a.m_ds, phi.corr, g.X, g.Y, g.Z, B, phi.corr_stride, G::PW, TY + 2)))
     return st;
   unsigned bytes = a.has_phi ? (unsigned)(G::PHI * sizeof(T)) : 0u;
   if (a.has_sigma) bytes += (unsigned)((G::SXN + G::SYN + G::SZN) * sizeof(T));
   if (a.has_f) bytes += (unsigned)(G::FN * sizeof(T));
-  if (corr) bytes += (unsigned)(G::CCN * sizeof(T));
+  if (corr) bytes += (unsigned)((corr == 1 ? G::CCN : G::PHI) * sizeof(T));
   a.stage_bytes = bytes;
   a.wait_budget = g_wait_budget.load();
   a.op = op;
@@ -891,6 +901,7 @@ int tma_launch(int kind, int mode, const DevOp &op, const PhiSrc<T> &phi, const 
 #define HFM_TMA_GO(KIND, MODE, CORR) return go<KIND, T, MODE, CORR>(a, grid, s)
 #define HFM_TMA_MODES(KIND)                                              \
   if (mode == M_SMOOTH) {                                                \
+    if (corr == 2) HFM_TMA_GO(KIND, M_SMOOTH, 2);                        \
     if (corr) HFM_TMA_GO(KIND, M_SMOOTH, 1);                             \
     HFM_TMA_GO(KIND, M_SMOOTH, 0);                                       \
   } else if (mode == M_RESID) {                                          \

@@ -98,3 +98,33 @@ def test_fused_coarse_levels_few_slots(hfm, T, shape, form, cycle, nu):
             outs.append(np.stack([h.fetch(s).cpu().numpy() for s in range(B)]))
     # three cycles of a few dozen float32 roundings per value, damped by the smoothing
     assert np.abs(outs[0] - outs[1]).max() <= 1e-5 * np.abs(outs[1]).max()
+
+
+# the reference cycle with its small levels in one launch against one launch per step: the
+# iterate and every level's restricted residual and correction
+@pytest.mark.parametrize("shape", [(16, 16, 16), (64, 64, 64), (40, 8, 8), (24, 12, 20), (64, 128, 128)])
+@pytest.mark.parametrize("form", ["const7", "k27", "sigma7"])
+@pytest.mark.parametrize("sweeps,xend", [(1, False), (2, False), (1, True)])
+def test_fused_sawtooth_levels(hfm, T, shape, form, sweeps, xend):
+    M, ops = hfm.multigrid, hfm.ops
+    rng = np.random.default_rng(23)
+    f = dev(T, rng.standard_normal(shape))
+    sig = np.exp(0.5 * rng.standard_normal((3,) + shape))
+    op = {"const7": lambda: ops.Const7(0.5, 1.0, 2.0), "k27": lambda: ops.Stencil27(W.w5_pressure27()),
+          "sigma7": lambda: ops.Sigma7(*(dev(T, sig[k]) for k in range(3)))}[form]()
+    n_levels = int(np.log2(min(shape))) + 1
+    outs = []
+    for fused in (True, False):
+        cfg = M.SolverConfig.reference(n_levels=n_levels, cycles=100, coarse_sweeps=sweeps, zero_xend=xend,
+                                       fine_smooth=not xend)
+        cfg.fused_coarse = fused
+        with M.Multigrid(shape, op.kind, cfg, slots=1) as h:
+            h.set_operator(op)
+            h.load(0, f, f)
+            h.run(3)
+            got = [h.fetch(0)]
+            for l in range(1, len(h.levels)):
+                got += [h.read_level(0, l, 0), h.read_level(0, l, 1)]
+            outs.append([g.cpu().numpy() for g in got])
+    for a, b in zip(*outs):  # float32 rounding of three cycles, as the other parity tests allow
+        assert np.abs(a - b).max() <= 1e-5 * max(np.abs(b).max(), 1e-3 * np.abs(outs[1][0]).max())
