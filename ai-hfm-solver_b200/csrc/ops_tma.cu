@@ -26,6 +26,7 @@
 #include <cuda.h>
 
 #include <atomic>
+#include <map>
 #include <mutex>
 #include <type_traits>
 #include <vector>
@@ -578,56 +579,79 @@ int make_map(CUtensorMap *m, const void *ptr, int X, int Y, int Z, int B, int64_
   return HFM_OK;
 }
 
-template <int KIND, class T, int MODE, int CORR>
-int go(const TmaArgs<T> &a, dim3 grid, cudaStream_t s) {
-  using G = Geo<T, KIND == HFM_OP_SIGMA7, CORR == 1, MODE == M_PRE2 || CORR == 2>;
-  const int smem = G::NS * G::STAGE;
-  int st = set_max_dynamic_smem((const void *)k_tma<KIND, T, MODE, CORR>, smem,
-                                "cudaFuncSetAttribute(k_tma)");
-  if (st) return st;
-  k_tma<KIND, T, MODE, CORR><<<grid, G::THREADS, smem, s>>>(a);
-  HFM_CHECK_LAUNCH("k_tma");
-  return HFM_OK;
-}
-
-template <class T, int MODE, int CORR>
-int go_face(const TmaArgs<T> &a, dim3 grid, cudaStream_t s) {
-  using G = GeoF<CORR != 0, MODE == M_PRE2>;
-  const int smem = G::NS * G::STAGE;
-  int st = set_max_dynamic_smem((const void *)k_tma_face<T, MODE, CORR>, smem,
-                                "cudaFuncSetAttribute(k_tma_face)");
-  if (st) return st;
-  k_tma_face<T, MODE, CORR><<<grid, G::THREADS, smem, s>>>(a);
-  HFM_CHECK_LAUNCH("k_tma_face");
-  return HFM_OK;
+// Blocks of a kernel an SM holds (its registers and shared memory decide), at most 8 - the
+// partial sums per instance are sized for that - looked up once per kernel and device.
+int tma_resident(const void *kernel, int threads, int smem) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void *>, int> cache;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = cache.find({dev, kernel});
+  if (it != cache.end()) return it->second;
+  int nb = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, smem) != cudaSuccess || nb < 1) nb = 1;
+  return cache[{dev, kernel}] = nb > 8 ? 8 : nb;
 }
 
 // Grid (plane tiles, z chunks, instances).  The z chunk length (even, at least 2) minimises
 // (rounds of resident blocks) x (planes a block marches + 2 for its two halo planes and the
 // pipeline fill): a last round that is only partly filled costs a whole round, and every
 // chunk re-reads its halo planes.  (A fixed four waves left the 64^3 levels of 64 instances
-// at 3.03 waves - a fourth round for 3 % of the blocks.)
+// at 3.03 waves - a fourth round for 3 % of the blocks.)  The kernels without conductivity
+// tiles hold 8 blocks per SM, not the 4 all are compiled for at least: a single 128^3 instance
+// then marches 4 planes per block instead of 8 (CONST7 residual + restriction 8.7 -> 7.5 us,
+// 27-point convolution 12.5 -> 10.9 us), and eight 48^3 instances of the fused first two sweeps
+// fit one round (10.7 -> 7.6 us).
 template <class T>
-dim3 tma_grid(TmaArgs<T> &a, Grid3 g, int B) {
+dim3 tma_grid(TmaArgs<T> &a, int B, int per_sm) {
   constexpr int TY = Geo<T>::TY;
-  a.tiles_x = (g.X + TX - 1) / TX;
-  const int tiles = a.tiles_x * ((g.Y + TY - 1) / TY);
+  a.tiles_x = (a.X + TX - 1) / TX;
+  const int tiles = a.tiles_x * ((a.Y + TY - 1) / TY);
   const int64_t per = (int64_t)tiles * B;
-  const int64_t cap = (int64_t)sm_count() * Geo<T>::MINB;
-  int zc = g.Z;
+  const int64_t cap = (int64_t)sm_count() * per_sm;
+  int zc = a.Z;
   int64_t best = -1;
-  for (int c = 2; c < g.Z + 2; c += 2) {
-    const int zcc = c > g.Z ? g.Z : c;
-    const int64_t chunks = (g.Z + zcc - 1) / zcc;
+  for (int c = 2; c < a.Z + 2; c += 2) {
+    const int zcc = c > a.Z ? a.Z : c;
+    const int64_t chunks = (a.Z + zcc - 1) / zcc;
     const int64_t cost = ((per * chunks + cap - 1) / cap) * (zcc + 2);
     if (best < 0 || cost <= best) {
       best = cost;
       zc = zcc;
     }
-    if (zcc == g.Z) break;
+    if (zcc == a.Z) break;
   }
   a.zc = zc;
-  return dim3(tiles, (g.Z + zc - 1) / zc, B);
+  return dim3(tiles, (a.Z + zc - 1) / zc, B);
+}
+
+template <int KIND, class T, int MODE, int CORR>
+int go(TmaArgs<T> &a, int B, int *nblk_out, cudaStream_t s) {
+  using G = Geo<T, KIND == HFM_OP_SIGMA7, CORR == 1, MODE == M_PRE2 || CORR == 2>;
+  const int smem = G::NS * G::STAGE;
+  const void *fn = (const void *)k_tma<KIND, T, MODE, CORR>;
+  int st = set_max_dynamic_smem(fn, smem, "cudaFuncSetAttribute(k_tma)");
+  if (st) return st;
+  const dim3 grid = tma_grid(a, B, tma_resident(fn, G::THREADS, smem));
+  if (nblk_out) *nblk_out = grid.x * grid.y;
+  k_tma<KIND, T, MODE, CORR><<<grid, G::THREADS, smem, s>>>(a);
+  HFM_CHECK_LAUNCH("k_tma");
+  return HFM_OK;
+}
+
+template <class T, int MODE, int CORR>
+int go_face(TmaArgs<T> &a, int B, int *nblk_out, cudaStream_t s) {
+  using G = GeoF<CORR != 0, MODE == M_PRE2>;
+  const int smem = G::NS * G::STAGE;
+  const void *fn = (const void *)k_tma_face<T, MODE, CORR>;
+  int st = set_max_dynamic_smem(fn, smem, "cudaFuncSetAttribute(k_tma_face)");
+  if (st) return st;
+  const dim3 grid = tma_grid(a, B, tma_resident(fn, G::THREADS, smem));
+  if (nblk_out) *nblk_out = grid.x * grid.y;
+  k_tma_face<T, MODE, CORR><<<grid, G::THREADS, smem, s>>>(a);
+  HFM_CHECK_LAUNCH("k_tma_face");
+  return HFM_OK;
 }
 
 }  // namespace
@@ -702,15 +726,13 @@ int tma_launch_face(int mode, const DevOp &op, const PhiSrc<T> &phi, const T *rh
   a.omega = omega;
   a.corr_sign = phi.corr_sign;
   a.dot_rhs = ((mode == M_SMOOTH || pre2) && (flags & HFM_INT_DOT_RHS) && partials) ? 1 : 0;
-  dim3 grid = tma_grid(a, g, B);
-  if (nblk_out) *nblk_out = grid.x * grid.y;
-  if (pre2) return go_face<T, M_PRE2, 0>(a, grid, s);
+  if (pre2) return go_face<T, M_PRE2, 0>(a, B, nblk_out, s);
   if (mode == M_SMOOTH) {
-    if (corr) return go_face<T, M_SMOOTH, 1>(a, grid, s);
-    return go_face<T, M_SMOOTH, 0>(a, grid, s);
+    if (corr) return go_face<T, M_SMOOTH, 1>(a, B, nblk_out, s);
+    return go_face<T, M_SMOOTH, 0>(a, B, nblk_out, s);
   }
-  if (mode == M_RESID) return go_face<T, M_RESID, 0>(a, grid, s);
-  return go_face<T, M_RESTRICT, 0>(a, grid, s);
+  if (mode == M_RESID) return go_face<T, M_RESID, 0>(a, B, nblk_out, s);
+  return go_face<T, M_RESTRICT, 0>(a, B, nblk_out, s);
 }
 
 template <class T, int PAIR, int CORR, int W>
@@ -896,9 +918,7 @@ int tma_launch(int kind, int mode, const DevOp &op, const PhiSrc<T> &phi, const 
   a.top_copy = (mode == M_SMOOTH && (flags & HFM_FLAG_TOP_COPY)) ? 1 : 0;
   a.dot_phi = (mode == M_RESID && (flags & HFM_INT_DOT_PHI)) ? 1 : 0;
   a.dot_rhs = (mode == M_SMOOTH && (flags & HFM_INT_DOT_RHS) && partials) ? 1 : 0;
-  dim3 grid = tma_grid(a, g, B);
-  if (nblk_out) *nblk_out = grid.x * grid.y;
-#define HFM_TMA_GO(KIND, MODE, CORR) return go<KIND, T, MODE, CORR>(a, grid, s)
+#define HFM_TMA_GO(KIND, MODE, CORR) return go<KIND, T, MODE, CORR>(a, B, nblk_out, s)
 #define HFM_TMA_MODES(KIND)                                              \
   if (mode == M_SMOOTH) {                                                \
     if (corr == 2) HFM_TMA_GO(KIND, M_SMOOTH, 2);                        \
@@ -956,8 +976,7 @@ int tma_launch_pre2(int kind, const DevOp &op, const T *f, const T *invd, T *out
   a.Y = g.Y;
   a.X = g.X;
   a.omega = omega;
-  dim3 grid = tma_grid(a, g, B);
-  return go<HFM_OP_SIGMA7, T, M_PRE2, 0>(a, grid, s);
+  return go<HFM_OP_SIGMA7, T, M_PRE2, 0>(a, B, nullptr, s);
 }
 
 #define HFM_TMA_INST(T)                                                                       \
