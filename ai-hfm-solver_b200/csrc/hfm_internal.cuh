@@ -237,12 +237,16 @@ int launch_coarse_jacobi(int kind, const DevOp &op, const T *rhs, int64_t rhs_st
                          int sweeps, const int *active, cudaStream_t s);
 int coarse_smem_limit();  // max cells for launch_coarse_jacobi
 
-// Plane-marching kernels (ops_fast.cu) for X % 4 == 0; mode 0 smooth, 1 residual,
-// 2 residual + restriction.  The generic launchers call them when fast_eligible().
+// Register-queue plane-marching kernels (ops_fast.cu); mode 0 smooth, 1 residual, 2 residual +
+// restriction.  fast_eligible: the extents allow 4 cells per thread; fast_width: cells per
+// thread for a grid and its pointers (4, 2 or 1), 0 where the generic kernels serve.
 enum { FAST_SMOOTH = 0, FAST_RESID = 1, FAST_RESTRICT = 2 };
 bool fast_eligible(int kind, Grid3 g, bool restrict_mode);
 template <class T>
-int fast_launch(int kind, int mode, const DevOp &op, const PhiSrc<T> &phi, const T *rhs,
+int fast_width(int kind, const DevOp &op, const PhiSrc<T> &phi, const T *rhs, const T *out,
+               const T *coarse, int64_t stride, Grid3 g, bool restrict_mode);
+template <class T>
+int fast_launch(int kind, int mode, int V, const DevOp &op, const PhiSrc<T> &phi, const T *rhs,
                 T *out, T *coarse, int64_t stride, int64_t coarse_stride, int B, Grid3 g,
                 float omega, unsigned flags, const int *active, double *partials,
                 int *nblk_out, cudaStream_t s);

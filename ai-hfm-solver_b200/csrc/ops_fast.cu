@@ -1,9 +1,9 @@
-// Plane-marching stencil kernels for grids with X % 4 == 0 (the fine and most coarse
-// levels).  Layout and semantics are those of ops_generic.cu; these kernels differ only in
-// how they move data:
-//   * a thread owns 4 consecutive x (one 16-byte float32 / 8-byte 16-bit load) on R rows and
-//     marches along z through a chunk of planes, so z neighbours, the z-face coefficient and
-//     27-point partial sums stay in registers;
+// Register-queue plane-marching stencil kernels.  Layout and semantics are those of
+// ops_generic.cu; these kernels differ only in how they move data:
+//   * a thread owns V consecutive x (V = 4 where rows and pointers allow it: one 16-byte
+//     float32 / 8-byte 16-bit load; else 2 or 1, for the ragged grids) on R rows and marches
+//     along z through a chunk of planes, so z neighbours, the z-face coefficient and 27-point
+//     partial sums stay in registers;
 //   * x neighbours come from the adjacent lanes by warp shuffle (lanes hold consecutive
 //     vectors of the flattened (row, x-vector) index); only lanes 0 / 31 load them;
 //   * y neighbours are vector loads served mostly by L1 (the rows belong to the same block).
@@ -23,62 +23,61 @@ constexpr int kFastThreads = 256;
 enum { M_SMOOTH = FAST_SMOOTH, M_RESID = FAST_RESID, M_RESTRICT = FAST_RESTRICT };
 enum { C_NONE = 0, C_COARSE = 1, C_SAME = 2 };
 
-struct F4 {
-  float v[4];
+template <int V> struct FV {
+  float v[V];
 };
 
-template <class T> __device__ __forceinline__ F4 ld4(const T *p);
-template <> __device__ __forceinline__ F4 ld4<float>(const float *p) {
-  float4 a = __ldg(reinterpret_cast<const float4 *>(p));
-  return F4{{a.x, a.y, a.z, a.w}};
-}
-template <> __device__ __forceinline__ F4 ld4<__nv_bfloat16>(const __nv_bfloat16 *p) {
-  uint2 u = __ldg(reinterpret_cast<const uint2 *>(p));
-  __nv_bfloat162 a = *reinterpret_cast<__nv_bfloat162 *>(&u.x);
-  __nv_bfloat162 b = *reinterpret_cast<__nv_bfloat162 *>(&u.y);
-  float2 fa = __bfloat1622float2(a), fb = __bfloat1622float2(b);
-  return F4{{fa.x, fa.y, fb.x, fb.y}};
-}
-template <> __device__ __forceinline__ F4 ld4<__half>(const __half *p) {
-  uint2 u = __ldg(reinterpret_cast<const uint2 *>(p));
-  __half2 a = *reinterpret_cast<__half2 *>(&u.x);
-  __half2 b = *reinterpret_cast<__half2 *>(&u.y);
-  float2 fa = __half22float2(a), fb = __half22float2(b);
-  return F4{{fa.x, fa.y, fb.x, fb.y}};
+// V consecutive values (V sizeof(T)-byte access).
+template <class T, int V> __device__ __forceinline__ FV<V> ldv(const T *p) {
+  FV<V> r;
+  if constexpr (V == 1) {
+    r.v[0] = St<T>::ld(p);
+  } else if constexpr (sizeof(T) == 4) {
+    if constexpr (V == 4) {
+      const float4 a = __ldg(reinterpret_cast<const float4 *>(p));
+      r.v[0] = a.x; r.v[1] = a.y; r.v[2] = a.z; r.v[3] = a.w;
+    } else {
+      const float2 a = __ldg(reinterpret_cast<const float2 *>(p));
+      r.v[0] = a.x; r.v[1] = a.y;
+    }
+  } else {
+    unsigned u[V / 2];
+    if constexpr (V == 4) {
+      const uint2 q = __ldg(reinterpret_cast<const uint2 *>(p));
+      u[0] = q.x;
+      u[1] = q.y;
+    } else {
+      u[0] = __ldg(reinterpret_cast<const unsigned *>(p));
+    }
+#pragma unroll
+    for (int k = 0; k < V / 2; ++k) {
+      const T *h = reinterpret_cast<const T *>(&u[k]);
+      r.v[2 * k] = St<T>::to(h[0]);
+      r.v[2 * k + 1] = St<T>::to(h[1]);
+    }
+  }
+  return r;
 }
 
-template <class T> __device__ __forceinline__ float2 ld2(const T *p);
-template <> __device__ __forceinline__ float2 ld2<float>(const float *p) {
-  return __ldg(reinterpret_cast<const float2 *>(p));
+template <class T, int V> __device__ __forceinline__ void stv(T *p, const FV<V> &v) {
+  if constexpr (V == 1) {
+    *p = St<T>::from(v.v[0]);
+  } else if constexpr (sizeof(T) == 4) {
+    if constexpr (V == 4) *reinterpret_cast<float4 *>(p) = make_float4(v.v[0], v.v[1], v.v[2], v.v[3]);
+    else *reinterpret_cast<float2 *>(p) = make_float2(v.v[0], v.v[1]);
+  } else {
+    alignas(8) T h[V];
+#pragma unroll
+    for (int k = 0; k < V; ++k) h[k] = St<T>::from(v.v[k]);
+    if constexpr (V == 4) *reinterpret_cast<uint2 *>(p) = *reinterpret_cast<const uint2 *>(h);
+    else *reinterpret_cast<unsigned *>(p) = *reinterpret_cast<const unsigned *>(h);
+  }
 }
-template <> __device__ __forceinline__ float2 ld2<__nv_bfloat16>(const __nv_bfloat16 *p) {
-  unsigned u = __ldg(reinterpret_cast<const unsigned *>(p));
-  return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162 *>(&u));
-}
-template <> __device__ __forceinline__ float2 ld2<__half>(const __half *p) {
-  unsigned u = __ldg(reinterpret_cast<const unsigned *>(p));
-  return __half22float2(*reinterpret_cast<__half2 *>(&u));
-}
-
-template <class T> __device__ __forceinline__ void st4(T *p, const F4 &v);
-template <> __device__ __forceinline__ void st4<float>(float *p, const F4 &v) {
-  *reinterpret_cast<float4 *>(p) = make_float4(v.v[0], v.v[1], v.v[2], v.v[3]);
-}
-template <> __device__ __forceinline__ void st4<__nv_bfloat16>(__nv_bfloat16 *p, const F4 &v) {
-  __nv_bfloat162 a = __floats2bfloat162_rn(v.v[0], v.v[1]);
-  __nv_bfloat162 b = __floats2bfloat162_rn(v.v[2], v.v[3]);
-  uint2 u;
-  u.x = *reinterpret_cast<unsigned *>(&a);
-  u.y = *reinterpret_cast<unsigned *>(&b);
-  *reinterpret_cast<uint2 *>(p) = u;
-}
-template <> __device__ __forceinline__ void st4<__half>(__half *p, const F4 &v) {
-  __half2 a = __floats2half2_rn(fminf(fmaxf(v.v[0], -65504.f), 65504.f), fminf(fmaxf(v.v[1], -65504.f), 65504.f));
-  __half2 b = __floats2half2_rn(fminf(fmaxf(v.v[2], -65504.f), 65504.f), fminf(fmaxf(v.v[3], -65504.f), 65504.f));
-  uint2 u;
-  u.x = *reinterpret_cast<unsigned *>(&a);
-  u.y = *reinterpret_cast<unsigned *>(&b);
-  *reinterpret_cast<uint2 *>(p) = u;
+template <int V> __device__ __forceinline__ FV<V> filled(float x) {
+  FV<V> r;
+#pragma unroll
+  for (int e = 0; e < V; ++e) r.v[e] = x;
+  return r;
 }
 
 template <class T> struct FastArgs {
@@ -113,55 +112,54 @@ __device__ __forceinline__ float phi_scalar(const FastArgs<T> &a, int64_t ib, in
   return v;
 }
 
-// Load phi' (4-vector) at (z, y, x0); zero outside the grid.  `inb` must be warp-uniform
-// only for the shuffle that follows; loads are guarded per lane.
-template <class T, int CORR>
-__device__ __forceinline__ F4 phi_vec(const FastArgs<T> &a, int64_t ib, int64_t ic, int z, int y,
-                                      int x0, bool inb) {
-  F4 v{{0.f, 0.f, 0.f, 0.f}};
+// Load phi' (V-vector) at (z, y, x0); zero outside the grid.
+template <class T, int CORR, int V>
+__device__ __forceinline__ FV<V> phi_vec(const FastArgs<T> &a, int64_t ib, int64_t ic, int z, int y,
+                                         int x0, bool inb) {
+  FV<V> v = filled<V>(0.f);
   if (!inb) return v;
-  if (a.base) v = ld4<T>(a.base + ib + ((int64_t)z * a.Y + y) * a.X + x0);
+  if (a.base) v = ldv<T, V>(a.base + ib + ((int64_t)z * a.Y + y) * a.X + x0);
   if (CORR == C_COARSE) {
-    float2 c = ld2<T>(a.corr + ic + ((int64_t)(z >> 1) * (a.Y >> 1) + (y >> 1)) * (a.X >> 1) + (x0 >> 1));
-    v.v[0] += a.corr_sign * c.x;
-    v.v[1] += a.corr_sign * c.x;
-    v.v[2] += a.corr_sign * c.y;
-    v.v[3] += a.corr_sign * c.y;
-  } else if (CORR == C_SAME) {
-    F4 c = ld4<T>(a.corr + ic + ((int64_t)z * a.Y + y) * a.X + x0);
+    const T *p = a.corr + ic + ((int64_t)(z >> 1) * (a.Y >> 1) + (y >> 1)) * (a.X >> 1) + (x0 >> 1);
+    constexpr int H = V > 1 ? V / 2 : 1;
+    const FV<H> c = ldv<T, H>(p);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) v.v[e] += a.corr_sign * c.v[e];
+    for (int e = 0; e < V; ++e) v.v[e] += a.corr_sign * c.v[e >> 1];
+  } else if (CORR == C_SAME) {
+    const FV<V> c = ldv<T, V>(a.corr + ic + ((int64_t)z * a.Y + y) * a.X + x0);
+#pragma unroll
+    for (int e = 0; e < V; ++e) v.v[e] += a.corr_sign * c.v[e];
   }
-  if (a.zero_xend && x0 + 4 == a.X) v.v[3] = 0.f;
+  if (a.zero_xend && x0 + V == a.X) v.v[V - 1] = 0.f;
   return v;
 }
 
 // Neighbours across the vector boundary by shuffle (all lanes must call).
-template <class T, int CORR>
+template <class T, int CORR, int V>
 __device__ __forceinline__ void halo_x(const FastArgs<T> &a, int64_t ib, int64_t ic, int z, int y,
-                                       int x0, bool inb, const F4 &c, float &l, float &r) {
+                                       int x0, bool inb, const FV<V> &c, float &l, float &r) {
   const int lane = threadIdx.x & 31;
-  float sl = __shfl_up_sync(0xffffffffu, c.v[3], 1);
+  float sl = __shfl_up_sync(0xffffffffu, c.v[V - 1], 1);
   float sr = __shfl_down_sync(0xffffffffu, c.v[0], 1);
   l = 0.f;
   r = 0.f;
   if (inb) {
     if (x0 > 0) l = lane > 0 ? sl : phi_scalar<T, CORR>(a, ib, ic, z, y, x0 - 1);
-    if (x0 + 4 < a.X) r = lane < 31 ? sr : phi_scalar<T, CORR>(a, ib, ic, z, y, x0 + 4);
+    if (x0 + V < a.X) r = lane < 31 ? sr : phi_scalar<T, CORR>(a, ib, ic, z, y, x0 + V);
   }
 }
 
-template <class T>
+template <class T, int V>
 __device__ __forceinline__ void coef_halo_x(const T *s, int64_t base_off, int x0, int X, bool inb,
-                                            const F4 &c, float &l, float &r) {
+                                            const FV<V> &c, float &l, float &r) {
   const int lane = threadIdx.x & 31;
-  float sl = __shfl_up_sync(0xffffffffu, c.v[3], 1);
+  float sl = __shfl_up_sync(0xffffffffu, c.v[V - 1], 1);
   float sr = __shfl_down_sync(0xffffffffu, c.v[0], 1);
   l = c.v[0];  // wall: ghost sigma = interior sigma
-  r = c.v[3];
+  r = c.v[V - 1];
   if (inb) {
     if (x0 > 0) l = lane > 0 ? sl : St<T>::ld(s + base_off - 1);
-    if (x0 + 4 < X) r = lane < 31 ? sr : St<T>::ld(s + base_off + 4);
+    if (x0 + V < X) r = lane < 31 ? sr : St<T>::ld(s + base_off + V);
   }
 }
 
@@ -176,42 +174,46 @@ __device__ __forceinline__ double block_reduce(double v) {
   return t;
 }
 
-// RESTRICT: the two coarse cells of a thread's vector gain plane z of its residuals (x pairs
-// within the vector, y pairs across the two rows); an odd plane completes and stores them.
-template <class T, int R>
+// RESTRICT: the coarse cells of a thread's vector gain plane z of its residuals (x pairs within
+// the vector, y pairs across the two rows); an odd plane completes and stores them.
+template <class T, int R, int V>
 __device__ __forceinline__ void coarse_cells(const FastArgs<T> &a, int64_t inst, int z, int g, int x0,
-                                             bool valid, const F4 (&res)[R], float (&cpart)[2]) {
-  cpart[0] += 0.125f * ((res[0].v[0] + res[0].v[1]) + (res[R - 1].v[0] + res[R - 1].v[1]));
-  cpart[1] += 0.125f * ((res[0].v[2] + res[0].v[3]) + (res[R - 1].v[2] + res[R - 1].v[3]));
-  if (!(z & 1)) return;
-  if (valid) {
-    const int Yc = a.Y >> 1, Xc = a.X >> 1;
-    T *cp = a.coarse + inst * a.coarse_stride + ((int64_t)(z >> 1) * Yc + g) * Xc + (x0 >> 1);
-    if (sizeof(T) == 4) {
-      *reinterpret_cast<float2 *>(cp) = make_float2(cpart[0], cpart[1]);
-    } else {
-      cp[0] = St<T>::from(cpart[0]);
-      cp[1] = St<T>::from(cpart[1]);
+                                             bool valid, const FV<V> (&res)[R], float (&cpart)[2]) {
+  if constexpr (V > 1) {
+#pragma unroll
+    for (int k = 0; k < V / 2; ++k)
+      cpart[k] += 0.125f * ((res[0].v[2 * k] + res[0].v[2 * k + 1]) + (res[R - 1].v[2 * k] + res[R - 1].v[2 * k + 1]));
+    if (!(z & 1)) return;
+    if (valid) {
+      const int Yc = a.Y >> 1, Xc = a.X >> 1;
+      T *cp = a.coarse + inst * a.coarse_stride + ((int64_t)(z >> 1) * Yc + g) * Xc + (x0 >> 1);
+      if (sizeof(T) == 4 && V == 4) {
+        *reinterpret_cast<float2 *>(cp) = make_float2(cpart[0], cpart[1]);
+      } else {
+        cp[0] = St<T>::from(cpart[0]);
+        if (V == 4) cp[1] = St<T>::from(cpart[1]);
+      }
     }
+    cpart[0] = cpart[1] = 0.f;
   }
-  cpart[0] = cpart[1] = 0.f;
 }
 
 // ---------------------------------------------------------------------------------------
 // 7-point forms (CONST7, SIGMA7).  R rows per thread.
 // ---------------------------------------------------------------------------------------
-template <int KIND, class T, int MODE, int CORR, int R>
+template <int KIND, class T, int MODE, int CORR, int R, int V>
 __global__ void __launch_bounds__(kFastThreads, R == 1 ? 4 : 2)
     k_fast7(FastArgs<T> a) {
+  using F4 = FV<V>;  // a thread's cells of a row
   const int64_t inst = blockIdx.z;
   if (a.active && !a.active[inst]) return;
   const int X = a.X, Y = a.Y, Z = a.Z;
-  const int nvx = X >> 2;
+  const int nvx = X / V;
   const int ngroups = (Y + R - 1) / R;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = i < ngroups * nvx;
   const int g = valid ? i / nvx : 0;
-  const int x0 = valid ? (i - g * nvx) * 4 : 0;
+  const int x0 = valid ? (i - g * nvx) * V : 0;
   const int64_t ib = inst * a.stride, ic = inst * a.corr_stride;
   const int64_t plane = (int64_t)Y * X;
   const int z0 = blockIdx.y * a.zc;
@@ -249,25 +251,25 @@ __global__ void __launch_bounds__(kFastThreads, R == 1 ? 4 : 2)
   for (int r = 0; r < R; ++r) {
     yr[r] = g * R + r;
     rin[r] = valid && yr[r] < Y;
-    pm[r] = (z0 > 0) ? phi_vec<T, CORR>(a, ib, ic, z0 - 1, yr[r], x0, rin[r]) : F4{{0.f, 0.f, 0.f, 0.f}};
-    pc[r] = phi_vec<T, CORR>(a, ib, ic, z0, yr[r], x0, rin[r]);
+    pm[r] = (z0 > 0) ? phi_vec<T, CORR, V>(a, ib, ic, z0 - 1, yr[r], x0, rin[r]) : filled<V>(0.f);
+    pc[r] = phi_vec<T, CORR, V>(a, ib, ic, z0, yr[r], x0, rin[r]);
     if (KIND == HFM_OP_SIGMA7) {
       const int64_t off = (int64_t)z0 * plane + (int64_t)yr[r] * X + x0;
-      szc[r] = rin[r] ? ld4<T>(sz + off) : F4{{1.f, 1.f, 1.f, 1.f}};
+      szc[r] = rin[r] ? ldv<T, V>(sz + off) : filled<V>(1.f);
       if (z0 > 0 && rin[r]) {
-        F4 sm = ld4<T>(sz + off - plane);
+        F4 sm = ldv<T, V>(sz + off - plane);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) azlo[r].v[e] = cz * 0.5f * (szc[r].v[e] + sm.v[e]);
+        for (int e = 0; e < V; ++e) azlo[r].v[e] = cz * 0.5f * (szc[r].v[e] + sm.v[e]);
       } else {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) azlo[r].v[e] = cz * szc[r].v[e];
+        for (int e = 0; e < V; ++e) azlo[r].v[e] = cz * szc[r].v[e];
       }
     } else if (KIND == HFM_OP_FACE7) {
       // the z face below plane z0 (wall faces included in the array), times the scale
       const float s = a.op.scale;
-      const F4 fz = rin[r] ? ld4<T>(sz + (int64_t)z0 * plane + (int64_t)yr[r] * X + x0) : F4{{0.f, 0.f, 0.f, 0.f}};
+      const F4 fz = rin[r] ? ldv<T, V>(sz + (int64_t)z0 * plane + (int64_t)yr[r] * X + x0) : filled<V>(0.f);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) azlo[r].v[e] = s * fz.v[e];
+      for (int e = 0; e < V; ++e) azlo[r].v[e] = s * fz.v[e];
     }
   }
   double acc = 0.0;
@@ -279,18 +281,18 @@ __global__ void __launch_bounds__(kFastThreads, R == 1 ? 4 : 2)
     for (int r = 0; r < R; ++r) {
       const int y = yr[r];
       const bool in = rin[r];
-      pp[r] = (z + 1 < Z) ? phi_vec<T, CORR>(a, ib, ic, z + 1, y, x0, in) : F4{{0.f, 0.f, 0.f, 0.f}};
+      pp[r] = (z + 1 < Z) ? phi_vec<T, CORR, V>(a, ib, ic, z + 1, y, x0, in) : filled<V>(0.f);
       float pl, pr;
-      halo_x<T, CORR>(a, ib, ic, z, y, x0, in, pc[r], pl, pr);
-      F4 pym = phi_vec<T, CORR>(a, ib, ic, z, y - 1, x0, in && y > 0);
-      F4 pyp = phi_vec<T, CORR>(a, ib, ic, z, y + 1, x0, in && y + 1 < Y);
+      halo_x<T, CORR, V>(a, ib, ic, z, y, x0, in, pc[r], pl, pr);
+      F4 pym = phi_vec<T, CORR, V>(a, ib, ic, z, y - 1, x0, in && y > 0);
+      F4 pyp = phi_vec<T, CORR, V>(a, ib, ic, z, y + 1, x0, in && y + 1 < Y);
       const int64_t off = (int64_t)z * plane + (int64_t)y * X + x0;
       F4 Ax, dg;
       if (KIND == HFM_OP_CONST7) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
+        for (int e = 0; e < V; ++e) {
           float xm = e == 0 ? pl : pc[r].v[e - 1];
-          float xp = e == 3 ? pr : pc[r].v[e + 1];
+          float xp = e == V - 1 ? pr : pc[r].v[e + 1];
           Ax.v[e] = dconst * pc[r].v[e] - kz * (pm[r].v[e] + pp[r].v[e]) -
                     ky * (pym.v[e] + pyp.v[e]) - kx * (xm + xp);
           dg.v[e] = dconst;
@@ -301,20 +303,20 @@ __global__ void __launch_bounds__(kFastThreads, R == 1 ? 4 : 2)
         const float s = a.op.scale;
         const int64_t rx = ((int64_t)z * Y + y) * (X + 8) + x0;
         const int64_t ry = ((int64_t)z * (Y + 1) + y) * X + x0;
-        const F4 zero4{{0.f, 0.f, 0.f, 0.f}};
-        const F4 fx = in ? ld4<T>(sx + rx) : zero4;
-        const float fx4 = in ? St<T>::ld(sx + rx + 4) : 0.f;
-        const F4 fyl = in ? ld4<T>(sy + ry) : zero4;
-        const F4 fyh = in ? ld4<T>(sy + ry + X) : zero4;
-        const F4 fzh = in ? ld4<T>(sz + off + plane) : zero4;
+        const F4 zero4 = filled<V>(0.f);
+        const F4 fx = in ? ldv<T, V>(sx + rx) : zero4;
+        const float fx4 = in ? St<T>::ld(sx + rx + V) : 0.f;
+        const F4 fyl = in ? ldv<T, V>(sy + ry) : zero4;
+        const F4 fyh = in ? ldv<T, V>(sy + ry + X) : zero4;
+        const F4 fzh = in ? ldv<T, V>(sz + off + plane) : zero4;
         F4 azhi;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float axm = s * fx.v[e], axp = s * (e == 3 ? fx4 : fx.v[e + 1]);
+        for (int e = 0; e < V; ++e) {
+          const float axm = s * fx.v[e], axp = s * (e == V - 1 ? fx4 : fx.v[e + 1]);
           const float aym = s * fyl.v[e], ayp = s * fyh.v[e];
           azhi.v[e] = s * fzh.v[e];
           const float xm = e == 0 ? pl : pc[r].v[e - 1];
-          const float xp = e == 3 ? pr : pc[r].v[e + 1];
+          const float xp = e == V - 1 ? pr : pc[r].v[e + 1];
           const float p = pc[r].v[e];
           Ax.v[e] = axm * (p - xm) + axp * (p - xp) + aym * (p - pym.v[e]) + ayp * (p - pyp.v[e]) +
                     azlo[r].v[e] * (p - pm[r].v[e]) + azhi.v[e] * (p - pp[r].v[e]);
@@ -322,19 +324,19 @@ __global__ void __launch_bounds__(kFastThreads, R == 1 ? 4 : 2)
         }
         azlo[r] = azhi;
       } else {
-        F4 sxc = in ? ld4<T>(sx + off) : F4{{1.f, 1.f, 1.f, 1.f}};
+        F4 sxc = in ? ldv<T, V>(sx + off) : filled<V>(1.f);
         float sxl, sxr;
-        coef_halo_x<T>(sx, off, x0, X, in, sxc, sxl, sxr);
-        F4 syc = in ? ld4<T>(sy + off) : F4{{1.f, 1.f, 1.f, 1.f}};
-        F4 sym = (in && y > 0) ? ld4<T>(sy + off - X) : syc;
-        F4 syp = (in && y + 1 < Y) ? ld4<T>(sy + off + X) : syc;
-        F4 szp = (in && z + 1 < Z) ? ld4<T>(sz + off + plane) : szc[r];
+        coef_halo_x<T, V>(sx, off, x0, X, in, sxc, sxl, sxr);
+        F4 syc = in ? ldv<T, V>(sy + off) : filled<V>(1.f);
+        F4 sym = (in && y > 0) ? ldv<T, V>(sy + off - X) : syc;
+        F4 syp = (in && y + 1 < Y) ? ldv<T, V>(sy + off + X) : syc;
+        F4 szp = (in && z + 1 < Z) ? ldv<T, V>(sz + off + plane) : szc[r];
         F4 azhi;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
+        for (int e = 0; e < V; ++e) {
           const float sxe = sxc.v[e];
           const float sxm = e == 0 ? sxl : sxc.v[e - 1];
-          const float sxp = e == 3 ? sxr : sxc.v[e + 1];
+          const float sxp = e == V - 1 ? sxr : sxc.v[e + 1];
           // wall faces use the interior sigma (sxl / sxr already do at x = 0 / X-1)
           const float axm = cx * 0.5f * (sxe + sxm);
           const float axp = cx * 0.5f * (sxe + sxp);
@@ -342,7 +344,7 @@ __global__ void __launch_bounds__(kFastThreads, R == 1 ? 4 : 2)
           const float ayp = cy * 0.5f * (syc.v[e] + syp.v[e]);
           azhi.v[e] = cz * 0.5f * (szc[r].v[e] + szp.v[e]);
           const float xm = e == 0 ? pl : pc[r].v[e - 1];
-          const float xp = e == 3 ? pr : pc[r].v[e + 1];
+          const float xp = e == V - 1 ? pr : pc[r].v[e + 1];
           const float p = pc[r].v[e];
           Ax.v[e] = axm * (p - xm) + axp * (p - xp) + aym * (p - pym.v[e]) + ayp * (p - pyp.v[e]) +
                     azlo[r].v[e] * (p - pm[r].v[e]) + azhi.v[e] * (p - pp[r].v[e]);
@@ -351,34 +353,186 @@ __global__ void __launch_bounds__(kFastThreads, R == 1 ? 4 : 2)
         azlo[r] = azhi;
         szc[r] = szp;
       }
-      F4 f{{0.f, 0.f, 0.f, 0.f}};
-      if (a.rhs && in) f = ld4<T>(a.rhs + ib + off);
+      F4 f = filled<V>(0.f);
+      if (a.rhs && in) f = ldv<T, V>(a.rhs + ib + off);
       if (MODE == M_SMOOTH) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) res[r].v[e] = pc[r].v[e] + a.omega * __fdividef(f.v[e] - Ax.v[e], dg.v[e]);
+        for (int e = 0; e < V; ++e) res[r].v[e] = pc[r].v[e] + a.omega * __fdividef(f.v[e] - Ax.v[e], dg.v[e]);
         if (a.dot_rhs && in) {
 #pragma unroll
-          for (int e = 0; e < 4; ++e) acc += (double)res[r].v[e] * f.v[e];
+          for (int e = 0; e < V; ++e) acc += (double)res[r].v[e] * f.v[e];
         }
       } else {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) res[r].v[e] = Ax.v[e] - f.v[e];
-        if (a.zero_xend_out && x0 + 4 == X) res[r].v[3] = 0.f;
+        for (int e = 0; e < V; ++e) res[r].v[e] = Ax.v[e] - f.v[e];
+        if (a.zero_xend_out && x0 + V == X) res[r].v[V - 1] = 0.f;
         if (in) {
 #pragma unroll
-          for (int e = 0; e < 4; ++e) acc += (double)res[r].v[e] * (a.dot_phi ? pc[r].v[e] : res[r].v[e]);
+          for (int e = 0; e < V; ++e) acc += (double)res[r].v[e] * (a.dot_phi ? pc[r].v[e] : res[r].v[e]);
         }
       }
       if (in && a.out) {
-        if (MODE == M_SMOOTH && a.top_copy && z == 1) st4<T>(a.out + ib + y * X + x0, res[r]);
-        if (!(MODE == M_SMOOTH && a.top_copy && z == 0 && Z > 1)) st4<T>(a.out + ib + off, res[r]);
+        if (MODE == M_SMOOTH && a.top_copy && z == 1) stv<T, V>(a.out + ib + y * X + x0, res[r]);
+        if (!(MODE == M_SMOOTH && a.top_copy && z == 0 && Z > 1)) stv<T, V>(a.out + ib + off, res[r]);
       }
       pm[r] = pc[r];
       pc[r] = pp[r];
     }
-    if (MODE == M_RESTRICT) coarse_cells<T, R>(a, inst, z, g, x0, valid, res, cpart);
+    if (MODE == M_RESTRICT) coarse_cells<T, R, V>(a, inst, z, g, x0, valid, res, cpart);
   }
   if ((MODE != M_SMOOTH || a.dot_rhs) && a.partials) {
+    double t = block_reduce(acc);
+    if (threadIdx.x == 0) a.partials[inst * (gridDim.x * gridDim.y) + blockIdx.y * gridDim.x + blockIdx.x] = t;
+  }
+}
+
+// ---------------------------------------------------------------------------------------
+// 7-point forms on rows of an odd number of cells (or off every vector boundary): one column
+// of cells per thread.  Nine 4-byte loads per cell are then the least the pass can do, so it is
+// bound by their latency unless they are issued early: the loads of plane z + 1 go out before
+// plane z is computed, and the index arithmetic is kept to 32-bit byte offsets from the
+// instance's pointers (64-bit element offsets made 257 instructions per cell, these 173).
+// 4 x 75 x 90 x 101, SIGMA7: a sweep 19.6 us, 3.9 TB/s (k_fast7 with one cell per thread, loads
+// and use in one plane, 40 us; one thread per cell with 64-bit divisions 53 us).  The arithmetic
+// is k_fast7's.
+// ---------------------------------------------------------------------------------------
+template <int KIND, class T, int MODE, int CORR>
+__global__ void __launch_bounds__(kFastThreads, 4) k_column7(FastArgs<T> a) {
+  const int64_t inst = blockIdx.z;
+  if (a.active && !a.active[inst]) return;
+  constexpr bool SIG = KIND == HFM_OP_SIGMA7;
+  constexpr unsigned ES = sizeof(T);
+  const int X = a.X, Y = a.Y, Z = a.Z;
+  const int lane = threadIdx.x & 31;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = i < X * Y;
+  const int y = valid ? i / X : 0, x = valid ? i - y * X : 0;
+  const int z0 = blockIdx.y * a.zc, z1 = min(Z, z0 + a.zc);
+  const T *phi = a.base + inst * a.stride;  // not read when base is null
+  const T *cor = a.corr + inst * a.corr_stride;
+  const T *rhs = a.rhs + inst * a.stride;
+  T *out = a.out + inst * a.stride;
+  const T *sx = nullptr, *sy = nullptr, *sz = nullptr;
+  float cx = 0.f, cy = 0.f, cz = 0.f, kx = 0.f, ky = 0.f, kz = 0.f;
+  if (SIG) {
+    sx = (const T *)a.op.coef[0] + inst * a.op.coef_stride;
+    sy = (const T *)a.op.coef[1] + inst * a.op.coef_stride;
+    sz = (const T *)a.op.coef[2] + inst * a.op.coef_stride;
+    cz = a.op.c[0] * a.op.scale;
+    cy = a.op.c[1] * a.op.scale;
+    cx = a.op.c[2] * a.op.scale;
+  } else {
+    kz = a.op.k[0];
+    ky = a.op.k[1];
+    kx = a.op.k[2];
+  }
+  // value at a byte offset from an instance pointer (uniform base, 32-bit offset)
+  auto ld = [](const T *base, unsigned off) {
+    return St<T>::ld(reinterpret_cast<const T *>(reinterpret_cast<const char *>(base) + off));
+  };
+  // phi' at byte offset o, cell (zz, yy, xx); `p`: the cell is in the grid and not zeroed by the
+  // x-end rule
+  const bool has = a.base != nullptr;
+  auto at = [&](bool p, int zz, int yy, int xx, unsigned o) -> float {
+    float v = 0.f;
+    if (has && p) v = ld(phi, o);
+    if (CORR == C_COARSE && p)
+      v += a.corr_sign * ld(cor, ES * (unsigned)(((zz >> 1) * (Y >> 1) + (yy >> 1)) * (X >> 1) + (xx >> 1)));
+    if (CORR == C_SAME && p) v += a.corr_sign * ld(cor, o);
+    return v;
+  };
+  // lanes 0 and 31 load the row neighbour the shuffles cannot give
+  const int dx = lane == 0 ? -1 : 1;
+  const bool edge = valid && ((lane == 0 && x > 0) || (lane == 31 && x + 1 < X));
+  const bool live = valid && !(a.zero_xend && x == X - 1);
+  const bool live_lo = live && y > 0, live_hi = live && y + 1 < Y;
+  const bool live_e = edge && !(a.zero_xend && x + dx == X - 1);
+  const bool f_in = a.rhs && valid;
+  const unsigned row = ES * (unsigned)X, plane = row * (unsigned)Y;
+  const unsigned ylo = valid && y > 0 ? row : 0u, yhi = valid && y + 1 < Y ? row : 0u;  // wall: own sigma
+  const unsigned xe = edge ? (unsigned)((int)ES * dx) : 0u;
+  struct Plane {
+    float pp, ym, yp, pe, f;           // phi' above, before / after in y, at the edge; rhs
+    float sxc, sxe, syc, sym, syp, szp;
+  };
+  auto load = [&](int z, unsigned o, Plane &q) {
+    q.pp = at(live && z + 1 < Z, z + 1, y, x, o + plane);
+    q.ym = at(live_lo, z, y - 1, x, o - row);
+    q.yp = at(live_hi, z, y + 1, x, o + row);
+    q.pe = at(live_e, z, y, x + dx, o + (unsigned)((int)ES * dx));
+    q.f = f_in ? ld(rhs, o) : 0.f;
+    if (SIG) {
+      q.sxc = ld(sx, o);
+      q.sxe = edge ? ld(sx, o + xe) : q.sxc;
+      q.syc = ld(sy, o);
+      q.sym = ld(sy, o - ylo);
+      q.syp = ld(sy, o + yhi);
+      q.szp = ld(sz, z + 1 < Z ? o + plane : o);
+    }
+  };
+  // threads past the plane read cell (z, 0, 0)'s conductivities and store nothing
+  unsigned o = ES * (unsigned)(z0 * X * Y + (valid ? i : 0));
+  float pm = at(live && z0 > 0, z0 - 1, y, x, o - plane);
+  float pc = at(live, z0, y, x, o);
+  Plane nx;
+  load(z0, o, nx);
+  float szc = 1.f, azlo = 0.f;
+  if (SIG) {
+    szc = ld(sz, o);
+    azlo = z0 > 0 ? cz * 0.5f * (szc + ld(sz, o - plane)) : cz * szc;
+  }
+  const bool sums = a.partials && (MODE != M_SMOOTH || a.dot_rhs);
+  double acc = 0.0;
+  for (int z = z0; z < z1; ++z) {
+    const Plane q = nx;
+    const unsigned here = o;
+    o += plane;
+    if (z + 1 < z1) load(z + 1, o, nx);
+    float l = __shfl_up_sync(0xffffffffu, pc, 1), r = __shfl_down_sync(0xffffffffu, pc, 1);
+    l = lane == 0 ? q.pe : l;
+    r = lane == 31 ? q.pe : r;
+    if (x == 0) l = 0.f;
+    if (x + 1 == X) r = 0.f;
+    float Ax, dg;
+    if (SIG) {
+      float sl = __shfl_up_sync(0xffffffffu, q.sxc, 1), sr = __shfl_down_sync(0xffffffffu, q.sxc, 1);
+      sl = lane == 0 ? q.sxe : sl;
+      sr = lane == 31 ? q.sxe : sr;
+      if (x == 0) sl = q.sxc;  // wall: ghost sigma = interior sigma
+      if (x + 1 == X) sr = q.sxc;
+      const float axm = cx * 0.5f * (q.sxc + sl), axp = cx * 0.5f * (q.sxc + sr);
+      const float aym = cy * 0.5f * (q.syc + q.sym), ayp = cy * 0.5f * (q.syc + q.syp);
+      const float azhi = cz * 0.5f * (szc + q.szp);
+      Ax = axm * (pc - l) + axp * (pc - r) + aym * (pc - q.ym) + ayp * (pc - q.yp) + azlo * (pc - pm) +
+           azhi * (pc - q.pp);
+      dg = axm + axp + aym + ayp + azlo + azhi;
+      azlo = azhi;
+      szc = q.szp;
+    } else {
+      dg = 2.f * (kx + ky + kz);
+      Ax = dg * pc - kz * (pm + q.pp) - ky * (q.ym + q.yp) - kx * (l + r);
+    }
+    float v;
+    if (MODE == M_SMOOTH) {
+      v = pc + a.omega * __fdividef(q.f - Ax, dg);
+    } else {
+      v = Ax - q.f;
+      if (a.zero_xend_out && x == X - 1) v = 0.f;
+    }
+    if (sums && valid) acc += (double)v * (MODE == M_SMOOTH ? q.f : a.dot_phi ? pc : v);
+    if (valid) {
+      T *dst = reinterpret_cast<T *>(reinterpret_cast<char *>(out) + here);
+      if (MODE == M_SMOOTH && a.top_copy && Z > 1) {
+        if (z > 0) *dst = St<T>::from(v);
+        if (z == 1) out[i] = St<T>::from(v);
+      } else {
+        *dst = St<T>::from(v);
+      }
+    }
+    pm = pc;
+    pc = q.pp;
+  }
+  if (sums) {
     double t = block_reduce(acc);
     if (threadIdx.x == 0) a.partials[inst * (gridDim.x * gridDim.y) + blockIdx.y * gridDim.x + blockIdx.x] = t;
   }
@@ -391,19 +545,20 @@ __global__ void __launch_bounds__(kFastThreads, R == 1 ? 4 : 2)
 // chain of dependent loads; a thread per coarse cell with 216 bounds-checked loads took 21 us
 // (and 82 us on 64 x 128 x 128, where the plane-marching TMA kernel takes 8 us).
 // ---------------------------------------------------------------------------------------
-template <class T, int MODE, int CORR, int R>
+template <class T, int MODE, int CORR, int R, int V>
 __global__ void __launch_bounds__(kFastThreads)
     k_fast27(FastArgs<T> a) {
+  using F4 = FV<V>;  // a thread's cells of a row
   const int64_t inst = blockIdx.z;
   if (a.active && !a.active[inst]) return;
   const int X = a.X, Y = a.Y, Z = a.Z;
-  const int nvx = X >> 2;
+  const int nvx = X / V;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int ngroups = (Y + R - 1) / R;
   const bool valid = i < ngroups * nvx;
   const int g = valid ? i / nvx : 0;
   const int y0 = g * R;  // RESTRICT: Y is even, so both rows are inside
-  const int x0 = valid ? (i - g * nvx) * 4 : 0;
+  const int x0 = valid ? (i - g * nvx) * V : 0;
   const int64_t ib = inst * a.stride, ic = inst * a.corr_stride;
   const int64_t plane = (int64_t)Y * X;
   const int z0 = blockIdx.y * a.zc;
@@ -418,20 +573,20 @@ __global__ void __launch_bounds__(kFastThreads)
     for (int b = 0; b < R + 2; ++b) {
       const int yy = y0 + b - 1;
       const bool in = valid && p >= 0 && p < Z && yy >= 0 && yy < Y;
-      rows[b] = phi_vec<T, CORR>(a, ib, ic, p, yy, x0, in);
-      halo_x<T, CORR>(a, ib, ic, p, yy, x0, in, rows[b], ls[b], rs[b]);
+      rows[b] = phi_vec<T, CORR, V>(a, ib, ic, p, yy, x0, in);
+      halo_x<T, CORR, V>(a, ib, ic, p, yy, x0, in, rows[b], ls[b], rs[b]);
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       centre[r] = rows[r + 1];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
+      for (int e = 0; e < V; ++e) {
         float t0 = 0.f, t1 = 0.f, t2 = 0.f;
 #pragma unroll
         for (int b = 0; b < 3; ++b) {
           const float xm = e == 0 ? ls[r + b] : rows[r + b].v[e - 1];
           const float xc = rows[r + b].v[e];
-          const float xp = e == 3 ? rs[r + b] : rows[r + b].v[e + 1];
+          const float xp = e == V - 1 ? rs[r + b] : rows[r + b].v[e + 1];
           t0 += K[3 * b + 0] * xm + K[3 * b + 1] * xc + K[3 * b + 2] * xp;
           t1 += K[9 + 3 * b + 0] * xm + K[9 + 3 * b + 1] * xc + K[9 + 3 * b + 2] * xp;
           t2 += K[18 + 3 * b + 0] * xm + K[18 + 3 * b + 1] * xc + K[18 + 3 * b + 2] * xp;
@@ -452,7 +607,7 @@ __global__ void __launch_bounds__(kFastThreads)
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
+      for (int e = 0; e < V; ++e) {
         acc_cur[r].v[e] = d0[r].v[e] + s1[r].v[e];
         acc_next[r].v[e] = s0[r].v[e];
       }
@@ -469,39 +624,39 @@ __global__ void __launch_bounds__(kFastThreads)
       const bool in = valid && y < Y;
       F4 Ax;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) Ax.v[e] = acc_cur[r].v[e] + n2[r].v[e];
+      for (int e = 0; e < V; ++e) Ax.v[e] = acc_cur[r].v[e] + n2[r].v[e];
       const int64_t off = (int64_t)z * plane + (int64_t)y * X + x0;
-      F4 f{{0.f, 0.f, 0.f, 0.f}};
-      if (a.rhs && in) f = ld4<T>(a.rhs + ib + off);
+      F4 f = filled<V>(0.f);
+      if (a.rhs && in) f = ldv<T, V>(a.rhs + ib + off);
       if (MODE == M_SMOOTH) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) res[r].v[e] = cen_cur[r].v[e] + a.omega * __fdividef(f.v[e] - Ax.v[e], diag);
+        for (int e = 0; e < V; ++e) res[r].v[e] = cen_cur[r].v[e] + a.omega * __fdividef(f.v[e] - Ax.v[e], diag);
         if (a.dot_rhs && in) {
 #pragma unroll
-          for (int e = 0; e < 4; ++e) acc2 += (double)res[r].v[e] * f.v[e];
+          for (int e = 0; e < V; ++e) acc2 += (double)res[r].v[e] * f.v[e];
         }
       } else {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) res[r].v[e] = Ax.v[e] - f.v[e];
-        if (a.zero_xend_out && x0 + 4 == X) res[r].v[3] = 0.f;
+        for (int e = 0; e < V; ++e) res[r].v[e] = Ax.v[e] - f.v[e];
+        if (a.zero_xend_out && x0 + V == X) res[r].v[V - 1] = 0.f;
         if (in) {
 #pragma unroll
-          for (int e = 0; e < 4; ++e)
+          for (int e = 0; e < V; ++e)
             acc2 += (double)res[r].v[e] * (a.dot_phi ? cen_cur[r].v[e] : res[r].v[e]);
         }
       }
       if (in && a.out) {
-        if (MODE == M_SMOOTH && a.top_copy && z == 1) st4<T>(a.out + ib + y * X + x0, res[r]);
-        if (!(MODE == M_SMOOTH && a.top_copy && z == 0 && Z > 1)) st4<T>(a.out + ib + off, res[r]);
+        if (MODE == M_SMOOTH && a.top_copy && z == 1) stv<T, V>(a.out + ib + y * X + x0, res[r]);
+        if (!(MODE == M_SMOOTH && a.top_copy && z == 0 && Z > 1)) stv<T, V>(a.out + ib + off, res[r]);
       }
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
+      for (int e = 0; e < V; ++e) {
         acc_cur[r].v[e] = acc_next[r].v[e] + n1[r].v[e];
         acc_next[r].v[e] = n0[r].v[e];
       }
       cen_cur[r] = cen_next[r];
     }
-    if (MODE == M_RESTRICT) coarse_cells<T, R>(a, inst, z, g, x0, valid, res, cpart);
+    if (MODE == M_RESTRICT) coarse_cells<T, R, V>(a, inst, z, g, x0, valid, res, cpart);
   }
   if ((MODE != M_SMOOTH || a.dot_rhs) && a.partials) {
     double t = block_reduce(acc2);
@@ -533,8 +688,8 @@ int resident_blocks(const void *kernel) {
 // chunks and 3.2 us with one-plane chunks.  Chunks of fewer than 4 planes are taken only while
 // the whole launch is resident, which also bounds the partial sums per instance.
 template <class T>
-dim3 fast_grid(FastArgs<T> &a, int B, int rows, bool even_chunks, int per_sm) {
-  const int nvx = a.X >> 2;
+dim3 fast_grid(FastArgs<T> &a, int B, int rows, int V, bool even_chunks, int per_sm) {
+  const int nvx = a.X / V;
   const int64_t vecs = (int64_t)((a.Y + rows - 1) / rows) * nvx;
   const int tiles = (int)((vecs + kFastThreads - 1) / kFastThreads);
   const int64_t target = (int64_t)sm_count() * per_sm;
@@ -559,8 +714,63 @@ bool fast_eligible(int kind, Grid3 g, bool restrict_mode) {
   return true;
 }
 
+// Cells per thread of the register-queue kernels for a grid and its pointers, 0: the generic
+// kernels.  V = 4 needs rows of a multiple of 4 and pointers aligned to 4 elements; the other
+// grids of the 7- and 27-point forms take V = 2 (even rows, pointers aligned to 2 elements) or
+// V = 1 from 8 columns up: 4 x 75 x 90 x 101, a SIGMA7 sweep 53 -> 20 us.  Narrower rows, of
+// a few hundred cells at most where they occur, stay with one thread per cell.  A correction
+// on a coarse grid of a fine grid with odd extents does too (nearest prolongation past the
+// last coarse cell).
 template <class T>
-int fast_launch(int kind, int mode, const DevOp &op, const PhiSrc<T> &phi, const T *rhs,
+int fast_width(int kind, const DevOp &op, const PhiSrc<T> &phi, const T *rhs, const T *out,
+               const T *coarse, int64_t stride, Grid3 g, bool restrict_mode) {
+  const int64_t es = (int64_t)sizeof(T);
+  if (fast_eligible(kind, g, restrict_mode) && vec_aligned<T>(kind, op, phi, rhs, out, coarse, stride, 4 * es))
+    return 4;
+  if ((kind != HFM_OP_CONST7 && kind != HFM_OP_SIGMA7 && kind != HFM_OP_K27) || g.X < 8) return 0;
+  if ((restrict_mode || (phi.corr && phi.corr_coarse)) && ((g.Z | g.Y | g.X) & 1)) return 0;
+  if (!(g.X & 1) && vec_aligned<T>(kind, op, phi, rhs, out, coarse, stride, 2 * es)) return 2;
+  // k_column7 keeps 32-bit byte offsets within an instance
+  return restrict_mode || g.n() * es >= ((int64_t)1 << 32) || g.n() >= ((int64_t)1 << 31) ? 0 : 1;
+}
+
+template <class T, int V, int KIND>
+int fast_go(int mode, int corr, FastArgs<T> &a, int B, int *nblk_out, cudaStream_t s) {
+#define HFM_FAST_GO(KER, ROWS)                                                                 \
+  do {                                                                                         \
+    const dim3 grid = fast_grid<T>(a, B, ROWS, V, mode == M_RESTRICT,                          \
+                                   resident_blocks((const void *)KER));                        \
+    if (nblk_out) *nblk_out = grid.x * grid.y;                                                 \
+    KER<<<grid, kFastThreads, 0, s>>>(a);                                                      \
+  } while (0)
+#define HFM_FAST_K(M, C, R)                                                                    \
+  do {                                                                                         \
+    if constexpr (KIND == HFM_OP_K27) HFM_FAST_GO((k_fast27<T, M, C, R, V>), R);               \
+    else if constexpr (V == 1) HFM_FAST_GO((k_column7<KIND, T, M, C>), R);                     \
+    else HFM_FAST_GO((k_fast7<KIND, T, M, C, R, V>), R);                                       \
+  } while (0)
+  if (mode == M_SMOOTH) {
+    if (corr == C_NONE) HFM_FAST_K(M_SMOOTH, C_NONE, 1);
+    else if (corr == C_COARSE) HFM_FAST_K(M_SMOOTH, C_COARSE, 1);
+    else HFM_FAST_K(M_SMOOTH, C_SAME, 1);
+  } else {
+    if (corr != C_NONE) return fail(HFM_ERR_UNSUPPORTED, "fast path: corrected residual");
+    if (mode == M_RESID) {
+      HFM_FAST_K(M_RESID, C_NONE, 1);
+    } else if constexpr (V > 1) {
+      HFM_FAST_K(M_RESTRICT, C_NONE, 2);
+    } else {
+      return fail(HFM_ERR_UNSUPPORTED, "fast path: restriction of odd rows");
+    }
+  }
+#undef HFM_FAST_K
+#undef HFM_FAST_GO
+  HFM_CHECK_LAUNCH("fast stencil kernel");
+  return HFM_OK;
+}
+
+template <class T>
+int fast_launch(int kind, int mode, int V, const DevOp &op, const PhiSrc<T> &phi, const T *rhs,
                 T *out, T *coarse, int64_t stride, int64_t coarse_stride, int B, Grid3 g,
                 float omega, unsigned flags, const int *active, double *partials,
                 int *nblk_out, cudaStream_t s) {
@@ -589,55 +799,22 @@ int fast_launch(int kind, int mode, const DevOp &op, const PhiSrc<T> &phi, const
   a.zc = 0;
   if (phi.base && phi.base_stride != stride) return fail(HFM_ERR_BAD_ARG, "fast path: stride mismatch");
   const int corr = phi.corr ? (phi.corr_coarse ? C_COARSE : C_SAME) : C_NONE;
-  const int rows = (mode == M_RESTRICT) ? 2 : 1;
-#define HFM_FAST_GO(KER)                                                                       \
-  do {                                                                                         \
-    const dim3 grid = fast_grid<T>(a, B, rows, mode == M_RESTRICT,                             \
-                                   resident_blocks((const void *)KER));                        \
-    if (nblk_out) *nblk_out = grid.x * grid.y;                                                 \
-    KER<<<grid, kFastThreads, 0, s>>>(a);                                                      \
-  } while (0)
-  // dispatch
-  if (kind == HFM_OP_K27) {
-    if (mode == M_SMOOTH) {
-      if (corr == C_NONE) HFM_FAST_GO((k_fast27<T, M_SMOOTH, C_NONE, 1>));
-      else if (corr == C_COARSE) HFM_FAST_GO((k_fast27<T, M_SMOOTH, C_COARSE, 1>));
-      else HFM_FAST_GO((k_fast27<T, M_SMOOTH, C_SAME, 1>));
-    } else {
-      if (corr != C_NONE) return fail(HFM_ERR_UNSUPPORTED, "fast path: corrected residual");
-      if (mode == M_RESID) HFM_FAST_GO((k_fast27<T, M_RESID, C_NONE, 1>));
-      else HFM_FAST_GO((k_fast27<T, M_RESTRICT, C_NONE, 2>));
-    }
-  } else {
-#define HFM_FAST7(KIND)                                                                        \
-  if (mode == M_SMOOTH) {                                                                      \
-    if (corr == C_NONE) HFM_FAST_GO((k_fast7<KIND, T, M_SMOOTH, C_NONE, 1>));                  \
-    else if (corr == C_COARSE) HFM_FAST_GO((k_fast7<KIND, T, M_SMOOTH, C_COARSE, 1>));         \
-    else HFM_FAST_GO((k_fast7<KIND, T, M_SMOOTH, C_SAME, 1>));                                 \
-  } else if (mode == M_RESID) {                                                                \
-    if (corr != C_NONE) return fail(HFM_ERR_UNSUPPORTED, "fast path: corrected residual");     \
-    HFM_FAST_GO((k_fast7<KIND, T, M_RESID, C_NONE, 1>));                                       \
-  } else {                                                                                     \
-    if (corr != C_NONE) return fail(HFM_ERR_UNSUPPORTED, "fast path: corrected residual");     \
-    HFM_FAST_GO((k_fast7<KIND, T, M_RESTRICT, C_NONE, 2>));                                    \
-  }
-    if (kind == HFM_OP_CONST7) {
-      HFM_FAST7(HFM_OP_CONST7)
-    } else if (kind == HFM_OP_FACE7) {
-      HFM_FAST7(HFM_OP_FACE7)
-    } else {
-      HFM_FAST7(HFM_OP_SIGMA7)
-    }
-#undef HFM_FAST7
-  }
-#undef HFM_FAST_GO
-  HFM_CHECK_LAUNCH("fast stencil kernel");
-  return HFM_OK;
+#define HFM_FAST_V(KIND)                                                          \
+  (V == 4 ? fast_go<T, 4, KIND>(mode, corr, a, B, nblk_out, s)                    \
+   : V == 2 ? fast_go<T, 2, KIND>(mode, corr, a, B, nblk_out, s)                  \
+            : fast_go<T, 1, KIND>(mode, corr, a, B, nblk_out, s))
+  if (kind == HFM_OP_FACE7) return fast_go<T, 4, HFM_OP_FACE7>(mode, corr, a, B, nblk_out, s);
+  if (kind == HFM_OP_K27) return HFM_FAST_V(HFM_OP_K27);
+  if (kind == HFM_OP_CONST7) return HFM_FAST_V(HFM_OP_CONST7);
+  return HFM_FAST_V(HFM_OP_SIGMA7);
+#undef HFM_FAST_V
 }
 
 #define HFM_FAST_INST(T)                                                                       \
-  template int fast_launch<T>(int, int, const DevOp &, const PhiSrc<T> &, const T *, T *, T *, \
-                              int64_t, int64_t, int, Grid3, float, unsigned, const int *,      \
+  template int fast_width<T>(int, const DevOp &, const PhiSrc<T> &, const T *, const T *,      \
+                             const T *, int64_t, Grid3, bool);                                 \
+  template int fast_launch<T>(int, int, int, const DevOp &, const PhiSrc<T> &, const T *, T *, \
+                              T *, int64_t, int64_t, int, Grid3, float, unsigned, const int *, \
                               double *, int *, cudaStream_t);
 HFM_FAST_INST(float)
 HFM_FAST_INST(__nv_bfloat16)

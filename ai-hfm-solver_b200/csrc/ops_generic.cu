@@ -1,8 +1,8 @@
 // Generic stencil / transfer kernels: one thread per output cell, any grid extent.
 //
-// These kernels serve every extent (odd sizes, the 1^3 / 2^3 / 5x1x1 coarse levels of the
-// reference cycles, X not a multiple of 4).  Fine levels with X % 4 == 0 are served by the
-// plane-marching kernels in ops_fast.cu.
+// These kernels serve every extent (the 1^3 / 2^3 / 5x1x1 coarse levels of the reference
+// cycles, rows of fewer than 8 cells) and the directional form; the other grids are served by
+// the plane-marching kernels in ops_tma.cu and ops_fast.cu.
 #include "hfm_internal.cuh"
 
 namespace hfm {
@@ -346,8 +346,10 @@ __global__ void k_coarse_jacobi(DevOp op, const T *__restrict__ rhs, int64_t rhs
 int coarse_smem_limit() { return 4096; }
 
 int64_t max_partial_blocks(Grid3 g, int B) {
-  // generic kernels: blocks_for() <= 8 per SM; fast kernels: plane tiles x z chunks
-  const int64_t tiles = ((int64_t)g.Y * (g.X / 4) + 255) / 256 + 1;
+  // generic kernels: blocks_for() <= 8 per SM; fast kernels: plane tiles x z chunks (chunks of
+  // fewer than 4 planes only while the whole launch is resident)
+  const int V = g.X % 4 == 0 ? 4 : g.X % 2 == 0 ? 2 : 1;
+  const int64_t tiles = ((int64_t)g.Y * (g.X / V) + 255) / 256 + 1;
   const int64_t chunks = (g.Z + 3) / 4 + 1;
   int64_t v = tiles * chunks;
   const int64_t tma_tiles = ((int64_t)(g.X + 63) / 64) * ((g.Y + 7) / 8);
@@ -379,10 +381,11 @@ int launch_smooth(int kind, const DevOp &op, const PhiSrc<T> &phi, const T *rhs,
       vec_aligned<T>(kind, op, phi, rhs, out, nullptr, out_stride, 16))
     return tma_launch<T>(kind, FAST_SMOOTH, op, phi, rhs, out, nullptr, out_stride, 0, B, g,
                          omega, flags, active, partials, nblk_out, s);
-  if (fast_eligible(kind, g, false) && (!rhs || rhs_stride == out_stride) &&
-      (!phi.base || phi.base_stride == out_stride) && (!phi.corr || phi.corr_coarse || phi.corr_stride == out_stride) &&
-      vec_aligned<T>(kind, op, phi, rhs, out, nullptr, out_stride, 4 * (int64_t)sizeof(T)))
-    return fast_launch<T>(kind, FAST_SMOOTH, op, phi, rhs, out, nullptr, out_stride, 0, B, g,
+  int V;
+  if ((!rhs || rhs_stride == out_stride) && (!phi.base || phi.base_stride == out_stride) &&
+      (!phi.corr || phi.corr_coarse || phi.corr_stride == out_stride) &&
+      (V = fast_width<T>(kind, op, phi, rhs, out, nullptr, out_stride, g, false)))
+    return fast_launch<T>(kind, FAST_SMOOTH, V, op, phi, rhs, out, nullptr, out_stride, 0, B, g,
                           omega, flags, active, partials, nblk_out, s);
   const int nb = blocks_for(g.n(), B);
   if (nblk_out) *nblk_out = nb;
@@ -404,10 +407,10 @@ int launch_residual(int kind, const DevOp &op, const PhiSrc<T> &phi, const T *b,
       vec_aligned<T>(kind, op, phi, b, r, nullptr, r_stride, 16))
     return tma_launch<T>(kind, FAST_RESID, op, phi, b, r, nullptr, r_stride, 0, B, g, 0.f,
                          flags, active, partials, nblk_out, s);
-  if (fast_eligible(kind, g, false) && !phi.corr && r &&
-      (!b || b_stride == r_stride) && (!phi.base || phi.base_stride == r_stride) &&
-      vec_aligned<T>(kind, op, phi, b, r, nullptr, r_stride, 4 * (int64_t)sizeof(T)))
-    return fast_launch<T>(kind, FAST_RESID, op, phi, b, r, nullptr, r_stride, 0, B, g, 0.f,
+  int V;
+  if (!phi.corr && r && (!b || b_stride == r_stride) && (!phi.base || phi.base_stride == r_stride) &&
+      (V = fast_width<T>(kind, op, phi, b, r, nullptr, r_stride, g, false)))
+    return fast_launch<T>(kind, FAST_RESID, V, op, phi, b, r, nullptr, r_stride, 0, B, g, 0.f,
                           flags, active, partials, nblk_out, s);
   int nb = blocks_for(g.n(), B);
   if (nblk_out) *nblk_out = nb;
@@ -440,11 +443,11 @@ int launch_residual_restrict(int kind, const DevOp &op, const PhiSrc<T> &phi, co
       vec_aligned<T>(kind, op, phi, b, r_fine, nullptr, b_stride, 16))
     return tma_launch<T>(kind, FAST_RESTRICT, op, phi, b, r_fine, r_coarse, b_stride, rc_stride,
                          B, g, 0.f, flags, active, partials, nblk_out, s);
-  if (fast_eligible(kind, g, true) && !phi.corr && b &&
-      (!r_fine || rf_stride == b_stride) && (!phi.base || phi.base_stride == b_stride) &&
+  int V;
+  if (!phi.corr && b && (!r_fine || rf_stride == b_stride) && (!phi.base || phi.base_stride == b_stride) &&
       rc_stride == b_stride / 8 &&
-      vec_aligned<T>(kind, op, phi, b, r_fine, r_coarse, b_stride, 4 * (int64_t)sizeof(T)))
-    return fast_launch<T>(kind, FAST_RESTRICT, op, phi, b, r_fine, r_coarse, b_stride, rc_stride,
+      (V = fast_width<T>(kind, op, phi, b, r_fine, r_coarse, b_stride, g, true)))
+    return fast_launch<T>(kind, FAST_RESTRICT, V, op, phi, b, r_fine, r_coarse, b_stride, rc_stride,
                           B, g, 0.f, flags, active, partials, nblk_out, s);
   int64_t nc = g.n() / 8;
   int nb = blocks_for(nc, B);

@@ -128,3 +128,55 @@ def test_fused_sawtooth_levels(hfm, T, shape, form, sweeps, xend):
             outs.append([g.cpu().numpy() for g in got])
     for a, b in zip(*outs):  # float32 rounding of three cycles, as the other parity tests allow
         assert np.abs(a - b).max() <= 1e-5 * max(np.abs(b).max(), 1e-3 * np.abs(outs[1][0]).max())
+
+
+# rows that are no multiple of 4 cells, and views off a 16-byte boundary: two cells or one per
+# thread in the register-queue kernels
+@pytest.mark.parametrize("shape", [(3, 4, 8), (5, 7, 9), (4, 6, 10), (6, 33, 31), (8, 10, 34), (9, 8, 101), (34, 20, 70)])
+@pytest.mark.parametrize("form", ["const7", "k27", "sigma7"])
+@pytest.mark.parametrize("offset", [0, 1, 2])
+def test_ragged_rows(hfm, T, shape, form, offset):
+    ops, L = hfm.ops, hfm._lib
+    rng = np.random.default_rng(29)
+    B, n = 2, 2 * int(np.prod(shape))
+
+    def field(a):  # `offset` floats past a 16-byte boundary
+        t = T.zeros(n + 4, device="cuda")[offset:offset + n].view((B,) + shape)
+        return t.copy_(T.from_numpy(np.ascontiguousarray(a, dtype=np.float32)))
+
+    x, f = (rng.standard_normal((B,) + shape).astype(np.float32) for _ in range(2))
+    sig = np.exp(rng.standard_normal((3, B) + shape)).astype(np.float32)
+    K = rng.standard_normal((3, 3, 3)).astype(np.float32)
+    K[1, 1, 1] = 20.0
+    op = {"const7": lambda: ops.Const7(0.5, 1.0, 2.0), "k27": lambda: ops.Stencil27(K),
+          "sigma7": lambda: ops.Sigma7(*(field(sig[k]) for k in range(3)))}[form]()
+    even = not any(e & 1 for e in shape)
+    w = rng.standard_normal((B,) + tuple(e // 2 for e in shape)).astype(np.float32)
+    for flags in (0, L.FLAG_ZERO_XEND, L.FLAG_TOP_COPY):
+        y = ops.jacobi(op, field(x), field(f), 2.0 / 3.0, flags=flags)
+        r = ops.residual(op, field(x), field(f), flags=flags & L.FLAG_ZERO_XEND)
+        if even:
+            c = ops.residual_restrict(op, field(x), field(f), flags=flags & L.FLAG_ZERO_XEND)
+            p = ops.prolong_correct_smooth(op, field(x), dev(T, w), field(f), 2.0 / 3.0)
+        for b in range(B):
+            o = {"const7": lambda: mg.const7(0.5, 1.0, 2.0, dtype=np.float64),
+                 "k27": lambda: mg.Stencil27(K, dtype=np.float64),
+                 "sigma7": lambda: mg.Sigma7(*(sig[k, b] for k in range(3)), dtype=np.float64)}[form]()
+            xb = x[b].astype(np.float64)
+            if flags == L.FLAG_ZERO_XEND:
+                xb[..., -1] = 0
+            ref = mg.jacobi(o, xb, f[b], 2.0 / 3.0)
+            if flags == L.FLAG_TOP_COPY:
+                ref[0] = ref[1]
+            res = mg.residual(o, x[b], f[b])
+            if flags == L.FLAG_ZERO_XEND:
+                res[..., -1] = 0
+            pairs = [(y, ref), (r, res)]
+            if even:
+                s = tuple(e // 2 for e in shape)
+                pairs.append((c, res.reshape(s[0], 2, s[1], 2, s[2], 2).mean(axis=(1, 3, 5))))
+                up = w[b].repeat(2, 0).repeat(2, 1).repeat(2, 2)
+                pairs.append((p, mg.jacobi(o, x[b] - up.astype(np.float64), f[b], 2.0 / 3.0)))
+            for got, want in pairs:  # at most 28 roundings of 6e-8 of the largest term
+                scale = max(np.abs(want).max(), np.abs(res).max())
+                assert np.abs(got[b].cpu().numpy() - want).max() <= 1e-5 * scale
