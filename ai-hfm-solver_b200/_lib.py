@@ -199,4 +199,5 @@ def check(status, what=""):
 
 
 def call(name, *args):
-    return check(getattr(lib(), name)(*args), name)
+    status = getattr(_lib or lib(), name)(*args)
+    return status if status == OK else check(status, name)

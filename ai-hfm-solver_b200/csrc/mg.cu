@@ -2000,7 +2000,6 @@ int hfm_mg_create(const hfm_mg_config *cfg, int Z, int Y, int X, int slots, hfm_
     m->x64 = (double *)dalloc(m.get(), nf * 8, &st);
     m->b64 = (double *)dalloc(m.get(), nf * 8, &st);
   }
-  m->outer = (int *)dalloc(m.get(), (size_t)slots * 4, &st);
   if (cfg->accel != HFM_ACCEL_NONE) {
     for (int i = 0; i < 4; ++i) m->cg[i] = (float *)dalloc(m.get(), nf * 4, &st);
     m->fine_b = dalloc(m.get(), nf * 4, &st);
@@ -2014,9 +2013,11 @@ int hfm_mg_create(const hfm_mg_config *cfg, int Z, int Y, int X, int slots, hfm_
   m->partials = (double *)dalloc(m.get(), (size_t)slots * m->partials_per_slot * 8, &st);
   if (cfg->accel != HFM_ACCEL_NONE)
     m->partials2 = (double *)dalloc(m.get(), (size_t)slots * m->partials_per_slot * 8, &st);
-  m->active = (int *)dalloc(m.get(), (size_t)slots * 4, &st);
   m->small_ctr = (int *)dalloc(m.get(), (size_t)(slots + 1) * 4, &st);
-  m->state = (SlotState *)dalloc(m.get(), (size_t)slots * sizeof(SlotState), &st);
+  // states, active and outer masks in one block, so that a query is one copy
+  m->state = (SlotState *)dalloc(m.get(), (size_t)slots * (sizeof(SlotState) + 8), &st);
+  m->active = (int *)(m->state + slots);
+  m->outer = m->active + slots;
   m->stats_dev = (hfm_slot_stats *)dalloc(m.get(), (size_t)slots * sizeof(hfm_slot_stats), &st);
   m->scal = (double *)dalloc(m.get(), (size_t)(slots + 1) * 8, &st);
   m->gscale = (double *)dalloc(m.get(), (size_t)slots * 8, &st);
@@ -2129,13 +2130,14 @@ int hfm_mg_run(hfm_mg *m, int cycles, hfm_stream_t stream) {
 
 int hfm_mg_query(hfm_mg *m, hfm_slot_stats *out, hfm_stream_t stream) {
   if (!m || !out) return fail(HFM_ERR_BAD_ARG, "hfm_mg_query: bad argument");
-  std::vector<SlotState> st(m->slots);
-  std::vector<int> act(m->slots), outer(m->slots);
+  // one copy of the block that holds states, active and outer masks
   cudaStream_t s = (cudaStream_t)stream;
-  HFM_CUDA(cudaMemcpyAsync(st.data(), m->state, m->slots * sizeof(SlotState), cudaMemcpyDeviceToHost, s));
-  HFM_CUDA(cudaMemcpyAsync(act.data(), m->active, m->slots * 4, cudaMemcpyDeviceToHost, s));
-  HFM_CUDA(cudaMemcpyAsync(outer.data(), m->outer, m->slots * 4, cudaMemcpyDeviceToHost, s));
+  std::vector<SlotState> buf(m->slots + (m->slots * 8 + sizeof(SlotState) - 1) / sizeof(SlotState));
+  HFM_CUDA(cudaMemcpyAsync(buf.data(), m->state, (size_t)m->slots * (sizeof(SlotState) + 8),
+                           cudaMemcpyDeviceToHost, s));
   HFM_CUDA(cudaStreamSynchronize(s));
+  const SlotState *st = buf.data();
+  const int *act = (const int *)(st + m->slots), *outer = act + m->slots;
   for (int i = 0; i < m->slots; ++i) {
     out[i].active = act[i] | outer[i];
     out[i].status = st[i].status;

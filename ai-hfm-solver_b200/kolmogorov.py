@@ -35,7 +35,7 @@ _DT = {"f32": (L.F32, torch.float32), "bf16": (L.BF16, torch.bfloat16)}
 
 
 def _p(t):
-    return C.c_void_p(t.data_ptr() if t is not None else 0)
+    return t.data_ptr() if t is not None else 0
 
 
 def _w9(w):

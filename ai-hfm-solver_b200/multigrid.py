@@ -158,8 +158,8 @@ class Multigrid:
         _check_field(rhs, "rhs")
         if phi0 is not None:
             _check_field(phi0, "phi0")
-        L.call("hfm_mg_load", self._h, int(slot), C.c_void_p(rhs.data_ptr()),
-               C.c_void_p(phi0.data_ptr() if phi0 is not None else 0), _stream())
+        L.call("hfm_mg_load", self._h, int(slot), rhs.data_ptr(),
+               phi0.data_ptr() if phi0 is not None else 0, _stream())
 
     def run(self, cycles):
         L.call("hfm_mg_run", self._h, int(cycles), _stream())
@@ -173,7 +173,7 @@ class Multigrid:
         """Enqueue a copy of all slots' statistics into ``host_buf`` (pinned uint8 tensor of
         ``slots * sizeof(HfmSlotStats)`` bytes); decode with ``decode_stats`` once the stream
         has passed this point."""
-        L.call("hfm_mg_query_async", self._h, C.c_void_p(host_buf.data_ptr()), _stream())
+        L.call("hfm_mg_query_async", self._h, host_buf.data_ptr(), _stream())
 
     def decode_stats(self, host_buf):
         arr = (L.HfmSlotStats * self.slots).from_address(host_buf.data_ptr())
@@ -182,7 +182,7 @@ class Multigrid:
 
     def fetch(self, slot, out=None):
         out = torch.empty(self.shape, dtype=torch.float32, device="cuda") if out is None else out
-        L.call("hfm_mg_fetch", self._h, int(slot), C.c_void_p(out.data_ptr()), _stream())
+        L.call("hfm_mg_fetch", self._h, int(slot), out.data_ptr(), _stream())
         return out
 
     def load_f64(self, slot, rhs, phi0=None):
@@ -190,12 +190,12 @@ class Multigrid:
         for t in (rhs, phi0):
             if t is not None and (t.dtype != torch.float64 or not t.is_cuda or not t.is_contiguous()):
                 raise TypeError("load_f64 takes contiguous float64 CUDA tensors")
-        L.call("hfm_mg_load_f64", self._h, int(slot), C.c_void_p(rhs.data_ptr()),
-               C.c_void_p(phi0.data_ptr() if phi0 is not None else 0), _stream())
+        L.call("hfm_mg_load_f64", self._h, int(slot), rhs.data_ptr(),
+               phi0.data_ptr() if phi0 is not None else 0, _stream())
 
     def fetch_f64(self, slot, out=None):
         out = torch.empty(self.shape, dtype=torch.float64, device="cuda") if out is None else out
-        L.call("hfm_mg_fetch_f64", self._h, int(slot), C.c_void_p(out.data_ptr()), _stream())
+        L.call("hfm_mg_fetch_f64", self._h, int(slot), out.data_ptr(), _stream())
         return out
 
     def cancel(self, slot):
@@ -205,7 +205,7 @@ class Multigrid:
         shp = self.levels[level]
         out = torch.empty(shp, dtype=torch.float32, device="cuda")
         L.call("hfm_mg_read_level", self._h, int(slot), int(level), int(which),
-               C.c_void_p(out.data_ptr()), _stream())
+               out.data_ptr(), _stream())
         return out
 
     def solve(self, rhs):
@@ -214,7 +214,7 @@ class Multigrid:
         its status in stats (no exception)."""
         _check_field(rhs, "rhs")
         phi = torch.empty_like(rhs)
-        st = L.lib().hfm_mg_solve(self._h, C.c_void_p(rhs.data_ptr()), C.c_void_p(phi.data_ptr()),
+        st = L.lib().hfm_mg_solve(self._h, rhs.data_ptr(), phi.data_ptr(),
                                   self._stats, _stream())
         if st not in (L.OK, L.ERR_NOT_CONVERGED, L.ERR_NAN, L.ERR_TIMEOUT):
             L.check(st, "hfm_mg_solve")

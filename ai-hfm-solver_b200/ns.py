@@ -13,7 +13,6 @@ coarsest 2^3, no fine-level Jacobi on w, residual and pressure zeroed on x = X-1
 ``multi_itr`` cycles); ``pressure="fcycle"`` runs F(2,2) cycles on the same operator to a
 relative residual ``p_tol`` each step.
 """
-import ctypes as C
 import os
 from dataclasses import dataclass
 
@@ -23,16 +22,11 @@ import torch
 from . import _lib as L
 from . import weights as W
 from .multigrid import Multigrid, SolverConfig
-from .ops import Stencil27, _stream
+from .ops import Stencil27, _stream, _w27 as _w
 
 
 def _p(t):
-    return C.c_void_p(t.data_ptr())
-
-
-def _w(K):
-    a = np.ascontiguousarray(np.asarray(K, np.float32).reshape(27))
-    return a, a.ctypes.data_as(C.c_void_p)
+    return t.data_ptr()
 
 
 def _shape(t):

@@ -18,21 +18,30 @@ from . import _lib as L
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current torch stream of the current device, as an address."""
+    return _raw_stream(_device())
+
+
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device = getattr(torch._C, "_cuda_getDevice", None)
+if _raw_stream is None or _device is None:  # a torch build without the raw accessors
+    def _stream():  # noqa: F811
+        return torch.cuda.current_stream().cuda_stream
 
 
 def _grid(x):
     """Return (B, Z, Y, X) for a reference-shaped or batched tensor."""
-    s = tuple(x.shape)
-    if len(s) == 5:
+    s = x.shape
+    n = len(s)
+    if n == 4:
+        return s
+    if n == 5:
         if s[-1] != 1:
             raise ValueError("expected a single channel (..., 1)")
-        return s[0], s[1], s[2], s[3]
-    if len(s) == 4:
-        return s
-    if len(s) == 3:
-        return (1,) + s
-    raise ValueError("expected (1,Z,Y,X,1), (B,Z,Y,X) or (Z,Y,X), got %s" % (s,))
+        return s[:4]
+    if n == 3:
+        return (1, s[0], s[1], s[2])
+    raise ValueError("expected (1,Z,Y,X,1), (B,Z,Y,X) or (Z,Y,X), got %s" % (tuple(s),))
 
 
 def _check_field(x, name="x"):
@@ -45,15 +54,22 @@ def _check_field(x, name="x"):
 
 
 def _ptr(x):
-    return C.c_void_p(x.data_ptr()) if x is not None else C.c_void_p(0)
+    return x.data_ptr() if x is not None else 0
 
 
 def _w27(K):
-    a = np.ascontiguousarray(np.asarray(K, dtype=np.float32).reshape(27))
-    return a, a.ctypes.data_as(C.c_void_p)
+    """27 weights as a contiguous float32 array (kept alive by the caller) and its address."""
+    a = K if type(K) is np.ndarray and K.dtype == np.float32 and K.flags.c_contiguous else \
+        np.ascontiguousarray(K, dtype=np.float32)
+    if a.size != 27:
+        raise ValueError("expected 27 weights, got shape %s" % (a.shape,))
+    return a, a.__array_interface__["data"][0]
 
 
 # ---------------------------------------------------------------------------- operators
+_K_OFFSET = L.HfmOperator.k.offset
+
+
 class Operator:
     """A discretised operator A as passed to the library (``hfm_operator``)."""
 
@@ -104,8 +120,8 @@ class Stencil27(Operator):
     def struct(self):
         s = L.HfmOperator()
         s.kind, s.coef_dtype, s.scale = self.kind, L.F32, self.scale
-        for i, v in enumerate(self.K.reshape(27)):
-            s.k[i] = float(v)
+        _keep, address = _w27(self.K)
+        C.memmove(C.addressof(s) + _K_OFFSET, address, 27 * 4)
         return s
 
 
@@ -194,6 +210,12 @@ def dir7_from_mesh(D, mesh_x, mesh_y, mesh_z, device="cuda"):
                  for k, v in a.items()})
 
 
+def _resized(x, Z, Y, X):
+    """The shape of ``x`` with other extents."""
+    n = x.dim()
+    return (Z, Y, X) if n == 3 else (x.shape[0], Z, Y, X) if n == 4 else (x.shape[0], Z, Y, X, 1)
+
+
 # ---------------------------------------------------------------------------- functions
 def conv3d_same(x, K, out=None):
     """``Conv3D(1, kernel_size=3, strides=1, padding='SAME')`` with frozen kernel ``K``."""
@@ -209,12 +231,7 @@ def restrict_avg(x):
     """``CNN3D_res_<n>``: 2x2x2 average, stride 2, VALID (odd trailing cells dropped)."""
     _check_field(x)
     B, Z, Y, X = _grid(x)
-    shp = list(x.shape)
-    if len(shp) == 5:
-        shp[1:4] = [Z // 2, Y // 2, X // 2]
-    else:
-        shp[-3:] = [Z // 2, Y // 2, X // 2]
-    out = torch.empty(shp, dtype=x.dtype, device=x.device)
+    out = x.new_empty(_resized(x, Z // 2, Y // 2, X // 2))
     L.call("hfm_restrict_avg", _ptr(x), _ptr(out), B, Z, Y, X, _stream())
     return out
 
@@ -223,12 +240,7 @@ def prolong_nearest(x):
     """``CNN3D_prol_<n>``: ``UpSampling3D(size=(2, 2, 2))``."""
     _check_field(x)
     B, Z, Y, X = _grid(x)
-    shp = list(x.shape)
-    if len(shp) == 5:
-        shp[1:4] = [2 * Z, 2 * Y, 2 * X]
-    else:
-        shp[-3:] = [2 * Z, 2 * Y, 2 * X]
-    out = torch.empty(shp, dtype=x.dtype, device=x.device)
+    out = x.new_empty(_resized(x, 2 * Z, 2 * Y, 2 * X))
     L.call("hfm_prolong_nearest", _ptr(x), _ptr(out), B, Z, Y, X, _stream())
     return out
 
@@ -277,7 +289,7 @@ def residual_restrict(op, phi, b, flags=0, want_fine=False):
     _check_field(phi, "phi")
     _check_field(b, "b")
     B, Z, Y, X = _grid(phi)
-    rc = torch.empty((B, Z // 2, Y // 2, X // 2), dtype=phi.dtype, device=phi.device)
+    rc = phi.new_empty((B, Z // 2, Y // 2, X // 2))
     rf = torch.empty_like(phi) if want_fine else None
     s = op.struct()
     L.call("hfm_residual_restrict", C.byref(s), _ptr(phi), _ptr(b), _ptr(rf), _ptr(rc),
