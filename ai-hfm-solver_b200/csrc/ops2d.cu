@@ -344,7 +344,7 @@ template <class T>
 __global__ void __launch_bounds__(kT2) k2_coarse_jacobi(W9 w, const T *__restrict__ f, T *__restrict__ out,
                                                         int Y, int X, float omega, int sweeps,
                                                         int periodic) {
-  extern __shared__ float sm2[];
+  extern __shared__ __align__(16) float sm2[];
   const int n = Y * X;
   float *a = sm2, *c = sm2 + n, *ff = sm2 + 2 * n;
   const int64_t b = blockIdx.x;
@@ -382,9 +382,13 @@ __global__ void __launch_bounds__(kT2) k2_coarse_jacobi(W9 w, const T *__restric
 
 // ------------------------------------------------------------------ fused coarse cycle
 // The V-cycle of the levels of at most 4096 cells (64^2 .. 4^2 of a 512^2 grid) in one
-// launch: one 1024-thread block per instance, every field of those levels in shared memory
-// (float32), sweeps separated by __syncthreads(); a coarsest level of at most 32 cells runs
-// on one warp with its iterate in registers (shuffles, no barriers).  The steps and their
+// launch: one 512-thread block per instance, every field of those levels in shared memory
+// (float32), sweeps separated by __syncthreads(); levels of 1024 cells or more with even rows
+// of whole quads are worked by a thread per 4 x 2 cells (16-byte accesses, row neighbours by
+// shuffle, the restriction inside the thread), the smaller ones cell by cell; a coarsest level
+// of at most 32 cells runs on one warp with its iterate in registers (shuffles, no barriers).
+// 64^2 .. 4^2: 19 us a launch against 32 us with padded fields, cell by cell on 1024
+// threads.  The steps and their
 // arithmetic are those of the per-level kernels (hfm_jacobi2d, hfm_residual_restrict2d,
 // hfm_coarse_jacobi2d): nu_pre sweeps from zero, residual + 2 x 2 averaging restriction
 // (0.25 x the sum), recursion, coarse_sweeps sweeps from zero on the coarsest level, then
@@ -392,14 +396,7 @@ __global__ void __launch_bounds__(kT2) k2_coarse_jacobi(W9 w, const T *__restric
 // between sweeps (the per-level path stores them in the storage type, so float32 storage
 // gives the same bits).
 constexpr int kSub2Levels = 8;
-constexpr int kSub2Threads = 1024;
-struct Sub2Args {
-  W9 w[kSub2Levels];
-  int Y[kSub2Levels], X[kSub2Levels];
-  int nlev, periodic, nu_pre, nu_post, coarse_sweeps;
-  int smem_floats;  // shared memory of all levels, in floats
-  float omega;
-};
+constexpr int kSub2Threads = 512;
 
 // This thread's first cell of a Y x X level and the step between its cells, for walks by
 // the whole block (thread t visits cells t, t + nt, ...; one division per level visit).
@@ -516,20 +513,28 @@ __device__ __forceinline__ float sub2_coarsest_warp(const W9 &w9, const float *_
   if (!live) ok = 0;
   int src[9];
   float w[9];
+  // A neighbour outside the grid is read from a lane past the level, whose value stays zero;
+  // a full warp of cells (n = 32) has none and masks the values instead.
+  const bool mask = n == 32;
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
-    src[k] = (ok >> k) & 1 ? r[k / 3] * X + c[k % 3] : lane;
+    src[k] = (ok >> k) & 1 ? r[k / 3] * X + c[k % 3] : (mask ? lane : 31);
     w[k] = w9.w[k];
   }
-  const float fv = live ? f[lane] : 0.f;
+  // lanes past the level divide a number that is not zero and drop the result: a zero numerator
+  // sends the whole warp down the division's slow path (424 cycles a sweep)
+  const float fv = live ? f[lane] : 1.f;
   float ph = 0.f;
   for (int s = 0; s < sweeps; ++s) {
-    float acc = 0.f;
+    float v[9], acc = 0.f;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) {
-      const float v = __shfl_sync(0xffffffffu, ph, src[k]);
-      acc += w[k] * ((ok >> k) & 1 ? v : 0.f);
+    for (int k = 0; k < 9; ++k) v[k] = __shfl_sync(0xffffffffu, ph, src[k]);
+    if (mask) {
+#pragma unroll
+      for (int k = 0; k < 9; ++k) v[k] = (ok >> k) & 1 ? v[k] : 0.f;
     }
+#pragma unroll
+    for (int k = 0; k < 9; ++k) acc += w[k] * v[k];
     const float nv = ph + omega * (fv - acc) / w[4];
     ph = live ? nv : 0.f;
   }
@@ -538,10 +543,155 @@ __device__ __forceinline__ float sub2_coarsest_warp(const W9 &w9, const float *_
 
 // One level of the fused cycle: extents, row pitch of the padded iterates P = X + 2, their
 // size np = (Y + 2) P, the level's offset in shared memory (two iterates, then the rhs of
-// Y X floats) and its weights, held in registers while the level runs.
+// Y X floats) and its weights, held in registers while the level runs.  The iterates of a level
+// worked in quads or with one cell per thread have no ring: Y rows of X and one row of zeros
+// (P = X, np = (Y + 1) X); `at` is cell (0, 0).
+enum { LV2_RING = 0, LV2_QUAD = 1, LV2_CELL = 2 };
 struct Lv2 {
-  int Y, X, P, np, off;
+  int Y, X, P, np, off, kind, at;
   W9 w;
+};
+inline int kind2(int Y, int X) {
+  if (Y * X <= kSub2Threads) return LV2_CELL;
+  return X % 4 == 0 && Y % 2 == 0 && Y * X <= 8 * kSub2Threads ? LV2_QUAD : LV2_RING;
+}
+inline int field2(int Y, int X) {
+  return ((kind2(Y, X) != LV2_RING ? (Y + 1) * X : (Y + 2) * (X + 2)) + 3) & ~3;
+}
+inline int level2(int Y, int X) { return 2 * field2(Y, X) + ((Y * X + 3) & ~3); }
+
+// A thread's cell of a level of at most 512 cells: its place and those of its nine neighbours
+// (rows, then columns; the periodic images, or the row of zeros outside a zero-padded grid).
+struct Cell2 {
+  int i, nb[9], y, x;
+  bool on;
+};
+__device__ __forceinline__ Cell2 cell2_of(const Lv2 &L, int periodic) {
+  Cell2 q;
+  const int t = threadIdx.x;
+  q.on = t < L.Y * L.X;
+  q.i = q.on ? t : 0;
+  q.y = (L.X & (L.X - 1)) == 0 ? q.i >> (__ffs(L.X) - 1) : q.i / L.X;
+  q.x = q.i - q.y * L.X;
+  const int zero = L.Y * L.X;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    int y = q.y + k / 3 - 1, x = q.x + k % 3 - 1;
+    if (periodic) {
+      y = y < 0 ? L.Y - 1 : (y >= L.Y ? 0 : y);
+      x = x < 0 ? L.X - 1 : (x >= L.X ? 0 : x);
+      q.nb[k] = y * L.X + x;
+    } else {
+      q.nb[k] = y < 0 || y >= L.Y || x < 0 || x >= L.X ? zero : y * L.X + x;
+    }
+  }
+  return q;
+}
+__device__ __forceinline__ float cell2_apply(const Lv2 &L, const Cell2 &q, const float *fld) {
+  float acc = 0.f;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) acc += L.w.w[k] * fld[q.nb[k]];
+  return acc;
+}
+__device__ __forceinline__ void cell2_sweep(const Lv2 &L, const Cell2 &q, const float *in, const float *f,
+                                            float *out, float omega) {
+  if (q.on) {
+    const float ax = in ? cell2_apply(L, q, in) : 0.f, pc = in ? in[q.i] : 0.f;
+    out[q.i] = pc + omega * (f[q.i] - ax) / L.w.w[4];
+  }
+  __syncthreads();
+}
+
+// A thread's 4 x 2 cells of a quad level: columns x0 .. x0 + 3 of rows y and y + 1.
+struct Quad2 {
+  int x0, y, rm, rp;     // rm / rp: offsets of the rows before and after (the zero row outside)
+  int lane_l, lane_h;    // lanes of the row neighbours (whole rows in a warp)
+  int xl, xh;            // their columns otherwise
+  bool on, work, shfl, zl, zh;  // zl / zh: the neighbour is outside a zero-padded grid
+};
+__device__ __forceinline__ Quad2 quad2_of(const Lv2 &L, int periodic) {
+  Quad2 q;
+  const int nvx = L.X >> 2, nq = (L.Y >> 1) * nvx, t = threadIdx.x;
+  q.on = t < nq;
+  q.work = (t & ~31) < nq;
+  const int k = q.on ? t : 0;
+  int r;
+  if ((nvx & (nvx - 1)) == 0) r = k >> (__ffs(nvx) - 1);
+  else r = k / nvx;
+  const int v = k - r * nvx, lane = t & 31;
+  q.x0 = 4 * v;
+  q.y = 2 * r;
+  q.rm = q.y > 0 ? (q.y - 1) * L.X : (periodic ? L.Y - 1 : L.Y) * L.X;
+  q.rp = q.y + 2 < L.Y ? (q.y + 2) * L.X : (periodic ? 0 : L.Y) * L.X;
+  q.shfl = 32 % nvx == 0;
+  q.lane_l = v == 0 ? lane + nvx - 1 : lane - 1;
+  q.lane_h = v == nvx - 1 ? lane - nvx + 1 : lane + 1;
+  q.xl = v == 0 ? L.X - 1 : q.x0 - 1;
+  q.xh = v == nvx - 1 ? 0 : q.x0 + 4;
+  q.zl = !periodic && v == 0;
+  q.zh = !periodic && v == nvx - 1;
+  return q;
+}
+__device__ __forceinline__ void ld4s(const float *p, float *v) {
+  const float4 m = *reinterpret_cast<const float4 *>(p);
+  v[0] = m.x; v[1] = m.y; v[2] = m.z; v[3] = m.w;
+}
+// A phi on the thread's cells and phi there; the additions in the order of conv9.  Every lane
+// of a working warp calls it.
+__device__ __forceinline__ void quad2_apply(const Lv2 &L, const Quad2 &q, const float *fld, float (&A)[2][4],
+                                            float (&c)[2][4]) {
+  float v[4][6];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float *row = fld + (j == 0 ? q.rm : j == 3 ? q.rp : (q.y + j - 1) * L.X);
+    ld4s(row + q.x0, v[j] + 1);
+    if (q.shfl) {
+      v[j][0] = __shfl_sync(0xffffffffu, v[j][4], q.lane_l);
+      v[j][5] = __shfl_sync(0xffffffffu, v[j][1], q.lane_h);
+    } else {
+      v[j][0] = row[q.xl];
+      v[j][5] = row[q.xh];
+    }
+    if (q.zl) v[j][0] = 0.f;
+    if (q.zh) v[j][5] = 0.f;
+  }
+#pragma unroll
+  for (int g = 0; g < 2; ++g)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float acc = 0.f;
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) acc += L.w.w[3 * a + b] * v[g + a][e + b];
+      A[g][e] = acc;
+      c[g][e] = v[g + 1][e + 1];
+    }
+}
+// out = in + omega (f - A in) / w[4] on a quad level (in == nullptr: a zero iterate)
+__device__ __forceinline__ void quad2_sweep(const Lv2 &L, const Quad2 &q, const float *in, const float *f,
+                                            float *out, float omega) {
+  if (q.work) {
+    float A[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, c[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+    if (in) quad2_apply(L, q, in, A, c);
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      const int i = (q.y + g) * L.X + q.x0;
+      float fv[4], v[4];
+      ld4s(f + i, fv);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] = c[g][e] + omega * (fv[e] - A[g][e]) / L.w.w[4];
+      if (q.on) *reinterpret_cast<float4 *>(out + i) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+  }
+  __syncthreads();
+}
+
+struct Sub2Args {
+  Lv2 lv[kSub2Levels];
+  int nlev, periodic, nu_pre, nu_post, coarse_sweeps;
+  int smem_floats;  // shared memory of all levels, in floats (whole quads)
+  float omega;
 };
 
 // pre-sweeps from zero, then the coarse rhs 0.25 * sum over the 2 x 2 cells of (A phi - f);
@@ -551,6 +701,57 @@ __device__ __forceinline__ void sub2_down(float *sm, const Lv2 &L, const Lv2 &Lc
   float *const b0 = sm + L.off, *const b1 = b0 + L.np;
   auto buf = [&](int k) { return k ? b1 : b0; };  // selects: no local-memory array
   const float *f = sm + L.off + 2 * L.np;
+  if (L.kind == LV2_CELL) {
+    const Cell2 q = cell2_of(L, a.periodic);
+    int c = 0;
+    cell2_sweep(L, q, nullptr, f, buf(0), a.omega);
+    for (int k = 1; k < a.nu_pre; ++k) {
+      cell2_sweep(L, q, buf(c), f, buf(c ^ 1), a.omega);
+      c ^= 1;
+    }
+    if (q.on) buf(c ^ 1)[q.i] = cell2_apply(L, q, buf(c)) - f[q.i];
+    __syncthreads();
+    if (threadIdx.x < Lc.Y * Lc.X) {  // the coarse cells: half the extents, so one per thread too
+      const int yc = (Lc.X & (Lc.X - 1)) == 0 ? threadIdx.x >> (__ffs(Lc.X) - 1) : threadIdx.x / Lc.X;
+      const float *r = buf(c ^ 1) + 2 * yc * L.X + 2 * (threadIdx.x - yc * Lc.X);
+      float sum = 0.f;
+      sum += r[0];
+      sum += r[1];
+      sum += r[L.X];
+      sum += r[L.X + 1];
+      sm[Lc.off + 2 * Lc.np + threadIdx.x] = 0.25f * sum;
+    }
+    __syncthreads();
+    return;
+  }
+  if (L.kind == LV2_QUAD) {
+    const Quad2 q = quad2_of(L, a.periodic);
+    int c = 0;
+    quad2_sweep(L, q, nullptr, f, buf(0), a.omega);
+    for (int k = 1; k < a.nu_pre; ++k) {
+      quad2_sweep(L, q, buf(c), f, buf(c ^ 1), a.omega);
+      c ^= 1;
+    }
+    if (q.work) {
+      float A[2][4], p[2][4], f0[4], f1[4];
+      quad2_apply(L, q, buf(c), A, p);
+      ld4s(f + q.y * L.X + q.x0, f0);
+      ld4s(f + (q.y + 1) * L.X + q.x0, f1);
+      float s[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {  // the order of the cell-by-cell sum
+        s[k] = 0.f + (A[0][2 * k] - f0[2 * k]);
+        s[k] += A[0][2 * k + 1] - f0[2 * k + 1];
+        s[k] += A[1][2 * k] - f1[2 * k];
+        s[k] += A[1][2 * k + 1] - f1[2 * k + 1];
+      }
+      if (q.on)
+        *reinterpret_cast<float2 *>(sm + Lc.off + 2 * Lc.np + (q.y >> 1) * Lc.X + (q.x0 >> 1)) =
+            make_float2(0.25f * s[0], 0.25f * s[1]);
+    }
+    __syncthreads();
+    return;
+  }
   const Walk2 wk = walk2_of(L.X);
   int c = 0;
   sub2_sweep(L.w, nullptr, f, buf(0), L.Y, L.X, wk, a.periodic, a.omega);
@@ -586,14 +787,30 @@ __device__ __forceinline__ int sub2_coarsest(float *sm, const Lv2 &L, const Sub2
     if (threadIdx.x < 32) {
       const float v = sub2_coarsest_warp(L.w, f, L.Y, L.X, a.periodic, a.omega, a.coarse_sweeps);
       const int y = threadIdx.x / L.X, x = threadIdx.x - y * L.X;
-      if (threadIdx.x < n) buf(0)[(y + 1) * L.P + x + 1] = v;
+      if (threadIdx.x < n) buf(0)[y * L.P + x + L.at] = v;
     }
     __syncthreads();
     return 0;
   }
   // buf(0) holds zeros (shared memory is cleared at the start)
-  const Walk2 wk = walk2_of(L.X);
   int c = 0;
+  if (L.kind == LV2_CELL) {
+    const Cell2 q = cell2_of(L, a.periodic);
+    for (int k = 0; k < a.coarse_sweeps; ++k) {
+      cell2_sweep(L, q, buf(c), f, buf(c ^ 1), a.omega);
+      c ^= 1;
+    }
+    return c;
+  }
+  if (L.kind == LV2_QUAD) {
+    const Quad2 q = quad2_of(L, a.periodic);
+    for (int k = 0; k < a.coarse_sweeps; ++k) {
+      quad2_sweep(L, q, buf(c), f, buf(c ^ 1), a.omega);
+      c ^= 1;
+    }
+    return c;
+  }
+  const Walk2 wk = walk2_of(L.X);
   for (int k = 0; k < a.coarse_sweeps; ++k) {
     sub2_sweep(L.w, buf(c), f, buf(c ^ 1), L.Y, L.X, wk, a.periodic, a.omega);
     c ^= 1;
@@ -608,12 +825,49 @@ __device__ __forceinline__ int sub2_up(float *sm, const Lv2 &L, const Lv2 &Lc, i
   float *const b0 = sm + L.off, *const b1 = b0 + L.np;
   auto buf = [&](int k) { return k ? b1 : b0; };  // selects: no local-memory array
   const float *f = sm + L.off + 2 * L.np;
-  const float *wc = sm + Lc.off + cc * Lc.np;
-  const Walk2 wk = walk2_of(L.X);
+  const float *wc = sm + Lc.off + cc * Lc.np + Lc.at;
   const int P = L.P, Pc = Lc.P;
   float *ph = buf(c);
+  if (L.kind == LV2_CELL) {
+    const Cell2 q = cell2_of(L, a.periodic);
+    if (q.on) ph[q.i] -= wc[(q.y >> 1) * Pc + (q.x >> 1)];
+    __syncthreads();
+    cell2_sweep(L, q, buf(c), f, buf(c ^ 1), a.nu_post ? a.omega : 0.f);
+    c ^= 1;
+    for (int k = 1; k < a.nu_post; ++k) {
+      cell2_sweep(L, q, buf(c), f, buf(c ^ 1), a.omega);
+      c ^= 1;
+    }
+    return c;
+  }
+  if (L.kind == LV2_QUAD) {
+    const Quad2 q = quad2_of(L, a.periodic);
+    if (q.on) {
+      const float *w = wc + (q.y >> 1) * Pc + (q.x0 >> 1);
+      const float w0 = w[0], w1 = w[1];
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        float4 *d = reinterpret_cast<float4 *>(ph + (q.y + g) * L.X + q.x0);
+        float4 v = *d;
+        v.x -= w0;
+        v.y -= w0;
+        v.z -= w1;
+        v.w -= w1;
+        *d = v;
+      }
+    }
+    __syncthreads();
+    quad2_sweep(L, q, buf(c), f, buf(c ^ 1), a.nu_post ? a.omega : 0.f);
+    c ^= 1;
+    for (int k = 1; k < a.nu_post; ++k) {
+      quad2_sweep(L, q, buf(c), f, buf(c ^ 1), a.omega);
+      c ^= 1;
+    }
+    return c;
+  }
+  const Walk2 wk = walk2_of(L.X);
   walk2(wk, L.Y, L.X, [&](int, int y, int x) {
-    const float v = ph[(y + 1) * P + x + 1] - wc[((y >> 1) + 1) * Pc + (x >> 1) + 1];
+    const float v = ph[(y + 1) * P + x + 1] - wc[(y >> 1) * Pc + (x >> 1)];
     put2(ph, P, L.Y, L.X, y, x, v, a.periodic);
   });
   __syncthreads();
@@ -630,53 +884,51 @@ template <class T>
 __global__ void __launch_bounds__(kSub2Threads) k2_subcycle(const __grid_constant__ Sub2Args a,
                                                             const T *__restrict__ rhs,
                                                             T *__restrict__ out) {
-  extern __shared__ float sm2[];
-  __shared__ Lv2 lv[kSub2Levels];
+  extern __shared__ __align__(16) float sm2[];
   const int nl = a.nlev;
-  if (threadIdx.x < nl) {
-    const int l = threadIdx.x;
-    int o = 0;
-    for (int k = 0; k < l; ++k) o += 2 * (a.Y[k] + 2) * (a.X[k] + 2) + a.Y[k] * a.X[k];
-    Lv2 L;
-    L.Y = a.Y[l];
-    L.X = a.X[l];
-    L.P = L.X + 2;
-    L.np = (L.Y + 2) * L.P;
-    L.off = o;
-    L.w = a.w[l];
-    lv[l] = L;
-  }
-  for (int i = threadIdx.x; i < a.smem_floats; i += blockDim.x) sm2[i] = 0.f;
-  __syncthreads();  // the zeros land before the rhs below
   const int64_t b = blockIdx.x;
-  const int Y0 = a.Y[0], X0 = a.X[0], n0 = Y0 * X0, P0 = X0 + 2;
-  float *f0 = sm2 + 2 * (Y0 + 2) * P0;
-  for (int i = threadIdx.x; i < n0; i += blockDim.x) f0[i] = St<T>::to(rhs[b * n0 + i]);
+  const int Y0 = a.lv[0].Y, X0 = a.lv[0].X, n0 = Y0 * X0;
+  float *f0 = sm2 + 2 * a.lv[0].np;
+  // the right-hand side (at most 8 values a thread) is on its way while the block clears its
+  // shared memory
+  float r[4096 / kSub2Threads];
+#pragma unroll
+  for (int k = 0; k < 4096 / kSub2Threads; ++k) {
+    const int i = threadIdx.x + k * kSub2Threads;
+    r[k] = i < n0 ? St<T>::to(rhs[b * n0 + i]) : 0.f;
+  }
+  for (int i = threadIdx.x; i < a.smem_floats / 4; i += kSub2Threads)
+    reinterpret_cast<float4 *>(sm2)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncthreads();  // the zeros land before the rhs below
+#pragma unroll
+  for (int k = 0; k < 4096 / kSub2Threads; ++k) {
+    const int i = threadIdx.x + k * kSub2Threads;
+    if (i < n0) f0[i] = r[k];
+  }
   __syncthreads();
   for (int l = 0; l < nl - 1; ++l) {
-    const Lv2 L = lv[l], Lc = lv[l + 1];
+    const Lv2 L = a.lv[l], Lc = a.lv[l + 1];
     sub2_down(sm2, L, Lc, a);
   }
   const int cd = (a.nu_pre - 1) & 1;  // a level's iterate after its pre-sweeps
   int cc;
   {
-    const Lv2 L = lv[nl - 1];
+    const Lv2 L = a.lv[nl - 1];
     cc = sub2_coarsest(sm2, L, a);
   }
   for (int l = nl - 2; l >= 0; --l) {
-    const Lv2 L = lv[l], Lc = lv[l + 1];
+    const Lv2 L = a.lv[l], Lc = a.lv[l + 1];
     cc = sub2_up(sm2, L, Lc, cd, cc, a);
   }
-  const float *res = sm2 + cc * (Y0 + 2) * P0;
-  walk2(walk2_of(X0), Y0, X0, [&](int i, int y, int x) {
-    out[b * n0 + i] = St<T>::from(res[(y + 1) * P0 + x + 1]);
-  });
+  const float *res = sm2 + cc * a.lv[0].np + a.lv[0].at;
+  const int P0 = a.lv[0].P;
+  walk2(walk2_of(X0), Y0, X0, [&](int i, int y, int x) { out[b * n0 + i] = St<T>::from(res[y * P0 + x]); });
 }
 
 // Shared-memory bytes of k2_subcycle for nlev levels from Y x X (each coarser level halved)
 size_t sub2_smem_bytes(int Y, int X, int nlev) {
   size_t n = 0;
-  for (int l = 0; l < nlev; ++l, Y /= 2, X /= 2) n += (size_t)2 * (Y + 2) * (X + 2) + (size_t)Y * X;
+  for (int l = 0; l < nlev; ++l, Y /= 2, X /= 2) n += (size_t)level2(Y, X);
   return n * sizeof(float);
 }
 constexpr size_t kSub2MaxSmem = 200 * 1024;
@@ -1027,16 +1279,24 @@ int hfm_subcycle2d(int dtype, const float *w9_levels, const void *rhs, void *out
   a.nu_post = nu_post;
   a.coarse_sweeps = coarse_sweeps;
   a.omega = omega;
+  int off = 0;
   for (int l = 0; l < nlev; ++l) {
-    a.Y[l] = l ? a.Y[l - 1] / 2 : Y;
-    a.X[l] = l ? a.X[l - 1] / 2 : X;
-    if (a.Y[l] < 1 || a.X[l] < 1) return fail(HFM_ERR_BAD_ARG, "hfm_subcycle2d: too many levels");
-    if (l + 1 < nlev && ((a.Y[l] & 1) || (a.X[l] & 1)))
+    Lv2 &L = a.lv[l];
+    L.Y = l ? a.lv[l - 1].Y / 2 : Y;
+    L.X = l ? a.lv[l - 1].X / 2 : X;
+    if (L.Y < 1 || L.X < 1) return fail(HFM_ERR_BAD_ARG, "hfm_subcycle2d: too many levels");
+    if (l + 1 < nlev && ((L.Y & 1) || (L.X & 1)))
       return fail(HFM_ERR_BAD_ARG, "hfm_subcycle2d: odd extent above the coarsest level");
     if (w9_levels[9 * l + 4] == 0.f) return fail(HFM_ERR_BAD_ARG, "hfm_subcycle2d: zero diagonal weight");
-    a.w[l] = w9_of(w9_levels + 9 * l);
+    L.w = w9_of(w9_levels + 9 * l);
+    L.kind = kind2(L.Y, L.X);
+    L.P = L.kind == LV2_RING ? L.X + 2 : L.X;
+    L.at = L.kind == LV2_RING ? L.P + 1 : 0;
+    L.np = field2(L.Y, L.X);
+    L.off = off;
+    off += level2(L.Y, L.X);
   }
-  for (int l = nlev; l < kSub2Levels; ++l) a.Y[l] = a.X[l] = 0;
+  for (int l = nlev; l < kSub2Levels; ++l) a.lv[l] = a.lv[nlev - 1];
   const size_t smem = sub2_smem_bytes(Y, X, nlev);
   if (smem > kSub2MaxSmem) return fail(HFM_ERR_UNSUPPORTED, "hfm_subcycle2d: levels exceed shared memory");
   a.smem_floats = (int)(smem / sizeof(float));

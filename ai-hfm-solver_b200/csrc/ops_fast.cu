@@ -73,6 +73,10 @@ template <class T, int V> __device__ __forceinline__ void stv(T *p, const FV<V> 
     else *reinterpret_cast<unsigned *>(p) = *reinterpret_cast<const unsigned *>(h);
   }
 }
+// The sweep's quotient: the ragged grids (V < 4) keep the IEEE division of the generic kernels.
+template <int V> __device__ __forceinline__ float quotient(float n, float d) {
+  return V < 4 ? n / d : __fdividef(n, d);
+}
 template <int V> __device__ __forceinline__ FV<V> filled(float x) {
   FV<V> r;
 #pragma unroll
@@ -357,7 +361,7 @@ __global__ void __launch_bounds__(kFastThreads, R == 1 ? 4 : 2)
       if (a.rhs && in) f = ldv<T, V>(a.rhs + ib + off);
       if (MODE == M_SMOOTH) {
 #pragma unroll
-        for (int e = 0; e < V; ++e) res[r].v[e] = pc[r].v[e] + a.omega * __fdividef(f.v[e] - Ax.v[e], dg.v[e]);
+        for (int e = 0; e < V; ++e) res[r].v[e] = pc[r].v[e] + a.omega * quotient<V>(f.v[e] - Ax.v[e], dg.v[e]);
         if (a.dot_rhs && in) {
 #pragma unroll
           for (int e = 0; e < V; ++e) acc += (double)res[r].v[e] * f.v[e];
@@ -514,7 +518,7 @@ __global__ void __launch_bounds__(kFastThreads, 4) k_column7(FastArgs<T> a) {
     }
     float v;
     if (MODE == M_SMOOTH) {
-      v = pc + a.omega * __fdividef(q.f - Ax, dg);
+      v = pc + a.omega * quotient<1>(q.f - Ax, dg);
     } else {
       v = Ax - q.f;
       if (a.zero_xend_out && x == X - 1) v = 0.f;
@@ -630,7 +634,7 @@ __global__ void __launch_bounds__(kFastThreads)
       if (a.rhs && in) f = ldv<T, V>(a.rhs + ib + off);
       if (MODE == M_SMOOTH) {
 #pragma unroll
-        for (int e = 0; e < V; ++e) res[r].v[e] = cen_cur[r].v[e] + a.omega * __fdividef(f.v[e] - Ax.v[e], diag);
+        for (int e = 0; e < V; ++e) res[r].v[e] = cen_cur[r].v[e] + a.omega * quotient<V>(f.v[e] - Ax.v[e], diag);
         if (a.dot_rhs && in) {
 #pragma unroll
           for (int e = 0; e < V; ++e) acc2 += (double)res[r].v[e] * f.v[e];

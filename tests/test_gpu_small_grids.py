@@ -180,3 +180,26 @@ def test_ragged_rows(hfm, T, shape, form, offset):
             for got, want in pairs:  # at most 28 roundings of 6e-8 of the largest term
                 scale = max(np.abs(want).max(), np.abs(res).max())
                 assert np.abs(got[b].cpu().numpy() - want).max() <= 1e-5 * scale
+
+
+# the 2D fused coarse cycle against one launch per level step, bit for bit: levels in quads
+# with whole and straddling rows, one cell per thread, ringed levels (X % 4 != 0 above 512
+# cells), coarsest levels on a warp (a full one too) and above
+@pytest.mark.parametrize("periodic", [True, False])
+@pytest.mark.parametrize("shape,min_edge", [((64, 64), 4), ((56, 56), 4), ((48, 80), 5), ((52, 46), 4), ((40, 24), 3),
+                                            ((16, 128), 4), ((64, 32), 8), ((60, 44), 30)])
+def test_2d_fused_levels_same_bits(hfm, T, periodic, shape, min_edge):
+    KM = hfm.kolmogorov
+    rng = np.random.default_rng(31)
+    w = KM.laplace5(0.1)
+    w += 0.02 * rng.standard_normal((3, 3))  # no zero weights
+    w[1, 1] *= 1.2
+    f = T.from_numpy(rng.standard_normal((2,) + shape).astype(np.float32)).cuda()
+    outs = []
+    for fused in (True, False):
+        m = KM.Multigrid2D(shape, w, periodic=periodic, slots=2, min_edge=min_edge, fused_coarse=fused, coarse_sweeps=7)
+        p = T.zeros((2,) + shape, device="cuda")
+        for _ in range(2):
+            m.iterate(p, f)
+        outs.append(p.cpu().numpy())
+    np.testing.assert_array_equal(outs[0], outs[1])
