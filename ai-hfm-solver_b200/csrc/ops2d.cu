@@ -118,101 +118,200 @@ __global__ void __launch_bounds__(kT2) k2_two_sweeps(W9 w, Sweep1Src<T> s, T *__
   }
 }
 
-// Two Jacobi sweeps in one pass from phi = base + sign P(coarse) (Src2): a 32 x 8 tile of
-// the first sweep and its one-cell ring in shared memory (each value computed as the
-// one-sweep launch computes it and rounded to T as it stores it), then the second sweep from
-// there; the bits of two hfm_jacobi2d launches.
+// Row or column i of a tile's ring on an axis of n cells, -3 <= i <= n + 2: its periodic image
+// (one wrap serves from 3 cells up; shorter axes take the remainder).
+__device__ __forceinline__ int ring2(int i, int n) {
+  if (n < 3) return ((i % n) + n) % n;
+  return i < 0 ? i + n : (i >= n ? i - n : i);
+}
+
+// Two Jacobi sweeps in one pass from phi = base + sign P(coarse) (Src2): a 32 x 8 tile holds
+// phi on a two-cell ring and the first sweep on a one-cell ring in shared memory (each value
+// computed as the one-sweep launch computes it and rounded to T as it stores it), then the
+// second sweep from there; the bits of two hfm_jacobi2d launches.  All global loads of a block
+// are issued before its first barrier: the pass is bound by that one latency.  256^2 and 128^2,
+// correction included: 2.4 us a launch, 512^2 with the update 5.1 us (6.9 us on average, and 2.2 us
+// for the update, when every first-sweep cell read its nine phi and nine coarse values from
+// L2).  With UPDATE the second sweep's result w is not stored
+// but applied, p += update_sign w, as hfm_update2d does.
 constexpr int kTwoTX = 32, kTwoTY = 8;
 static_assert(kTwoTX * kTwoTY == kT2, "one thread per output cell of a tile");
-template <class T>
+template <class T, bool UPDATE>
 __global__ void __launch_bounds__(kT2) k2_two_sweeps_tile(W9 w, Src2<T> s, const T *__restrict__ f,
-                                                          T *__restrict__ out, float omega) {
-  __shared__ float mid[kTwoTY + 2][kTwoTX + 2];
+                                                          T *__restrict__ out, float *__restrict__ p,
+                                                          float update_sign, float omega) {
+  constexpr int PX = kTwoTX + 4, PY = kTwoTY + 4, MX = kTwoTX + 2, MY = kTwoTY + 2;
+  constexpr int NP = (PX * PY + kT2 - 1) / kT2, NM = (MX * MY + kT2 - 1) / kT2;
+  __shared__ float phi[PY][PX];
+  __shared__ float mid[MY][MX];
   const int64_t b = blockIdx.z;
   const int x0 = blockIdx.x * kTwoTX, y0 = blockIdx.y * kTwoTY;
-  for (int k = threadIdx.x; k < (kTwoTY + 2) * (kTwoTX + 2); k += blockDim.x) {
-    const int ty = k / (kTwoTX + 2), tx = k - ty * (kTwoTX + 2);
-    int y = y0 + ty - 1, x = x0 + tx - 1;  // -1 <= y <= y0 + kTwoTY, likewise x
-    float v = 0.f;
-    // cells past row Y / column X neighbour no cell of the grid: left at 0
-    bool live = y <= s.Y && x <= s.X;
+  const int Y = s.Y, X = s.X;
+  const T *base = s.base ? s.base + b * s.stride : nullptr;
+  const T *coarse = s.coarse ? s.coarse + b * s.cstride : nullptr;
+  const T *fb = f + b * s.stride;
+  // cell (y, x) of a ring, wrapped; false: outside a zero-padded grid, or past the ring of the
+  // last tile
+  auto place = [&](int &y, int &x, int ring) {
+    bool in = y < Y + ring && x < X + ring;
     if (s.periodic) {
-      y = y < 0 ? y + s.Y : (y >= s.Y ? y - s.Y : y);
-      x = x < 0 ? x + s.X : (x >= s.X ? x - s.X : x);
+      if (in) {
+        y = ring2(y, Y);
+        x = ring2(x, X);
+      }
     } else {
-      live = live && y >= 0 && y < s.Y && x >= 0 && x < s.X;
+      in = y >= 0 && y < Y && x >= 0 && x < X;
     }
-    if (live) {
-      float pc;
-      const float ax = conv9(w, s, b, y, x, &pc);
-      const float fv = St<T>::ld(f + b * s.stride + (int64_t)y * s.X + x);
-      v = St<T>::to(St<T>::from(pc + omega * (fv - ax) / w.w[4]));
-    }
-    mid[ty][tx] = v;
+    return in;
+  };
+  float pv[NP], cv[NP], fv[NM];
+#pragma unroll
+  for (int j = 0; j < NP; ++j) {
+    const int k = threadIdx.x + j * kT2, ty = k / PX;
+    int y = y0 + ty - 2, x = x0 + (k - ty * PX) - 2;
+    const bool in = k < PX * PY && place(y, x, 2);
+    pv[j] = in && base ? St<T>::ld(base + (int64_t)y * X + x) : 0.f;
+    cv[j] = in && coarse ? St<T>::ld(coarse + (int64_t)(y >> s.cshift) * s.Xc + (x >> s.cshift)) : 0.f;
+  }
+  unsigned live = 0;
+#pragma unroll
+  for (int j = 0; j < NM; ++j) {
+    const int k = threadIdx.x + j * kT2, ty = k / MX;
+    int y = y0 + ty - 1, x = x0 + (k - ty * MX) - 1;
+    const bool in = k < MX * MY && place(y, x, 1);
+    if (in) live |= 1u << j;
+    fv[j] = in ? St<T>::ld(fb + (int64_t)y * X + x) : 0.f;
+  }
+  const int tx = threadIdx.x % kTwoTX, ty = threadIdx.x / kTwoTX;
+  const int yo = y0 + ty, xo = x0 + tx;
+  const bool mine = yo < Y && xo < X;
+  const int64_t i = b * s.stride + (int64_t)yo * X + xo;
+  const float fo = mine ? St<T>::ld(f + i) : 1.f;
+  const float po = UPDATE && mine ? p[i] : 0.f;
+#pragma unroll
+  for (int j = 0; j < NP; ++j) {
+    const int k = threadIdx.x + j * kT2;
+    float v = pv[j];
+    if (coarse) v += s.sign * cv[j];
+    if (k < PX * PY) (&phi[0][0])[k] = v;
   }
   __syncthreads();
-  const int tx = threadIdx.x % kTwoTX, ty = threadIdx.x / kTwoTX;
-  const int y = y0 + ty, x = x0 + tx;
-  if (y < s.Y && x < s.X) {
+  auto sweep = [&](const float *c, int P, float fvv) {
     float acc = 0.f;
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
-      for (int c = 0; c < 3; ++c) acc += w.w[3 * a + c] * mid[ty + a][tx + c];
-    const float pc = mid[ty + 1][tx + 1];
-    const int64_t i = b * s.stride + (int64_t)y * s.X + x;
-    out[i] = St<T>::from(pc + omega * (St<T>::ld(f + i) - acc) / w.w[4]);
+      for (int e = 0; e < 3; ++e) acc += w.w[3 * a + e] * c[(a - 1) * P + e - 1];
+    return c[0] + omega * (fvv - acc) / w.w[4];
+  };
+#pragma unroll
+  for (int j = 0; j < NM; ++j) {
+    const int k = threadIdx.x + j * kT2, my = k / MX, mx = k - my * MX;
+    if (k < MX * MY) {
+      float v = 0.f;
+      if ((live >> j) & 1) v = St<T>::to(St<T>::from(sweep(&phi[my + 1][mx + 1], PX, fv[j])));
+      mid[my][mx] = v;
+    }
+  }
+  __syncthreads();
+  if (mine) {
+    const T r = St<T>::from(sweep(&mid[ty + 1][tx + 1], MX, fo));
+    if (UPDATE) p[i] = po + update_sign * St<T>::to(r);
+    else out[i] = r;
   }
 }
 
 // The down leg of a level with two pre-sweeps in one pass: phi = two Jacobi sweeps from zero
-// and the coarse rhs 0.25 * sum over 2 x 2 cells of (A phi - f).  A 32 x 8 tile holds the
+// and the coarse rhs 0.25 * sum over 2 x 2 cells of (A phi - f).  A 32 x 8 tile holds f and the
 // first sweep on a two-cell ring, the second on a one-cell ring (each value computed and
 // rounded to T as the one-sweep launches store it) and the tile's residuals in shared memory;
 // the bits of hfm_jacobi2d (HFM_FLAG_TWO_SWEEPS) followed by hfm_residual_restrict2d.
 // Even extents: the tile's coarse cells lie inside the grid or wholly outside it.
-template <class T>
+// With OUTER f is the outer defect of a mixed-precision solve, formed here: f = A q - g of the
+// float32 iterate q (on a three-cell ring) and right-hand side g, rounded to T, and stored in
+// f_out (hfm_outer_residual2d's bits).  256^2 and 128^2: 2.5 us a launch, 512^2 with the outer
+// defect 6.3 us (4.7 us on average and 7.2 us for the defect apart, with integer remainders per
+// ring cell and the loads waited for one by one).
+template <class T, bool OUTER>
 __global__ void __launch_bounds__(kT2) k2_pre2_restrict(W9 w, Sweep1Src<T> s, T *__restrict__ phi,
-                                                        T *__restrict__ coarse) {
-  __shared__ float s1[kTwoTY + 4][kTwoTX + 4];
+                                                        T *__restrict__ coarse, const float *__restrict__ q,
+                                                        const float *__restrict__ g, T *__restrict__ f_out) {
+  constexpr int QX = kTwoTX + 6, QY = kTwoTY + 6, FX = kTwoTX + 4, FY = kTwoTY + 4;
+  constexpr int NQ = (QX * QY + kT2 - 1) / kT2, NF = (FX * FY + kT2 - 1) / kT2;
+  __shared__ float qs[OUTER ? QY : 1][OUTER ? QX : 1];
+  __shared__ float fs[FY][FX];
+  __shared__ float s1[FY][FX];
   __shared__ float s2[kTwoTY + 2][kTwoTX + 2];
   __shared__ float rr[kTwoTY][kTwoTX];
   const int64_t b = blockIdx.z;
   const int Y = s.Y, X = s.X;
   const int x0 = blockIdx.x * kTwoTX, y0 = blockIdx.y * kTwoTY;
-  // first sweep on the tile and a two-cell ring (s(b, y, x) wraps or pads, -2 <= y - y0 <= 9)
-  for (int k = threadIdx.x; k < (kTwoTY + 4) * (kTwoTX + 4); k += blockDim.x) {
-    const int ty = k / (kTwoTX + 4), tx = k - ty * (kTwoTX + 4);
-    int y = y0 + ty - 2, x = x0 + tx - 2;
-    if (s.periodic) {  // a ring cell may lie more than one period out on a grid of 1 row
-      y = ((y % Y) + Y) % Y;
-      x = ((x % X) + X) % X;
+  auto place = [&](int &y, int &x, int ring) {  // as in k2_two_sweeps_tile
+    bool in = y < Y + ring && x < X + ring;
+    if (s.periodic) {
+      if (in) {
+        y = ring2(y, Y);
+        x = ring2(x, X);
+      }
+    } else {
+      in = y >= 0 && y < Y && x >= 0 && x < X;
     }
-    s1[ty][tx] = s(b, y, x);
+    return in;
+  };
+  auto nine = [&](const float *c, int P) {
+    float acc = 0.f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int e = 0; e < 3; ++e) acc += w.w[3 * a + e] * c[(a - 1) * P + e - 1];
+    return acc;
+  };
+  // f on the tile and a two-cell ring, and the first sweep there
+  float fv[NF];
+  unsigned live = 0;
+#pragma unroll
+  for (int j = 0; j < NF; ++j) {
+    const int k = threadIdx.x + j * kT2, ty = k / FX;
+    int y = y0 + ty - 2, x = x0 + (k - ty * FX) - 2;
+    const bool in = k < FX * FY && place(y, x, 2);
+    if (in) live |= 1u << j;
+    const int64_t i = b * s.stride + (int64_t)y * X + x;
+    if (OUTER) fv[j] = in ? g[i] : 0.f;
+    else fv[j] = in ? St<T>::ld(s.f + i) : 0.f;
+  }
+  if (OUTER) {
+    float qv[NQ];
+#pragma unroll
+    for (int j = 0; j < NQ; ++j) {
+      const int k = threadIdx.x + j * kT2, ty = k / QX;
+      int y = y0 + ty - 3, x = x0 + (k - ty * QX) - 3;
+      qv[j] = k < QX * QY && place(y, x, 3) ? q[b * s.stride + (int64_t)y * X + x] : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < NQ; ++j) {
+      const int k = threadIdx.x + j * kT2;
+      if (k < QX * QY) (&qs[0][0])[k] = qv[j];
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int j = 0; j < NF; ++j) {
+    const int k = threadIdx.x + j * kT2, ty = k / FX, tx = k - ty * FX;
+    if (k < FX * FY) {
+      float f = fv[j];
+      if (OUTER) f = St<T>::to(St<T>::from(nine(&qs[OUTER ? ty + 1 : 0][OUTER ? tx + 1 : 0], QX) - fv[j]));
+      fs[ty][tx] = f;
+      s1[ty][tx] = (live >> j) & 1 ? St<T>::to(St<T>::from(0.f + s.omega * f / s.diag)) : 0.f;
+    }
   }
   __syncthreads();
   // second sweep on the tile and a one-cell ring
-  for (int k = threadIdx.x; k < (kTwoTY + 2) * (kTwoTX + 2); k += blockDim.x) {
+  for (int k = threadIdx.x; k < (kTwoTY + 2) * (kTwoTX + 2); k += kT2) {
     const int ty = k / (kTwoTX + 2), tx = k - ty * (kTwoTX + 2);
     int y = y0 + ty - 1, x = x0 + tx - 1;
-    bool live = true;
-    if (s.periodic) {
-      y = ((y % Y) + Y) % Y;
-      x = ((x % X) + X) % X;
-    } else {
-      live = y >= 0 && y < Y && x >= 0 && x < X;
-    }
     float v = 0.f;
-    if (live) {
-      float acc = 0.f;
-#pragma unroll
-      for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) acc += w.w[3 * a + c] * s1[ty + a][tx + c];
-      const float pc = s1[ty + 1][tx + 1];
-      const float fv = St<T>::ld(s.f + b * s.stride + (int64_t)y * X + x);
-      v = St<T>::to(St<T>::from(pc + s.omega * (fv - acc) / w.w[4]));
-    }
+    if (place(y, x, 1))
+      v = St<T>::to(St<T>::from(s1[ty + 1][tx + 1] + s.omega * (fs[ty + 1][tx + 1] - nine(&s1[ty + 1][tx + 1], FX)) / w.w[4]));
     s2[ty][tx] = v;
   }
   __syncthreads();
@@ -220,15 +319,11 @@ __global__ void __launch_bounds__(kT2) k2_pre2_restrict(W9 w, Sweep1Src<T> s, T 
     const int tx = threadIdx.x % kTwoTX, ty = threadIdx.x / kTwoTX;
     const int y = y0 + ty, x = x0 + tx;
     if (y < Y && x < X) {
-      float acc = 0.f;
-#pragma unroll
-      for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) acc += w.w[3 * a + c] * s2[ty + a][tx + c];
       const int64_t i = b * s.stride + (int64_t)y * X + x;
       phi[i] = St<T>::from(s2[ty + 1][tx + 1]);
-      float r = acc;
-      r -= St<T>::ld(s.f + i);
+      if (OUTER) f_out[i] = St<T>::from(fs[ty + 2][tx + 2]);
+      float r = nine(&s2[ty + 1][tx + 1], kTwoTX + 2);
+      r -= fs[ty + 2][tx + 2];
       rr[ty][tx] = r;
     }
   }
@@ -383,7 +478,7 @@ __global__ void __launch_bounds__(kT2) k2_coarse_jacobi(W9 w, const T *__restric
 // ------------------------------------------------------------------ fused coarse cycle
 // The V-cycle of the levels of at most 4096 cells (64^2 .. 4^2 of a 512^2 grid) in one
 // launch: one 512-thread block per instance, every field of those levels in shared memory
-// (float32), sweeps separated by __syncthreads(); levels of 1024 cells or more with even rows
+// (float32), sweeps separated by __syncthreads(); levels of more than 512 cells with even rows
 // of whole quads are worked by a thread per 4 x 2 cells (16-byte accesses, row neighbours by
 // shuffle, the restriction inside the thread), the smaller ones cell by cell; a coarsest level
 // of at most 32 cells runs on one warp with its iterate in registers (shuffles, no barriers).
@@ -937,8 +1032,10 @@ constexpr size_t kSub2MaxSmem = 200 * 1024;
 // thread-block cluster of kMeanCluster blocks per instance: each block sums its contiguous
 // share in a fixed order (thread-strided, warp tree, warps in order), the blocks read the
 // cluster's partial sums from each other's shared memory in rank order, and each subtracts
-// the mean from its share - a single block per instance spent 89 us on a 512^2 grid.
+// the mean from its share - a single block per instance spent 89 us on a 512^2 grid, one load in
+// flight per thread 11.7 us, kMeanHold of them 7.7 us.
 constexpr int kMeanCluster = 8;
+constexpr int kMeanHold = 32;
 __global__ void __cluster_dims__(kMeanCluster, 1, 1) __launch_bounds__(1024)
     k2_mean_subtract(float *p, int64_t n) {
   namespace cg = cooperative_groups;
@@ -949,8 +1046,17 @@ __global__ void __cluster_dims__(kMeanCluster, 1, 1) __launch_bounds__(1024)
   const int rank = (int)cl.block_rank();
   float *q = p + (int64_t)(blockIdx.x / kMeanCluster) * n;
   const int64_t lo = n * rank / kMeanCluster, hi = n * (rank + 1) / kMeanCluster;
+  // kMeanHold loads per thread in flight, added in the order of a plain strided walk; a share
+  // of at most kMeanHold * 1024 values (512^2 cells) stays in registers for the subtraction
   double acc = 0.0;
-  for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) acc += q[i];
+  float v[kMeanHold];
+  for (int64_t i0 = lo + threadIdx.x; i0 < hi; i0 += (int64_t)kMeanHold * 1024) {
+#pragma unroll
+    for (int k = 0; k < kMeanHold; ++k) v[k] = i0 + 1024 * k < hi ? q[i0 + 1024 * k] : 0.f;
+#pragma unroll
+    for (int k = 0; k < kMeanHold; ++k)
+      if (i0 + 1024 * k < hi) acc += v[k];
+  }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
   __syncthreads();
@@ -966,7 +1072,15 @@ __global__ void __cluster_dims__(kMeanCluster, 1, 1) __launch_bounds__(1024)
     mean = (float)(t / (double)n);
   }
   cl.sync();  // no block leaves while another may still read its partial
-  for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) q[i] -= mean;
+  if (hi - lo <= (int64_t)kMeanHold * 1024) {
+#pragma unroll
+    for (int k = 0; k < kMeanHold; ++k) {
+      const int64_t i = lo + threadIdx.x + 1024 * k;
+      if (i < hi) q[i] = v[k] - mean;
+    }
+  } else {
+    for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) q[i] -= mean;
+  }
 }
 
 // ------------------------------------------------------------------ Kolmogorov stepper
@@ -1068,6 +1182,19 @@ Src2<T> src2(const void *base, const void *coarse, float sign, int Y, int X, uns
   return s;
 }
 
+template <class T>
+Sweep1Src<T> sweep1(const void *f, float omega, float diag, int Y, int X, unsigned flags) {
+  Sweep1Src<T> s;
+  s.f = (const T *)f;
+  s.omega = omega;
+  s.diag = diag;
+  s.stride = (int64_t)Y * X;
+  s.Y = Y;
+  s.X = X;
+  s.periodic = (flags & HFM_FLAG_PERIODIC) ? 1 : 0;
+  return s;
+}
+
 }  // namespace
 }  // namespace hfm
 
@@ -1140,21 +1267,14 @@ int hfm_jacobi2d(int dtype, const float *w9_host, const void *base, const void *
     if (base || coarse) {
       const dim3 grid((X + kTwoTX - 1) / kTwoTX, (Y + kTwoTY - 1) / kTwoTY, B);
       if (grid.y > 65535) return fail(HFM_ERR_BAD_ARG, "hfm_jacobi2d: two sweeps: Y too large");
-      HFM2_DT(dtype, (k2_two_sweeps_tile<T><<<grid, kT2, 0, (cudaStream_t)stream>>>(
+      HFM2_DT(dtype, (k2_two_sweeps_tile<T, false><<<grid, kT2, 0, (cudaStream_t)stream>>>(
                          w9_of(w9_host), src2<T>(base, coarse, coarse_sign, Y, X, flags),
-                         (const T *)rhs, (T *)out, omega)));
+                         (const T *)rhs, (T *)out, nullptr, 0.f, omega)));
       HFM_CHECK_LAUNCH("k2_two_sweeps_tile");
       return HFM_OK;
     }
     HFM2_DT(dtype, {
-      Sweep1Src<T> s;
-      s.f = (const T *)rhs;
-      s.omega = omega;
-      s.diag = w9_host[4];
-      s.stride = n;
-      s.Y = Y;
-      s.X = X;
-      s.periodic = (flags & HFM_FLAG_PERIODIC) ? 1 : 0;
+      const Sweep1Src<T> s = sweep1<T>(rhs, omega, w9_host[4], Y, X, flags);
       k2_two_sweeps<T><<<dim3(blocks2(n, B), B), kT2, 0, (cudaStream_t)stream>>>(w9_of(w9_host), s, (T *)out);
     });
     HFM_CHECK_LAUNCH("k2_two_sweeps");
@@ -1207,19 +1327,52 @@ int hfm_pre2_restrict2d(int dtype, const float *w9_host, const void *rhs, void *
   if ((Y | X) & 1) return fail(HFM_ERR_BAD_ARG, "hfm_pre2_restrict2d: extents must be even");
   const dim3 grid((X + kTwoTX - 1) / kTwoTX, (Y + kTwoTY - 1) / kTwoTY, B);
   if (grid.y > 65535) return fail(HFM_ERR_BAD_ARG, "hfm_pre2_restrict2d: Y too large");
-  HFM2_DT(dtype, {
-    Sweep1Src<T> s;
-    s.f = (const T *)rhs;
-    s.omega = omega;
-    s.diag = w9_host[4];
-    s.stride = (int64_t)Y * X;
-    s.Y = Y;
-    s.X = X;
-    s.periodic = (flags & HFM_FLAG_PERIODIC) ? 1 : 0;
-    k2_pre2_restrict<T><<<grid, kT2, 0, (cudaStream_t)stream>>>(w9_of(w9_host), s, (T *)phi,
-                                                               (T *)coarse_rhs);
-  });
+  HFM2_DT(dtype, (k2_pre2_restrict<T, false><<<grid, kT2, 0, (cudaStream_t)stream>>>(
+                     w9_of(w9_host), sweep1<T>(rhs, omega, w9_host[4], Y, X, flags), (T *)phi,
+                     (T *)coarse_rhs, nullptr, nullptr, nullptr)));
   HFM_CHECK_LAUNCH("k2_pre2_restrict");
+  return HFM_OK;
+}
+
+int hfm_outer_pre2_restrict2d(int dtype, const float *w9_host, const float *p, const float *rhs,
+                              void *r, void *phi, void *coarse_rhs, int B, int Y, int X, float omega,
+                              unsigned flags, hfm_stream_t stream) {
+  int st;
+  if ((st = check2(B, Y, X)) || (st = check_dtype2(dtype))) return st;
+  const void *f[5] = {p, rhs, r, phi, coarse_rhs};
+  if (!w9_host) return fail(HFM_ERR_BAD_ARG, "hfm_outer_pre2_restrict2d: NULL weights");
+  for (int i = 0; i < 5; ++i) {
+    if (!f[i]) return fail(HFM_ERR_BAD_ARG, "hfm_outer_pre2_restrict2d: NULL field");
+    for (int j = 0; j < i; ++j)
+      if (f[i] == f[j] && (i > 1)) return fail(HFM_ERR_BAD_ARG, "hfm_outer_pre2_restrict2d: aliased fields");
+  }
+  if (w9_host[4] == 0.f) return fail(HFM_ERR_BAD_ARG, "hfm_outer_pre2_restrict2d: zero diagonal weight");
+  if ((Y | X) & 1) return fail(HFM_ERR_BAD_ARG, "hfm_outer_pre2_restrict2d: extents must be even");
+  const dim3 grid((X + kTwoTX - 1) / kTwoTX, (Y + kTwoTY - 1) / kTwoTY, B);
+  if (grid.y > 65535) return fail(HFM_ERR_BAD_ARG, "hfm_outer_pre2_restrict2d: Y too large");
+  HFM2_DT(dtype, (k2_pre2_restrict<T, true><<<grid, kT2, 0, (cudaStream_t)stream>>>(
+                     w9_of(w9_host), sweep1<T>(nullptr, omega, w9_host[4], Y, X, flags), (T *)phi,
+                     (T *)coarse_rhs, p, rhs, (T *)r)));
+  HFM_CHECK_LAUNCH("k2_pre2_restrict");
+  return HFM_OK;
+}
+
+int hfm_post2_update2d(int dtype, const float *w9_host, const void *base, const void *coarse,
+                       float coarse_sign, const void *rhs, float *p, float update_sign, int B, int Y,
+                       int X, float omega, unsigned flags, hfm_stream_t stream) {
+  int st;
+  if ((st = check2(B, Y, X)) || (st = check_dtype2(dtype))) return st;
+  if (!w9_host || !base || !rhs || !p) return fail(HFM_ERR_BAD_ARG, "hfm_post2_update2d: NULL argument");
+  if (p == base || p == coarse || p == rhs) return fail(HFM_ERR_BAD_ARG, "hfm_post2_update2d: p aliases an input");
+  if (w9_host[4] == 0.f) return fail(HFM_ERR_BAD_ARG, "hfm_post2_update2d: zero diagonal weight");
+  if (coarse && !(flags & HFM_FLAG_SAME_LEVEL_CORR) && ((Y | X) & 1))
+    return fail(HFM_ERR_BAD_ARG, "hfm_post2_update2d: coarse correction needs even extents");
+  const dim3 grid((X + kTwoTX - 1) / kTwoTX, (Y + kTwoTY - 1) / kTwoTY, B);
+  if (grid.y > 65535) return fail(HFM_ERR_BAD_ARG, "hfm_post2_update2d: Y too large");
+  HFM2_DT(dtype, (k2_two_sweeps_tile<T, true><<<grid, kT2, 0, (cudaStream_t)stream>>>(
+                     w9_of(w9_host), src2<T>(base, coarse, coarse_sign, Y, X, flags), (const T *)rhs,
+                     nullptr, p, update_sign, omega)));
+  HFM_CHECK_LAUNCH("k2_two_sweeps_tile");
   return HFM_OK;
 }
 

@@ -157,6 +157,15 @@ class Multigrid2D:
     def iterate(self, p, f):
         """p -= V(A p - f): float32 p and f of shape (slots, Y, X)."""
         Y, X = self.shapes[0]
+        if (self.fused_pairs and self.nu_pre == 2 and self.nu_post == 2 and Y % 2 == 0 and X % 2 == 0
+                and self.L > 1 and not (self.fused_coarse and self.l_sub == 0)):
+            # the fine level's two legs with the outer defect and the update inside them
+            L.call("hfm_outer_pre2_restrict2d", self.code, self.ws[0], _p(p), _p(f), _p(self.rhs[0]),
+                   _p(self.w[0]), _p(self.rhs[1]), self.slots, Y, X, self.omega, self.flags, _stream())
+            wc = self._cycle(1)
+            L.call("hfm_post2_update2d", self.code, self.ws[0], _p(self.w[0]), _p(wc), -1.0,
+                   _p(self.rhs[0]), _p(p), -1.0, self.slots, Y, X, self.omega, self.flags, _stream())
+            return
         L.call("hfm_outer_residual2d", self.ws[0], _p(p), _p(f), self.code, _p(self.rhs[0]),
                self.slots, Y, X, self.flags, None, None, _stream())
         w = self._cycle(0)

@@ -389,6 +389,18 @@ int hfm_jacobi2d(int dtype, const float *w9_host, const void *base, const void *
 int hfm_pre2_restrict2d(int dtype, const float *w9_host, const void *rhs, void *phi,
                         void *coarse_rhs, int B, int Y, int X, float omega, unsigned flags,
                         hfm_stream_t stream);
+/* hfm_outer_residual2d (r = A p - rhs of float32 p and rhs, stored in dtype) and
+ * hfm_pre2_restrict2d on r in one launch, the same bits.  Even extents; r, phi and coarse_rhs
+ * distinct from each other and from p and rhs. */
+int hfm_outer_pre2_restrict2d(int dtype, const float *w9_host, const float *p, const float *rhs,
+                              void *r, void *phi, void *coarse_rhs, int B, int Y, int X, float omega,
+                              unsigned flags, hfm_stream_t stream);
+/* hfm_jacobi2d with HFM_FLAG_TWO_SWEEPS (base not NULL) followed by hfm_update2d in one launch,
+ * the same bits: w = two sweeps from base + coarse_sign * P(coarse) on rhs is not stored, p +=
+ * update_sign * w.  p distinct from the other fields. */
+int hfm_post2_update2d(int dtype, const float *w9_host, const void *base, const void *coarse,
+                       float coarse_sign, const void *rhs, float *p, float update_sign, int B, int Y,
+                       int X, float omega, unsigned flags, hfm_stream_t stream);
 /* r = A phi - rhs (rhs NULL = 0): Multigrid_2D.ipynb#c18 `CNN3D_A_128(values) - b`. */
 int hfm_residual2d(int dtype, const float *w9_host, const void *phi, const void *rhs, void *r,
                    int B, int Y, int X, unsigned flags, hfm_stream_t stream);

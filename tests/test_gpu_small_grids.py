@@ -186,7 +186,7 @@ def test_ragged_rows(hfm, T, shape, form, offset):
 # with whole and straddling rows, one cell per thread, ringed levels (X % 4 != 0 above 512
 # cells), coarsest levels on a warp (a full one too) and above
 @pytest.mark.parametrize("periodic", [True, False])
-@pytest.mark.parametrize("shape,min_edge", [((64, 64), 4), ((56, 56), 4), ((48, 80), 5), ((52, 46), 4), ((40, 24), 3),
+@pytest.mark.parametrize("shape,min_edge", [((64, 64), 4), ((56, 56), 4), ((48, 80), 5), ((52, 46), 23), ((40, 24), 3),
                                             ((16, 128), 4), ((64, 32), 8), ((60, 44), 30)])
 def test_2d_fused_levels_same_bits(hfm, T, periodic, shape, min_edge):
     KM = hfm.kolmogorov
@@ -203,3 +203,32 @@ def test_2d_fused_levels_same_bits(hfm, T, periodic, shape, min_edge):
             m.iterate(p, f)
         outs.append(p.cpu().numpy())
     np.testing.assert_array_equal(outs[0], outs[1])
+
+
+# the fine level's two legs with the outer defect and the update inside, against the separate
+# launches, bit for bit: tile edges, axes shorter than a ring
+@pytest.mark.parametrize("periodic", [True, False])
+@pytest.mark.parametrize("storage", ["f32", "bf16"])
+@pytest.mark.parametrize("shape", [(2, 2), (2, 34), (4, 6), (8, 32), (10, 66), (130, 96)])
+def test_2d_outer_legs_same_bits(hfm, T, periodic, storage, shape):
+    L, KM = hfm._lib, hfm.kolmogorov
+    code, dt = KM._DT[storage]
+    Y, X = shape
+    rng = np.random.default_rng(37)
+    w = KM._w9(KM.laplace5(0.3) + 0.1 * rng.standard_normal((3, 3)))
+    fl = L.FLAG_PERIODIC if periodic else 0
+    st, P = hfm.ops._stream(), KM._p
+    p, f = (T.from_numpy(rng.standard_normal((2, Y, X)).astype(np.float32)).cuda() for _ in range(2))
+    wc = T.from_numpy(rng.standard_normal((2, Y // 2, X // 2)).astype(np.float32)).cuda().to(dt)
+    new = lambda *s: T.zeros((2,) + s, device="cuda", dtype=dt)
+    a, b = [(new(Y, X), new(Y, X), new(Y // 2, X // 2)) for _ in range(2)]
+    L.call("hfm_outer_pre2_restrict2d", code, w, P(p), P(f), *(P(t) for t in a), 2, Y, X, 0.8, fl, st)
+    L.call("hfm_outer_residual2d", w, P(p), P(f), code, P(b[0]), 2, Y, X, fl, None, None, st)
+    L.call("hfm_pre2_restrict2d", code, w, P(b[0]), P(b[1]), P(b[2]), 2, Y, X, 0.8, fl, st)
+    for s, t in zip(a, b):
+        assert T.equal(s, t)
+    pa, pb, out = p.clone(), p.clone(), new(Y, X)
+    L.call("hfm_post2_update2d", code, w, P(a[1]), P(wc), -1.0, P(a[0]), P(pa), -1.0, 2, Y, X, 0.8, fl, st)
+    L.call("hfm_jacobi2d", code, w, P(a[1]), P(wc), -1.0, P(a[0]), P(out), 2, Y, X, 0.8, fl | L.FLAG_TWO_SWEEPS, st)
+    L.call("hfm_update2d", P(pb), code, P(out), -1.0, 2 * Y * X, st)
+    assert T.equal(pa, pb)
