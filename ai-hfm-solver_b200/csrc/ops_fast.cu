@@ -1,14 +1,15 @@
 // Register-queue plane-marching stencil kernels.  Layout and semantics are those of
 // ops_generic.cu; these kernels differ only in how they move data:
 //   * a thread owns V consecutive x (V = 4 where rows and pointers allow it: one 16-byte
-//     float32 / 8-byte 16-bit load; else 2 or 1, for the ragged grids) on R rows and marches
+//     float32 / 8-byte 16-bit load; else 2 or 1, for the ragged grids) of a row and marches
 //     along z through a chunk of planes, so z neighbours, the z-face coefficient and 27-point
 //     partial sums stay in registers;
 //   * x neighbours come from the adjacent lanes by warp shuffle (lanes hold consecutive
 //     vectors of the flattened (row, x-vector) index); only lanes 0 / 31 load them;
 //   * y neighbours are vector loads served mostly by L1 (the rows belong to the same block).
 // Modes: SMOOTH (weighted Jacobi), RESID (A phi - b, optional norm partials), RESTRICT
-// (residual of R = 2 rows x 2 planes x 2 columns averaged into the coarse grid).
+// (residuals of 2 rows x 2 planes x 2 columns averaged into the coarse grid; a lane pair
+// holds the two rows).
 #include <map>
 #include <mutex>
 
@@ -138,32 +139,33 @@ __device__ __forceinline__ FV<V> phi_vec(const FastArgs<T> &a, int64_t ib, int64
   return v;
 }
 
-// Neighbours across the vector boundary by shuffle (all lanes must call).
-template <class T, int CORR, int V>
+// Neighbours across the vector boundary by shuffle (all lanes must call).  LS: lanes between a
+// row's vectors (2 in the restriction, where a lane pair holds a pair of rows).
+template <class T, int CORR, int V, int LS>
 __device__ __forceinline__ void halo_x(const FastArgs<T> &a, int64_t ib, int64_t ic, int z, int y,
                                        int x0, bool inb, const FV<V> &c, float &l, float &r) {
   const int lane = threadIdx.x & 31;
-  float sl = __shfl_up_sync(0xffffffffu, c.v[V - 1], 1);
-  float sr = __shfl_down_sync(0xffffffffu, c.v[0], 1);
+  float sl = __shfl_up_sync(0xffffffffu, c.v[V - 1], LS);
+  float sr = __shfl_down_sync(0xffffffffu, c.v[0], LS);
   l = 0.f;
   r = 0.f;
   if (inb) {
-    if (x0 > 0) l = lane > 0 ? sl : phi_scalar<T, CORR>(a, ib, ic, z, y, x0 - 1);
-    if (x0 + V < a.X) r = lane < 31 ? sr : phi_scalar<T, CORR>(a, ib, ic, z, y, x0 + V);
+    if (x0 > 0) l = lane >= LS ? sl : phi_scalar<T, CORR>(a, ib, ic, z, y, x0 - 1);
+    if (x0 + V < a.X) r = lane < 32 - LS ? sr : phi_scalar<T, CORR>(a, ib, ic, z, y, x0 + V);
   }
 }
 
-template <class T, int V>
+template <class T, int V, int LS>
 __device__ __forceinline__ void coef_halo_x(const T *s, int64_t base_off, int x0, int X, bool inb,
                                             const FV<V> &c, float &l, float &r) {
   const int lane = threadIdx.x & 31;
-  float sl = __shfl_up_sync(0xffffffffu, c.v[V - 1], 1);
-  float sr = __shfl_down_sync(0xffffffffu, c.v[0], 1);
+  float sl = __shfl_up_sync(0xffffffffu, c.v[V - 1], LS);
+  float sr = __shfl_down_sync(0xffffffffu, c.v[0], LS);
   l = c.v[0];  // wall: ghost sigma = interior sigma
   r = c.v[V - 1];
   if (inb) {
-    if (x0 > 0) l = lane > 0 ? sl : St<T>::ld(s + base_off - 1);
-    if (x0 + V < X) r = lane < 31 ? sr : St<T>::ld(s + base_off + V);
+    if (x0 > 0) l = lane >= LS ? sl : St<T>::ld(s + base_off - 1);
+    if (x0 + V < X) r = lane < 32 - LS ? sr : St<T>::ld(s + base_off + V);
   }
 }
 
@@ -178,19 +180,40 @@ __device__ __forceinline__ double block_reduce(double v) {
   return t;
 }
 
-// RESTRICT: the coarse cells of a thread's vector gain plane z of its residuals (x pairs within
-// the vector, y pairs across the two rows); an odd plane completes and stores them.
-template <class T, int R, int V>
-__device__ __forceinline__ void coarse_cells(const FastArgs<T> &a, int64_t inst, int z, int g, int x0,
-                                             bool valid, const FV<V> (&res)[R], float (&cpart)[2]) {
+// The (y, x0) of a thread: consecutive lanes hold consecutive vectors of a row; in RESTRICT a
+// lane pair holds the two rows of a coarse row at one x0, so that neither a second row per
+// thread (123 registers, half the warps) nor shared memory is needed to average them: one
+// 32^3 SIGMA7 instance, float32, 7.6 -> 4.1 us.
+constexpr int lane_step(int mode) { return mode == M_RESTRICT ? 2 : 1; }
+template <int MODE, int V>
+__device__ __forceinline__ bool thread_row(int X, int Y, int &y, int &x0) {
+  constexpr int LS = lane_step(MODE);
+  const int nvx = X / V;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = i < Y * nvx;  // RESTRICT: Y is even
+  const int j = valid ? i / LS : 0;
+  const int g = j / nvx;
+  y = g * LS + (valid ? i % LS : 0);
+  x0 = (j - g * nvx) * V;
+  return valid;
+}
+
+// RESTRICT: a lane pair holds the two rows of its coarse cells; they gain plane z of the
+// residuals (x pairs within the vector, y pairs across the two lanes), and an odd plane
+// completes and stores them.
+template <class T, int V>
+__device__ __forceinline__ void coarse_cells(const FastArgs<T> &a, int64_t inst, int z, int y, int x0,
+                                             bool valid, const FV<V> &res, float (&cpart)[2]) {
   if constexpr (V > 1) {
 #pragma unroll
-    for (int k = 0; k < V / 2; ++k)
-      cpart[k] += 0.125f * ((res[0].v[2 * k] + res[0].v[2 * k + 1]) + (res[R - 1].v[2 * k] + res[R - 1].v[2 * k + 1]));
+    for (int k = 0; k < V / 2; ++k) {
+      const float pk = res.v[2 * k] + res.v[2 * k + 1];
+      cpart[k] += 0.125f * (pk + __shfl_xor_sync(0xffffffffu, pk, 1));
+    }
     if (!(z & 1)) return;
-    if (valid) {
+    if (valid && !(y & 1)) {
       const int Yc = a.Y >> 1, Xc = a.X >> 1;
-      T *cp = a.coarse + inst * a.coarse_stride + ((int64_t)(z >> 1) * Yc + g) * Xc + (x0 >> 1);
+      T *cp = a.coarse + inst * a.coarse_stride + ((int64_t)(z >> 1) * Yc + (y >> 1)) * Xc + (x0 >> 1);
       if (sizeof(T) == 4 && V == 4) {
         *reinterpret_cast<float2 *>(cp) = make_float2(cpart[0], cpart[1]);
       } else {
@@ -203,21 +226,19 @@ __device__ __forceinline__ void coarse_cells(const FastArgs<T> &a, int64_t inst,
 }
 
 // ---------------------------------------------------------------------------------------
-// 7-point forms (CONST7, SIGMA7).  R rows per thread.
+// 7-point forms (CONST7, SIGMA7, FACE7).
 // ---------------------------------------------------------------------------------------
-template <int KIND, class T, int MODE, int CORR, int R, int V>
-__global__ void __launch_bounds__(kFastThreads, R == 1 ? 4 : 2)
+template <int KIND, class T, int MODE, int CORR, int V>
+__global__ void __launch_bounds__(kFastThreads, MODE == M_RESTRICT ? 2 : 4)
     k_fast7(FastArgs<T> a) {
   using F4 = FV<V>;  // a thread's cells of a row
+  constexpr int LS = lane_step(MODE);
+  constexpr int NP = MODE == M_RESTRICT ? 2 : 1;  // planes whose loads are in flight together
   const int64_t inst = blockIdx.z;
   if (a.active && !a.active[inst]) return;
   const int X = a.X, Y = a.Y, Z = a.Z;
-  const int nvx = X / V;
-  const int ngroups = (Y + R - 1) / R;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = i < ngroups * nvx;
-  const int g = valid ? i / nvx : 0;
-  const int x0 = valid ? (i - g * nvx) * V : 0;
+  int y, x0;
+  const bool valid = thread_row<MODE, V>(X, Y, y, x0);
   const int64_t ib = inst * a.stride, ic = inst * a.corr_stride;
   const int64_t plane = (int64_t)Y * X;
   const int z0 = blockIdx.y * a.zc;
@@ -247,142 +268,160 @@ __global__ void __launch_bounds__(kFastThreads, R == 1 ? 4 : 2)
     }
   }
 
-  // per-row z queue: phi' at z-1, z, z+1; for SIGMA7 also sigma_z at z and the z- face
-  F4 pm[R], pc[R], pp[R], szc[R], azlo[R];
-  bool rin[R];
-  int yr[R];
+  // z queue: phi' at z-1, z, z+1; for SIGMA7 also sigma_z at z, and the z- face
+  F4 pm, pc, szc, azlo;
+  pm = (z0 > 0) ? phi_vec<T, CORR, V>(a, ib, ic, z0 - 1, y, x0, valid) : filled<V>(0.f);
+  pc = phi_vec<T, CORR, V>(a, ib, ic, z0, y, x0, valid);
+  const int64_t off0 = (int64_t)z0 * plane + (int64_t)y * X + x0;
+  if (KIND == HFM_OP_SIGMA7) {
+    szc = valid ? ldv<T, V>(sz + off0) : filled<V>(1.f);
+    if (z0 > 0 && valid) {
+      F4 sm = ldv<T, V>(sz + off0 - plane);
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    yr[r] = g * R + r;
-    rin[r] = valid && yr[r] < Y;
-    pm[r] = (z0 > 0) ? phi_vec<T, CORR, V>(a, ib, ic, z0 - 1, yr[r], x0, rin[r]) : filled<V>(0.f);
-    pc[r] = phi_vec<T, CORR, V>(a, ib, ic, z0, yr[r], x0, rin[r]);
-    if (KIND == HFM_OP_SIGMA7) {
-      const int64_t off = (int64_t)z0 * plane + (int64_t)yr[r] * X + x0;
-      szc[r] = rin[r] ? ldv<T, V>(sz + off) : filled<V>(1.f);
-      if (z0 > 0 && rin[r]) {
-        F4 sm = ldv<T, V>(sz + off - plane);
+      for (int e = 0; e < V; ++e) azlo.v[e] = cz * 0.5f * (szc.v[e] + sm.v[e]);
+    } else {
 #pragma unroll
-        for (int e = 0; e < V; ++e) azlo[r].v[e] = cz * 0.5f * (szc[r].v[e] + sm.v[e]);
-      } else {
-#pragma unroll
-        for (int e = 0; e < V; ++e) azlo[r].v[e] = cz * szc[r].v[e];
-      }
-    } else if (KIND == HFM_OP_FACE7) {
-      // the z face below plane z0 (wall faces included in the array), times the scale
-      const float s = a.op.scale;
-      const F4 fz = rin[r] ? ldv<T, V>(sz + (int64_t)z0 * plane + (int64_t)yr[r] * X + x0) : filled<V>(0.f);
-#pragma unroll
-      for (int e = 0; e < V; ++e) azlo[r].v[e] = s * fz.v[e];
+      for (int e = 0; e < V; ++e) azlo.v[e] = cz * szc.v[e];
     }
+  } else if (KIND == HFM_OP_FACE7) {
+    // the z face below plane z0 (wall faces included in the array), times the scale
+    const float s = a.op.scale;
+    const F4 fz = valid ? ldv<T, V>(sz + off0) : filled<V>(0.f);
+#pragma unroll
+    for (int e = 0; e < V; ++e) azlo.v[e] = s * fz.v[e];
   }
   double acc = 0.0;
   float cpart[2] = {0.f, 0.f};  // RESTRICT: the two coarse cells of this vector, summed over planes
 
-  for (int z = z0; z < z1; ++z) {
-    F4 res[R];
+  for (int zb = z0; zb < z1; zb += NP) {
+    // what plane z reads besides the queue; RESTRICT (whole plane pairs) loads two planes'
+    // before it uses either, and the y neighbour the lane pair holds comes by shuffle
+    F4 pp[NP], pyo[NP], f[NP], c0[NP], c1[NP], c2[NP], c3[NP], c4[NP];
+    F4 pym, pyp;
+    float fx4[NP], pl, pr;
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int y = yr[r];
-      const bool in = rin[r];
-      pp[r] = (z + 1 < Z) ? phi_vec<T, CORR, V>(a, ib, ic, z + 1, y, x0, in) : filled<V>(0.f);
-      float pl, pr;
-      halo_x<T, CORR, V>(a, ib, ic, z, y, x0, in, pc[r], pl, pr);
-      F4 pym = phi_vec<T, CORR, V>(a, ib, ic, z, y - 1, x0, in && y > 0);
-      F4 pyp = phi_vec<T, CORR, V>(a, ib, ic, z, y + 1, x0, in && y + 1 < Y);
+    for (int n = 0; n < NP; ++n) {
+      const int z = zb + n;
       const int64_t off = (int64_t)z * plane + (int64_t)y * X + x0;
-      F4 Ax, dg;
-      if (KIND == HFM_OP_CONST7) {
-#pragma unroll
-        for (int e = 0; e < V; ++e) {
-          float xm = e == 0 ? pl : pc[r].v[e - 1];
-          float xp = e == V - 1 ? pr : pc[r].v[e + 1];
-          Ax.v[e] = dconst * pc[r].v[e] - kz * (pm[r].v[e] + pp[r].v[e]) -
-                    ky * (pym.v[e] + pyp.v[e]) - kx * (xm + xp);
-          dg.v[e] = dconst;
-        }
-      } else if (KIND == HFM_OP_FACE7) {
-        // stored faces (scale applied here): the x faces of the 4 cells and the one right of
+      pp[n] = (z + 1 < Z) ? phi_vec<T, CORR, V>(a, ib, ic, z + 1, y, x0, valid) : filled<V>(0.f);
+      if (MODE == M_RESTRICT) {
+        const int yo = (y & 1) ? y + 1 : y - 1;
+        pyo[n] = phi_vec<T, CORR, V>(a, ib, ic, z, yo, x0, valid && yo >= 0 && yo < Y);
+      } else {
+        halo_x<T, CORR, V, LS>(a, ib, ic, z, y, x0, valid, pc, pl, pr);
+        pym = phi_vec<T, CORR, V>(a, ib, ic, z, y - 1, x0, valid && y > 0);
+        pyp = phi_vec<T, CORR, V>(a, ib, ic, z, y + 1, x0, valid && y + 1 < Y);
+      }
+      if (KIND == HFM_OP_FACE7) {
+        // stored faces (scale applied later): the x faces of the V cells and the one right of
         // the last, the y faces below and above, the z face above (the one below is carried)
-        const float s = a.op.scale;
         const int64_t rx = ((int64_t)z * Y + y) * (X + 8) + x0;
         const int64_t ry = ((int64_t)z * (Y + 1) + y) * X + x0;
         const F4 zero4 = filled<V>(0.f);
-        const F4 fx = in ? ldv<T, V>(sx + rx) : zero4;
-        const float fx4 = in ? St<T>::ld(sx + rx + V) : 0.f;
-        const F4 fyl = in ? ldv<T, V>(sy + ry) : zero4;
-        const F4 fyh = in ? ldv<T, V>(sy + ry + X) : zero4;
-        const F4 fzh = in ? ldv<T, V>(sz + off + plane) : zero4;
-        F4 azhi;
+        c0[n] = valid ? ldv<T, V>(sx + rx) : zero4;
+        fx4[n] = valid ? St<T>::ld(sx + rx + V) : 0.f;
+        c1[n] = valid ? ldv<T, V>(sy + ry) : zero4;
+        c2[n] = valid ? ldv<T, V>(sy + ry + X) : zero4;
+        c3[n] = valid ? ldv<T, V>(sz + off + plane) : zero4;
+      } else if (KIND == HFM_OP_SIGMA7) {
+        c0[n] = valid ? ldv<T, V>(sx + off) : filled<V>(1.f);
+        c1[n] = valid ? ldv<T, V>(sy + off) : filled<V>(1.f);
+        c2[n] = (valid && y > 0) ? ldv<T, V>(sy + off - X) : c1[n];
+        c3[n] = (valid && y + 1 < Y) ? ldv<T, V>(sy + off + X) : c1[n];
+        if (z + 1 < Z && valid) c4[n] = ldv<T, V>(sz + off + plane);
+        else c4[n] = n ? c4[0] : szc;
+      }
+      if (MODE == M_RESTRICT) f[n] = a.rhs && valid ? ldv<T, V>(a.rhs + ib + off) : filled<V>(0.f);
+    }
+#pragma unroll
+    for (int n = 0; n < NP; ++n) {
+      const int z = zb + n;
+      const int64_t off = (int64_t)z * plane + (int64_t)y * X + x0;
+      if (MODE == M_RESTRICT) {
+        halo_x<T, CORR, V, LS>(a, ib, ic, z, y, x0, valid, pc, pl, pr);
 #pragma unroll
         for (int e = 0; e < V; ++e) {
-          const float axm = s * fx.v[e], axp = s * (e == V - 1 ? fx4 : fx.v[e + 1]);
-          const float aym = s * fyl.v[e], ayp = s * fyh.v[e];
-          azhi.v[e] = s * fzh.v[e];
-          const float xm = e == 0 ? pl : pc[r].v[e - 1];
-          const float xp = e == V - 1 ? pr : pc[r].v[e + 1];
-          const float p = pc[r].v[e];
-          Ax.v[e] = axm * (p - xm) + axp * (p - xp) + aym * (p - pym.v[e]) + ayp * (p - pyp.v[e]) +
-                    azlo[r].v[e] * (p - pm[r].v[e]) + azhi.v[e] * (p - pp[r].v[e]);
-          dg.v[e] = ((axm + axp) + (aym + ayp)) + (azlo[r].v[e] + azhi.v[e]);
+          const float o = __shfl_xor_sync(0xffffffffu, pc.v[e], 1);
+          pym.v[e] = (y & 1) ? o : pyo[n].v[e];
+          pyp.v[e] = (y & 1) ? pyo[n].v[e] : o;
         }
-        azlo[r] = azhi;
-      } else {
-        F4 sxc = in ? ldv<T, V>(sx + off) : filled<V>(1.f);
-        float sxl, sxr;
-        coef_halo_x<T, V>(sx, off, x0, X, in, sxc, sxl, sxr);
-        F4 syc = in ? ldv<T, V>(sy + off) : filled<V>(1.f);
-        F4 sym = (in && y > 0) ? ldv<T, V>(sy + off - X) : syc;
-        F4 syp = (in && y + 1 < Y) ? ldv<T, V>(sy + off + X) : syc;
-        F4 szp = (in && z + 1 < Z) ? ldv<T, V>(sz + off + plane) : szc[r];
+      }
+      F4 Ax, dg, res;
+      if (KIND == HFM_OP_CONST7) {
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          float xm = e == 0 ? pl : pc.v[e - 1];
+          float xp = e == V - 1 ? pr : pc.v[e + 1];
+          Ax.v[e] = dconst * pc.v[e] - kz * (pm.v[e] + pp[n].v[e]) - ky * (pym.v[e] + pyp.v[e]) -
+                    kx * (xm + xp);
+          dg.v[e] = dconst;
+        }
+      } else if (KIND == HFM_OP_FACE7) {
+        const float s = a.op.scale;
         F4 azhi;
 #pragma unroll
         for (int e = 0; e < V; ++e) {
-          const float sxe = sxc.v[e];
-          const float sxm = e == 0 ? sxl : sxc.v[e - 1];
-          const float sxp = e == V - 1 ? sxr : sxc.v[e + 1];
+          const float axm = s * c0[n].v[e], axp = s * (e == V - 1 ? fx4[n] : c0[n].v[e + 1]);
+          const float aym = s * c1[n].v[e], ayp = s * c2[n].v[e];
+          azhi.v[e] = s * c3[n].v[e];
+          const float xm = e == 0 ? pl : pc.v[e - 1];
+          const float xp = e == V - 1 ? pr : pc.v[e + 1];
+          const float p = pc.v[e];
+          Ax.v[e] = axm * (p - xm) + axp * (p - xp) + aym * (p - pym.v[e]) + ayp * (p - pyp.v[e]) +
+                    azlo.v[e] * (p - pm.v[e]) + azhi.v[e] * (p - pp[n].v[e]);
+          dg.v[e] = ((axm + axp) + (aym + ayp)) + (azlo.v[e] + azhi.v[e]);
+        }
+        azlo = azhi;
+      } else {
+        float sxl, sxr;
+        coef_halo_x<T, V, LS>(sx, off, x0, X, valid, c0[n], sxl, sxr);
+        F4 azhi;
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          const float sxe = c0[n].v[e];
+          const float sxm = e == 0 ? sxl : c0[n].v[e - 1];
+          const float sxp = e == V - 1 ? sxr : c0[n].v[e + 1];
           // wall faces use the interior sigma (sxl / sxr already do at x = 0 / X-1)
           const float axm = cx * 0.5f * (sxe + sxm);
           const float axp = cx * 0.5f * (sxe + sxp);
-          const float aym = cy * 0.5f * (syc.v[e] + sym.v[e]);
-          const float ayp = cy * 0.5f * (syc.v[e] + syp.v[e]);
-          azhi.v[e] = cz * 0.5f * (szc[r].v[e] + szp.v[e]);
-          const float xm = e == 0 ? pl : pc[r].v[e - 1];
-          const float xp = e == V - 1 ? pr : pc[r].v[e + 1];
-          const float p = pc[r].v[e];
+          const float aym = cy * 0.5f * (c1[n].v[e] + c2[n].v[e]);
+          const float ayp = cy * 0.5f * (c1[n].v[e] + c3[n].v[e]);
+          azhi.v[e] = cz * 0.5f * (szc.v[e] + c4[n].v[e]);
+          const float xm = e == 0 ? pl : pc.v[e - 1];
+          const float xp = e == V - 1 ? pr : pc.v[e + 1];
+          const float p = pc.v[e];
           Ax.v[e] = axm * (p - xm) + axp * (p - xp) + aym * (p - pym.v[e]) + ayp * (p - pyp.v[e]) +
-                    azlo[r].v[e] * (p - pm[r].v[e]) + azhi.v[e] * (p - pp[r].v[e]);
-          dg.v[e] = axm + axp + aym + ayp + azlo[r].v[e] + azhi.v[e];
+                    azlo.v[e] * (p - pm.v[e]) + azhi.v[e] * (p - pp[n].v[e]);
+          dg.v[e] = axm + axp + aym + ayp + azlo.v[e] + azhi.v[e];
         }
-        azlo[r] = azhi;
-        szc[r] = szp;
+        azlo = azhi;
+        szc = c4[n];
       }
-      F4 f = filled<V>(0.f);
-      if (a.rhs && in) f = ldv<T, V>(a.rhs + ib + off);
+      if (MODE != M_RESTRICT) f[n] = a.rhs && valid ? ldv<T, V>(a.rhs + ib + off) : filled<V>(0.f);
       if (MODE == M_SMOOTH) {
 #pragma unroll
-        for (int e = 0; e < V; ++e) res[r].v[e] = pc[r].v[e] + a.omega * quotient<V>(f.v[e] - Ax.v[e], dg.v[e]);
-        if (a.dot_rhs && in) {
+        for (int e = 0; e < V; ++e) res.v[e] = pc.v[e] + a.omega * quotient<V>(f[n].v[e] - Ax.v[e], dg.v[e]);
+        if (a.dot_rhs && valid) {
 #pragma unroll
-          for (int e = 0; e < V; ++e) acc += (double)res[r].v[e] * f.v[e];
+          for (int e = 0; e < V; ++e) acc += (double)res.v[e] * f[n].v[e];
         }
       } else {
 #pragma unroll
-        for (int e = 0; e < V; ++e) res[r].v[e] = Ax.v[e] - f.v[e];
-        if (a.zero_xend_out && x0 + V == X) res[r].v[V - 1] = 0.f;
-        if (in) {
+        for (int e = 0; e < V; ++e) res.v[e] = Ax.v[e] - f[n].v[e];
+        if (a.zero_xend_out && x0 + V == X) res.v[V - 1] = 0.f;
+        if (valid) {
 #pragma unroll
-          for (int e = 0; e < V; ++e) acc += (double)res[r].v[e] * (a.dot_phi ? pc[r].v[e] : res[r].v[e]);
+          for (int e = 0; e < V; ++e) acc += (double)res.v[e] * (a.dot_phi ? pc.v[e] : res.v[e]);
         }
       }
-      if (in && a.out) {
-        if (MODE == M_SMOOTH && a.top_copy && z == 1) stv<T, V>(a.out + ib + y * X + x0, res[r]);
-        if (!(MODE == M_SMOOTH && a.top_copy && z == 0 && Z > 1)) stv<T, V>(a.out + ib + off, res[r]);
+      if (valid && a.out) {
+        if (MODE == M_SMOOTH && a.top_copy && z == 1) stv<T, V>(a.out + ib + y * X + x0, res);
+        if (!(MODE == M_SMOOTH && a.top_copy && z == 0 && Z > 1)) stv<T, V>(a.out + ib + off, res);
       }
-      pm[r] = pc[r];
-      pc[r] = pp[r];
+      pm = pc;
+      pc = pp[n];
+      if (MODE == M_RESTRICT) coarse_cells<T, V>(a, inst, z, y, x0, valid, res, cpart);
     }
-    if (MODE == M_RESTRICT) coarse_cells<T, R, V>(a, inst, z, g, x0, valid, res, cpart);
   }
   if ((MODE != M_SMOOTH || a.dot_rhs) && a.partials) {
     double t = block_reduce(acc);
@@ -543,124 +582,104 @@ __global__ void __launch_bounds__(kFastThreads, 4) k_column7(FastArgs<T> a) {
 }
 
 // ---------------------------------------------------------------------------------------
-// 27-point form (K27): per-plane partial sums into three pending outputs.  R rows per thread:
-// one for sweeps and residuals, two for the residual + restriction, whose four input rows per
-// plane serve both.  On one instance of 16 x 32 x 32 the latter takes 7.8 us, bound by its
-// chain of dependent loads; a thread per coarse cell with 216 bounds-checked loads took 21 us
-// (and 82 us on 64 x 128 x 128, where the plane-marching TMA kernel takes 8 us).
+// 27-point form (K27): per-plane partial sums into three pending outputs.  On one instance of
+// 16 x 32 x 32 the residual + restriction takes 5.2 us, bound by its chain of dependent loads
+// (7.8 us with two rows per thread; a thread per coarse cell with 216 bounds-checked loads took
+// 21 us, and 82 us on 64 x 128 x 128, where the plane-marching TMA kernel takes 8 us).
 // ---------------------------------------------------------------------------------------
-template <class T, int MODE, int CORR, int R, int V>
+template <class T, int MODE, int CORR, int V>
 __global__ void __launch_bounds__(kFastThreads)
     k_fast27(FastArgs<T> a) {
   using F4 = FV<V>;  // a thread's cells of a row
   const int64_t inst = blockIdx.z;
   if (a.active && !a.active[inst]) return;
   const int X = a.X, Y = a.Y, Z = a.Z;
-  const int nvx = X / V;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ngroups = (Y + R - 1) / R;
-  const bool valid = i < ngroups * nvx;
-  const int g = valid ? i / nvx : 0;
-  const int y0 = g * R;  // RESTRICT: Y is even, so both rows are inside
-  const int x0 = valid ? (i - g * nvx) * V : 0;
+  int y, x0;
+  const bool valid = thread_row<MODE, V>(X, Y, y, x0);
   const int64_t ib = inst * a.stride, ic = inst * a.corr_stride;
   const int64_t plane = (int64_t)Y * X;
   const int z0 = blockIdx.y * a.zc;
   const int z1 = min(Z, z0 + a.zc);
   const float *K = a.op.k;
 
-  // s[a][r] of plane p = sum_{b,c} K[a][b][c] phi'(p, y0+r+b-1, x+c-1)
-  auto plane_sums = [&](int p, F4 (&s0)[R], F4 (&s1)[R], F4 (&s2)[R], F4 (&centre)[R]) {
-    F4 rows[R + 2];
-    float ls[R + 2], rs[R + 2];
+  // s_a of plane p = sum_{b,c} K[a][b][c] phi'(p, y+b-1, x+c-1)
+  auto plane_sums = [&](int p, F4 &s0, F4 &s1, F4 &s2, F4 &centre) {
+    F4 rows[3];
+    float ls[3], rs[3];
 #pragma unroll
-    for (int b = 0; b < R + 2; ++b) {
-      const int yy = y0 + b - 1;
+    for (int b = 0; b < 3; ++b) {
+      const int yy = y + b - 1;
       const bool in = valid && p >= 0 && p < Z && yy >= 0 && yy < Y;
       rows[b] = phi_vec<T, CORR, V>(a, ib, ic, p, yy, x0, in);
-      halo_x<T, CORR, V>(a, ib, ic, p, yy, x0, in, rows[b], ls[b], rs[b]);
+      halo_x<T, CORR, V, lane_step(MODE)>(a, ib, ic, p, yy, x0, in, rows[b], ls[b], rs[b]);
     }
+    centre = rows[1];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      centre[r] = rows[r + 1];
+    for (int e = 0; e < V; ++e) {
+      float t0 = 0.f, t1 = 0.f, t2 = 0.f;
 #pragma unroll
-      for (int e = 0; e < V; ++e) {
-        float t0 = 0.f, t1 = 0.f, t2 = 0.f;
-#pragma unroll
-        for (int b = 0; b < 3; ++b) {
-          const float xm = e == 0 ? ls[r + b] : rows[r + b].v[e - 1];
-          const float xc = rows[r + b].v[e];
-          const float xp = e == V - 1 ? rs[r + b] : rows[r + b].v[e + 1];
-          t0 += K[3 * b + 0] * xm + K[3 * b + 1] * xc + K[3 * b + 2] * xp;
-          t1 += K[9 + 3 * b + 0] * xm + K[9 + 3 * b + 1] * xc + K[9 + 3 * b + 2] * xp;
-          t2 += K[18 + 3 * b + 0] * xm + K[18 + 3 * b + 1] * xc + K[18 + 3 * b + 2] * xp;
-        }
-        s0[r].v[e] = t0;
-        s1[r].v[e] = t1;
-        s2[r].v[e] = t2;
+      for (int b = 0; b < 3; ++b) {
+        const float xm = e == 0 ? ls[b] : rows[b].v[e - 1];
+        const float xc = rows[b].v[e];
+        const float xp = e == V - 1 ? rs[b] : rows[b].v[e + 1];
+        t0 += K[3 * b + 0] * xm + K[3 * b + 1] * xc + K[3 * b + 2] * xp;
+        t1 += K[9 + 3 * b + 0] * xm + K[9 + 3 * b + 1] * xc + K[9 + 3 * b + 2] * xp;
+        t2 += K[18 + 3 * b + 0] * xm + K[18 + 3 * b + 1] * xc + K[18 + 3 * b + 2] * xp;
       }
+      s0.v[e] = t0;
+      s1.v[e] = t1;
+      s2.v[e] = t2;
     }
   };
 
   // pending: out(z) = s0(z-1) + s1(z) + s2(z+1)
-  F4 acc_cur[R], acc_next[R], cen_cur[R], cen_next[R];
+  F4 acc_cur, acc_next, cen_cur, cen_next;
   {
-    F4 d0[R], d1[R], d2[R], dc[R], s0[R], s1[R], s2[R];
+    F4 d0, d1, d2, dc, s1;
     plane_sums(z0 - 1, d0, d1, d2, dc);
-    plane_sums(z0, s0, s1, s2, cen_cur);
+    plane_sums(z0, acc_next, s1, d2, cen_cur);
 #pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-      for (int e = 0; e < V; ++e) {
-        acc_cur[r].v[e] = d0[r].v[e] + s1[r].v[e];
-        acc_next[r].v[e] = s0[r].v[e];
-      }
+    for (int e = 0; e < V; ++e) acc_cur.v[e] = d0.v[e] + s1.v[e];
   }
   const float diag = K[13];
   double acc2 = 0.0;
   float cpart[2] = {0.f, 0.f};  // RESTRICT: the two coarse cells of this vector, summed over planes
   for (int z = z0; z < z1; ++z) {
-    F4 n0[R], n1[R], n2[R], res[R];
+    const int64_t off = (int64_t)z * plane + (int64_t)y * X + x0;
+    F4 f = filled<V>(0.f);
+    if (a.rhs && valid) f = ldv<T, V>(a.rhs + ib + off);
+    F4 n0, n1, n2, res;
     plane_sums(z + 1, n0, n1, n2, cen_next);
+    F4 Ax;
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int y = y0 + r;
-      const bool in = valid && y < Y;
-      F4 Ax;
+    for (int e = 0; e < V; ++e) Ax.v[e] = acc_cur.v[e] + n2.v[e];
+    if (MODE == M_SMOOTH) {
 #pragma unroll
-      for (int e = 0; e < V; ++e) Ax.v[e] = acc_cur[r].v[e] + n2[r].v[e];
-      const int64_t off = (int64_t)z * plane + (int64_t)y * X + x0;
-      F4 f = filled<V>(0.f);
-      if (a.rhs && in) f = ldv<T, V>(a.rhs + ib + off);
-      if (MODE == M_SMOOTH) {
+      for (int e = 0; e < V; ++e) res.v[e] = cen_cur.v[e] + a.omega * quotient<V>(f.v[e] - Ax.v[e], diag);
+      if (a.dot_rhs && valid) {
 #pragma unroll
-        for (int e = 0; e < V; ++e) res[r].v[e] = cen_cur[r].v[e] + a.omega * quotient<V>(f.v[e] - Ax.v[e], diag);
-        if (a.dot_rhs && in) {
-#pragma unroll
-          for (int e = 0; e < V; ++e) acc2 += (double)res[r].v[e] * f.v[e];
-        }
-      } else {
-#pragma unroll
-        for (int e = 0; e < V; ++e) res[r].v[e] = Ax.v[e] - f.v[e];
-        if (a.zero_xend_out && x0 + V == X) res[r].v[V - 1] = 0.f;
-        if (in) {
-#pragma unroll
-          for (int e = 0; e < V; ++e)
-            acc2 += (double)res[r].v[e] * (a.dot_phi ? cen_cur[r].v[e] : res[r].v[e]);
-        }
+        for (int e = 0; e < V; ++e) acc2 += (double)res.v[e] * f.v[e];
       }
-      if (in && a.out) {
-        if (MODE == M_SMOOTH && a.top_copy && z == 1) stv<T, V>(a.out + ib + y * X + x0, res[r]);
-        if (!(MODE == M_SMOOTH && a.top_copy && z == 0 && Z > 1)) stv<T, V>(a.out + ib + off, res[r]);
-      }
+    } else {
 #pragma unroll
-      for (int e = 0; e < V; ++e) {
-        acc_cur[r].v[e] = acc_next[r].v[e] + n1[r].v[e];
-        acc_next[r].v[e] = n0[r].v[e];
+      for (int e = 0; e < V; ++e) res.v[e] = Ax.v[e] - f.v[e];
+      if (a.zero_xend_out && x0 + V == X) res.v[V - 1] = 0.f;
+      if (valid) {
+#pragma unroll
+        for (int e = 0; e < V; ++e) acc2 += (double)res.v[e] * (a.dot_phi ? cen_cur.v[e] : res.v[e]);
       }
-      cen_cur[r] = cen_next[r];
     }
-    if (MODE == M_RESTRICT) coarse_cells<T, R, V>(a, inst, z, g, x0, valid, res, cpart);
+    if (valid && a.out) {
+      if (MODE == M_SMOOTH && a.top_copy && z == 1) stv<T, V>(a.out + ib + y * X + x0, res);
+      if (!(MODE == M_SMOOTH && a.top_copy && z == 0 && Z > 1)) stv<T, V>(a.out + ib + off, res);
+    }
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      acc_cur.v[e] = acc_next.v[e] + n1.v[e];
+      acc_next.v[e] = n0.v[e];
+    }
+    cen_cur = cen_next;
+    if (MODE == M_RESTRICT) coarse_cells<T, V>(a, inst, z, y, x0, valid, res, cpart);
   }
   if ((MODE != M_SMOOTH || a.dot_rhs) && a.partials) {
     double t = block_reduce(acc2);
@@ -692,9 +711,8 @@ int resident_blocks(const void *kernel) {
 // chunks and 3.2 us with one-plane chunks.  Chunks of fewer than 4 planes are taken only while
 // the whole launch is resident, which also bounds the partial sums per instance.
 template <class T>
-dim3 fast_grid(FastArgs<T> &a, int B, int rows, int V, bool even_chunks, int per_sm) {
-  const int nvx = a.X / V;
-  const int64_t vecs = (int64_t)((a.Y + rows - 1) / rows) * nvx;
+dim3 fast_grid(FastArgs<T> &a, int B, int V, bool even_chunks, int per_sm) {
+  const int64_t vecs = (int64_t)a.Y * (a.X / V);
   const int tiles = (int)((vecs + kFastThreads - 1) / kFastThreads);
   const int64_t target = (int64_t)sm_count() * per_sm;
   int64_t chunks = std::max<int64_t>(1, target / ((int64_t)tiles * B));
@@ -740,29 +758,29 @@ int fast_width(int kind, const DevOp &op, const PhiSrc<T> &phi, const T *rhs, co
 
 template <class T, int V, int KIND>
 int fast_go(int mode, int corr, FastArgs<T> &a, int B, int *nblk_out, cudaStream_t s) {
-#define HFM_FAST_GO(KER, ROWS)                                                                 \
+#define HFM_FAST_GO(KER)                                                                       \
   do {                                                                                         \
-    const dim3 grid = fast_grid<T>(a, B, ROWS, V, mode == M_RESTRICT,                          \
+    const dim3 grid = fast_grid<T>(a, B, V, mode == M_RESTRICT,                                \
                                    resident_blocks((const void *)KER));                        \
     if (nblk_out) *nblk_out = grid.x * grid.y;                                                 \
     KER<<<grid, kFastThreads, 0, s>>>(a);                                                      \
   } while (0)
-#define HFM_FAST_K(M, C, R)                                                                    \
+#define HFM_FAST_K(M, C)                                                                       \
   do {                                                                                         \
-    if constexpr (KIND == HFM_OP_K27) HFM_FAST_GO((k_fast27<T, M, C, R, V>), R);               \
-    else if constexpr (V == 1) HFM_FAST_GO((k_column7<KIND, T, M, C>), R);                     \
-    else HFM_FAST_GO((k_fast7<KIND, T, M, C, R, V>), R);                                       \
+    if constexpr (KIND == HFM_OP_K27) HFM_FAST_GO((k_fast27<T, M, C, V>));                     \
+    else if constexpr (V == 1) HFM_FAST_GO((k_column7<KIND, T, M, C>));                        \
+    else HFM_FAST_GO((k_fast7<KIND, T, M, C, V>));                                             \
   } while (0)
   if (mode == M_SMOOTH) {
-    if (corr == C_NONE) HFM_FAST_K(M_SMOOTH, C_NONE, 1);
-    else if (corr == C_COARSE) HFM_FAST_K(M_SMOOTH, C_COARSE, 1);
-    else HFM_FAST_K(M_SMOOTH, C_SAME, 1);
+    if (corr == C_NONE) HFM_FAST_K(M_SMOOTH, C_NONE);
+    else if (corr == C_COARSE) HFM_FAST_K(M_SMOOTH, C_COARSE);
+    else HFM_FAST_K(M_SMOOTH, C_SAME);
   } else {
     if (corr != C_NONE) return fail(HFM_ERR_UNSUPPORTED, "fast path: corrected residual");
     if (mode == M_RESID) {
-      HFM_FAST_K(M_RESID, C_NONE, 1);
+      HFM_FAST_K(M_RESID, C_NONE);
     } else if constexpr (V > 1) {
-      HFM_FAST_K(M_RESTRICT, C_NONE, 2);
+      HFM_FAST_K(M_RESTRICT, C_NONE);
     } else {
       return fail(HFM_ERR_UNSUPPORTED, "fast path: restriction of odd rows");
     }
