@@ -237,6 +237,123 @@ int launch_coarse_jacobi(int kind, const DevOp &op, const T *rhs, int64_t rhs_st
                          int sweeps, const int *active, cudaStream_t s);
 int coarse_smem_limit();  // max cells for launch_coarse_jacobi
 
+// z chunks of a plane-marching launch over B instances, of which an activity mask may leave
+// only some working.  The grid (tiles, chunks, B) is sized for all of them; with a mask its
+// blocks are dealt to the active instances on the device, each of which then gets chunks as
+// short as zc[] says for that many.  (A handle of 64 slots with one 128^3 solve in it had 16
+// blocks marching 128 planes each: 24 us a sweep, 4.9 with this.)  Partial sums are
+// taken per `seg` planes, whatever the chunks, so an instance's sums do not depend on how many
+// others are active.
+struct ZPlan {
+  int chunk;               // planes per block with all instances working
+  int seg;                 // planes per partial sum; chunks are multiples of it where sums are taken
+  int step;                // active counts per entry of zc; 0: no table, always `chunk`
+  unsigned short zc[64];   // planes per block with up to (i + 1) * step active instances
+};
+
+// Fills the table: pick(n, limit) is the chunk length for n instances in at most limit chunks.
+// Without a table (no mask; one instance; more than 256, which a block would take longer to
+// count than it gains) the blocks keep their own instance.
+template <class F> void fill_zplan(ZPlan &p, int Z, int B, bool masked, int seg, F pick) {
+  p.chunk = pick(B, (int64_t)Z);
+  p.step = 0;
+  p.seg = p.chunk;
+  if (!masked || B < 2 || B > 256 || Z > 65535) return;
+  p.seg = seg;
+  p.step = (B + 63) / 64;
+  const int64_t total = (int64_t)((Z + p.chunk - 1) / p.chunk) * B;
+  for (int i = 0; i < 64; ++i) {
+    const int n = (i + 1) * p.step < B ? (i + 1) * p.step : B;
+    p.zc[i] = (unsigned short)(n == B ? p.chunk : pick(n, total / n));
+  }
+}
+
+// How many of the B instances `on` holds for, and which is the rank-th of them.  Called by whole
+// warps, whose lanes look at 32 instances at a time.
+template <class F> __device__ __forceinline__ int count_active(int B, F on) {
+  const int lane = threadIdx.x & 31;
+  int n = 0;
+  for (int b = 0; b < B; b += 32) n += __popc(__ballot_sync(0xffffffffu, b + lane < B && on(b + lane)));
+  return n;
+}
+template <class F> __device__ __forceinline__ int nth_active(int B, int rank, F on) {
+  const int lane = threadIdx.x & 31;
+  for (int b = 0; b < B; b += 32) {
+    const bool v = b + lane < B && on(b + lane);
+    const unsigned m = __ballot_sync(0xffffffffu, v);
+    const int c = __popc(m);
+    if (rank < c) {
+      const bool me = v && __popc(m & ((1u << lane) - 1u)) == rank;
+      return b + __ffs(__ballot_sync(0xffffffffu, me)) - 1;
+    }
+    rank -= c;
+  }
+  return 0;  // rank >= count_active: not called so
+}
+
+// (instance, chunk, planes per chunk) of this block among the active instances; instance -1
+// when it has none.  Not inlined: a launch over one instance does not carry its code.
+static __device__ __noinline__ int3 deal_block(const ZPlan &p, const int *active, int Z) {
+  auto on = [active](int i) { return active[i] != 0; };
+  const int n = count_active(gridDim.z, on);
+  if (n == (int)gridDim.z) return make_int3(blockIdx.z, blockIdx.y, p.chunk);  // without the divisions
+  if (n == 0) return make_int3(-1, 0, 0);
+  const int zc = p.zc[p.step == 1 ? n - 1 : (n - 1) / p.step];
+  const int chunks = (Z + zc - 1) / zc, l = blockIdx.z * gridDim.y + blockIdx.y;
+  const int rank = l / chunks;
+  if (rank >= n) return make_int3(-1, 0, 0);
+  return make_int3(nth_active(gridDim.z, rank, on), l - rank * chunks, zc);
+}
+
+// The instance and planes of this block: false when it has none.  All threads of the block
+// call it (whole warps).
+__device__ __forceinline__ bool block_planes(const ZPlan &p, const int *active, int Z, int64_t &inst,
+                                             int &z0, int &z1) {
+  int3 w = make_int3(blockIdx.z, blockIdx.y, p.chunk);
+  if (active) {
+    if (p.step == 0) {
+      if (!active[w.x]) return false;
+    } else {
+      w = deal_block(p, active, Z);
+      if (w.x < 0) return false;
+    }
+  }
+  inst = w.x;
+  z0 = w.y * w.z;
+  z1 = min(Z, z0 + w.z);
+  return true;
+}
+
+// Partial sums of a block of NW warps that marches planes z0 .. z1 - 1, one per segment of
+// p.seg planes (a chunk is a whole number of segments, so a segment has one block): called by
+// the whole block after plane z = next - 1 with the thread's sum since the last segment; the
+// result is the next call's.  The warps' sums wait in shared memory and are written 16 segments
+// at a time, after a barrier.  (The end of a segment is counted up to, not found by a division:
+// that alone cost the float32 SIGMA7 residual 8 % of its issue slots.)
+template <int NW>
+__device__ __forceinline__ int segment_sum(const ZPlan &p, double *partials, int64_t inst, int Z, int next,
+                                           int z0, int z1, double &acc) {
+  __shared__ double sh[16][NW];
+  const int seg = (next - 1) / p.seg, k = (seg - z0 / p.seg) & 15;
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+  if ((threadIdx.x & 31) == 0) sh[k][threadIdx.x >> 5] = acc;
+  acc = 0.0;
+  if (k == 15 || next == z1) {
+    __syncthreads();
+    if ((int)threadIdx.x <= k) {
+      double t = 0.0;
+      for (int w = 0; w < NW; ++w) t += sh[threadIdx.x][w];
+      partials[(inst * ((Z + p.seg - 1) / p.seg) + seg - k + threadIdx.x) * gridDim.x + blockIdx.x] = t;
+    }
+    if (next != z1) __syncthreads();
+  }
+  return min(next + p.seg, z1);
+}
+// the first segment's end, or none where nothing is summed
+__device__ __forceinline__ int first_segment(const ZPlan &p, bool sums, int z0, int z1) {
+  return sums ? min(z0 + p.seg, z1) : -1;
+}
+
 // Register-queue plane-marching kernels (ops_fast.cu); mode 0 smooth, 1 residual, 2 residual +
 // restriction.  fast_eligible: the extents allow 4 cells per thread; fast_width: cells per
 // thread for a grid and its pointers (4, 2 or 1), 0 where the generic kernels serve.

@@ -207,14 +207,30 @@ __global__ void k_check_outer(const double *__restrict__ partials, int nblk, Slo
 }
 
 // float64 outer residual r = b - A x (sigma / kernel read as float32), partial sums of r^2.
-// Work items of the vector kernels: (slot, chunk) pairs.  A block takes items blockIdx.x,
-// blockIdx.x + gridDim.x, ...; chunk c of a slot covers elements [n c / CH, n (c+1) / CH).
-// Items of inactive slots are skipped, so however few slots are active the whole grid works
-// on them; reductions produce one partial per (slot, chunk), independent of which block
-// handled the item, so the summation order is fixed.
+// Work items of the vector kernels: (slot, chunk) pairs of the active slots, dealt to the blocks
+// in contiguous ranges, so that however few slots are active the whole grid works on them and
+// a block meets one slot or two; chunk c of a slot covers elements [n c / CH, n (c+1) / CH).
+// Reductions produce one partial per (slot, chunk), independent of which block handled the
+// item, so the summation order is fixed.  new_slot: the item is the first of its slot in this
+// block (what a kernel reads or sums per slot is done then, not per item).  More than 256
+// slots are not listed but skipped one by one: counting them would cost more than it saves.
 struct Items {
   int B, CH;
   int64_t n;
+  // chunk bounds: the first `rem` chunks have q + 1 units, the others q; a unit is 4 elements
+  // when n is a multiple of 4, so that the kernels can move 16 bytes of float32 (8 of 16-bit)
+  // per access (v4 loops run i over lo, lo + 4, ... with vector loads)
+  int64_t q;
+  int rem;
+  Items(int slots, int chunks, int64_t elements) : B(slots), CH(chunks), n(elements) {
+    const int64_t units = (n & 3) ? n : n >> 2;
+    q = units / CH;
+    rem = (int)(units % CH);
+  }
+  __device__ __forceinline__ int64_t bound(int ch) const {
+    const int64_t u = q * ch + (ch < rem ? ch : rem);
+    return (n & 3) ? u : 4 * u;
+  }
 };
 
 __device__ __forceinline__ double block_reduce_sum(double v) {
@@ -229,20 +245,41 @@ __device__ __forceinline__ double block_reduce_sum(double v) {
   return t;
 }
 
-// When n is a multiple of 4 the chunk bounds are too, so the kernels below can move 16 bytes of
-// float32 (8 of 16-bit) per access: v4 loops run i over lo, lo + 4, ... with vector loads.
-__host__ __device__ __forceinline__ int64_t item_bound(int64_t n, int ch, int CH) {
-  return (n & 3) ? n * ch / CH : 4 * ((n >> 2) * ch / CH);
-}
+#define HFM_ITEM_RANGE(it, MASK)                                                  \
+  auto on_ = [&](int slot) -> bool { return MASK; };                             \
+  const bool listed_ = (it).B <= 256;                                            \
+  const int slots_ = (it).B == 1 ? (on_(0) ? 1 : 0) : listed_ ? count_active((it).B, on_) : (it).B; \
+  const int per_ = slots_ * (it).CH / (int)gridDim.x, left_ = slots_ * (it).CH - per_ * (int)gridDim.x; \
+  int w_ = per_ * (int)blockIdx.x + min((int)blockIdx.x, left_);                 \
+  const int last_ = w_ + per_ + ((int)blockIdx.x < left_ ? 1 : 0);
+#define HFM_ITEM_SLOT(it, rk) (slots_ == (it).B ? (rk) : nth_active((it).B, rk, on_))
 #define HFM_FOR_ITEMS(it, MASK)                                                   \
-  for (int w_ = blockIdx.x; w_ < (it).B * (it).CH; w_ += gridDim.x) {            \
-    const int slot = w_ / (it).CH, ch = w_ - slot * (it).CH;                     \
-    if (!(MASK)) continue;                                                        \
-    const int64_t lo = item_bound((it).n, ch, (it).CH), hi = item_bound((it).n, ch + 1, (it).CH); \
+  HFM_ITEM_RANGE(it, MASK)                                                        \
+  int rank_ = -1, slot = 0;                                                      \
+  for (; w_ < last_; ++w_) {                                                     \
+    const int rk_ = w_ / (it).CH, ch = w_ - rk_ * (it).CH;                       \
+    const bool new_slot = rk_ != rank_;                                          \
+    rank_ = rk_;                                                                 \
+    if (new_slot) slot = HFM_ITEM_SLOT(it, rk_);                                 \
+    if (!listed_ && !on_(slot)) continue;                                        \
+    const int64_t lo = (it).bound(ch), hi = (it).bound(ch + 1);                  \
     const int64_t base = (int64_t)slot * (it).n;                                  \
     const bool v4 = ((it).n & 3) == 0;                                            \
     (void)base;                                                                   \
+    (void)new_slot;                                                               \
     (void)v4;
+// The same where nothing is summed per chunk: a block's consecutive chunks of a slot as one span
+// [lo, hi).
+#define HFM_FOR_SPANS(it, MASK)                                                   \
+  HFM_ITEM_RANGE(it, MASK)                                                        \
+  for (int next_; w_ < last_; w_ = next_) {                                       \
+    const int rk_ = w_ / (it).CH, ch = w_ - rk_ * (it).CH;                       \
+    next_ = min(last_, (rk_ + 1) * (it).CH);                                     \
+    const int slot = HFM_ITEM_SLOT(it, rk_);                                     \
+    if (!listed_ && !on_(slot)) continue;                                        \
+    const int64_t lo = (it).bound(ch), hi = (it).bound(ch + next_ - w_);         \
+    const int64_t base = (int64_t)slot * (it).n;                                  \
+    const bool v4 = ((it).n & 3) == 0;
 #define HFM_END_ITEMS }
 
 // Four consecutive values as float4 / stored from float4 (16-byte float32, 8-byte 16-bit).
@@ -274,7 +311,7 @@ template <class T> __device__ __forceinline__ void st4v(T *p, float4 v) {
 // x64 += x_in for slots whose outer step is due (not before the first inner solve).
 __global__ void k_ir_update(double *__restrict__ x64, const float *__restrict__ xin, Items it,
                             const SlotState *st, const int *outer_mask) {
-  HFM_FOR_ITEMS(it, outer_mask[slot] && !st[slot].first)
+  HFM_FOR_SPANS(it, outer_mask[slot] && !st[slot].first)
   if (v4) {
     for (int64_t i = lo + 4 * threadIdx.x; i < hi; i += 4 * blockDim.x) {
       const float4 v = ld4v<float>(xin + base + i);
@@ -642,8 +679,9 @@ template <class TZ>
 __global__ void k_dot_partials(const float *__restrict__ a, const TZ *__restrict__ b, Items it,
                                double *partials, const int *active, const SlotState *st,
                                int scaled, const double *gscale) {
+  double zs = 1.0;
   HFM_FOR_ITEMS(it, active[slot])
-  const double zs = st ? pc_out(st[slot], it.n, scaled, gscale, slot) : 1.0;
+  if (new_slot && st) zs = pc_out(st[slot], it.n, scaled, gscale, slot);
   double acc = 0.0;
   if (v4) {
     for (int64_t i = lo + 4 * threadIdx.x; i < hi; i += 4 * blockDim.x) {
@@ -680,14 +718,14 @@ __device__ double slot_sum(const double *__restrict__ p, int nblk) {
 }
 
 // p = z + beta p (beta = rz_new / rz; first iteration p = z).  rz_new = r . z is summed here
-// from the slot's nblk_rz partials (every item of the slot sums them in the same order) and
+// from the slot's nblk_rz partials (every block of the slot sums them in the same order) and
 // stored in rz_new[slot] by the slot's first chunk; the check at the end of the iteration
 // makes it the current rz.
 template <class TZ>
 __global__ void k_cg_p(const TZ *__restrict__ z, float *__restrict__ p, Items it, SlotState *st,
                        const double *__restrict__ rz_part, int nblk_rz, double *rz_new,
                        const int *active, int scaled, const double *gscale) {
-  HFM_FOR_ITEMS(it, active[slot])
+  HFM_FOR_SPANS(it, active[slot])
   const double rzn = slot_sum(rz_part + (int64_t)slot * nblk_rz, nblk_rz);
   if (ch == 0 && threadIdx.x == 0) rz_new[slot] = rzn;
   const SlotState s = st[slot];
@@ -744,22 +782,44 @@ __global__ void k_cg_xr(float *__restrict__ x, float *__restrict__ r, const floa
                         const double *__restrict__ pq_part, int nblk_pq,
                         const double *__restrict__ rz_new, double *partials, const int *active,
                         const SlotState *st, int fresh) {
+  float alpha = 0.f;
+  bool zx = false;
   HFM_FOR_ITEMS(it, active[slot])
-  const double pq = slot_sum(pq_part + (int64_t)slot * nblk_pq, nblk_pq);
-  const float alpha = (pq != 0.0) ? (float)(rz_new[slot] / pq) : 0.f;
-  const bool zx = fresh && st[slot].inner_cycles == 0;
+  if (new_slot) {
+    const double pq = slot_sum(pq_part + (int64_t)slot * nblk_pq, nblk_pq);
+    alpha = (pq != 0.0) ? (float)(rz_new[slot] / pq) : 0.f;
+    zx = fresh && st[slot].inner_cycles == 0;
+  }
   double acc = 0.0;
   if (v4) {
-    for (int64_t i = lo + 4 * threadIdx.x; i < hi; i += 4 * blockDim.x) {
-      const int64_t k = base + i;
-      float4 xv = zx ? make_float4(0.f, 0.f, 0.f, 0.f) : ld4v<float>(x + k), rv = ld4v<float>(r + k);
-      const float4 pv = ld4v<float>(p + k), qv = ld4v<float>(q + k);
-      xv.x += alpha * pv.x; xv.y += alpha * pv.y; xv.z += alpha * pv.z; xv.w += alpha * pv.w;
-      rv.x -= alpha * qv.x; rv.y -= alpha * qv.y; rv.z -= alpha * qv.z; rv.w -= alpha * qv.w;
-      st4v<float>(x + k, xv);
-      st4v<float>(r + k, rv);
-      if (rstore) st4v<T>(rstore + k, rv);
-      acc += (double)rv.x * rv.x + (double)rv.y * rv.y + (double)rv.z * rv.z + (double)rv.w * rv.w;
+    // two 4-element groups at a time, as in k_cg_p
+    const int64_t step = 4 * (int64_t)blockDim.x;
+    for (int64_t i = lo + 4 * threadIdx.x; i < hi; i += 2 * step) {
+      const int64_t k0 = base + i;
+      const bool two = i + step < hi;
+      float4 xv[2], rv[2], pv[2], qv[2];
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        xv[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (g == 1 && !two) break;
+        const int64_t k = k0 + g * step;
+        if (!zx) xv[g] = ld4v<float>(x + k);
+        rv[g] = ld4v<float>(r + k);
+        pv[g] = ld4v<float>(p + k);
+        qv[g] = ld4v<float>(q + k);
+      }
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        if (g == 1 && !two) break;
+        const int64_t k = k0 + g * step;
+        xv[g].x += alpha * pv[g].x; xv[g].y += alpha * pv[g].y; xv[g].z += alpha * pv[g].z; xv[g].w += alpha * pv[g].w;
+        rv[g].x -= alpha * qv[g].x; rv[g].y -= alpha * qv[g].y; rv[g].z -= alpha * qv[g].z; rv[g].w -= alpha * qv[g].w;
+        st4v<float>(x + k, xv[g]);
+        st4v<float>(r + k, rv[g]);
+        if (rstore) st4v<T>(rstore + k, rv[g]);
+        acc += (double)rv[g].x * rv[g].x + (double)rv[g].y * rv[g].y + (double)rv[g].z * rv[g].z +
+               (double)rv[g].w * rv[g].w;
+      }
     }
   } else {
     for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
@@ -786,7 +846,7 @@ __global__ void k_negate(float *__restrict__ v, int64_t n) {
 template <class T>
 __global__ void k_to_storage(const float *__restrict__ a, T *__restrict__ b, Items it,
                              const int *active, const SlotState *st, int scaled) {
-  HFM_FOR_ITEMS(it, active[slot])
+  HFM_FOR_SPANS(it, active[slot])
   const float inv = 1.f / pc_in(st[slot], it.n, scaled);
   if (v4) {
     for (int64_t i = lo + 4 * threadIdx.x; i < hi; i += 4 * blockDim.x) {
@@ -800,13 +860,15 @@ __global__ void k_to_storage(const float *__restrict__ a, T *__restrict__ b, Ite
   HFM_END_ITEMS
 }
 
-// Chunks per slot for the vector kernels and their grid: about 4096 elements each, and down to
-// 1024 (one 16-byte access per thread) while all slots together make fewer than two chunks
+// Chunks per slot for the vector kernels and their grid: about 2048 elements each (one active
+// 128^3 slot then makes 1024 items for the 1184 blocks; with chunks of 4096, each of which
+// summed the slot's partials anew, k_cg_xr took 19.4 us there, now 12.1), and down to 1024 (one
+// 16-byte access per thread) while all slots together make fewer than two chunks
 // per SM - one 64^3 slot is 64 chunks of 4096, which left more than half of the SMs idle
 // (k_cg_xr 4.4 -> 3.6 us, k_cg_p, whose chunks were four times longer, 6.7 -> 3.5 us).
 int item_chunks(int64_t n, int B) {
   const int64_t fill = (2 * (int64_t)sm_count() + B - 1) / B;
-  const int64_t c = std::max((n + 4095) / 4096, std::min((n + 1023) / 1024, fill));
+  const int64_t c = std::max((n + 2047) / 2048, std::min((n + 1023) / 1024, fill));
   return (int)std::max<int64_t>(1, std::min<int64_t>(c, 4096));
 }
 int item_blocks(int B, int CH) {
@@ -1388,7 +1450,7 @@ class Engine : public EngineBase {
   int outer_step(cudaStream_t s) {
     const int B = m_->slots;
     const int64_t nf = n(0);
-    const Items it{B, item_chunks(nf, B), nf};
+    const Items it(B, item_chunks(nf, B), nf);
     const int vb = it.CH, ib = item_blocks(B, it.CH);
     k_ir_update<<<ib, 256, 0, s>>>(m_->x64, m_->cg[0], it, m_->state, m_->outer);
     HFM_CHECK_LAUNCH("k_ir_update");
@@ -1424,7 +1486,7 @@ class Engine : public EngineBase {
     const int B = m_->slots;
     const int64_t nf = n(0);
     float *x = m_->cg[0], *r = m_->cg[1], *p = m_->cg[2], *q = m_->cg[3];
-    const Items it{B, item_chunks(nf, B), nf};
+    const Items it(B, item_chunks(nf, B), nf);
     const int vb = it.CH, ib = item_blocks(B, it.CH);
     const int scaled = std::is_same<T, __half>::value ? 2 : 0;
     int st;
@@ -1452,13 +1514,8 @@ class Engine : public EngineBase {
       HFM_CHECK_LAUNCH("k_dot_partials");
       nblk_rz = vb;
     }
-    // k_cg_p writes no per-chunk partials, so it takes chunks four times longer where those
-    // still fill the GPU: every chunk re-sums the slot's r . z partials (three block barriers),
-    // which at 4096 elements held it near 0.7 of the copy bandwidth
-    const bool fills = (int64_t)B * (it.CH / 4) >= 2 * (int64_t)sm_count();
-    const Items itp{B, fills ? it.CH / 4 : it.CH, nf};
-    k_cg_p<T><<<item_blocks(B, itp.CH), 256, 0, s>>>(z, p, itp, m_->state, rz_part, nblk_rz,
-                                                     m_->scal, m_->active, scaled, m_->gscale);
+    k_cg_p<T><<<ib, 256, 0, s>>>(z, p, it, m_->state, rz_part, nblk_rz, m_->scal, m_->active, scaled,
+                                 m_->gscale);
     HFM_CHECK_LAUNCH("k_cg_p");
     // q = A p with the partial sums of p . q in the same pass (float32 operator on the fine
     // level), into a partials buffer of their own

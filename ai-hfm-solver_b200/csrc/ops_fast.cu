@@ -95,13 +95,14 @@ template <class T> struct FastArgs {
   double *partials;   // [inst][blocks] squared-residual partial sums (nullable)
   const int *active;
   int64_t stride, corr_stride, coarse_stride;
-  int Z, Y, X, zc;    // extents, planes per z-chunk
+  int Z, Y, X;
   float omega, corr_sign;
   int zero_xend;      // input: phi' = 0 on x = X-1 (NS correction before the sweep)
   int zero_xend_out;  // output: residual = 0 on x = X-1 (NS residual)
   int top_copy;
   int dot_phi;        // partials of res * phi instead of res^2 (RESID)
   int dot_rhs;        // partials of out * rhs (SMOOTH)
+  ZPlan zp;           // planes of a block (last: its table would lie between the scalars)
 };
 
 template <class T, int CORR>
@@ -169,17 +170,6 @@ __device__ __forceinline__ void coef_halo_x(const T *s, int64_t base_off, int x0
   }
 }
 
-__device__ __forceinline__ double block_reduce(double v) {
-  __shared__ double sh[kFastThreads / 32];
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double t = 0.0;
-  if (threadIdx.x == 0)
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sh[w];
-  return t;
-}
-
 // The (y, x0) of a thread: consecutive lanes hold consecutive vectors of a row; in RESTRICT a
 // lane pair holds the two rows of a coarse row at one x0, so that neither a second row per
 // thread (123 registers, half the warps) nor shared memory is needed to average them: one
@@ -230,19 +220,18 @@ __device__ __forceinline__ void coarse_cells(const FastArgs<T> &a, int64_t inst,
 // ---------------------------------------------------------------------------------------
 template <int KIND, class T, int MODE, int CORR, int V>
 __global__ void __launch_bounds__(kFastThreads, MODE == M_RESTRICT ? 2 : 4)
-    k_fast7(FastArgs<T> a) {
+    k_fast7(const __grid_constant__ FastArgs<T> a) {
   using F4 = FV<V>;  // a thread's cells of a row
   constexpr int LS = lane_step(MODE);
   constexpr int NP = MODE == M_RESTRICT ? 2 : 1;  // planes whose loads are in flight together
-  const int64_t inst = blockIdx.z;
-  if (a.active && !a.active[inst]) return;
+  int64_t inst;
+  int z0, z1;
+  if (!block_planes(a.zp, a.active, a.Z, inst, z0, z1)) return;
   const int X = a.X, Y = a.Y, Z = a.Z;
   int y, x0;
   const bool valid = thread_row<MODE, V>(X, Y, y, x0);
   const int64_t ib = inst * a.stride, ic = inst * a.corr_stride;
   const int64_t plane = (int64_t)Y * X;
-  const int z0 = blockIdx.y * a.zc;
-  const int z1 = min(Z, z0 + a.zc);
 
   // coefficient setup
   float kx = 0.f, ky = 0.f, kz = 0.f, dconst = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
@@ -268,15 +257,40 @@ __global__ void __launch_bounds__(kFastThreads, MODE == M_RESTRICT ? 2 : 4)
     }
   }
 
+  // offsets of (z, y, x0) that advance by a plane, so that a load costs one addition, not the
+  // 64-bit products of its coordinates
+  const T *phi = a.base + ib, *cor = a.corr + ic, *rhs = a.rhs + ib;  // read only where not null
+  int64_t o = (int64_t)z0 * plane + (int64_t)y * X + x0;
+  int64_t ox = ((int64_t)z0 * Y + y) * (X + 8) + x0, oy = ((int64_t)z0 * (Y + 1) + y) * X + x0;  // FACE7
+  const int Xc = X >> 1;
+  const int64_t plane_c = (int64_t)(Y >> 1) * Xc;
+  // phi' of row y + dy of plane zz, at offset oo
+  auto phi_at = [&](int64_t oo, int zz, int dy, bool in) {
+    F4 v = filled<V>(0.f);
+    if (!in) return v;
+    if (a.base) v = ldv<T, V>(phi + oo);
+    if (CORR == C_COARSE) {
+      constexpr int H = V > 1 ? V / 2 : 1;
+      const FV<H> c = ldv<T, H>(cor + (zz >> 1) * plane_c + ((y + dy) >> 1) * Xc + (x0 >> 1));
+#pragma unroll
+      for (int e = 0; e < V; ++e) v.v[e] += a.corr_sign * c.v[e >> 1];
+    } else if (CORR == C_SAME) {
+      const FV<V> c = ldv<T, V>(cor + oo);
+#pragma unroll
+      for (int e = 0; e < V; ++e) v.v[e] += a.corr_sign * c.v[e];
+    }
+    if (a.zero_xend && x0 + V == X) v.v[V - 1] = 0.f;
+    return v;
+  };
+
   // z queue: phi' at z-1, z, z+1; for SIGMA7 also sigma_z at z, and the z- face
   F4 pm, pc, szc, azlo;
-  pm = (z0 > 0) ? phi_vec<T, CORR, V>(a, ib, ic, z0 - 1, y, x0, valid) : filled<V>(0.f);
-  pc = phi_vec<T, CORR, V>(a, ib, ic, z0, y, x0, valid);
-  const int64_t off0 = (int64_t)z0 * plane + (int64_t)y * X + x0;
+  pm = phi_at(o - plane, z0 - 1, 0, valid && z0 > 0);
+  pc = phi_at(o, z0, 0, valid);
   if (KIND == HFM_OP_SIGMA7) {
-    szc = valid ? ldv<T, V>(sz + off0) : filled<V>(1.f);
+    szc = valid ? ldv<T, V>(sz + o) : filled<V>(1.f);
     if (z0 > 0 && valid) {
-      F4 sm = ldv<T, V>(sz + off0 - plane);
+      F4 sm = ldv<T, V>(sz + o - plane);
 #pragma unroll
       for (int e = 0; e < V; ++e) azlo.v[e] = cz * 0.5f * (szc.v[e] + sm.v[e]);
     } else {
@@ -286,11 +300,12 @@ __global__ void __launch_bounds__(kFastThreads, MODE == M_RESTRICT ? 2 : 4)
   } else if (KIND == HFM_OP_FACE7) {
     // the z face below plane z0 (wall faces included in the array), times the scale
     const float s = a.op.scale;
-    const F4 fz = valid ? ldv<T, V>(sz + off0) : filled<V>(0.f);
+    const F4 fz = valid ? ldv<T, V>(sz + o) : filled<V>(0.f);
 #pragma unroll
     for (int e = 0; e < V; ++e) azlo.v[e] = s * fz.v[e];
   }
   double acc = 0.0;
+  int seg_end = first_segment(a.zp, (MODE != M_SMOOTH || a.dot_rhs) && a.partials, z0, z1);
   float cpart[2] = {0.f, 0.f};  // RESTRICT: the two coarse cells of this vector, summed over planes
 
   for (int zb = z0; zb < z1; zb += NP) {
@@ -299,51 +314,55 @@ __global__ void __launch_bounds__(kFastThreads, MODE == M_RESTRICT ? 2 : 4)
     F4 pp[NP], pyo[NP], f[NP], c0[NP], c1[NP], c2[NP], c3[NP], c4[NP];
     F4 pym, pyp;
     float fx4[NP], pl, pr;
+    const int64_t ob = o;
 #pragma unroll
     for (int n = 0; n < NP; ++n) {
       const int z = zb + n;
-      const int64_t off = (int64_t)z * plane + (int64_t)y * X + x0;
-      pp[n] = (z + 1 < Z) ? phi_vec<T, CORR, V>(a, ib, ic, z + 1, y, x0, valid) : filled<V>(0.f);
+      pp[n] = phi_at(o + plane, z + 1, 0, valid && z + 1 < Z);
       if (MODE == M_RESTRICT) {
-        const int yo = (y & 1) ? y + 1 : y - 1;
-        pyo[n] = phi_vec<T, CORR, V>(a, ib, ic, z, yo, x0, valid && yo >= 0 && yo < Y);
+        const int dy = (y & 1) ? 1 : -1;
+        pyo[n] = phi_at(o + dy * X, z, dy, valid && y + dy >= 0 && y + dy < Y);
       } else {
         halo_x<T, CORR, V, LS>(a, ib, ic, z, y, x0, valid, pc, pl, pr);
-        pym = phi_vec<T, CORR, V>(a, ib, ic, z, y - 1, x0, valid && y > 0);
-        pyp = phi_vec<T, CORR, V>(a, ib, ic, z, y + 1, x0, valid && y + 1 < Y);
+        pym = phi_at(o - X, z, -1, valid && y > 0);
+        pyp = phi_at(o + X, z, 1, valid && y + 1 < Y);
       }
       if (KIND == HFM_OP_FACE7) {
         // stored faces (scale applied later): the x faces of the V cells and the one right of
         // the last, the y faces below and above, the z face above (the one below is carried)
-        const int64_t rx = ((int64_t)z * Y + y) * (X + 8) + x0;
-        const int64_t ry = ((int64_t)z * (Y + 1) + y) * X + x0;
-        const F4 zero4 = filled<V>(0.f);
-        c0[n] = valid ? ldv<T, V>(sx + rx) : zero4;
-        fx4[n] = valid ? St<T>::ld(sx + rx + V) : 0.f;
-        c1[n] = valid ? ldv<T, V>(sy + ry) : zero4;
-        c2[n] = valid ? ldv<T, V>(sy + ry + X) : zero4;
-        c3[n] = valid ? ldv<T, V>(sz + off + plane) : zero4;
+        c0[n] = c1[n] = c2[n] = c3[n] = filled<V>(0.f);
+        fx4[n] = 0.f;
+        if (valid) {
+          c0[n] = ldv<T, V>(sx + ox);
+          fx4[n] = St<T>::ld(sx + ox + V);
+          c1[n] = ldv<T, V>(sy + oy);
+          c2[n] = ldv<T, V>(sy + oy + X);
+          c3[n] = ldv<T, V>(sz + o + plane);
+        }
+        ox += (int64_t)Y * (X + 8);
+        oy += plane + X;
       } else if (KIND == HFM_OP_SIGMA7) {
-        c0[n] = valid ? ldv<T, V>(sx + off) : filled<V>(1.f);
-        c1[n] = valid ? ldv<T, V>(sy + off) : filled<V>(1.f);
-        c2[n] = (valid && y > 0) ? ldv<T, V>(sy + off - X) : c1[n];
-        c3[n] = (valid && y + 1 < Y) ? ldv<T, V>(sy + off + X) : c1[n];
-        if (z + 1 < Z && valid) c4[n] = ldv<T, V>(sz + off + plane);
+        c0[n] = valid ? ldv<T, V>(sx + o) : filled<V>(1.f);
+        c1[n] = valid ? ldv<T, V>(sy + o) : filled<V>(1.f);
+        c2[n] = (valid && y > 0) ? ldv<T, V>(sy + o - X) : c1[n];
+        c3[n] = (valid && y + 1 < Y) ? ldv<T, V>(sy + o + X) : c1[n];
+        if (z + 1 < Z && valid) c4[n] = ldv<T, V>(sz + o + plane);
         else c4[n] = n ? c4[0] : szc;
       }
-      if (MODE == M_RESTRICT) f[n] = a.rhs && valid ? ldv<T, V>(a.rhs + ib + off) : filled<V>(0.f);
+      if (MODE == M_RESTRICT) f[n] = a.rhs && valid ? ldv<T, V>(rhs + o) : filled<V>(0.f);
+      o += plane;
     }
 #pragma unroll
     for (int n = 0; n < NP; ++n) {
       const int z = zb + n;
-      const int64_t off = (int64_t)z * plane + (int64_t)y * X + x0;
+      const int64_t off = ob + n * plane;
       if (MODE == M_RESTRICT) {
         halo_x<T, CORR, V, LS>(a, ib, ic, z, y, x0, valid, pc, pl, pr);
 #pragma unroll
         for (int e = 0; e < V; ++e) {
-          const float o = __shfl_xor_sync(0xffffffffu, pc.v[e], 1);
-          pym.v[e] = (y & 1) ? o : pyo[n].v[e];
-          pyp.v[e] = (y & 1) ? pyo[n].v[e] : o;
+          const float sh = __shfl_xor_sync(0xffffffffu, pc.v[e], 1);
+          pym.v[e] = (y & 1) ? sh : pyo[n].v[e];
+          pyp.v[e] = (y & 1) ? pyo[n].v[e] : sh;
         }
       }
       F4 Ax, dg, res;
@@ -397,7 +416,7 @@ __global__ void __launch_bounds__(kFastThreads, MODE == M_RESTRICT ? 2 : 4)
         azlo = azhi;
         szc = c4[n];
       }
-      if (MODE != M_RESTRICT) f[n] = a.rhs && valid ? ldv<T, V>(a.rhs + ib + off) : filled<V>(0.f);
+      if (MODE != M_RESTRICT) f[n] = a.rhs && valid ? ldv<T, V>(rhs + off) : filled<V>(0.f);
       if (MODE == M_SMOOTH) {
 #pragma unroll
         for (int e = 0; e < V; ++e) res.v[e] = pc.v[e] + a.omega * quotient<V>(f[n].v[e] - Ax.v[e], dg.v[e]);
@@ -421,11 +440,8 @@ __global__ void __launch_bounds__(kFastThreads, MODE == M_RESTRICT ? 2 : 4)
       pm = pc;
       pc = pp[n];
       if (MODE == M_RESTRICT) coarse_cells<T, V>(a, inst, z, y, x0, valid, res, cpart);
+      if (z + 1 == seg_end) seg_end = segment_sum<kFastThreads / 32>(a.zp, a.partials, inst, Z, seg_end, z0, z1, acc);
     }
-  }
-  if ((MODE != M_SMOOTH || a.dot_rhs) && a.partials) {
-    double t = block_reduce(acc);
-    if (threadIdx.x == 0) a.partials[inst * (gridDim.x * gridDim.y) + blockIdx.y * gridDim.x + blockIdx.x] = t;
   }
 }
 
@@ -440,9 +456,10 @@ __global__ void __launch_bounds__(kFastThreads, MODE == M_RESTRICT ? 2 : 4)
 // is k_fast7's.
 // ---------------------------------------------------------------------------------------
 template <int KIND, class T, int MODE, int CORR>
-__global__ void __launch_bounds__(kFastThreads, 4) k_column7(FastArgs<T> a) {
-  const int64_t inst = blockIdx.z;
-  if (a.active && !a.active[inst]) return;
+__global__ void __launch_bounds__(kFastThreads, 4) k_column7(const __grid_constant__ FastArgs<T> a) {
+  int64_t inst;
+  int z0, z1;
+  if (!block_planes(a.zp, a.active, a.Z, inst, z0, z1)) return;
   constexpr bool SIG = KIND == HFM_OP_SIGMA7;
   constexpr unsigned ES = sizeof(T);
   const int X = a.X, Y = a.Y, Z = a.Z;
@@ -450,7 +467,6 @@ __global__ void __launch_bounds__(kFastThreads, 4) k_column7(FastArgs<T> a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = i < X * Y;
   const int y = valid ? i / X : 0, x = valid ? i - y * X : 0;
-  const int z0 = blockIdx.y * a.zc, z1 = min(Z, z0 + a.zc);
   const T *phi = a.base + inst * a.stride;  // not read when base is null
   const T *cor = a.corr + inst * a.corr_stride;
   const T *rhs = a.rhs + inst * a.stride;
@@ -525,6 +541,7 @@ __global__ void __launch_bounds__(kFastThreads, 4) k_column7(FastArgs<T> a) {
     azlo = z0 > 0 ? cz * 0.5f * (szc + ld(sz, o - plane)) : cz * szc;
   }
   const bool sums = a.partials && (MODE != M_SMOOTH || a.dot_rhs);
+  int seg_end = first_segment(a.zp, sums, z0, z1);
   double acc = 0.0;
   for (int z = z0; z < z1; ++z) {
     const Plane q = nx;
@@ -574,10 +591,7 @@ __global__ void __launch_bounds__(kFastThreads, 4) k_column7(FastArgs<T> a) {
     }
     pm = pc;
     pc = q.pp;
-  }
-  if (sums) {
-    double t = block_reduce(acc);
-    if (threadIdx.x == 0) a.partials[inst * (gridDim.x * gridDim.y) + blockIdx.y * gridDim.x + blockIdx.x] = t;
+    if (z + 1 == seg_end) seg_end = segment_sum<kFastThreads / 32>(a.zp, a.partials, inst, Z, seg_end, z0, z1, acc);
   }
 }
 
@@ -589,17 +603,16 @@ __global__ void __launch_bounds__(kFastThreads, 4) k_column7(FastArgs<T> a) {
 // ---------------------------------------------------------------------------------------
 template <class T, int MODE, int CORR, int V>
 __global__ void __launch_bounds__(kFastThreads)
-    k_fast27(FastArgs<T> a) {
+    k_fast27(const __grid_constant__ FastArgs<T> a) {
   using F4 = FV<V>;  // a thread's cells of a row
-  const int64_t inst = blockIdx.z;
-  if (a.active && !a.active[inst]) return;
+  int64_t inst;
+  int z0, z1;
+  if (!block_planes(a.zp, a.active, a.Z, inst, z0, z1)) return;
   const int X = a.X, Y = a.Y, Z = a.Z;
   int y, x0;
   const bool valid = thread_row<MODE, V>(X, Y, y, x0);
   const int64_t ib = inst * a.stride, ic = inst * a.corr_stride;
   const int64_t plane = (int64_t)Y * X;
-  const int z0 = blockIdx.y * a.zc;
-  const int z1 = min(Z, z0 + a.zc);
   const float *K = a.op.k;
 
   // s_a of plane p = sum_{b,c} K[a][b][c] phi'(p, y+b-1, x+c-1)
@@ -643,6 +656,7 @@ __global__ void __launch_bounds__(kFastThreads)
   }
   const float diag = K[13];
   double acc2 = 0.0;
+  int seg_end = first_segment(a.zp, (MODE != M_SMOOTH || a.dot_rhs) && a.partials, z0, z1);
   float cpart[2] = {0.f, 0.f};  // RESTRICT: the two coarse cells of this vector, summed over planes
   for (int z = z0; z < z1; ++z) {
     const int64_t off = (int64_t)z * plane + (int64_t)y * X + x0;
@@ -680,10 +694,7 @@ __global__ void __launch_bounds__(kFastThreads)
     }
     cen_cur = cen_next;
     if (MODE == M_RESTRICT) coarse_cells<T, V>(a, inst, z, y, x0, valid, res, cpart);
-  }
-  if ((MODE != M_SMOOTH || a.dot_rhs) && a.partials) {
-    double t = block_reduce(acc2);
-    if (threadIdx.x == 0) a.partials[inst * (gridDim.x * gridDim.y) + blockIdx.y * gridDim.x + blockIdx.x] = t;
+    if (z + 1 == seg_end) seg_end = segment_sum<kFastThreads / 32>(a.zp, a.partials, inst, Z, seg_end, z0, z1, acc2);
   }
 }
 
@@ -711,17 +722,23 @@ int resident_blocks(const void *kernel) {
 // chunks and 3.2 us with one-plane chunks.  Chunks of fewer than 4 planes are taken only while
 // the whole launch is resident, which also bounds the partial sums per instance.
 template <class T>
-dim3 fast_grid(FastArgs<T> &a, int B, int V, bool even_chunks, int per_sm) {
+dim3 fast_grid(FastArgs<T> &a, int B, int V, bool even_chunks, bool sums, int per_sm, int *nblk_out) {
   const int64_t vecs = (int64_t)a.Y * (a.X / V);
   const int tiles = (int)((vecs + kFastThreads - 1) / kFastThreads);
   const int64_t target = (int64_t)sm_count() * per_sm;
-  int64_t chunks = std::max<int64_t>(1, target / ((int64_t)tiles * B));
-  int zc = (int)((a.Z + chunks - 1) / chunks);
-  if (zc < 4 && (int64_t)tiles * B * ((a.Z + zc - 1) / zc) > target) zc = 4;
-  if (even_chunks && (zc & 1)) ++zc;
-  if (zc > a.Z) zc = a.Z;
-  a.zc = zc;
-  return dim3(tiles, (a.Z + zc - 1) / zc, B);
+  // sums per plane on the small grids, where a block that must march 4 is a chain 4 long
+  // (32^3: 8.1 us with a few of 64 instances active, 5.0 per plane), else per 4 planes
+  const int seg = tiles * a.Z <= 64 ? 1 : 4;
+  const int Z = a.Z, step = std::max(sums && a.active && B > 1 ? seg : 1, even_chunks ? 2 : 1);
+  fill_zplan(a.zp, Z, B, a.active != nullptr, seg, [&](int n, int64_t limit) {
+    const int64_t chunks = std::min(std::max<int64_t>(1, target / ((int64_t)tiles * n)), limit);
+    int zc = (int)((Z + chunks - 1) / chunks);
+    if (zc < 4 && (int64_t)tiles * n * ((Z + zc - 1) / zc) > target) zc = 4;
+    zc = (zc + step - 1) / step * step;
+    return zc > Z ? Z : zc;
+  });
+  if (nblk_out) *nblk_out = tiles * ((Z + a.zp.seg - 1) / a.zp.seg);
+  return dim3(tiles, (Z + a.zp.chunk - 1) / a.zp.chunk, B);
 }
 
 }  // namespace
@@ -760,9 +777,9 @@ template <class T, int V, int KIND>
 int fast_go(int mode, int corr, FastArgs<T> &a, int B, int *nblk_out, cudaStream_t s) {
 #define HFM_FAST_GO(KER)                                                                       \
   do {                                                                                         \
-    const dim3 grid = fast_grid<T>(a, B, V, mode == M_RESTRICT,                                \
-                                   resident_blocks((const void *)KER));                        \
-    if (nblk_out) *nblk_out = grid.x * grid.y;                                                 \
+    const bool sums = (mode != M_SMOOTH || a.dot_rhs) && a.partials;                           \
+    const dim3 grid = fast_grid<T>(a, B, V, mode == M_RESTRICT, sums,                          \
+                                   resident_blocks((const void *)KER), nblk_out);              \
     KER<<<grid, kFastThreads, 0, s>>>(a);                                                      \
   } while (0)
 #define HFM_FAST_K(M, C)                                                                       \
@@ -818,7 +835,6 @@ int fast_launch(int kind, int mode, int V, const DevOp &op, const PhiSrc<T> &phi
   a.top_copy = (mode == M_SMOOTH && (flags & HFM_FLAG_TOP_COPY)) ? 1 : 0;
   a.dot_phi = (mode == M_RESID && (flags & HFM_INT_DOT_PHI)) ? 1 : 0;
   a.dot_rhs = (mode == M_SMOOTH && (flags & HFM_INT_DOT_RHS) && partials) ? 1 : 0;
-  a.zc = 0;
   if (phi.base && phi.base_stride != stride) return fail(HFM_ERR_BAD_ARG, "fast path: stride mismatch");
   const int corr = phi.corr ? (phi.corr_coarse ? C_COARSE : C_SAME) : C_NONE;
 #define HFM_FAST_V(KIND)                                                          \

@@ -93,11 +93,12 @@ template <class T> struct TmaArgs {
   double *partials;
   const int *active;
   int64_t stride, coarse_stride;
-  int Z, Y, X, zc, tiles_x;
+  int Z, Y, X, zc, tiles_x;  // zc: k_tma_face2's
   float omega, corr_sign;
   int has_phi, has_f, has_sigma, zero_xend, zero_xend_out, top_copy, dot_phi, dot_rhs;
   unsigned stage_bytes;
   int wait_budget;  // polls of a plane wait before the block gives up (hfm_set_wait_budget)
+  ZPlan zp;         // last: its table would lie between the scalars every launch reads
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -236,12 +237,12 @@ __global__ void __launch_bounds__(Geo<T>::THREADS, Geo<T>::MINB) k_tma(const __g
   constexpr int TY = G::TY, V = G::VEC, NS = G::NS;
   extern __shared__ __align__(128) char smem[];
   __shared__ __align__(8) uint64_t bars[NS];
-  const int64_t inst = blockIdx.z;
-  if (a.active && !a.active[inst]) return;
   const int X = a.X, Y = a.Y, Z = a.Z;
+  int64_t inst;
+  int z0, z1;
+  if (!block_planes(a.zp, a.active, Z, inst, z0, z1)) return;
   const int tx = blockIdx.x % a.tiles_x, ty = blockIdx.x / a.tiles_x;
   const int x0 = tx * TX, y0 = ty * TY;
-  const int z0 = blockIdx.y * a.zc, z1 = min(Z, z0 + a.zc);
   const int tid = threadIdx.x;
   const int r = tid / G::TPR, c = tid % G::TPR;
   const int gx = x0 + V * c, gy = y0 + r;
@@ -347,6 +348,7 @@ __global__ void __launch_bounds__(Geo<T>::THREADS, Geo<T>::MINB) k_tma(const __g
     for (int e = 0; e < V; ++e) azlo[e] = z0 > 0 ? hz * (szc[e] + szm[e]) : cz * szc[e];
   }
   double acc = 0.0;
+  int seg_end = first_segment(a.zp, (MODE != M_SMOOTH || a.dot_rhs) && a.partials, z0, z1);
   float cpart[V / 2];
 #pragma unroll
   for (int e = 0; e < V / 2; ++e) cpart[e] = 0.f;
@@ -516,6 +518,7 @@ __global__ void __launch_bounds__(Geo<T>::THREADS, Geo<T>::MINB) k_tma(const __g
         for (int k = 0; k < V / 2; ++k) cpart[k] = 0.f;
       }
     }
+    if (z + 1 == seg_end) seg_end = segment_sum<G::THREADS / 32>(a.zp, a.partials, inst, Z, seg_end, z0, z1, acc);
   }
   if (ok && __syncthreads_or(!mine)) ok = false;  // the last plane's wait
   if (!ok) {
@@ -527,11 +530,6 @@ __global__ void __launch_bounds__(Geo<T>::THREADS, Geo<T>::MINB) k_tma(const __g
       for (int p = p_waited + 1; p < p_next; ++p) drained = wait_plane(p, kMaxSpin) && drained;
       if (!drained) atomicAdd(&g_tma_wait_fail[1], 1);
     }
-    return;
-  }
-  if ((MODE != M_SMOOTH || a.dot_rhs) && a.partials) {
-    double t = block_sum(acc);
-    if (tid == 0) a.partials[inst * (gridDim.x * gridDim.y) + blockIdx.y * gridDim.x + blockIdx.x] = t;
   }
 }
 
@@ -604,26 +602,32 @@ int tma_resident(const void *kernel, int threads, int smem) {
 // 27-point convolution 12.5 -> 10.9 us), and eight 48^3 instances of the fused first two sweeps
 // fit one round (10.7 -> 7.6 us).
 template <class T>
-dim3 tma_grid(TmaArgs<T> &a, int B, int per_sm) {
+dim3 tma_grid(TmaArgs<T> &a, int B, int per_sm, bool sums, int *nblk_out) {
   constexpr int TY = Geo<T>::TY;
   a.tiles_x = (a.X + TX - 1) / TX;
   const int tiles = a.tiles_x * ((a.Y + TY - 1) / TY);
-  const int64_t per = (int64_t)tiles * B;
   const int64_t cap = (int64_t)sm_count() * per_sm;
-  int zc = a.Z;
-  int64_t best = -1;
-  for (int c = 2; c < a.Z + 2; c += 2) {
-    const int zcc = c > a.Z ? a.Z : c;
-    const int64_t chunks = (a.Z + zcc - 1) / zcc;
-    const int64_t cost = ((per * chunks + cap - 1) / cap) * (zcc + 2);
-    if (best < 0 || cost <= best) {
-      best = cost;
-      zc = zcc;
+  const int Z = a.Z;
+  int seg = 8;  // planes per partial sum: as many as leave one instance a block for half the SMs
+  while (seg > 2 && 2 * tiles * ((Z + seg - 1) / seg) < sm_count()) seg /= 2;
+  const int step = sums && a.active && B > 1 ? seg : 2;
+  fill_zplan(a.zp, Z, B, a.active != nullptr, seg, [&](int n, int64_t limit) {
+    int zc = Z;
+    int64_t best = -1;
+    for (int c = step; c < Z + step; c += step) {
+      const int zcc = c > Z ? Z : c;
+      const int64_t chunks = (Z + zcc - 1) / zcc;
+      if (chunks > limit) continue;
+      const int64_t cost = (((int64_t)tiles * n * chunks + cap - 1) / cap) * (zcc + 2);
+      if (best < 0 || cost <= best) {
+        best = cost;
+        zc = zcc;
+      }
     }
-    if (zcc == a.Z) break;
-  }
-  a.zc = zc;
-  return dim3(tiles, (a.Z + zc - 1) / zc, B);
+    return zc;
+  });
+  if (nblk_out) *nblk_out = tiles * ((Z + a.zp.seg - 1) / a.zp.seg);
+  return dim3(tiles, (Z + a.zp.chunk - 1) / a.zp.chunk, B);
 }
 
 template <int KIND, class T, int MODE, int CORR>
@@ -633,8 +637,8 @@ int go(TmaArgs<T> &a, int B, int *nblk_out, cudaStream_t s) {
   const void *fn = (const void *)k_tma<KIND, T, MODE, CORR>;
   int st = set_max_dynamic_smem(fn, smem, "cudaFuncSetAttribute(k_tma)");
   if (st) return st;
-  const dim3 grid = tma_grid(a, B, tma_resident(fn, G::THREADS, smem));
-  if (nblk_out) *nblk_out = grid.x * grid.y;
+  const dim3 grid = tma_grid(a, B, tma_resident(fn, G::THREADS, smem),
+                             (MODE != M_SMOOTH || a.dot_rhs) && a.partials, nblk_out);
   k_tma<KIND, T, MODE, CORR><<<grid, G::THREADS, smem, s>>>(a);
   HFM_CHECK_LAUNCH("k_tma");
   return HFM_OK;
@@ -647,8 +651,8 @@ int go_face(TmaArgs<T> &a, int B, int *nblk_out, cudaStream_t s) {
   const void *fn = (const void *)k_tma_face<T, MODE, CORR>;
   int st = set_max_dynamic_smem(fn, smem, "cudaFuncSetAttribute(k_tma_face)");
   if (st) return st;
-  const dim3 grid = tma_grid(a, B, tma_resident(fn, G::THREADS, smem));
-  if (nblk_out) *nblk_out = grid.x * grid.y;
+  const dim3 grid = tma_grid(a, B, tma_resident(fn, G::THREADS, smem),
+                             (MODE != M_SMOOTH || a.dot_rhs) && a.partials, nblk_out);
   k_tma_face<T, MODE, CORR><<<grid, G::THREADS, smem, s>>>(a);
   HFM_CHECK_LAUNCH("k_tma_face");
   return HFM_OK;

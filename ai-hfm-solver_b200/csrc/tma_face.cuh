@@ -224,12 +224,12 @@ __global__ void __launch_bounds__(GeoF<false, false>::THREADS, GeoF<false, false
   constexpr int TY = G::TY, V = G::VEC, NS = G::NS;
   extern __shared__ __align__(128) char smem[];
   __shared__ __align__(8) uint64_t bars[NS];
-  const int64_t inst = blockIdx.z;
-  if (a.active && !a.active[inst]) return;
   const int X = a.X, Y = a.Y, Z = a.Z;
+  int64_t inst;
+  int z0, z1;
+  if (!block_planes(a.zp, a.active, Z, inst, z0, z1)) return;
   const int tx = blockIdx.x % a.tiles_x, ty = blockIdx.x / a.tiles_x;
   const int x0 = tx * TX, y0 = ty * TY;
-  const int z0 = blockIdx.y * a.zc, z1 = min(Z, z0 + a.zc);
   const int tid = threadIdx.x;
   const int r = tid / G::TPR, c = tid % G::TPR;
   const int gx = x0 + V * c, gy = y0 + r;
@@ -308,6 +308,7 @@ __global__ void __launch_bounds__(GeoF<false, false>::THREADS, GeoF<false, false
   uint32_t fzl[4] = {0u, 0u, 0u, 0u};
   if (ok) ld8w(stage_of(z0 - 1) + G::O_FZ + (r * TX + V * c) * 2, fzl);
   double acc = 0.0;
+  int seg_end = first_segment(a.zp, (MODE != M_SMOOTH || a.dot_rhs) && !PRE2 && a.partials, z0, z1);
   float cpart[V / 2];
 #pragma unroll
   for (int e = 0; e < V / 2; ++e) cpart[e] = 0.f;
@@ -514,6 +515,7 @@ __global__ void __launch_bounds__(GeoF<false, false>::THREADS, GeoF<false, false
         for (int k = 0; k < V / 2; ++k) cpart[k] = 0.f;
       }
     }
+    if (z + 1 == seg_end) seg_end = segment_sum<G::THREADS / 32>(a.zp, a.partials, inst, Z, seg_end, z0, z1, acc);
   }
   if (ok && __syncthreads_or(!mine)) ok = false;
   if (!ok) {
@@ -523,10 +525,5 @@ __global__ void __launch_bounds__(GeoF<false, false>::THREADS, GeoF<false, false
       for (int p = p_waited + 1; p < p_next; ++p) drained = wait_plane(p, kMaxSpin) && drained;
       if (!drained) atomicAdd(&g_tma_wait_fail[1], 1);
     }
-    return;
-  }
-  if ((MODE != M_SMOOTH || a.dot_rhs) && !PRE2 && a.partials) {
-    double t = block_sum(acc);
-    if (tid == 0) a.partials[inst * (gridDim.x * gridDim.y) + blockIdx.y * gridDim.x + blockIdx.x] = t;
   }
 }

@@ -232,3 +232,43 @@ def test_2d_outer_legs_same_bits(hfm, T, periodic, storage, shape):
     L.call("hfm_jacobi2d", code, w, P(a[1]), P(wc), -1.0, P(a[0]), P(out), 2, Y, X, 0.8, fl | L.FLAG_TWO_SWEEPS, st)
     L.call("hfm_update2d", P(pb), code, P(out), -1.0, 2 * Y * X, st)
     assert T.equal(pa, pb)
+
+
+# the blocks of a many-slot handle are dealt to its active slots: a slot's solve has the same
+# bits alone, in a few and with every slot at work (table of one and of several counts per
+# entry, more slots than are listed; register-queue and plane-marching kernels; planes that
+# are no multiple of a segment)
+@pytest.mark.parametrize("shape,slots,accel,storage", [
+    ((16, 16, 16), 2, "cg", "f32"), ((18, 12, 20), 33, "cg", "f32"), ((8, 8, 8), 70, "cg", "f32"),
+    ((8, 8, 8), 300, "cg", "f32"), ((32, 32, 32), 64, "ir", "bf16"), ((18, 32, 64), 3, "ir", "bf16"),
+    ((36, 16, 48), 40, "ir", "bf16"), ((16, 64, 64), 7, "cg", "f32"), ((20, 16, 72), 65, "none", "f32")])
+def test_active_slots_share_the_grid_same_bits(hfm, T, shape, slots, accel, storage):
+    rng = np.random.default_rng(9)
+    cfg = hfm.multigrid.SolverConfig(cycle="V", accel=accel, storage=storage, tol=1e-6, max_cycles=60,
+                                     inner_tol=1e-3)
+    sig = dev(T, np.exp(0.5 * rng.standard_normal((3,) + shape)))
+    rhs = dev(T, rng.standard_normal((slots,) + shape))
+    with hfm.multigrid.Multigrid(shape, hfm._lib.OP_SIGMA7, cfg, slots=slots) as h:
+        for k in range(slots):
+            h.set_operator(hfm.ops.Sigma7(sig[0], sig[1], sig[2]), slot=k)
+
+        def solve(which):
+            for k in which:
+                h.load(k, rhs[k])
+            for _ in range(40):
+                h.run(4)
+                st = h.query()
+                if not any(st[k]["active"] for k in which):
+                    break
+            return {k: (h.fetch(k).cpu().numpy(), st[k]["status"], st[k]["cycles"], st[k]["rel_resid"])
+                    for k in which}
+
+        probe = sorted({0, slots // 2, slots - 1})
+        every = solve(range(slots))
+        few = solve(probe)
+        for k in probe:
+            alone = solve([k])[k]
+            assert alone[1] == hfm._lib.OK and alone[3] <= 1e-6
+            for other in (few[k], every[k]):
+                np.testing.assert_array_equal(alone[0], other[0])
+                assert alone[1:] == other[1:]
