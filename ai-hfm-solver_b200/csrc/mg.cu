@@ -1460,7 +1460,9 @@ class Engine : public EngineBase {
     switch (kind()) {
       case HFM_OP_SIGMA7:
         if (vec4) {
-          k_residual64_sigma4<T><<<ib, 256, 0, s>>>(d, m_->x64, m_->b64, m_->cg[1], rs, g(0).Z,
+          // two blocks fit an SM (102 registers): with more, a launch that finds no slot due,
+          // as most do, still took four rounds of empty blocks (4.0 us, now 1.7)
+          k_residual64_sigma4<T><<<std::min(ib, 2 * sm_count()), 256, 0, s>>>(d, m_->x64, m_->b64, m_->cg[1], rs, g(0).Z,
                                                     g(0).Y, g(0).X, it, m_->outer, m_->partials);
           break;
         }

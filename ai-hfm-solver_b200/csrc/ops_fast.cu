@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(kFastThreads, MODE == M_RESTRICT ? 2 : 4)
 // is k_fast7's.
 // ---------------------------------------------------------------------------------------
 template <int KIND, class T, int MODE, int CORR>
-__global__ void __launch_bounds__(kFastThreads, 4) k_column7(const __grid_constant__ FastArgs<T> a) {
+__global__ void __launch_bounds__(kFastThreads, 3) k_column7(const __grid_constant__ FastArgs<T> a) {
   int64_t inst;
   int z0, z1;
   if (!block_planes(a.zp, a.active, a.Z, inst, z0, z1)) return;
