@@ -862,7 +862,7 @@ __global__ void k_to_storage(const float *__restrict__ a, T *__restrict__ b, Ite
 
 // Chunks per slot for the vector kernels and their grid: about 2048 elements each (one active
 // 128^3 slot then makes 1024 items for the 1184 blocks; with chunks of 4096, each of which
-// summed the slot's partials anew, k_cg_xr took 19.4 us there, now 12.1), and down to 1024 (one
+// summed the slot's partials anew, k_cg_xr took 19.4 us there, now 9.7), and down to 1024 (one
 // 16-byte access per thread) while all slots together make fewer than two chunks
 // per SM - one 64^3 slot is 64 chunks of 4096, which left more than half of the SMs idle
 // (k_cg_xr 4.4 -> 3.6 us, k_cg_p, whose chunks were four times longer, 6.7 -> 3.5 us).
@@ -875,6 +875,12 @@ int item_blocks(int B, int CH) {
   int64_t want = (int64_t)sm_count() * 8;
   return (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)B * CH));
 }
+
+// Blocks of the kernels that only stream (two vector groups in flight per thread): four per
+// SM are all resident and one range each, where eight made a second round: one of 64 slots of
+// 128^3 active, k_cg_xr 12.1 -> 9.7 us, k_cg_p 8.0 -> 6.0, an update with nothing due
+// 2.7 -> 2.2; all 64, 559 -> 549, 240 -> 237 (three per SM: 538 and 268).
+int stream_blocks(int B, int CH) { return std::min(item_blocks(B, CH), 4 * sm_count()); }
 
 int vec_blocks(int64_t n, int B) {
   int64_t want = (int64_t)sm_count() * 8 / std::max(B, 1);
@@ -1452,7 +1458,7 @@ class Engine : public EngineBase {
     const int64_t nf = n(0);
     const Items it(B, item_chunks(nf, B), nf);
     const int vb = it.CH, ib = item_blocks(B, it.CH);
-    k_ir_update<<<ib, 256, 0, s>>>(m_->x64, m_->cg[0], it, m_->state, m_->outer);
+    k_ir_update<<<stream_blocks(B, it.CH), 256, 0, s>>>(m_->x64, m_->cg[0], it, m_->state, m_->outer);
     HFM_CHECK_LAUNCH("k_ir_update");
     DevOp d = fine32_;
     T *rs = fused_rhs() ? rhs(0) : nullptr;
@@ -1516,7 +1522,7 @@ class Engine : public EngineBase {
       HFM_CHECK_LAUNCH("k_dot_partials");
       nblk_rz = vb;
     }
-    k_cg_p<T><<<ib, 256, 0, s>>>(z, p, it, m_->state, rz_part, nblk_rz, m_->scal, m_->active, scaled,
+    k_cg_p<T><<<stream_blocks(B, it.CH), 256, 0, s>>>(z, p, it, m_->state, rz_part, nblk_rz, m_->scal, m_->active, scaled,
                                  m_->gscale);
     HFM_CHECK_LAUNCH("k_cg_p");
     // q = A p with the partial sums of p . q in the same pass (float32 operator on the fine
@@ -1530,7 +1536,7 @@ class Engine : public EngineBase {
                                      m_->active, m_->partials2, &nblk_pq, s)))
       return st;
     // x += alpha p ; r -= alpha q ; ||r||  (alpha from rz_new and the p . q partials)
-    k_cg_xr<T><<<ib, 256, 0, s>>>(x, r, p, q, fused_rhs() ? rhs(0) : nullptr, it, m_->partials2,
+    k_cg_xr<T><<<stream_blocks(B, it.CH), 256, 0, s>>>(x, r, p, q, fused_rhs() ? rhs(0) : nullptr, it, m_->partials2,
                                   nblk_pq, m_->scal, m_->partials, m_->active, m_->state,
                                   ir ? 1 : 0);
     HFM_CHECK_LAUNCH("k_cg_xr");
