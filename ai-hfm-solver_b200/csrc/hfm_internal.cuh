@@ -349,11 +349,6 @@ __device__ __forceinline__ int segment_sum(const ZPlan &p, double *partials, int
   }
   return min(next + p.seg, z1);
 }
-// the first segment's end, or none where nothing is summed
-__device__ __forceinline__ int first_segment(const ZPlan &p, bool sums, int z0, int z1) {
-  return sums ? min(z0 + p.seg, z1) : -1;
-}
-
 // Register-queue plane-marching kernels (ops_fast.cu); mode 0 smooth, 1 residual, 2 residual +
 // restriction.  fast_eligible: the extents allow 4 cells per thread; fast_width: cells per
 // thread for a grid and its pointers (4, 2 or 1), 0 where the generic kernels serve.

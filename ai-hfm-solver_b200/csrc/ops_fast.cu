@@ -218,7 +218,7 @@ __device__ __forceinline__ void coarse_cells(const FastArgs<T> &a, int64_t inst,
 // ---------------------------------------------------------------------------------------
 // 7-point forms (CONST7, SIGMA7, FACE7).
 // ---------------------------------------------------------------------------------------
-template <int KIND, class T, int MODE, int CORR, int V>
+template <int KIND, class T, int MODE, int CORR, bool SUMS, int V>
 __global__ void __launch_bounds__(kFastThreads, MODE == M_RESTRICT ? 2 : 4)
     k_fast7(const __grid_constant__ FastArgs<T> a) {
   using F4 = FV<V>;  // a thread's cells of a row
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(kFastThreads, MODE == M_RESTRICT ? 2 : 4)
     for (int e = 0; e < V; ++e) azlo.v[e] = s * fz.v[e];
   }
   double acc = 0.0;
-  int seg_end = first_segment(a.zp, (MODE != M_SMOOTH || a.dot_rhs) && a.partials, z0, z1);
+  int seg_end = min(z0 + a.zp.seg, z1);
   float cpart[2] = {0.f, 0.f};  // RESTRICT: the two coarse cells of this vector, summed over planes
 
   for (int zb = z0; zb < z1; zb += NP) {
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(kFastThreads, MODE == M_RESTRICT ? 2 : 4)
       if (MODE == M_SMOOTH) {
 #pragma unroll
         for (int e = 0; e < V; ++e) res.v[e] = pc.v[e] + a.omega * quotient<V>(f[n].v[e] - Ax.v[e], dg.v[e]);
-        if (a.dot_rhs && valid) {
+        if (SUMS && valid) {
 #pragma unroll
           for (int e = 0; e < V; ++e) acc += (double)res.v[e] * f[n].v[e];
         }
@@ -428,7 +428,7 @@ __global__ void __launch_bounds__(kFastThreads, MODE == M_RESTRICT ? 2 : 4)
 #pragma unroll
         for (int e = 0; e < V; ++e) res.v[e] = Ax.v[e] - f[n].v[e];
         if (a.zero_xend_out && x0 + V == X) res.v[V - 1] = 0.f;
-        if (valid) {
+        if (SUMS && valid) {
 #pragma unroll
           for (int e = 0; e < V; ++e) acc += (double)res.v[e] * (a.dot_phi ? pc.v[e] : res.v[e]);
         }
@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(kFastThreads, MODE == M_RESTRICT ? 2 : 4)
       pm = pc;
       pc = pp[n];
       if (MODE == M_RESTRICT) coarse_cells<T, V>(a, inst, z, y, x0, valid, res, cpart);
-      if (z + 1 == seg_end) seg_end = segment_sum<kFastThreads / 32>(a.zp, a.partials, inst, Z, seg_end, z0, z1, acc);
+      if (SUMS && z + 1 == seg_end) seg_end = segment_sum<kFastThreads / 32>(a.zp, a.partials, inst, Z, seg_end, z0, z1, acc);
     }
   }
 }
@@ -451,11 +451,11 @@ __global__ void __launch_bounds__(kFastThreads, MODE == M_RESTRICT ? 2 : 4)
 // bound by their latency unless they are issued early: the loads of plane z + 1 go out before
 // plane z is computed, and the index arithmetic is kept to 32-bit byte offsets from the
 // instance's pointers (64-bit element offsets made 257 instructions per cell, these 173).
-// 4 x 75 x 90 x 101, SIGMA7: a sweep 19.6 us, 3.9 TB/s (k_fast7 with one cell per thread, loads
+// 4 x 75 x 90 x 101, SIGMA7: a sweep 18.5 us, 3.5 TB/s (k_fast7 with one cell per thread, loads
 // and use in one plane, 40 us; one thread per cell with 64-bit divisions 53 us).  The arithmetic
 // is k_fast7's.
 // ---------------------------------------------------------------------------------------
-template <int KIND, class T, int MODE, int CORR>
+template <int KIND, class T, int MODE, int CORR, bool SUMS>
 __global__ void __launch_bounds__(kFastThreads, 3) k_column7(const __grid_constant__ FastArgs<T> a) {
   int64_t inst;
   int z0, z1;
@@ -540,8 +540,7 @@ __global__ void __launch_bounds__(kFastThreads, 3) k_column7(const __grid_consta
     szc = ld(sz, o);
     azlo = z0 > 0 ? cz * 0.5f * (szc + ld(sz, o - plane)) : cz * szc;
   }
-  const bool sums = a.partials && (MODE != M_SMOOTH || a.dot_rhs);
-  int seg_end = first_segment(a.zp, sums, z0, z1);
+  int seg_end = min(z0 + a.zp.seg, z1);
   double acc = 0.0;
   for (int z = z0; z < z1; ++z) {
     const Plane q = nx;
@@ -579,7 +578,7 @@ __global__ void __launch_bounds__(kFastThreads, 3) k_column7(const __grid_consta
       v = Ax - q.f;
       if (a.zero_xend_out && x == X - 1) v = 0.f;
     }
-    if (sums && valid) acc += (double)v * (MODE == M_SMOOTH ? q.f : a.dot_phi ? pc : v);
+    if (SUMS && valid) acc += (double)v * (MODE == M_SMOOTH ? q.f : a.dot_phi ? pc : v);
     if (valid) {
       T *dst = reinterpret_cast<T *>(reinterpret_cast<char *>(out) + here);
       if (MODE == M_SMOOTH && a.top_copy && Z > 1) {
@@ -591,7 +590,7 @@ __global__ void __launch_bounds__(kFastThreads, 3) k_column7(const __grid_consta
     }
     pm = pc;
     pc = q.pp;
-    if (z + 1 == seg_end) seg_end = segment_sum<kFastThreads / 32>(a.zp, a.partials, inst, Z, seg_end, z0, z1, acc);
+    if (SUMS && z + 1 == seg_end) seg_end = segment_sum<kFastThreads / 32>(a.zp, a.partials, inst, Z, seg_end, z0, z1, acc);
   }
 }
 
@@ -601,7 +600,7 @@ __global__ void __launch_bounds__(kFastThreads, 3) k_column7(const __grid_consta
 // (7.8 us with two rows per thread; a thread per coarse cell with 216 bounds-checked loads took
 // 21 us, and 82 us on 64 x 128 x 128, where the plane-marching TMA kernel takes 8 us).
 // ---------------------------------------------------------------------------------------
-template <class T, int MODE, int CORR, int V>
+template <class T, int MODE, int CORR, bool SUMS, int V>
 __global__ void __launch_bounds__(kFastThreads)
     k_fast27(const __grid_constant__ FastArgs<T> a) {
   using F4 = FV<V>;  // a thread's cells of a row
@@ -656,7 +655,7 @@ __global__ void __launch_bounds__(kFastThreads)
   }
   const float diag = K[13];
   double acc2 = 0.0;
-  int seg_end = first_segment(a.zp, (MODE != M_SMOOTH || a.dot_rhs) && a.partials, z0, z1);
+  int seg_end = min(z0 + a.zp.seg, z1);
   float cpart[2] = {0.f, 0.f};  // RESTRICT: the two coarse cells of this vector, summed over planes
   for (int z = z0; z < z1; ++z) {
     const int64_t off = (int64_t)z * plane + (int64_t)y * X + x0;
@@ -670,7 +669,7 @@ __global__ void __launch_bounds__(kFastThreads)
     if (MODE == M_SMOOTH) {
 #pragma unroll
       for (int e = 0; e < V; ++e) res.v[e] = cen_cur.v[e] + a.omega * quotient<V>(f.v[e] - Ax.v[e], diag);
-      if (a.dot_rhs && valid) {
+      if (SUMS && valid) {
 #pragma unroll
         for (int e = 0; e < V; ++e) acc2 += (double)res.v[e] * f.v[e];
       }
@@ -694,7 +693,7 @@ __global__ void __launch_bounds__(kFastThreads)
     }
     cen_cur = cen_next;
     if (MODE == M_RESTRICT) coarse_cells<T, V>(a, inst, z, y, x0, valid, res, cpart);
-    if (z + 1 == seg_end) seg_end = segment_sum<kFastThreads / 32>(a.zp, a.partials, inst, Z, seg_end, z0, z1, acc2);
+    if (SUMS && z + 1 == seg_end) seg_end = segment_sum<kFastThreads / 32>(a.zp, a.partials, inst, Z, seg_end, z0, z1, acc2);
   }
 }
 
@@ -775,18 +774,23 @@ int fast_width(int kind, const DevOp &op, const PhiSrc<T> &phi, const T *rhs, co
 
 template <class T, int V, int KIND>
 int fast_go(int mode, int corr, FastArgs<T> &a, int B, int *nblk_out, cudaStream_t s) {
+  const bool sums = a.partials && (mode != M_SMOOTH || a.dot_rhs);
 #define HFM_FAST_GO(KER)                                                                       \
   do {                                                                                         \
-    const bool sums = (mode != M_SMOOTH || a.dot_rhs) && a.partials;                           \
     const dim3 grid = fast_grid<T>(a, B, V, mode == M_RESTRICT, sums,                          \
                                    resident_blocks((const void *)KER), nblk_out);              \
     KER<<<grid, kFastThreads, 0, s>>>(a);                                                      \
   } while (0)
+#define HFM_FAST_S(M, C, S)                                                                    \
+  do {                                                                                         \
+    if constexpr (KIND == HFM_OP_K27) HFM_FAST_GO((k_fast27<T, M, C, S, V>));                  \
+    else if constexpr (V == 1) HFM_FAST_GO((k_column7<KIND, T, M, C, S>));                     \
+    else HFM_FAST_GO((k_fast7<KIND, T, M, C, S, V>));                                          \
+  } while (0)
 #define HFM_FAST_K(M, C)                                                                       \
   do {                                                                                         \
-    if constexpr (KIND == HFM_OP_K27) HFM_FAST_GO((k_fast27<T, M, C, V>));                     \
-    else if constexpr (V == 1) HFM_FAST_GO((k_column7<KIND, T, M, C>));                        \
-    else HFM_FAST_GO((k_fast7<KIND, T, M, C, V>));                                             \
+    if (sums) HFM_FAST_S(M, C, true);                                                          \
+    else HFM_FAST_S(M, C, false);                                                              \
   } while (0)
   if (mode == M_SMOOTH) {
     if (corr == C_NONE) HFM_FAST_K(M_SMOOTH, C_NONE);
@@ -803,6 +807,7 @@ int fast_go(int mode, int corr, FastArgs<T> &a, int B, int *nblk_out, cudaStream
     }
   }
 #undef HFM_FAST_K
+#undef HFM_FAST_S
 #undef HFM_FAST_GO
   HFM_CHECK_LAUNCH("fast stencil kernel");
   return HFM_OK;

@@ -228,7 +228,10 @@ __device__ __forceinline__ double block_sum(double v) {
   return t;
 }
 
-template <int KIND, class T, int MODE, int CORR>
+// SUMS: with partial sums (of z . r in a sweep, else of res^2 or res * phi).  Kernels that have
+// none carry no code for them: 256^3 SIGMA7 passes 289 -> 284 us, ten one-slot 128^3 sawtooth
+// cycles 472 -> 459 us.
+template <int KIND, class T, int MODE, int CORR, bool SUMS>
 __global__ void __launch_bounds__(Geo<T>::THREADS, Geo<T>::MINB) k_tma(const __grid_constant__ TmaArgs<T> a) {
   constexpr bool SIG = KIND == HFM_OP_SIGMA7;
   constexpr bool PRE2 = MODE == M_PRE2;
@@ -348,7 +351,7 @@ __global__ void __launch_bounds__(Geo<T>::THREADS, Geo<T>::MINB) k_tma(const __g
     for (int e = 0; e < V; ++e) azlo[e] = z0 > 0 ? hz * (szc[e] + szm[e]) : cz * szc[e];
   }
   double acc = 0.0;
-  int seg_end = first_segment(a.zp, (MODE != M_SMOOTH || a.dot_rhs) && a.partials, z0, z1);
+  int seg_end = min(z0 + a.zp.seg, z1);
   float cpart[V / 2];
 #pragma unroll
   for (int e = 0; e < V / 2; ++e) cpart[e] = 0.f;
@@ -481,7 +484,7 @@ __global__ void __launch_bounds__(Geo<T>::THREADS, Geo<T>::MINB) k_tma(const __g
         res[e] = v.x;
         res[e + 1] = v.y;
       }
-      if (a.dot_rhs && valid) {
+      if (SUMS && valid) {
 #pragma unroll
         for (int e = 0; e < V; ++e) acc += (double)res[e] * f[e];
       }
@@ -489,7 +492,7 @@ __global__ void __launch_bounds__(Geo<T>::THREADS, Geo<T>::MINB) k_tma(const __g
 #pragma unroll
       for (int e = 0; e < V; ++e) res[e] = Ax[e] - f[e];
       if (a.zero_xend_out && gx + V == X) res[V - 1] = 0.f;
-      if (valid) {
+      if (SUMS && valid) {
 #pragma unroll
         for (int e = 0; e < V; ++e) acc += (double)res[e] * (a.dot_phi ? pc[e] : res[e]);
       }
@@ -518,7 +521,7 @@ __global__ void __launch_bounds__(Geo<T>::THREADS, Geo<T>::MINB) k_tma(const __g
         for (int k = 0; k < V / 2; ++k) cpart[k] = 0.f;
       }
     }
-    if (z + 1 == seg_end) seg_end = segment_sum<G::THREADS / 32>(a.zp, a.partials, inst, Z, seg_end, z0, z1, acc);
+    if (SUMS && z + 1 == seg_end) seg_end = segment_sum<G::THREADS / 32>(a.zp, a.partials, inst, Z, seg_end, z0, z1, acc);
   }
   if (ok && __syncthreads_or(!mine)) ok = false;  // the last plane's wait
   if (!ok) {
@@ -630,32 +633,49 @@ dim3 tma_grid(TmaArgs<T> &a, int B, int per_sm, bool sums, int *nblk_out) {
   return dim3(tiles, (Z + a.zp.chunk - 1) / a.zp.chunk, B);
 }
 
-template <int KIND, class T, int MODE, int CORR>
-int go(TmaArgs<T> &a, int B, int *nblk_out, cudaStream_t s) {
+// Whether a launch takes partial sums.
+template <class T> bool with_sums(const TmaArgs<T> &a, int mode) {
+  return mode != M_PRE2 && a.partials && (mode != M_SMOOTH || a.dot_rhs);
+}
+
+template <int KIND, class T, int MODE, int CORR, bool SUMS>
+int go_sums(TmaArgs<T> &a, int B, int *nblk_out, cudaStream_t s) {
   using G = Geo<T, KIND == HFM_OP_SIGMA7, CORR == 1, MODE == M_PRE2 || CORR == 2>;
   const int smem = G::NS * G::STAGE;
-  const void *fn = (const void *)k_tma<KIND, T, MODE, CORR>;
+  const void *fn = (const void *)k_tma<KIND, T, MODE, CORR, SUMS>;
   int st = set_max_dynamic_smem(fn, smem, "cudaFuncSetAttribute(k_tma)");
   if (st) return st;
-  const dim3 grid = tma_grid(a, B, tma_resident(fn, G::THREADS, smem),
-                             (MODE != M_SMOOTH || a.dot_rhs) && a.partials, nblk_out);
-  k_tma<KIND, T, MODE, CORR><<<grid, G::THREADS, smem, s>>>(a);
+  const dim3 grid = tma_grid(a, B, tma_resident(fn, G::THREADS, smem), SUMS, nblk_out);
+  k_tma<KIND, T, MODE, CORR, SUMS><<<grid, G::THREADS, smem, s>>>(a);
   HFM_CHECK_LAUNCH("k_tma");
+  return HFM_OK;
+}
+
+template <int KIND, class T, int MODE, int CORR>
+int go(TmaArgs<T> &a, int B, int *nblk_out, cudaStream_t s) {
+  if constexpr (MODE != M_PRE2)
+    if (with_sums(a, MODE)) return go_sums<KIND, T, MODE, CORR, true>(a, B, nblk_out, s);
+  return go_sums<KIND, T, MODE, CORR, false>(a, B, nblk_out, s);
+}
+
+template <class T, int MODE, int CORR, bool SUMS>
+int go_face_sums(TmaArgs<T> &a, int B, int *nblk_out, cudaStream_t s) {
+  using G = GeoF<CORR != 0, MODE == M_PRE2>;
+  const int smem = G::NS * G::STAGE;
+  const void *fn = (const void *)k_tma_face<T, MODE, CORR, SUMS>;
+  int st = set_max_dynamic_smem(fn, smem, "cudaFuncSetAttribute(k_tma_face)");
+  if (st) return st;
+  const dim3 grid = tma_grid(a, B, tma_resident(fn, G::THREADS, smem), SUMS, nblk_out);
+  k_tma_face<T, MODE, CORR, SUMS><<<grid, G::THREADS, smem, s>>>(a);
+  HFM_CHECK_LAUNCH("k_tma_face");
   return HFM_OK;
 }
 
 template <class T, int MODE, int CORR>
 int go_face(TmaArgs<T> &a, int B, int *nblk_out, cudaStream_t s) {
-  using G = GeoF<CORR != 0, MODE == M_PRE2>;
-  const int smem = G::NS * G::STAGE;
-  const void *fn = (const void *)k_tma_face<T, MODE, CORR>;
-  int st = set_max_dynamic_smem(fn, smem, "cudaFuncSetAttribute(k_tma_face)");
-  if (st) return st;
-  const dim3 grid = tma_grid(a, B, tma_resident(fn, G::THREADS, smem),
-                             (MODE != M_SMOOTH || a.dot_rhs) && a.partials, nblk_out);
-  k_tma_face<T, MODE, CORR><<<grid, G::THREADS, smem, s>>>(a);
-  HFM_CHECK_LAUNCH("k_tma_face");
-  return HFM_OK;
+  if constexpr (MODE != M_PRE2)
+    if (with_sums(a, MODE)) return go_face_sums<T, MODE, CORR, true>(a, B, nblk_out, s);
+  return go_face_sums<T, MODE, CORR, false>(a, B, nblk_out, s);
 }
 
 }  // namespace

@@ -1187,7 +1187,7 @@ template <class T> size_t layout_sub(int kind, SubArgs<T> &a) {
 // Level l1 of a V-cycle and the coarse end below it in one launch.  A block takes work items
 // in order from a global ticket: (step, instance, z tile) for the sweeps and the residual +
 // restriction of level l1, (SUB, instance) for the coarse end, which runs in the block's
-// shared memory exactly as k_subcycle does.  Items are numbered step by step, so an item
+// shared memory exactly as in k_subprog.  Items are numbered step by step, so an item
 // only waits for items with smaller numbers - items other running blocks have already taken
 // - and the waits always end; each is still bounded (the wait budget), and one that runs out
 // is counted in the device's wait-failure counters (the handle then ends its slots with

@@ -216,7 +216,7 @@ __device__ __forceinline__ void face_cells_f32(const float (&c)[8], float xl, fl
   }
 }
 
-template <class T, int MODE, int CORR>
+template <class T, int MODE, int CORR, bool SUMS>
 __global__ void __launch_bounds__(GeoF<false, false>::THREADS, GeoF<false, false>::MINB)
     k_tma_face(const __grid_constant__ TmaArgs<T> a) {
   constexpr bool PRE2 = MODE == M_PRE2;
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(GeoF<false, false>::THREADS, GeoF<false, false
   uint32_t fzl[4] = {0u, 0u, 0u, 0u};
   if (ok) ld8w(stage_of(z0 - 1) + G::O_FZ + (r * TX + V * c) * 2, fzl);
   double acc = 0.0;
-  int seg_end = first_segment(a.zp, (MODE != M_SMOOTH || a.dot_rhs) && !PRE2 && a.partials, z0, z1);
+  int seg_end = min(z0 + a.zp.seg, z1);
   float cpart[V / 2];
 #pragma unroll
   for (int e = 0; e < V / 2; ++e) cpart[e] = 0.f;
@@ -479,18 +479,18 @@ __global__ void __launch_bounds__(GeoF<false, false>::THREADS, GeoF<false, false
 #pragma unroll
     for (int k = 0; k < 4; ++k) packed[k] = pack2<T>(res[2 * k], res[2 * k + 1]);
     if (valid) {
-      if ((MODE == M_SMOOTH || PRE2) && a.dot_rhs) {
+      if (SUMS && MODE == M_SMOOTH) {
         // z . r of a preconditioner whose right-hand side is r: the stored z times r
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           pacc = M::template fma<0, 0>(packed[k], fr[k], pacc);
           pacc = M::template fma<1, 1>(packed[k], fr[k], pacc);
         }
-      } else if (MODE == M_RESID || MODE == M_RESTRICT) {
+      } else if (SUMS) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) pacc = fmaf(res[e], res[e], pacc);
       }
-      acc += (double)pacc;
+      if (SUMS) acc += (double)pacc;
       if (a.out) {
         uint4 u;
         u.x = packed[0]; u.y = packed[1]; u.z = packed[2]; u.w = packed[3];
@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(GeoF<false, false>::THREADS, GeoF<false, false
         for (int k = 0; k < V / 2; ++k) cpart[k] = 0.f;
       }
     }
-    if (z + 1 == seg_end) seg_end = segment_sum<G::THREADS / 32>(a.zp, a.partials, inst, Z, seg_end, z0, z1, acc);
+    if (SUMS && z + 1 == seg_end) seg_end = segment_sum<G::THREADS / 32>(a.zp, a.partials, inst, Z, seg_end, z0, z1, acc);
   }
   if (ok && __syncthreads_or(!mine)) ok = false;
   if (!ok) {
