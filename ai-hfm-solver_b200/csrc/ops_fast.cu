@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(kFastThreads, MODE == M_RESTRICT ? 2 : 4)
 // bound by their latency unless they are issued early: the loads of plane z + 1 go out before
 // plane z is computed, and the index arithmetic is kept to 32-bit byte offsets from the
 // instance's pointers (64-bit element offsets made 257 instructions per cell, these 173).
-// 4 x 75 x 90 x 101, SIGMA7: a sweep 18.5 us, 3.5 TB/s (k_fast7 with one cell per thread, loads
+// 4 x 75 x 90 x 101, SIGMA7: a sweep 19.3 us, 3.4 TB/s (k_fast7 with one cell per thread, loads
 // and use in one plane, 40 us; one thread per cell with 64-bit divisions 53 us).  The arithmetic
 // is k_fast7's.
 // ---------------------------------------------------------------------------------------
