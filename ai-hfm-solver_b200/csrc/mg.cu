@@ -16,6 +16,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -957,6 +958,8 @@ struct hfm_mg {
   const int *wait_fail = nullptr;  // the device's TMA wait-failure counters (read by checks)
   hfm_operator fine_desc;
   cudaStream_t cap = nullptr;
+  cudaEvent_t masks_done = nullptr;  // after the last call that reads or writes the activity masks
+  std::mutex masks_mu;
   std::map<int, cudaGraphExec_t> graphs;
   std::map<int, int64_t> graph_kernels;
   std::vector<void *> allocs;
@@ -2095,6 +2098,8 @@ int hfm_mg_create(const hfm_mg_config *cfg, int Z, int Y, int X, int slots, hfm_
   if (!st) st = wait_fail_counters(&m->wait_fail);
   if (!st && cudaStreamCreateWithFlags(&m->cap, cudaStreamNonBlocking) != cudaSuccess)
     st = fail(HFM_ERR_CUDA, "cudaStreamCreate failed");
+  if (!st && cudaEventCreateWithFlags(&m->masks_done, cudaEventDisableTiming) != cudaSuccess)
+    st = fail(HFM_ERR_CUDA, "cudaEventCreate failed");
   if (!st) {
     switch (cfg->storage) {
       case HFM_F32: m->eng.reset(new Engine<float>(m.get())); break;
@@ -2114,6 +2119,7 @@ int hfm_mg_create(const hfm_mg_config *cfg, int Z, int Y, int X, int slots, hfm_
   if (st) {
     for (void *p : m->allocs) cudaFree(p);
     if (m->cap) cudaStreamDestroy(m->cap);
+    if (m->masks_done) cudaEventDestroy(m->masks_done);
     return st;
   }
   // default constant operator so that CONST7 / K27 handles work after set_operator only
@@ -2129,6 +2135,7 @@ int hfm_mg_destroy(hfm_mg *m) {
     cudaStreamDestroy(m->cap);
   }
   cudaDeviceSynchronize();
+  if (m->masks_done) cudaEventDestroy(m->masks_done);
   for (void *p : m->allocs) cudaFree(p);
   delete m;
   return HFM_OK;
@@ -2149,13 +2156,53 @@ int hfm_mg_set_operator(hfm_mg *m, int slot, const hfm_operator *op, hfm_stream_
   return m->eng->set_operator(slot, *op, (cudaStream_t)stream);
 }
 
+}  // extern "C"
+
+namespace {
+// Orders the calls that write a many-slot handle's activity masks (load, cancel) and those that
+// read them (run) when a caller uses several streams or threads: the blocks of a launch share
+// out the active slots, so a mask that changed while it ran would take work from other slots.
+// A call waits on its stream for the one before it; on one stream that is no wait.  A caller's
+// own capture keeps the order of the captured stream.
+class MaskOrder {
+ public:
+  MaskOrder(hfm_mg *m, cudaStream_t s) : m_(m), s_(s), on_(m->slots > 1), lk_(m->masks_mu, std::defer_lock) {
+    if (!on_) return;
+    lk_.lock();
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &c) != cudaSuccess) {
+      cudaGetLastError();
+      on_ = false;
+    } else if (c != cudaStreamCaptureStatusNone) {
+      on_ = false;
+    }
+    if (on_) cudaStreamWaitEvent(s_, m_->masks_done, 0);
+  }
+  ~MaskOrder() {
+    if (on_) cudaEventRecord(m_->masks_done, s_);
+  }
+  MaskOrder(const MaskOrder &) = delete;
+  MaskOrder &operator=(const MaskOrder &) = delete;
+
+ private:
+  hfm_mg *m_;
+  cudaStream_t s_;
+  bool on_;
+  std::unique_lock<std::mutex> lk_;
+};
+}  // namespace
+
+extern "C" {
+
 int hfm_mg_load(hfm_mg *m, int slot, const float *rhs, const float *phi0, hfm_stream_t stream) {
   if (!m || !rhs || slot < 0 || slot >= m->slots) return fail(HFM_ERR_BAD_ARG, "hfm_mg_load: bad argument");
+  MaskOrder order(m, (cudaStream_t)stream);
   return m->eng->load(slot, rhs, phi0, (cudaStream_t)stream);
 }
 
 int hfm_mg_run(hfm_mg *m, int cycles, hfm_stream_t stream) {
   if (!m || cycles < 1) return fail(HFM_ERR_BAD_ARG, "hfm_mg_run: bad argument");
+  MaskOrder order(m, (cudaStream_t)stream);
   cudaGraphExec_t exec = nullptr;
   auto it = m->graphs.find(cycles);
   if (it != m->graphs.end()) {
@@ -2232,6 +2279,7 @@ int hfm_mg_fetch(hfm_mg *m, int slot, float *out, hfm_stream_t stream) {
 
 int hfm_mg_cancel(hfm_mg *m, int slot, hfm_stream_t stream) {
   if (!m || slot < 0 || slot >= m->slots) return fail(HFM_ERR_BAD_ARG, "hfm_mg_cancel: bad argument");
+  MaskOrder order(m, (cudaStream_t)stream);
   HFM_CUDA(cudaMemsetAsync(m->active + slot, 0, 4, (cudaStream_t)stream));
   HFM_CUDA(cudaMemsetAsync(m->outer + slot, 0, 4, (cudaStream_t)stream));
   return HFM_OK;
@@ -2240,6 +2288,7 @@ int hfm_mg_cancel(hfm_mg *m, int slot, hfm_stream_t stream) {
 int hfm_mg_load_f64(hfm_mg *m, int slot, const double *rhs, const double *phi0,
                     hfm_stream_t stream) {
   if (!m || !rhs || slot < 0 || slot >= m->slots) return fail(HFM_ERR_BAD_ARG, "hfm_mg_load_f64: bad argument");
+  MaskOrder order(m, (cudaStream_t)stream);
   return m->eng->load64(slot, rhs, phi0, (cudaStream_t)stream);
 }
 
@@ -2257,7 +2306,10 @@ int hfm_mg_solve(hfm_mg *m, const float *rhs, float *phi, hfm_slot_stats *stats_
                  hfm_stream_t stream) {
   if (!m || !rhs || !phi) return fail(HFM_ERR_BAD_ARG, "hfm_mg_solve: bad argument");
   int st;
-  if ((st = m->eng->load_all(rhs, (cudaStream_t)stream))) return st;
+  {
+    MaskOrder order(m, (cudaStream_t)stream);
+    if ((st = m->eng->load_all(rhs, (cudaStream_t)stream))) return st;
+  }
   std::vector<hfm_slot_stats> tmp(m->slots);
   hfm_slot_stats *ss = stats_host ? stats_host : tmp.data();
   const int per = m->cfg.cycles_per_launch;

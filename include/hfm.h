@@ -560,7 +560,8 @@ int hfm_mg_query(hfm_mg *mg, hfm_slot_stats *stats_host, hfm_stream_t stream);
 int hfm_mg_query_async(hfm_mg *mg, hfm_slot_stats *stats_host, hfm_stream_t stream);
 /* Copy a slot's current solution into phi_out (device, [Z][Y][X] float32). */
 int hfm_mg_fetch(hfm_mg *mg, int slot, float *phi_out, hfm_stream_t stream);
-/* Stop a slot (request cancelled); its memory can be reloaded at once. */
+/* Stop a slot (request cancelled); its memory can be reloaded at once.  From another stream or
+ * thread than the runs', it takes effect after the run in flight. */
 int hfm_mg_cancel(hfm_mg *mg, int slot, hfm_stream_t stream);
 /* Convenience: load all slots from rhs/phi ([slots][Z][Y][X]), run to completion, fetch the
  * solutions into phi, fill stats_host (may be NULL).  Synchronises `stream`. */

@@ -272,3 +272,34 @@ def test_active_slots_share_the_grid_same_bits(hfm, T, shape, slots, accel, stor
             for other in (few[k], every[k]):
                 np.testing.assert_array_equal(alone[0], other[0])
                 assert alone[1:] == other[1:]
+
+
+def test_cancel_on_another_stream_leaves_the_other_slots_alone(hfm, T):
+    """The blocks of a launch share out the active slots: a cancel from another stream takes
+    effect between launches, and the slots that stay keep their bits."""
+    shape, slots = (24, 32, 48), 6
+    rng = np.random.default_rng(13)
+    cfg = hfm.multigrid.SolverConfig(cycle="V", accel="cg", tol=1e-6, max_cycles=60)
+    sig = dev(T, np.exp(0.5 * rng.standard_normal((3,) + shape)))
+    rhs = dev(T, rng.standard_normal((slots,) + shape))
+    other = T.cuda.Stream()
+    with hfm.multigrid.Multigrid(shape, hfm._lib.OP_SIGMA7, cfg, slots=slots) as h:
+        for k in range(slots):
+            h.set_operator(hfm.ops.Sigma7(sig[0], sig[1], sig[2]), slot=k)
+
+        def solve(cancel):
+            for k in range(slots):
+                h.load(k, rhs[k])
+            for it in range(15):
+                h.run(4)
+                if cancel and it < slots - 2:
+                    with T.cuda.stream(other):
+                        h.cancel(it + 1)
+            st = h.query()
+            return h.fetch(0).cpu().numpy(), h.fetch(slots - 1).cpu().numpy(), st
+
+        a, b = solve(False), solve(True)
+        assert b[2][0]["status"] == hfm._lib.OK and b[2][slots - 1]["status"] == hfm._lib.OK
+        assert not any(s["active"] for s in b[2])
+        for x, y in zip(a[:2], b[:2]):
+            np.testing.assert_array_equal(x, y)
