@@ -340,6 +340,7 @@ int hfm_prolong_correct_smooth_typed(const hfm_operator *op, int dtype, const vo
     p.corr_stride = n / 8;
     p.corr_coarse = 1;
     p.corr_sign = phi ? -1.f : 1.f;
+    p.Zc = Z / 2;
     p.Yc = Y / 2;
     p.Xc = X / 2;
     return launch_smooth<T>(op->kind, d, p, (const T *)rhs, n, (T *)out, n, B, Grid3{Z, Y, X},
@@ -374,6 +375,7 @@ int hfm_face7_smooth2_typed(const hfm_operator *op, int dtype, const void *phi,
       p.corr_stride = n / 8;
       p.corr_coarse = 1;
       p.corr_sign = -1.f;
+      p.Zc = Z / 2;
       p.Yc = Y / 2;
       p.Xc = X / 2;
     }
@@ -412,6 +414,7 @@ int hfm_prolong_correct_smooth(const hfm_operator *op, const float *phi,
   p.corr_stride = n / 8;
   p.corr_coarse = 1;
   p.corr_sign = phi ? -1.f : 1.f;  // phi - P w, or P w alone (sawtooth coarse levels)
+  p.Zc = Z / 2;
   p.Yc = Y / 2;
   p.Xc = X / 2;
   return launch_smooth<float>(op->kind, d, p, rhs, n, out, n, B, Grid3{Z, Y, X}, omega, flags,
@@ -442,8 +445,8 @@ int hfm_prolong_nearest(const float *coarse, float *fine, int B, int Zc, int Yc,
   if ((st = check_grid(B, Zc, Yc, Xc))) return st;
   if (!fine || !coarse) return fail(HFM_ERR_BAD_ARG, "hfm_prolong_nearest: NULL field");
   const int64_t nc = (int64_t)Zc * Yc * Xc;
-  return launch_prolong<float>(coarse, nc, fine, nc * 8, B, Grid3{Zc, Yc, Xc}, nullptr,
-                               (cudaStream_t)stream);
+  return launch_prolong<float>(coarse, nc, fine, nc * 8, B, Grid3{2 * Zc, 2 * Yc, 2 * Xc},
+                               Grid3{Zc, Yc, Xc}, nullptr, (cudaStream_t)stream);
 }
 
 int hfm_stencil7_const_apply(const float *phi, float *out, int B, int Z, int Y, int X,

@@ -95,18 +95,22 @@ template <class T> struct PhiSrc {
   const T *corr;
   int64_t base_stride, corr_stride;
   float corr_sign;
-  int corr_coarse;  // corr lives on the coarse grid (Zc, Yc, Xc) = fine / 2
-  int Yc, Xc;
+  int corr_coarse;  // corr lives on the coarse grid (Zc, Yc, Xc) = fine / 2, rounded down
+  int Zc, Yc, Xc;
   int zero_xend;
   __device__ __forceinline__ float operator()(int64_t inst, int z, int y, int x, int Y,
                                               int X) const {
     if (zero_xend && x == X - 1) return 0.f;
     float v = 0.f;
     if (base) v = St<T>::ld(base + inst * base_stride + ((int64_t)z * Y + y) * X + x);
-    if (corr) {
-      int64_t ci = corr_coarse ? (((int64_t)(z >> 1) * Yc + (y >> 1)) * Xc + (x >> 1))
-                               : (((int64_t)z * Y + y) * X + x);
-      v += corr_sign * St<T>::ld(corr + inst * corr_stride + ci);
+    if (corr && corr_coarse) {
+      // the last cells of an odd extent have no coarse cell (the restriction drops them too):
+      // no correction there
+      const int zc = z >> 1, yc = y >> 1, xc = x >> 1;
+      if (zc < Zc && yc < Yc && xc < Xc)
+        v += corr_sign * St<T>::ld(corr + inst * corr_stride + ((int64_t)zc * Yc + yc) * Xc + xc);
+    } else if (corr) {
+      v += corr_sign * St<T>::ld(corr + inst * corr_stride + ((int64_t)z * Y + y) * X + x);
     }
     return v;
   }
@@ -222,8 +226,9 @@ int launch_residual_restrict(int kind, const DevOp &op, const PhiSrc<T> &phi, co
 template <class T>
 int launch_restrict(const T *fine, int64_t f_stride, T *coarse, int64_t c_stride, int B,
                     Grid3 g, const int *active, cudaStream_t s);
+// fine grid g, coarse grid gc (g / 2 rounded down); cells past the last coarse cell become zero
 template <class T>
-int launch_prolong(const T *coarse, int64_t c_stride, T *fine, int64_t f_stride, int B,
+int launch_prolong(const T *coarse, int64_t c_stride, T *fine, int64_t f_stride, int B, Grid3 g,
                    Grid3 gc, const int *active, cudaStream_t s);
 // Three same-shape arrays (the conductivities) restricted by one launch where the vector
 // kernel applies.

@@ -1008,6 +1008,7 @@ class Engine : public EngineBase {
     p.corr_stride = n(lc);
     p.corr_coarse = 1;
     p.corr_sign = sign;
+    p.Zc = m_->lv[lc].Z;
     p.Yc = m_->lv[lc].Y;
     p.Xc = m_->lv[lc].X;
     return p;
@@ -1438,7 +1439,7 @@ class Engine : public EngineBase {
       PhiSrc<T> p = with_coarse(src(nullptr, n(0)), 1, buf(1, 0), 1.f);
       if ((st = smooth(0, p, r0, w0, c.omega, 0u, s))) return st;
     } else {
-      if ((st = launch_prolong<T>(buf(1, 0), n(1), w0, n(0), m_->slots, g(1), m_->active, s)))
+      if ((st = launch_prolong<T>(buf(1, 0), n(1), w0, n(0), m_->slots, g(0), g(1), m_->active, s)))
         return st;
     }
     // 6. phi = J(phi - w) against b (NS: phi[..., X-1] = 0 before the sweep; _BC: top copy)

@@ -757,16 +757,16 @@ bool fast_eligible(int kind, Grid3 g, bool restrict_mode) {
 // grids of the 7- and 27-point forms take V = 2 (even rows, pointers aligned to 2 elements) or
 // V = 1 from 8 columns up: 4 x 75 x 90 x 101, a SIGMA7 sweep 53 -> 20 us.  Narrower rows, of
 // a few hundred cells at most where they occur, stay with one thread per cell.  A correction
-// on a coarse grid of a fine grid with odd extents does too (nearest prolongation past the
-// last coarse cell).
+// from the coarse grid of a fine grid with odd extents does too, at every width: its last cells
+// have no coarse cell, and these kernels do not test for that.
 template <class T>
 int fast_width(int kind, const DevOp &op, const PhiSrc<T> &phi, const T *rhs, const T *out,
                const T *coarse, int64_t stride, Grid3 g, bool restrict_mode) {
   const int64_t es = (int64_t)sizeof(T);
+  if ((restrict_mode || (phi.corr && phi.corr_coarse)) && ((g.Z | g.Y | g.X) & 1)) return 0;
   if (fast_eligible(kind, g, restrict_mode) && vec_aligned<T>(kind, op, phi, rhs, out, coarse, stride, 4 * es))
     return 4;
   if ((kind != HFM_OP_CONST7 && kind != HFM_OP_SIGMA7 && kind != HFM_OP_K27) || g.X < 8) return 0;
-  if ((restrict_mode || (phi.corr && phi.corr_coarse)) && ((g.Z | g.Y | g.X) & 1)) return 0;
   if (!(g.X & 1) && vec_aligned<T>(kind, op, phi, rhs, out, coarse, stride, 2 * es)) return 2;
   // k_column7 keeps 32-bit byte offsets within an instance
   return restrict_mode || g.n() * es >= ((int64_t)1 << 32) || g.n() >= ((int64_t)1 << 31) ? 0 : 1;

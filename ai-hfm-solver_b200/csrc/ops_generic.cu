@@ -168,19 +168,17 @@ __global__ void __launch_bounds__(kThreads)
 
 template <class T>
 __global__ void __launch_bounds__(kThreads)
-    k_prolong(const T *__restrict__ c, int64_t cs, T *__restrict__ f, int64_t fs, int Zc,
-              int Yc, int Xc, const int *__restrict__ active) {
+    k_prolong(const T *__restrict__ c, int64_t cs, T *__restrict__ f, int64_t fs, Grid3 g, Grid3 gc,
+              const int *__restrict__ active) {
   const int64_t inst = blockIdx.y;
   if (active && !active[inst]) return;
-  const int Y = 2 * Yc, X = 2 * Xc;
-  const int64_t n = (int64_t)8 * Zc * Yc * Xc;
+  const int64_t n = (int64_t)g.Z * g.Y * g.X;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
-    int x = (int)(i % X);
-    int64_t t = i / X;
-    int y = (int)(t % Y);
-    int z = (int)(t / Y);
-    f[inst * fs + i] = c[inst * cs + ((int64_t)(z >> 1) * Yc + (y >> 1)) * Xc + (x >> 1)];
+    const int64_t t = i / g.X;
+    const int x = (int)(i - t * g.X) >> 1, y = (int)(t % g.Y) >> 1, z = (int)(t / g.Y) >> 1;
+    const bool in = z < gc.Z && y < gc.Y && x < gc.X;  // else the last cell of an odd extent
+    f[inst * fs + i] = in ? c[inst * cs + ((int64_t)z * gc.Y + y) * gc.X + x] : St<T>::from(0.f);
   }
 }
 
@@ -505,18 +503,18 @@ int launch_restrict3(const T *const fine[3], int64_t f_stride, T *const coarse[3
 }
 
 template <class T>
-int launch_prolong(const T *coarse, int64_t c_stride, T *fine, int64_t f_stride, int B,
+int launch_prolong(const T *coarse, int64_t c_stride, T *fine, int64_t f_stride, int B, Grid3 g,
                    Grid3 gc, const int *active, cudaStream_t s) {
-  if (transfer_vec_ok<T>(fine, f_stride, coarse, c_stride, 2 * gc.X, B)) {
+  if (g.Z == 2 * gc.Z && g.Y == 2 * gc.Y && g.X == 2 * gc.X &&
+      transfer_vec_ok<T>(fine, f_stride, coarse, c_stride, g.X, B)) {
     dim3 grid(blocks_for(gc.n() / Vec16<T>::HC, B), B);
     k_prolong_v<T><<<grid, kThreads, 0, s>>>(coarse, c_stride, fine, f_stride, gc.Z, gc.Y,
                                              gc.X, active);
     HFM_CHECK_LAUNCH("k_prolong_v");
     return HFM_OK;
   }
-  dim3 grid(blocks_for(gc.n() * 8, B), B);
-  k_prolong<T><<<grid, kThreads, 0, s>>>(coarse, c_stride, fine, f_stride, gc.Z, gc.Y, gc.X,
-                                         active);
+  dim3 grid(blocks_for(g.n(), B), B);
+  k_prolong<T><<<grid, kThreads, 0, s>>>(coarse, c_stride, fine, f_stride, g, gc, active);
   HFM_CHECK_LAUNCH("k_prolong");
   return HFM_OK;
 }
@@ -553,8 +551,8 @@ int launch_coarse_jacobi(int kind, const DevOp &op, const T *rhs, int64_t rhs_st
                                    cudaStream_t);                                           \
   template int launch_restrict<T>(const T *, int64_t, T *, int64_t, int, Grid3, const int *, \
                                   cudaStream_t);                                             \
-  template int launch_prolong<T>(const T *, int64_t, T *, int64_t, int, Grid3, const int *,  \
-                                 cudaStream_t);                                              \
+  template int launch_prolong<T>(const T *, int64_t, T *, int64_t, int, Grid3, Grid3,        \
+                                 const int *, cudaStream_t);                                 \
   template int launch_coarse_jacobi<T>(int, const DevOp &, const T *, int64_t, const T *,    \
                                        T *, int64_t, int, Grid3, float, int, const int *,    \
                                        cudaStream_t);
