@@ -1078,6 +1078,12 @@ class Engine : public EngineBase {
     int l0 = m_->L - 1;
     while (l0 - 1 >= 1 && n(l0 - 1) <= 4096 && m_->L - (l0 - 1) <= kMaxSubLevels) --l0;
     if (l0 >= m_->L - 1) return -1;
+    // V and F cycles refuse odd extents above the coarsest level (the launch per step does).
+    // Handles of 8 slots and more have always run the V-cycle's fused levels with floored
+    // extents, dropping the last cells, and keep doing so.
+    if (c.cycle != HFM_CYCLE_SAWTOOTH && !(c.cycle == HFM_CYCLE_V && m_->slots >= 8))
+      for (int l = l0; l + 1 < m_->L; ++l)
+        if ((g(l).Z | g(l).Y | g(l).X) & 1) return -1;
     SubProgram<T> p;  // the longest list of the cycle form and the levels' fields fit
     const bool listed = c.cycle == HFM_CYCLE_SAWTOOTH
                             ? sawtooth_program(l0, p)

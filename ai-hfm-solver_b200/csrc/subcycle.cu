@@ -1386,10 +1386,11 @@ int go_subprog(const SubProgram<T> &p, int B, size_t smem, cudaStream_t s) {
   return HFM_OK;
 }
 
-// The quad form of level l0: whole quads per row, and at most one pair of quads per thread.
+// The quad form of level l0: whole quads per row, at most one pair of quads per thread, and two
+// rows and planes for its restriction to pair.
 template <class T> bool program_top(const SubProgram<T> &p) {
   const SubLevel<T> &L = p.a.lv[0];
-  return (L.X & 3) == 0 && ((L.Z + 1) >> 1) * L.Y * (L.X >> 2) <= kProgThreads;
+  return (L.X & 3) == 0 && L.Y > 1 && L.Z > 1 && ((L.Z + 1) >> 1) * L.Y * (L.X >> 2) <= kProgThreads;
 }
 
 // Shared-memory layout of a program: per level the fields, right-hand side and faces as

@@ -65,3 +65,62 @@ def test_sawtooth_on_odd_extents(hfm, shape, levels, form, fine_smooth):
         # a few dozen roundings of them, or some eight of the storage's 2^-9
         scale = max(np.abs(ref).max(), np.abs(f[s]).max(), w)
         assert np.abs(got[s] - ref).max() <= (16 * 2.0 ** -9 if bf16 else 1e-5) * scale
+
+
+def _vcycle(ops, l, f, phi):
+    if l == len(ops) - 1:
+        for _ in range(5):
+            phi = mg.jacobi(ops[l], phi, f, 2.0 / 3.0)
+        return phi
+    for _ in range(2):
+        phi = mg.jacobi(ops[l], phi, f, 2.0 / 3.0)
+    r = tfops.restrict_avg(mg.residual(ops[l], phi, f), np.float64)
+    phi = phi - _prolong(_vcycle(ops, l + 1, r, np.zeros_like(r)), phi.shape)
+    for _ in range(2):
+        phi = mg.jacobi(ops[l], phi, f, 2.0 / 3.0)
+    return phi
+
+
+ODD_BELOW = [((24, 24, 24), 5), ((20, 12, 40), 4), ((28, 20, 24), 4)]
+
+
+@pytest.mark.parametrize("shape,levels", ODD_BELOW)
+@pytest.mark.parametrize("cycle,slots,fused", [("V", 1, True), ("V", 7, True), ("V", 1, False), ("V", 8, False),
+                                               ("F", 1, True), ("F", 8, True), ("F", 1, False)])
+def test_v_and_f_cycles_refuse_odd_levels(hfm, shape, levels, cycle, slots, fused):
+    import torch
+    cfg = hfm.multigrid.SolverConfig(cycle=cycle, n_levels=levels, tol=1e-300, fused_coarse=fused)
+    op = hfm.ops.Const7(0.5, 1.0, 2.0)
+    with hfm.multigrid.Multigrid(shape, op.kind, cfg, slots=slots) as h:
+        h.set_operator(op)
+        h.load(0, torch.ones(shape, device="cuda"))
+        with pytest.raises(hfm._lib.HfmError, match="BAD_ARG"):
+            h.run(1)
+
+
+@pytest.mark.parametrize("shape,levels", ODD_BELOW)
+@pytest.mark.parametrize("form", ["const7", "k27", "sigma7"])
+def test_many_slot_v_cycles_floor_odd_levels(hfm, shape, levels, form):
+    import torch
+    ops, rng = hfm.ops, np.random.default_rng(43)
+    B = 8
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).cuda()
+    f = rng.standard_normal((B,) + shape).astype(np.float32)
+    sig = np.exp(0.5 * rng.standard_normal((3, B) + shape)).astype(np.float32)
+    K = W.w5_pressure27()
+    op = {"const7": lambda: ops.Const7(0.5, 1.0, 2.0), "k27": lambda: ops.Stencil27(K),
+          "sigma7": lambda: ops.Sigma7(*(dev(s) for s in sig))}[form]()
+    cfg = hfm.multigrid.SolverConfig(cycle="V", n_levels=levels, tol=1e-300, coarse_sweeps=5)
+    with hfm.multigrid.Multigrid(shape, op.kind, cfg, slots=B) as h:
+        h.set_operator(op)
+        for s in range(B):
+            h.load(s, dev(f[s]))
+        h.run(1)
+        got = [h.fetch(s).cpu().numpy() for s in range(B)]
+    for s in (0, B - 1):
+        oracle = {"const7": lambda: mg.const7(0.5, 1.0, 2.0, dtype=np.float64),
+                  "k27": lambda: mg.Stencil27(np.asarray(K, np.float32), dtype=np.float64),
+                  "sigma7": lambda: mg.Sigma7(*(a[s].astype(np.float64) for a in sig), dtype=np.float64)}[form]()
+        f64 = f[s].astype(np.float64)
+        ref = _vcycle(mg.hierarchy(oracle, levels, 0.5), 0, f64, np.zeros_like(f64))
+        assert np.abs(got[s] - ref).max() <= 1e-5 * max(np.abs(ref).max(), np.abs(f64).max())
