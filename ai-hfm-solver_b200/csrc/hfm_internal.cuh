@@ -437,8 +437,7 @@ template <class T> struct SubProgram {
   int nsteps;
   unsigned char op[kMaxSubSteps], lev[kMaxSubSteps], cnt[kMaxSubSteps];
   const T *phi0;  // initial iterate of level l0 (nullable: zero), instance stride lv[0].n
-  // with store_all, where the right-hand sides and iterates of the levels below l0 are written
-  int store_all;
+  // where the right-hand sides and iterates of the levels below l0 are written
   T *g_rhs[kMaxSubLevels], *g_phi[kMaxSubLevels];
   int o_top;      // float offset of the pair sums of level l0 (quad form)
   int clear;      // 16-byte words of shared memory in use

@@ -1099,8 +1099,7 @@ class Engine : public EngineBase {
     const hfm_mg_config &c = m_->cfg;
     for (int l = l0; l + 1 < m_->L; ++l)
       if (((g(l).Z | g(l).Y | g(l).X) & 1)) return false;
-    memset(&p, 0, sizeof(p));
-    p.a = make_sub(l0);
+    new_program(l0, p);
     p.a.coarse_omega = c.omega;
     const int last = p.a.nlev - 1;
     for (int l = 0; l < last; ++l)
@@ -1108,15 +1107,22 @@ class Engine : public EngineBase {
     if (!add_step(p, SO_COARSE, last, sawtooth_coarse_sweeps())) return false;
     for (int l = last - 1; l >= 0; --l)
       if (!add_step(p, SO_PROLONG, l, 1) || !add_step(p, SO_SWEEP, l, 1)) return false;
-    p.store_all = 1;
-    for (int l = 1; l <= last; ++l) {
-      p.g_rhs[l] = rhs(l0 + l);
-      p.g_phi[l] = buf(l0 + l, 0);
-    }
     return true;
   }
   int sawtooth_coarse_sweeps() const {
     return (m_->cfg.options & HFM_OPT_SAWTOOTH_COARSE_SWEEPS) ? m_->cfg.coarse_sweeps : 1;
+  }
+
+  // An empty program over the levels from l0 down.  The right-hand sides and iterates of the levels
+  // below l0 are written back at its end: hfm_mg_read_level shows them.
+  void new_program(int l0, SubProgram<T> &p) {
+    memset(&p, 0, sizeof(p));
+    p.a = make_sub(l0);
+    for (int l = 1; l < p.a.nlev; ++l) {
+      p.g_rhs[l] = rhs(l0 + l);
+      p.g_phi[l] = buf(l0 + l, 0);
+      cur_[l0 + l] = 0;
+    }
   }
 
   // Steps of the cycles vcycle() runs from level l down (l relative to l0): V from a zero or the
@@ -1153,8 +1159,7 @@ class Engine : public EngineBase {
     return launch_subprogram<T>(kind(), p, m_->slots, s);
   }
   bool fused_program(int l0, int what, SubProgram<T> &p) {
-    memset(&p, 0, sizeof(p));
-    p.a = make_sub(l0);
+    new_program(l0, p);
     if (!add_cycle(p, 0, what != SUB_V, what == SUB_F || what == SUB_FV)) return false;
     return what != SUB_FV || add_cycle(p, 0, false, false);
   }

@@ -1140,15 +1140,14 @@ __global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant_
       out[i] = St<T>::from(res[q.ip]);
     }
   }
-  if (P.store_all)
-    for (l = 1; l < nl; ++l) {
-      const SubLevel<T> &L = a.lv[l];
-      const float *res = F + (((cur >> l) & 1) ? L.o_tmp : L.o_phi);
-      HFM_FOR_CELLS(L, F)
-        P.g_rhs[l][inst * (int64_t)L.n + i] = St<T>::from(F[L.o_rhs + i]);
-        P.g_phi[l][inst * (int64_t)L.n + i] = St<T>::from(res[q.ip]);
-      }
+  for (l = 1; l < nl; ++l) {
+    const SubLevel<T> &L = a.lv[l];
+    const float *res = F + (((cur >> l) & 1) ? L.o_tmp : L.o_phi);
+    HFM_FOR_CELLS(L, F)
+      P.g_rhs[l][inst * (int64_t)L.n + i] = St<T>::from(F[L.o_rhs + i]);
+      P.g_phi[l][inst * (int64_t)L.n + i] = St<T>::from(res[q.ip]);
     }
+  }
 }
 
 }  // namespace
