@@ -401,6 +401,9 @@ int tma_launch(int kind, int mode, const DevOp &op, const PhiSrc<T> &phi, const 
 // CONST7 or K27 hierarchy, one block per instance, all fields in shared memory.
 constexpr int kMaxSubLevels = 8;
 constexpr size_t kSubcycleMaxSmem = 200 * 1024;
+// The program kernel also holds a cell table: with all of an SM's shared memory it serves every
+// hierarchy whose fields and faces alone take kSubcycleMaxSmem.
+constexpr size_t kProgramMaxSmem = 227 * 1024;
 template <class T> struct SubLevel {
   int Z, Y, X, n;
   float cz, cy, cx;          // SIGMA7: face multipliers of this level (c_d times its scale)
@@ -408,7 +411,8 @@ template <class T> struct SubLevel {
   const T *sx, *sy, *sz;     // the level's conductivities, instance stride n
   int o_phi, o_tmp, o_rhs;   // float offsets of the level's fields in shared memory
   int o_face;                // float offset of its face arrays and diagonal (SIGMA7)
-  int o_idx;                 // float offset of its cell table (8 bytes per cell)
+  int o_idx;                 // float offset of its cell table (4 bytes per cell)
+  int bx, by;                // bits of x and of y in the table's coordinates
 };
 template <class T> struct SubArgs {
   SubLevel<T> lv[kMaxSubLevels];
@@ -435,7 +439,8 @@ constexpr int kMaxSubSteps = 160;
 template <class T> struct SubProgram {
   SubArgs<T> a;
   int nsteps;
-  unsigned char op[kMaxSubSteps], lev[kMaxSubSteps], cnt[kMaxSubSteps];
+  unsigned char op[kMaxSubSteps], lev[kMaxSubSteps];
+  int cnt[kMaxSubSteps];
   const T *phi0;  // initial iterate of level l0 (nullable: zero), instance stride lv[0].n
   // where the right-hand sides and iterates of the levels below l0 are written
   T *g_rhs[kMaxSubLevels], *g_phi[kMaxSubLevels];

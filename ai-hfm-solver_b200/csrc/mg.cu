@@ -1128,10 +1128,10 @@ class Engine : public EngineBase {
   // Steps of the cycles vcycle() runs from level l down (l relative to l0): V from a zero or the
   // current iterate, F from zero.  Returns false when the list is full.
   static bool add_step(SubProgram<T> &p, SubOp op, int l, int cnt) {
-    if (p.nsteps >= kMaxSubSteps || cnt > 255) return false;
+    if (p.nsteps >= kMaxSubSteps) return false;
     p.op[p.nsteps] = op;
     p.lev[p.nsteps] = (unsigned char)l;
-    p.cnt[p.nsteps++] = (unsigned char)cnt;
+    p.cnt[p.nsteps++] = cnt;
     return true;
   }
   bool add_cycle(SubProgram<T> &p, int l, bool zero, bool fcycle) {

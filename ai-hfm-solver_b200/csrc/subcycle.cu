@@ -347,19 +347,22 @@ __device__ void subcycle_body(const SubArgs<T> &a, int64_t inst, unsigned char *
 // per sweep of 16^3.
 constexpr int kProgThreads = 512;
 
-// Cell i of a level: padded index and coordinates, from a table formed once per launch.
+// Cell i of a level: padded index and coordinates, from a table formed once per launch: 16 bits of
+// padded index (at most 36882, 1 x 1 x 4096) below the coordinates, whose bits add up to 15 at
+// most (a level has 4096 cells at most).
 struct Cell {
   int ip, z, y, x;
 };
-__device__ __forceinline__ Cell cell_of(const uint2 *tab, int i) {
-  const uint2 u = tab[i];
-  return Cell{(int)(u.x & 0xffffu), (int)(u.x >> 16), (int)(u.y >> 16), (int)(u.y & 0xffffu)};
+template <class T> __device__ __forceinline__ Cell cell_of(const SubLevel<T> &L, const float *F, int i) {
+  const unsigned u = reinterpret_cast<const unsigned *>(F + L.o_idx)[i], c = u >> 16;
+  return Cell{(int)(u & 0xffffu), (int)(c >> (L.bx + L.by)), (int)((c >> L.bx) & ((1u << L.by) - 1u)),
+              (int)(c & ((1u << L.bx) - 1u))};
 }
 
 // A thread-strided pass over the cells of level L.
 #define HFM_FOR_CELLS(L, F)                                                              \
   for (int i = threadIdx.x; i < (L).n; i += kProgThreads) {                              \
-    const Cell q = cell_of(reinterpret_cast<const uint2 *>((F) + (L).o_idx), i);
+    const Cell q = cell_of(L, F, i);
 
 // Cell i of level L: its table entry and, for SIGMA7, its face coefficients (the low ones,
 // and the high ones at the walls) and 1 / diagonal.  The global loads and the shared-memory
@@ -391,8 +394,8 @@ template <int KIND, class T> struct CellInit {
   }
   __device__ __forceinline__ void store(const SubLevel<T> &L, float *F) const {
     const int X = L.X, Y = L.Y, Z = L.Z, P = X * Y;
-    reinterpret_cast<uint2 *>(F + L.o_idx)[i] =
-        make_uint2((unsigned)pix(z, y, x, Y, X) | ((unsigned)z << 16), ((unsigned)y << 16) | (unsigned)x);
+    reinterpret_cast<unsigned *>(F + L.o_idx)[i] =
+        (unsigned)pix(z, y, x, Y, X) | ((unsigned)x << 16) | ((unsigned)y << (16 + L.bx)) | ((unsigned)z << (16 + L.bx + L.by));
     if (KIND == HFM_OP_SIGMA7) {
       const float axm = L.cx * (0.5f * (vx + xl)), axp = L.cx * (0.5f * (vx + xh));
       const float aym = L.cy * (0.5f * (vy + yl)), ayp = L.cy * (0.5f * (vy + yh));
@@ -613,7 +616,7 @@ __device__ __forceinline__ void coarse_cells7(const SubLevel<T> &L, float *F, fl
   const int X = L.X, Y = L.Y, Z = L.Z, PX = X + 2, PXY = PX * (Y + 2), P = X * Y;
   const bool in = (int)threadIdx.x < L.n;
   const int i = in ? threadIdx.x : L.n - 1;
-  const Cell q = cell_of(reinterpret_cast<const uint2 *>(F + L.o_idx), i);
+  const Cell q = cell_of(L, F, i);
   float c[6], od;
   if (KIND == HFM_OP_CONST7) {
     c[0] = c[1] = L.k[2];
@@ -1116,7 +1119,7 @@ __global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant_
         __syncthreads();
       } else if (mid && l == 1) {
         if (mc.valid) {
-          const Cell q = cell_of(reinterpret_cast<const uint2 *>(F + L1.o_idx), mc.i);
+          const Cell q = cell_of(L1, F, mc.i);
           const float d = sign * coarse[pix(q.z >> 1, q.y >> 1, q.x >> 1, Lc.Y, Lc.X)];
           mc.v[0] = zero ? d : mc.v[0] + d;
           mc.v[1] = !mc.two ? 0.f : zero ? d : mc.v[1] + d;
@@ -1377,7 +1380,7 @@ template int launch_small<__half>(int, SmallArgs<__half>, int, cudaStream_t);
 
 template <int KIND, class T, bool TOP>
 int go_subprog(const SubProgram<T> &p, int B, size_t smem, cudaStream_t s) {
-  int st = set_max_dynamic_smem((const void *)k_subprog<KIND, T, TOP>, (int)kSubcycleMaxSmem,
+  int st = set_max_dynamic_smem((const void *)k_subprog<KIND, T, TOP>, (int)kProgramMaxSmem,
                                 "cudaFuncSetAttribute(k_subprog)");
   if (st) return st;
   k_subprog<KIND, T, TOP><<<B, kProgThreads, smem, s>>>(p);
@@ -1401,6 +1404,13 @@ template <class T> size_t layout_program(int kind, SubProgram<T> &p) {
   for (int l = 0; l < p.a.nlev; ++l) {
     SubLevel<T> &q = p.a.lv[l];
     const int np = sub_padded(q.Z, q.Y, q.X);
+    auto bits = [](int e) {
+      int b = 0;
+      while ((1 << b) < e) ++b;
+      return b;
+    };
+    q.bx = bits(q.X);
+    q.by = bits(q.Y);
     q.o_phi = (int)off;
     if (top && l == 0) {
       const int nt = (q.Z + 2) * (q.Y + 2) * q.X;
@@ -1413,9 +1423,8 @@ template <class T> size_t layout_program(int kind, SubProgram<T> &p) {
     q.o_rhs = (int)off + 2 * np;
     q.o_face = q.o_rhs + q.n;
     off = q.o_face + (kind == HFM_OP_SIGMA7 ? sub_faces(q.Z, q.Y, q.X) + q.n : 0);
-    off = (off + 1) & ~1;
     q.o_idx = (int)off;
-    off = (off + 2 * q.n + 3) & ~3;
+    off = (off + q.n + 3) & ~3;
   }
   off = (off + 3) & ~3;
   p.clear = (int)(off / 4);
@@ -1423,14 +1432,14 @@ template <class T> size_t layout_program(int kind, SubProgram<T> &p) {
 }
 
 template <class T> bool subprogram_fits(int kind, SubProgram<T> &p) {
-  return layout_program<T>(kind, p) <= kSubcycleMaxSmem;
+  return layout_program<T>(kind, p) <= kProgramMaxSmem;
 }
 
 template <class T>
 int launch_subprogram(int kind, SubProgram<T> &p, int B, cudaStream_t s) {
   const bool top = program_top(p);
   const size_t smem = layout_program<T>(kind, p);
-  if (smem > kSubcycleMaxSmem) return fail(HFM_ERR_BAD_ARG, "subcycle: levels exceed shared memory");
+  if (smem > kProgramMaxSmem) return fail(HFM_ERR_BAD_ARG, "subcycle: levels exceed shared memory");
   switch (kind) {
     case HFM_OP_SIGMA7:
       return top ? go_subprog<HFM_OP_SIGMA7, T, true>(p, B, smem, s) : go_subprog<HFM_OP_SIGMA7, T, false>(p, B, smem, s);

@@ -67,15 +67,15 @@ def test_sawtooth_on_odd_extents(hfm, shape, levels, form, fine_smooth):
         assert np.abs(got[s] - ref).max() <= (16 * 2.0 ** -9 if bf16 else 1e-5) * scale
 
 
-def _vcycle(ops, l, f, phi):
+def _vcycle(ops, l, f, phi, coarse_sweeps=5):
     if l == len(ops) - 1:
-        for _ in range(5):
+        for _ in range(coarse_sweeps):
             phi = mg.jacobi(ops[l], phi, f, 2.0 / 3.0)
         return phi
     for _ in range(2):
         phi = mg.jacobi(ops[l], phi, f, 2.0 / 3.0)
     r = tfops.restrict_avg(mg.residual(ops[l], phi, f), np.float64)
-    phi = phi - _prolong(_vcycle(ops, l + 1, r, np.zeros_like(r)), phi.shape)
+    phi = phi - _prolong(_vcycle(ops, l + 1, r, np.zeros_like(r), coarse_sweeps), phi.shape)
     for _ in range(2):
         phi = mg.jacobi(ops[l], phi, f, 2.0 / 3.0)
     return phi
@@ -98,9 +98,10 @@ def test_v_and_f_cycles_refuse_odd_levels(hfm, shape, levels, cycle, slots, fuse
             h.run(1)
 
 
-@pytest.mark.parametrize("shape,levels", ODD_BELOW)
+# the last two: thin levels that fill an SM's shared memory, and a long coarsest solve
 @pytest.mark.parametrize("form", ["const7", "k27", "sigma7"])
-def test_many_slot_v_cycles_floor_odd_levels(hfm, shape, levels, form):
+@pytest.mark.parametrize("shape,levels,coarse_sweeps", [s + (5,) for s in ODD_BELOW] + [((4, 6, 1156), 3, 5), ((20, 12, 40), 4, 300)])
+def test_many_slot_v_cycles_floor_odd_levels(hfm, shape, levels, form, coarse_sweeps):
     import torch
     ops, rng = hfm.ops, np.random.default_rng(43)
     B = 8
@@ -110,7 +111,7 @@ def test_many_slot_v_cycles_floor_odd_levels(hfm, shape, levels, form):
     K = W.w5_pressure27()
     op = {"const7": lambda: ops.Const7(0.5, 1.0, 2.0), "k27": lambda: ops.Stencil27(K),
           "sigma7": lambda: ops.Sigma7(*(dev(s) for s in sig))}[form]()
-    cfg = hfm.multigrid.SolverConfig(cycle="V", n_levels=levels, tol=1e-300, coarse_sweeps=5)
+    cfg = hfm.multigrid.SolverConfig(cycle="V", n_levels=levels, tol=1e-300, coarse_sweeps=coarse_sweeps)
     with hfm.multigrid.Multigrid(shape, op.kind, cfg, slots=B) as h:
         h.set_operator(op)
         for s in range(B):
@@ -122,5 +123,5 @@ def test_many_slot_v_cycles_floor_odd_levels(hfm, shape, levels, form):
                   "k27": lambda: mg.Stencil27(np.asarray(K, np.float32), dtype=np.float64),
                   "sigma7": lambda: mg.Sigma7(*(a[s].astype(np.float64) for a in sig), dtype=np.float64)}[form]()
         f64 = f[s].astype(np.float64)
-        ref = _vcycle(mg.hierarchy(oracle, levels, 0.5), 0, f64, np.zeros_like(f64))
+        ref = _vcycle(mg.hierarchy(oracle, levels, 0.5), 0, f64, np.zeros_like(f64), coarse_sweeps)
         assert np.abs(got[s] - ref).max() <= 1e-5 * max(np.abs(ref).max(), np.abs(f64).max())
