@@ -411,8 +411,8 @@ template <class T> struct SubLevel {
   const T *sx, *sy, *sz;     // the level's conductivities, instance stride n
   int o_phi, o_tmp, o_rhs;   // float offsets of the level's fields in shared memory
   int o_face;                // float offset of its face arrays and diagonal (SIGMA7)
-  int o_idx;                 // float offset of its cell table (4 bytes per cell)
-  int bx, by;                // bits of x and of y in the table's coordinates
+  int o_idx;                 // float offset of its cell table (8 or 4 bytes per cell)
+  int bx, by;                // bits of x and of y in a 4-byte table's coordinates
 };
 template <class T> struct SubArgs {
   SubLevel<T> lv[kMaxSubLevels];

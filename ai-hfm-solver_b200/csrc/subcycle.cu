@@ -347,27 +347,43 @@ __device__ void subcycle_body(const SubArgs<T> &a, int64_t inst, unsigned char *
 // per sweep of 16^3.
 constexpr int kProgThreads = 512;
 
-// Cell i of a level: padded index and coordinates, from a table formed once per launch: 16 bits of
-// padded index (at most 36882, 1 x 1 x 4096) below the coordinates, whose bits add up to 15 at
-// most (a level has 4096 cells at most).
+// Cell i of a level: padded index and coordinates, from a table formed once per launch.  With level
+// l0 in quads (TOP) it takes 8 bytes a cell; without, where the levels may fill the shared memory,
+// 4: 16 bits of padded index (at most 36882, 1 x 1 x 4096) below the coordinates, whose bits add
+// up to 15 at most (a level has 4096 cells at most).  (4 bytes for both: the compiler then keeps
+// fewer of the 27-point weights in registers, and the 16 x 32 x 32 program takes 24 us, not 20.)
 struct Cell {
   int ip, z, y, x;
 };
-template <class T> __device__ __forceinline__ Cell cell_of(const SubLevel<T> &L, const float *F, int i) {
-  const unsigned u = reinterpret_cast<const unsigned *>(F + L.o_idx)[i], c = u >> 16;
-  return Cell{(int)(u & 0xffffu), (int)(c >> (L.bx + L.by)), (int)((c >> L.bx) & ((1u << L.by) - 1u)),
-              (int)(c & ((1u << L.bx) - 1u))};
+template <bool TOP, class T> __device__ __forceinline__ Cell cell_of(const SubLevel<T> &L, const float *F, int i) {
+  if constexpr (TOP) {
+    const uint2 u = reinterpret_cast<const uint2 *>(F + L.o_idx)[i];
+    return Cell{(int)(u.x & 0xffffu), (int)(u.x >> 16), (int)(u.y >> 16), (int)(u.y & 0xffffu)};
+  } else {
+    const unsigned u = reinterpret_cast<const unsigned *>(F + L.o_idx)[i], c = u >> 16;
+    return Cell{(int)(u & 0xffffu), (int)(c >> (L.bx + L.by)), (int)((c >> L.bx) & ((1u << L.by) - 1u)),
+                (int)(c & ((1u << L.bx) - 1u))};
+  }
+}
+template <bool TOP, class T>
+__device__ __forceinline__ void set_cell(const SubLevel<T> &L, float *F, int i, int z, int y, int x) {
+  const unsigned ip = (unsigned)pix(z, y, x, L.Y, L.X);
+  if constexpr (TOP)
+    reinterpret_cast<uint2 *>(F + L.o_idx)[i] = make_uint2(ip | ((unsigned)z << 16), ((unsigned)y << 16) | (unsigned)x);
+  else
+    reinterpret_cast<unsigned *>(F + L.o_idx)[i] =
+        ip | ((unsigned)x << 16) | ((unsigned)y << (16 + L.bx)) | ((unsigned)z << (16 + L.bx + L.by));
 }
 
 // A thread-strided pass over the cells of level L.
 #define HFM_FOR_CELLS(L, F)                                                              \
   for (int i = threadIdx.x; i < (L).n; i += kProgThreads) {                              \
-    const Cell q = cell_of(L, F, i);
+    const Cell q = cell_of<TOP>(L, F, i);
 
 // Cell i of level L: its table entry and, for SIGMA7, its face coefficients (the low ones,
 // and the high ones at the walls) and 1 / diagonal.  The global loads and the shared-memory
 // stores are apart, so that the loads can be in flight while the block clears its fields.
-template <int KIND, class T> struct CellInit {
+template <int KIND, class T, bool TOP> struct CellInit {
   int x, y, z, t, i;
   float vx, vy, vz, xl, xh, yl, yh, zl, zh;
   __device__ __forceinline__ void load(const SubLevel<T> &L, int64_t inst, int cell) {
@@ -394,8 +410,7 @@ template <int KIND, class T> struct CellInit {
   }
   __device__ __forceinline__ void store(const SubLevel<T> &L, float *F) const {
     const int X = L.X, Y = L.Y, Z = L.Z, P = X * Y;
-    reinterpret_cast<unsigned *>(F + L.o_idx)[i] =
-        (unsigned)pix(z, y, x, Y, X) | ((unsigned)x << 16) | ((unsigned)y << (16 + L.bx)) | ((unsigned)z << (16 + L.bx + L.by));
+    set_cell<TOP>(L, F, i, z, y, x);
     if (KIND == HFM_OP_SIGMA7) {
       const float axm = L.cx * (0.5f * (vx + xl)), axp = L.cx * (0.5f * (vx + xh));
       const float aym = L.cy * (0.5f * (vy + yl)), ayp = L.cy * (0.5f * (vy + yh));
@@ -534,7 +549,7 @@ template <int KIND> struct CellPair {
 };
 
 // One sweep of a level's iterate `in` (null: zero) into `out`.
-template <int KIND, class T>
+template <int KIND, bool TOP, class T>
 __device__ void prog_sweep(const SubLevel<T> &L, float *F, const float *in, float *out, float om) {
   const float *f = F + L.o_rhs, *Fc = F + L.o_face;
   const float *rd = Fc + sub_faces(L.Z, L.Y, L.X);
@@ -555,7 +570,7 @@ __device__ void prog_sweep(const SubLevel<T> &L, float *F, const float *in, floa
 
 // The second phase of a restriction: each coarse cell's eight fine residuals (padded field,
 // ordered z, y, x), averaged into the coarse level's right-hand side.
-template <class T>
+template <bool TOP, class T>
 __device__ void prog_sum8(const SubLevel<T> &L, float *F, const float *res, const SubLevel<T> &Lc) {
   __syncthreads();
   const int PX = L.X + 2, PXY = PX * (L.Y + 2);
@@ -571,7 +586,7 @@ __device__ void prog_sum8(const SubLevel<T> &L, float *F, const float *res, cons
 
 // Next level's right-hand side = R(A phi - f) (phi null: zero): every fine residual by its own
 // thread into `res`, then the sums.
-template <int KIND, class T>
+template <int KIND, bool TOP, class T>
 __device__ void prog_restrict(const SubLevel<T> &L, float *F, const float *ph, float *res,
                               const SubLevel<T> &Lc) {
   const float *f = F + L.o_rhs, *Fc = F + L.o_face;
@@ -580,11 +595,11 @@ __device__ void prog_restrict(const SubLevel<T> &L, float *F, const float *ph, f
     const float ax = ph ? sub_apply<KIND, T>(L, ph, Fc, q.z, q.y, q.x, q.ip, i, &dg) : 0.f;
     res[q.ip] = ax - f[i];
   }
-  prog_sum8<T>(L, F, res, Lc);
+  prog_sum8<TOP, T>(L, F, res, Lc);
 }
 
 // Next level's right-hand side = R f
-template <class T>
+template <bool TOP, class T>
 __device__ void prog_restrict_rhs(const SubLevel<T> &L, float *F, const SubLevel<T> &Lc) {
   const float *f = F + L.o_rhs;
   HFM_FOR_CELLS(Lc, F)
@@ -598,7 +613,7 @@ __device__ void prog_restrict_rhs(const SubLevel<T> &L, float *F, const SubLevel
 }
 
 // phi = [phi] + sign * P(coarse) on the level's interior (both padded)
-template <class T>
+template <bool TOP, class T>
 __device__ void prog_correct(const SubLevel<T> &L, float *F, float *ph, const SubLevel<T> &Lc,
                              const float *coarse, float sign, bool zero) {
   HFM_FOR_CELLS(L, F)
@@ -611,12 +626,12 @@ __device__ void prog_correct(const SubLevel<T> &L, float *F, float *ph, const Su
 // The coarsest level's sweeps of a 7-point operator, one cell per thread (a warp's chain of
 // dependent instructions sets the time of these sweeps: 218 cycles for 64 cells on two warps,
 // 456 in pairs on one warp).  Unrolled by two, so that each field's addresses are formed once.
-template <int KIND, class T>
+template <int KIND, bool TOP, class T>
 __device__ __forceinline__ void coarse_cells7(const SubLevel<T> &L, float *F, float om, int sweeps, int nthr) {
   const int X = L.X, Y = L.Y, Z = L.Z, PX = X + 2, PXY = PX * (Y + 2), P = X * Y;
   const bool in = (int)threadIdx.x < L.n;
   const int i = in ? threadIdx.x : L.n - 1;
-  const Cell q = cell_of(L, F, i);
+  const Cell q = cell_of<TOP>(L, F, i);
   float c[6], od;
   if (KIND == HFM_OP_CONST7) {
     c[0] = c[1] = L.k[2];
@@ -655,18 +670,18 @@ __device__ __forceinline__ void coarse_cells7(const SubLevel<T> &L, float *F, fl
 // Where the block has a thread for each cell (K27: for each pair of cells, whose 27 neighbours
 // mostly coincide), coefficients stay in registers and a barrier among the warps that hold
 // cells (a warp barrier when one does) parts the sweeps.
-template <int KIND, class T>
+template <int KIND, bool TOP, class T>
 __device__ int prog_coarse(const SubLevel<T> &L, float *F, float om, int sweeps) {
   const int np = KIND == HFM_OP_K27 ? cell_pairs(L.Z, L.Y, L.X) : L.n;
   if (np > kProgThreads) {
     for (int k = 0; k < sweeps; ++k)
-      prog_sweep<KIND, T>(L, F, k == 0 ? nullptr : F + (k & 1 ? L.o_tmp : L.o_phi), F + (k & 1 ? L.o_phi : L.o_tmp), om);
+      prog_sweep<KIND, TOP, T>(L, F, k == 0 ? nullptr : F + (k & 1 ? L.o_tmp : L.o_phi), F + (k & 1 ? L.o_phi : L.o_tmp), om);
     return sweeps & 1;
   }
   const int nthr = (np + 31) & ~31;
   if ((int)threadIdx.x < nthr) {
     if constexpr (KIND != HFM_OP_K27) {
-      coarse_cells7<KIND, T>(L, F, om, sweeps, nthr);
+      coarse_cells7<KIND, TOP, T>(L, F, om, sweeps, nthr);
     } else {
       CellPair<KIND> c;
       c.load(L, F, threadIdx.x);
@@ -960,7 +975,7 @@ __global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant_
   // cell is loaded, then its quads; meanwhile the block clears its shared memory (the ghosts
   // of the fields stay zero)
   constexpr int LB = TOP ? 1 : 0;
-  CellInit<KIND, T> ci;
+  CellInit<KIND, T, TOP> ci;
   int l = nl - 1, first = 0;
   int k = threadIdx.x;
   auto find = [&]() {
@@ -1009,7 +1024,7 @@ __global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant_
     float *other = F + (c ? L.o_phi : L.o_tmp);
     float *coarse = F + (((cur >> (l + 1)) & 1) ? Lc.o_tmp : Lc.o_phi);
     if (op == SO_COARSE) {
-      const int r = prog_coarse<KIND, T>(L, F, a.coarse_omega, cnt);
+      const int r = prog_coarse<KIND, TOP, T>(L, F, a.coarse_omega, cnt);
       cur = (cur & ~(1u << l)) | ((unsigned)r << l);
     } else if (op == SO_SWEEP0 || op == SO_SWEEP) {
       for (int n = 0; n < cnt; ++n) {
@@ -1041,7 +1056,7 @@ __global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant_
           }
           __syncthreads();
         } else {
-          prog_sweep<KIND, T>(L, F, zero ? nullptr : ph, other, a.omega);
+          prog_sweep<KIND, TOP, T>(L, F, zero ? nullptr : ph, other, a.omega);
         }
         float *t = ph;
         ph = other;
@@ -1083,9 +1098,9 @@ __global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant_
           }
           mc.store(L1, other, r);
         }
-        prog_sum8<T>(L1, F, other, Lc);
+        prog_sum8<TOP, T>(L1, F, other, Lc);
       } else {
-        prog_restrict<KIND, T>(L, F, zero ? nullptr : ph, other, Lc);
+        prog_restrict<KIND, TOP, T>(L, F, zero ? nullptr : ph, other, Lc);
       }
     } else if (op == SO_RESTRICT_RHS) {
       if (TOP && l == 0) {
@@ -1099,7 +1114,7 @@ __global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant_
         }
         __syncthreads();
       } else {
-        prog_restrict_rhs<T>(L, F, Lc);
+        prog_restrict_rhs<TOP, T>(L, F, Lc);
       }
     } else {  // SO_CORRECT0, SO_CORRECT, SO_PROLONG
       const float sign = op == SO_PROLONG ? 1.f : -1.f;
@@ -1119,7 +1134,7 @@ __global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant_
         __syncthreads();
       } else if (mid && l == 1) {
         if (mc.valid) {
-          const Cell q = cell_of(L1, F, mc.i);
+          const Cell q = cell_of<TOP>(L1, F, mc.i);
           const float d = sign * coarse[pix(q.z >> 1, q.y >> 1, q.x >> 1, Lc.Y, Lc.X)];
           mc.v[0] = zero ? d : mc.v[0] + d;
           mc.v[1] = !mc.two ? 0.f : zero ? d : mc.v[1] + d;
@@ -1127,7 +1142,7 @@ __global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant_
         }
         __syncthreads();
       } else {
-        prog_correct<T>(L, F, ph, Lc, coarse, sign, zero);
+        prog_correct<TOP, T>(L, F, ph, Lc, coarse, sign, zero);
       }
     }
   }
@@ -1423,8 +1438,9 @@ template <class T> size_t layout_program(int kind, SubProgram<T> &p) {
     q.o_rhs = (int)off + 2 * np;
     q.o_face = q.o_rhs + q.n;
     off = q.o_face + (kind == HFM_OP_SIGMA7 ? sub_faces(q.Z, q.Y, q.X) + q.n : 0);
+    off = (off + 1) & ~1;
     q.o_idx = (int)off;
-    off = (off + q.n + 3) & ~3;
+    off = (off + (top ? 2 : 1) * q.n + 3) & ~3;
   }
   off = (off + 3) & ~3;
   p.clear = (int)(off / 4);
