@@ -354,6 +354,16 @@ __device__ __forceinline__ int segment_sum(const ZPlan &p, double *partials, int
   }
   return min(next + p.seg, z1);
 }
+// Whether a 27-point restriction or a pass over ragged rows leaves out zero weights, so that an
+// infinite or NaN neighbour under one gives no NaN: stateless calls, which the one-thread-per-cell
+// kernels served so.  (A handle ends a slot whose residual is not finite, whatever its weights.)
+inline bool skips_zero_weights(int kind, const DevOp &op, const int *active) {
+  if (kind != HFM_OP_K27 || active) return false;
+  for (float w : op.k)
+    if (w == 0.f) return true;
+  return false;
+}
+
 // Register-queue plane-marching kernels (ops_fast.cu); mode 0 smooth, 1 residual, 2 residual +
 // restriction.  fast_eligible: the extents allow 4 cells per thread; fast_width: cells per
 // thread for a grid and its pointers (4, 2 or 1), 0 where the generic kernels serve.

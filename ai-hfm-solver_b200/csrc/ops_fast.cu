@@ -599,8 +599,9 @@ __global__ void __launch_bounds__(kFastThreads, 3) k_column7(const __grid_consta
 // 16 x 32 x 32 the residual + restriction takes 5.2 us, bound by its chain of dependent loads
 // (7.8 us with two rows per thread; a thread per coarse cell with 216 bounds-checked loads took
 // 21 us, and 82 us on 64 x 128 x 128, where the plane-marching TMA kernel takes 8 us).
+// SKIP: as skips_zero_weights() says.
 // ---------------------------------------------------------------------------------------
-template <class T, int MODE, int CORR, bool SUMS, int V>
+template <class T, int MODE, int CORR, bool SUMS, int V, bool SKIP>
 __global__ void __launch_bounds__(kFastThreads)
     k_fast27(const __grid_constant__ FastArgs<T> a) {
   using F4 = FV<V>;  // a thread's cells of a row
@@ -634,9 +635,10 @@ __global__ void __launch_bounds__(kFastThreads)
         const float xm = e == 0 ? ls[b] : rows[b].v[e - 1];
         const float xc = rows[b].v[e];
         const float xp = e == V - 1 ? rs[b] : rows[b].v[e + 1];
-        t0 += K[3 * b + 0] * xm + K[3 * b + 1] * xc + K[3 * b + 2] * xp;
-        t1 += K[9 + 3 * b + 0] * xm + K[9 + 3 * b + 1] * xc + K[9 + 3 * b + 2] * xp;
-        t2 += K[18 + 3 * b + 0] * xm + K[18 + 3 * b + 1] * xc + K[18 + 3 * b + 2] * xp;
+        auto wx = [&](int j, float x) { return K[j] * (SKIP && K[j] == 0.f ? 0.f : x); };
+        t0 += wx(3 * b, xm) + wx(3 * b + 1, xc) + wx(3 * b + 2, xp);
+        t1 += wx(9 + 3 * b, xm) + wx(9 + 3 * b + 1, xc) + wx(9 + 3 * b + 2, xp);
+        t2 += wx(18 + 3 * b, xm) + wx(18 + 3 * b + 1, xc) + wx(18 + 3 * b + 2, xp);
       }
       s0.v[e] = t0;
       s1.v[e] = t1;
@@ -783,8 +785,15 @@ int fast_go(int mode, int corr, FastArgs<T> &a, int B, int *nblk_out, cudaStream
   } while (0)
 #define HFM_FAST_S(M, C, S)                                                                    \
   do {                                                                                         \
-    if constexpr (KIND == HFM_OP_K27) HFM_FAST_GO((k_fast27<T, M, C, S, V>));                  \
-    else if constexpr (V == 1) HFM_FAST_GO((k_column7<KIND, T, M, C, S>));                     \
+    if constexpr (KIND == HFM_OP_K27) {                                                        \
+      if constexpr (!S && (V < 4 || M == M_RESTRICT)) {                                        \
+        if (skips_zero_weights(KIND, a.op, a.active)) {                                        \
+          HFM_FAST_GO((k_fast27<T, M, C, S, V, true>));                                        \
+          break;                                                                               \
+        }                                                                                      \
+      }                                                                                        \
+      HFM_FAST_GO((k_fast27<T, M, C, S, V, false>));                                           \
+    } else if constexpr (V == 1) HFM_FAST_GO((k_column7<KIND, T, M, C, S>));                     \
     else HFM_FAST_GO((k_fast7<KIND, T, M, C, S, V>));                                          \
   } while (0)
 #define HFM_FAST_K(M, C)                                                                       \

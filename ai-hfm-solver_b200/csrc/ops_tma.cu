@@ -230,8 +230,8 @@ __device__ __forceinline__ double block_sum(double v) {
 
 // SUMS: with partial sums (of z . r in a sweep, else of res^2 or res * phi).  Kernels that have
 // none carry no code for them: 256^3 SIGMA7 passes 289 -> 284 us, ten one-slot 128^3 sawtooth
-// cycles 472 -> 459 us.
-template <int KIND, class T, int MODE, int CORR, bool SUMS>
+// cycles 472 -> 459 us.  SKIP: as skips_zero_weights() says.
+template <int KIND, class T, int MODE, int CORR, bool SUMS, bool SKIP = false>
 __global__ void __launch_bounds__(Geo<T>::THREADS, Geo<T>::MINB) k_tma(const __grid_constant__ TmaArgs<T> a) {
   constexpr bool SIG = KIND == HFM_OP_SIGMA7;
   constexpr bool PRE2 = MODE == M_PRE2;
@@ -396,6 +396,13 @@ __global__ void __launch_bounds__(Geo<T>::THREADS, Geo<T>::MINB) k_tma(const __g
           for (int e = 0; e < V; ++e) row[e + 1] = mid[e];
           row[V + 1] = phiv(pl3[aa], r + bb, G::HX + V * c + V);
           const float k0 = K[9 * aa + 3 * bb], k1 = K[9 * aa + 3 * bb + 1], k2 = K[9 * aa + 3 * bb + 2];
+          if (SKIP) {
+            const bool on[3] = {k0 != 0.f, k1 != 0.f, k2 != 0.f};
+#pragma unroll
+            for (int e = 0; e < V; ++e)
+              Ax[e] += k0 * (on[0] ? row[e] : 0.f) + k1 * (on[1] ? row[e + 1] : 0.f) + k2 * (on[2] ? row[e + 2] : 0.f);
+            continue;
+          }
 #pragma unroll
           for (int e = 0; e < V; ++e) Ax[e] += k0 * row[e] + k1 * row[e + 1] + k2 * row[e + 2];
         }
@@ -638,15 +645,15 @@ template <class T> bool with_sums(const TmaArgs<T> &a, int mode) {
   return mode != M_PRE2 && a.partials && (mode != M_SMOOTH || a.dot_rhs);
 }
 
-template <int KIND, class T, int MODE, int CORR, bool SUMS>
+template <int KIND, class T, int MODE, int CORR, bool SUMS, bool SKIP>
 int go_sums(TmaArgs<T> &a, int B, int *nblk_out, cudaStream_t s) {
   using G = Geo<T, KIND == HFM_OP_SIGMA7, CORR == 1, MODE == M_PRE2 || CORR == 2>;
   const int smem = G::NS * G::STAGE;
-  const void *fn = (const void *)k_tma<KIND, T, MODE, CORR, SUMS>;
+  const void *fn = (const void *)k_tma<KIND, T, MODE, CORR, SUMS, SKIP>;
   int st = set_max_dynamic_smem(fn, smem, "cudaFuncSetAttribute(k_tma)");
   if (st) return st;
   const dim3 grid = tma_grid(a, B, tma_resident(fn, G::THREADS, smem), SUMS, nblk_out);
-  k_tma<KIND, T, MODE, CORR, SUMS><<<grid, G::THREADS, smem, s>>>(a);
+  k_tma<KIND, T, MODE, CORR, SUMS, SKIP><<<grid, G::THREADS, smem, s>>>(a);
   HFM_CHECK_LAUNCH("k_tma");
   return HFM_OK;
 }
@@ -654,8 +661,10 @@ int go_sums(TmaArgs<T> &a, int B, int *nblk_out, cudaStream_t s) {
 template <int KIND, class T, int MODE, int CORR>
 int go(TmaArgs<T> &a, int B, int *nblk_out, cudaStream_t s) {
   if constexpr (MODE != M_PRE2)
-    if (with_sums(a, MODE)) return go_sums<KIND, T, MODE, CORR, true>(a, B, nblk_out, s);
-  return go_sums<KIND, T, MODE, CORR, false>(a, B, nblk_out, s);
+    if (with_sums(a, MODE)) return go_sums<KIND, T, MODE, CORR, true, false>(a, B, nblk_out, s);
+  if constexpr (KIND == HFM_OP_K27 && MODE == M_RESTRICT)
+    if (skips_zero_weights(KIND, a.op, a.active)) return go_sums<KIND, T, MODE, CORR, false, true>(a, B, nblk_out, s);
+  return go_sums<KIND, T, MODE, CORR, false, false>(a, B, nblk_out, s);
 }
 
 template <class T, int MODE, int CORR, bool SUMS>
