@@ -12,6 +12,7 @@
 // below tol (or that fails, or reaches max_cycles) is switched off by the check kernel and
 // every later kernel skips it, so the host only polls between graph launches.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -43,7 +44,7 @@ namespace {
 
 constexpr int kMaxLevels = 24;
 
-__global__ void k_init_state(SlotState *st, int *active, int slot, const double *sumsq_b,
+__global__ void k_init_state(SlotState *st, int *active, int *cancel, int slot, const double *sumsq_b,
                              int status_if_zero, int *outer_mask) {
   double nb = sqrt(sumsq_b[0]);
   SlotState s;
@@ -68,12 +69,21 @@ __global__ void k_init_state(SlotState *st, int *active, int slot, const double 
     else s.status = status_if_zero;
   }
   st[slot] = s;
+  cancel[slot] = 0;
   if (outer_mask) {  // refinement starts with an outer step (residual of x0 in float64)
     outer_mask[slot] = act;
     active[slot] = 0;
   } else {
     active[slot] = act;
   }
+}
+
+// A cancelled slot: cancel[slot] is set by hfm_mg_cancel on any stream at any time, and the slot
+// is switched off by the next check, so that the masks themselves only change between the
+// launches that read them (whose blocks share out the active slots).  At the start of a run:
+__global__ void k_drop_cancelled(const int *cancel, int *active, int *outer_mask, int B) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < B && cancel[i]) active[i] = outer_mask[i] = 0;
 }
 
 // Sum the residual partials of each slot, update its state, switch it off when done.
@@ -85,7 +95,7 @@ __device__ __forceinline__ bool waits_failed(const int *wf) {
 }
 
 __global__ void k_check(const double *__restrict__ partials, int nblk, SlotState *st,
-                        int *active, double tol, int max_cycles, int which_buf, const int *wf,
+                        int *active, const int *cancel, double tol, int max_cycles, int which_buf, const int *wf,
                         const double *rz_new = nullptr) {
   const int inst = blockIdx.x;
   if (!active[inst]) return;
@@ -103,7 +113,10 @@ __global__ void k_check(const double *__restrict__ partials, int nblk, SlotState
     s.rel = rel;
     s.rr = tot;
     if (rz_new) s.rz = rz_new[inst];  // CG: this iteration's r . z becomes the current one
-    if (waits_failed(wf)) {
+    if (cancel[inst]) {
+      s.sol_buf = which_buf;
+      active[inst] = 0;
+    } else if (waits_failed(wf)) {
       s.status = HFM_ERR_TIMEOUT;
       s.sol_buf = which_buf;
       active[inst] = 0;
@@ -131,7 +144,7 @@ __global__ void k_check(const double *__restrict__ partials, int nblk, SlotState
 // reaches max(inner_tol * ||r0||, 0.3 tol ||b||) or after inner_max iterations, and hands
 // the slot to the outer (float64) step.
 __global__ void k_check_inner(const double *__restrict__ partials, int nblk, SlotState *st,
-                              int *active, int *outer_mask, double tol, double inner_tol,
+                              int *active, int *outer_mask, const int *cancel, double tol, double inner_tol,
                               int inner_max, const int *wf, const double *rz_new) {
   const int inst = blockIdx.x;
   if (!active[inst]) return;
@@ -151,7 +164,9 @@ __global__ void k_check_inner(const double *__restrict__ partials, int nblk, Slo
     s.inner_cycles += 1;
     const double r = sqrt(tot);
     const double target = fmax(inner_tol * s.inner_norm, 0.3 * tol * s.norm_b);
-    if (waits_failed(wf)) {
+    if (cancel[inst]) {
+      active[inst] = 0;
+    } else if (waits_failed(wf)) {
       s.status = HFM_ERR_TIMEOUT;
       active[inst] = 0;
     } else if (!(r == r) || isinf(r)) {
@@ -168,7 +183,7 @@ __global__ void k_check_inner(const double *__restrict__ partials, int nblk, Slo
 // Outer step bookkeeping: relative residual of the float64 solution; finish, or start the
 // next inner solve from its residual.
 __global__ void k_check_outer(const double *__restrict__ partials, int nblk, SlotState *st,
-                              int *active, int *outer_mask, double tol, int max_cycles,
+                              int *active, int *outer_mask, const int *cancel, double tol, int max_cycles,
                               const int *wf) {
   const int inst = blockIdx.x;
   if (!outer_mask[inst]) return;
@@ -188,7 +203,9 @@ __global__ void k_check_outer(const double *__restrict__ partials, int nblk, Slo
     s.outer += 1;
     s.first = 0;
     outer_mask[inst] = 0;
-    if (waits_failed(wf)) {
+    if (cancel[inst]) {
+      // no inner solve follows
+    } else if (waits_failed(wf)) {
       s.status = HFM_ERR_TIMEOUT;
     } else if (!(rel == rel) || isinf(rel)) {
       s.status = HFM_ERR_NAN;
@@ -508,12 +525,12 @@ __global__ void k_sumsq64(const double *__restrict__ x, int64_t n, double *__res
 }
 
 // Pack the public per-slot statistics (for the asynchronous query).
-__global__ void k_pack_stats(const SlotState *st, const int *active, const int *outer, int B,
-                             hfm_slot_stats *out) {
+__global__ void k_pack_stats(const SlotState *st, const int *active, const int *outer, const int *cancel,
+                             int B, hfm_slot_stats *out) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= B) return;
   hfm_slot_stats o;
-  o.active = active[i] | (outer ? outer[i] : 0);
+  o.active = cancel[i] ? 0 : active[i] | outer[i];
   o.status = st[i].status;
   o.cycles = st[i].cycles;
   o.outer = st[i].outer;
@@ -614,7 +631,7 @@ __global__ void k_copy_active(const T *__restrict__ src, T *__restrict__ dst, in
 }
 
 // Initial state of every slot from its ||b||^2 (batched load).
-__global__ void k_init_states(SlotState *st, int *active, int B, const double *sumsq_b,
+__global__ void k_init_states(SlotState *st, int *active, int *cancel, int B, const double *sumsq_b,
                               int *outer_mask) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= B) return;
@@ -640,6 +657,7 @@ __global__ void k_init_states(SlotState *st, int *active, int B, const double *s
     s.status = (nb != nb) ? HFM_ERR_NAN : HFM_OK;
   }
   st[i] = s;
+  cancel[i] = 0;
   if (outer_mask) {
     outer_mask[i] = act;
     active[i] = 0;
@@ -945,6 +963,7 @@ struct hfm_mg {
   void *saw[2] = {nullptr, nullptr};  // sawtooth: r, w in storage type
   int *active = nullptr;
   int *outer = nullptr;     // refinement: slots whose float64 outer step is due
+  int *cancel = nullptr;    // slots to switch off at their next check
   double *x64 = nullptr;    // refinement: float64 solution and right-hand side
   double *b64 = nullptr;
   hfm::SlotState *state = nullptr;
@@ -958,8 +977,11 @@ struct hfm_mg {
   const int *wait_fail = nullptr;  // the device's TMA wait-failure counters (read by checks)
   hfm_operator fine_desc;
   cudaStream_t cap = nullptr;
-  cudaEvent_t masks_done = nullptr;  // after the last call that reads or writes the activity masks
+  cudaEvent_t masks_done = nullptr;    // after the last call that reads or writes the activity masks
+  cudaEvent_t loads_done = nullptr;    // after the last load
+  cudaEvent_t cancels_done = nullptr;  // after the last cancel
   std::mutex masks_mu;
+  std::atomic<bool> cancelled{false};  // a cancel since the last run started
   std::map<int, cudaGraphExec_t> graphs;
   std::map<int, int64_t> graph_kernels;
   std::vector<void *> allocs;
@@ -1021,7 +1043,7 @@ class Engine : public EngineBase {
   }
 
   int check(int nblk, int which, cudaStream_t s, const double *rz_new = nullptr) {
-    k_check<<<m_->slots, 256, 0, s>>>(m_->partials, nblk, m_->state, m_->active, m_->cfg.tol,
+    k_check<<<m_->slots, 256, 0, s>>>(m_->partials, nblk, m_->state, m_->active, m_->cancel, m_->cfg.tol,
                                       m_->cfg.max_cycles, which, m_->wait_fail, rz_new);
     HFM_CHECK_LAUNCH("k_check");
     return HFM_OK;
@@ -1499,7 +1521,7 @@ class Engine : public EngineBase {
                                                         g(0).Y, g(0).X, it, m_->outer, m_->partials);
     }
     HFM_CHECK_LAUNCH("k_residual64");
-    k_check_outer<<<B, 256, 0, s>>>(m_->partials, vb, m_->state, m_->active, m_->outer,
+    k_check_outer<<<B, 256, 0, s>>>(m_->partials, vb, m_->state, m_->active, m_->outer, m_->cancel,
                                     m_->cfg.tol, m_->cfg.max_cycles, m_->wait_fail);
     HFM_CHECK_LAUNCH("k_check_outer");
     return HFM_OK;
@@ -1556,7 +1578,7 @@ class Engine : public EngineBase {
                                   ir ? 1 : 0);
     HFM_CHECK_LAUNCH("k_cg_xr");
     if (!ir) return check(vb, 0, s, m_->scal);
-    k_check_inner<<<B, 256, 0, s>>>(m_->partials, vb, m_->state, m_->active, m_->outer,
+    k_check_inner<<<B, 256, 0, s>>>(m_->partials, vb, m_->state, m_->active, m_->outer, m_->cancel,
                                     m_->cfg.tol, m_->cfg.inner_tol, m_->cfg.inner_max_cycles,
                                     m_->wait_fail, m_->scal);
     HFM_CHECK_LAUNCH("k_check_inner");
@@ -1776,9 +1798,9 @@ class Engine : public EngineBase {
     if ((st = launch_finalize_sum(m_->partials, nb, count, m_->scal + (count == 1 ? m_->slots : 0), s)))
       return st;
     if (count == 1)
-      k_init_state<<<1, 1, 0, s>>>(m_->state, m_->active, slot, m_->scal + m_->slots, HFM_OK, m_->outer);
+      k_init_state<<<1, 1, 0, s>>>(m_->state, m_->active, m_->cancel, slot, m_->scal + m_->slots, HFM_OK, m_->outer);
     else
-      k_init_states<<<(count + 127) / 128, 128, 0, s>>>(m_->state, m_->active, count, m_->scal, m_->outer);
+      k_init_states<<<(count + 127) / 128, 128, 0, s>>>(m_->state, m_->active, m_->cancel, count, m_->scal, m_->outer);
     HFM_CHECK_LAUNCH("k_init_state");
     return HFM_OK;
   }
@@ -1833,7 +1855,7 @@ class Engine : public EngineBase {
     int nb = 0;
     if ((st = launch_sumsq_partials<float>(b, nf, nf, 1, m_->partials, &nb, nullptr, s))) return st;
     if ((st = launch_finalize_sum(m_->partials, nb, 1, m_->scal + m_->slots, s))) return st;
-    k_init_state<<<1, 1, 0, s>>>(m_->state, m_->active, slot, m_->scal + m_->slots, HFM_OK, nullptr);
+    k_init_state<<<1, 1, 0, s>>>(m_->state, m_->active, m_->cancel, slot, m_->scal + m_->slots, HFM_OK, nullptr);
     HFM_CHECK_LAUNCH("k_init_state");
     return HFM_OK;
   }
@@ -1856,7 +1878,7 @@ class Engine : public EngineBase {
     int nb = 0;
     if ((st = launch_sumsq_partials<float>(b, nf, nf, B, m_->partials, &nb, nullptr, s))) return st;
     if ((st = launch_finalize_sum(m_->partials, nb, B, m_->scal, s))) return st;
-    k_init_states<<<(B + 127) / 128, 128, 0, s>>>(m_->state, m_->active, B, m_->scal, nullptr);
+    k_init_states<<<(B + 127) / 128, 128, 0, s>>>(m_->state, m_->active, m_->cancel, B, m_->scal, nullptr);
     HFM_CHECK_LAUNCH("k_init_states");
     return HFM_OK;
   }
@@ -2094,24 +2116,24 @@ int hfm_mg_create(const hfm_mg_config *cfg, int Z, int Y, int X, int slots, hfm_
   if (cfg->accel != HFM_ACCEL_NONE)
     m->partials2 = (double *)dalloc(m.get(), (size_t)slots * m->partials_per_slot * 8, &st);
   m->small_ctr = (int *)dalloc(m.get(), (size_t)(slots + 1) * 4, &st);
-  // states, active and outer masks in one block, so that a query is one copy
-  m->state = (SlotState *)dalloc(m.get(), (size_t)slots * (sizeof(SlotState) + 8), &st);
+  // states, active and outer masks and cancel requests in one block, so that a query is one copy
+  m->state = (SlotState *)dalloc(m.get(), (size_t)slots * (sizeof(SlotState) + 12), &st);
   m->active = (int *)(m->state + slots);
   m->outer = m->active + slots;
+  m->cancel = m->outer + slots;
   m->stats_dev = (hfm_slot_stats *)dalloc(m.get(), (size_t)slots * sizeof(hfm_slot_stats), &st);
   m->scal = (double *)dalloc(m.get(), (size_t)(slots + 1) * 8, &st);
   m->gscale = (double *)dalloc(m.get(), (size_t)slots * 8, &st);
   if (!st) {
-    if (cudaMemset(m->active, 0, (size_t)slots * 4) != cudaSuccess ||
-        cudaMemset(m->outer, 0, (size_t)slots * 4) != cudaSuccess ||
-        cudaMemset(m->state, 0, (size_t)slots * sizeof(SlotState)) != cudaSuccess)
+    if (cudaMemset(m->state, 0, (size_t)slots * (sizeof(SlotState) + 12)) != cudaSuccess)
       st = fail(HFM_ERR_CUDA, "cudaMemset failed");
   }
   if (!st) st = wait_fail_counters(&m->wait_fail);
   if (!st && cudaStreamCreateWithFlags(&m->cap, cudaStreamNonBlocking) != cudaSuccess)
     st = fail(HFM_ERR_CUDA, "cudaStreamCreate failed");
-  if (!st && cudaEventCreateWithFlags(&m->masks_done, cudaEventDisableTiming) != cudaSuccess)
-    st = fail(HFM_ERR_CUDA, "cudaEventCreate failed");
+  for (cudaEvent_t *e : {&m->masks_done, &m->loads_done, &m->cancels_done})
+    if (!st && cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess)
+      st = fail(HFM_ERR_CUDA, "cudaEventCreate failed");
   if (!st) {
     switch (cfg->storage) {
       case HFM_F32: m->eng.reset(new Engine<float>(m.get())); break;
@@ -2131,7 +2153,8 @@ int hfm_mg_create(const hfm_mg_config *cfg, int Z, int Y, int X, int slots, hfm_
   if (st) {
     for (void *p : m->allocs) cudaFree(p);
     if (m->cap) cudaStreamDestroy(m->cap);
-    if (m->masks_done) cudaEventDestroy(m->masks_done);
+    for (cudaEvent_t e : {m->masks_done, m->loads_done, m->cancels_done})
+      if (e) cudaEventDestroy(e);
     return st;
   }
   // default constant operator so that CONST7 / K27 handles work after set_operator only
@@ -2147,7 +2170,8 @@ int hfm_mg_destroy(hfm_mg *m) {
     cudaStreamDestroy(m->cap);
   }
   cudaDeviceSynchronize();
-  if (m->masks_done) cudaEventDestroy(m->masks_done);
+  for (cudaEvent_t e : {m->masks_done, m->loads_done, m->cancels_done})
+    if (e) cudaEventDestroy(e);
   for (void *p : m->allocs) cudaFree(p);
   delete m;
   return HFM_OK;
@@ -2171,14 +2195,18 @@ int hfm_mg_set_operator(hfm_mg *m, int slot, const hfm_operator *op, hfm_stream_
 }  // extern "C"
 
 namespace {
-// Orders the calls that write a many-slot handle's activity masks (load, cancel) and those that
-// read them (run) when a caller uses several streams or threads: the blocks of a launch share
-// out the active slots, so a mask that changed while it ran would take work from other slots.
-// A call waits on its stream for the one before it; on one stream that is no wait.  A caller's
-// own capture keeps the order of the captured stream.
+// Orders the calls on a many-slot handle when a caller uses several streams or threads.  The blocks
+// of a launch share out the active slots, so a mask that changed while it ran would take work
+// from other slots: loads, which write the masks, and runs, which read them, wait on their stream
+// for the ones before them (on one stream that is no wait).  A cancel only sets the slot's request,
+// which the checks of a run act on, so it waits for no run; it is ordered among the loads and
+// cancels before it, and a load among the cancels before it.  A caller's own capture keeps the order
+// of the captured stream.
+enum MaskCall { MASK_LOAD, MASK_RUN, MASK_CANCEL };
 class MaskOrder {
  public:
-  MaskOrder(hfm_mg *m, cudaStream_t s) : m_(m), s_(s), on_(m->slots > 1), lk_(m->masks_mu, std::defer_lock) {
+  MaskOrder(hfm_mg *m, MaskCall call, cudaStream_t s)
+      : m_(m), call_(call), s_(s), on_(m->slots > 1), lk_(m->masks_mu, std::defer_lock) {
     if (!on_) return;
     lk_.lock();
     cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
@@ -2188,16 +2216,21 @@ class MaskOrder {
     } else if (c != cudaStreamCaptureStatusNone) {
       on_ = false;
     }
-    if (on_) cudaStreamWaitEvent(s_, m_->masks_done, 0);
+    if (!on_) return;
+    cudaStreamWaitEvent(s_, call == MASK_CANCEL ? m->loads_done : m->masks_done, 0);
+    if (call != MASK_RUN) cudaStreamWaitEvent(s_, m->cancels_done, 0);
   }
   ~MaskOrder() {
-    if (on_) cudaEventRecord(m_->masks_done, s_);
+    if (!on_) return;
+    cudaEventRecord(call_ == MASK_CANCEL ? m_->cancels_done : m_->masks_done, s_);
+    if (call_ == MASK_LOAD) cudaEventRecord(m_->loads_done, s_);
   }
   MaskOrder(const MaskOrder &) = delete;
   MaskOrder &operator=(const MaskOrder &) = delete;
 
  private:
   hfm_mg *m_;
+  MaskCall call_;
   cudaStream_t s_;
   bool on_;
   std::unique_lock<std::mutex> lk_;
@@ -2208,13 +2241,18 @@ extern "C" {
 
 int hfm_mg_load(hfm_mg *m, int slot, const float *rhs, const float *phi0, hfm_stream_t stream) {
   if (!m || !rhs || slot < 0 || slot >= m->slots) return fail(HFM_ERR_BAD_ARG, "hfm_mg_load: bad argument");
-  MaskOrder order(m, (cudaStream_t)stream);
+  MaskOrder order(m, MASK_LOAD, (cudaStream_t)stream);
   return m->eng->load(slot, rhs, phi0, (cudaStream_t)stream);
 }
 
 int hfm_mg_run(hfm_mg *m, int cycles, hfm_stream_t stream) {
   if (!m || cycles < 1) return fail(HFM_ERR_BAD_ARG, "hfm_mg_run: bad argument");
-  MaskOrder order(m, (cudaStream_t)stream);
+  MaskOrder order(m, MASK_RUN, (cudaStream_t)stream);
+  if (m->cancelled.exchange(false)) {
+    k_drop_cancelled<<<(m->slots + 127) / 128, 128, 0, (cudaStream_t)stream>>>(m->cancel, m->active, m->outer,
+                                                                             m->slots);
+    HFM_CHECK_LAUNCH("k_drop_cancelled");
+  }
   cudaGraphExec_t exec = nullptr;
   auto it = m->graphs.find(cycles);
   if (it != m->graphs.end()) {
@@ -2254,16 +2292,16 @@ int hfm_mg_run(hfm_mg *m, int cycles, hfm_stream_t stream) {
 
 int hfm_mg_query(hfm_mg *m, hfm_slot_stats *out, hfm_stream_t stream) {
   if (!m || !out) return fail(HFM_ERR_BAD_ARG, "hfm_mg_query: bad argument");
-  // one copy of the block that holds states, active and outer masks
+  // one copy of the block that holds states, active and outer masks and cancel requests
   cudaStream_t s = (cudaStream_t)stream;
-  std::vector<SlotState> buf(m->slots + (m->slots * 8 + sizeof(SlotState) - 1) / sizeof(SlotState));
-  HFM_CUDA(cudaMemcpyAsync(buf.data(), m->state, (size_t)m->slots * (sizeof(SlotState) + 8),
+  std::vector<SlotState> buf(m->slots + (m->slots * 12 + sizeof(SlotState) - 1) / sizeof(SlotState));
+  HFM_CUDA(cudaMemcpyAsync(buf.data(), m->state, (size_t)m->slots * (sizeof(SlotState) + 12),
                            cudaMemcpyDeviceToHost, s));
   HFM_CUDA(cudaStreamSynchronize(s));
   const SlotState *st = buf.data();
-  const int *act = (const int *)(st + m->slots), *outer = act + m->slots;
+  const int *act = (const int *)(st + m->slots), *outer = act + m->slots, *cancel = outer + m->slots;
   for (int i = 0; i < m->slots; ++i) {
-    out[i].active = act[i] | outer[i];
+    out[i].active = cancel[i] ? 0 : act[i] | outer[i];
     out[i].status = st[i].status;
     out[i].cycles = st[i].cycles;
     out[i].outer = st[i].outer;
@@ -2276,7 +2314,7 @@ int hfm_mg_query(hfm_mg *m, hfm_slot_stats *out, hfm_stream_t stream) {
 int hfm_mg_query_async(hfm_mg *m, hfm_slot_stats *stats_host, hfm_stream_t stream) {
   if (!m || !stats_host) return fail(HFM_ERR_BAD_ARG, "hfm_mg_query_async: bad argument");
   cudaStream_t s = (cudaStream_t)stream;
-  k_pack_stats<<<(m->slots + 127) / 128, 128, 0, s>>>(m->state, m->active, m->outer, m->slots,
+  k_pack_stats<<<(m->slots + 127) / 128, 128, 0, s>>>(m->state, m->active, m->outer, m->cancel, m->slots,
                                                       m->stats_dev);
   HFM_CHECK_LAUNCH("k_pack_stats");
   HFM_CUDA(cudaMemcpyAsync(stats_host, m->stats_dev, m->slots * sizeof(hfm_slot_stats),
@@ -2291,16 +2329,16 @@ int hfm_mg_fetch(hfm_mg *m, int slot, float *out, hfm_stream_t stream) {
 
 int hfm_mg_cancel(hfm_mg *m, int slot, hfm_stream_t stream) {
   if (!m || slot < 0 || slot >= m->slots) return fail(HFM_ERR_BAD_ARG, "hfm_mg_cancel: bad argument");
-  MaskOrder order(m, (cudaStream_t)stream);
-  HFM_CUDA(cudaMemsetAsync(m->active + slot, 0, 4, (cudaStream_t)stream));
-  HFM_CUDA(cudaMemsetAsync(m->outer + slot, 0, 4, (cudaStream_t)stream));
+  MaskOrder order(m, MASK_CANCEL, (cudaStream_t)stream);
+  HFM_CUDA(cudaMemsetAsync(m->cancel + slot, 1, 4, (cudaStream_t)stream));
+  m->cancelled = true;
   return HFM_OK;
 }
 
 int hfm_mg_load_f64(hfm_mg *m, int slot, const double *rhs, const double *phi0,
                     hfm_stream_t stream) {
   if (!m || !rhs || slot < 0 || slot >= m->slots) return fail(HFM_ERR_BAD_ARG, "hfm_mg_load_f64: bad argument");
-  MaskOrder order(m, (cudaStream_t)stream);
+  MaskOrder order(m, MASK_LOAD, (cudaStream_t)stream);
   return m->eng->load64(slot, rhs, phi0, (cudaStream_t)stream);
 }
 
@@ -2319,7 +2357,7 @@ int hfm_mg_solve(hfm_mg *m, const float *rhs, float *phi, hfm_slot_stats *stats_
   if (!m || !rhs || !phi) return fail(HFM_ERR_BAD_ARG, "hfm_mg_solve: bad argument");
   int st;
   {
-    MaskOrder order(m, (cudaStream_t)stream);
+    MaskOrder order(m, MASK_LOAD, (cudaStream_t)stream);
     if ((st = m->eng->load_all(rhs, (cudaStream_t)stream))) return st;
   }
   std::vector<hfm_slot_stats> tmp(m->slots);

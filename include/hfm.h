@@ -547,7 +547,9 @@ int hfm_mg_level_shape(const hfm_mg *mg, int level, int *Z, int *Y, int *X);
  * hierarchy by the reference restriction (BGS_multigrid_v1.ipynb cell 38, lines 16-33).
  * SIGMA7 coefficient arrays hold one instance each ([Z][Y][X]); they are copied. */
 int hfm_mg_set_operator(hfm_mg *mg, int slot, const hfm_operator *op, hfm_stream_t stream);
-/* Copy rhs (and phi0, NULL = zero) into a slot, compute ||b|| and mark it active. */
+/* Copy rhs (and phi0, NULL = zero) into a slot, compute ||b|| and mark it active.  On a handle of
+ * several slots, loads and runs wait for the ones before them on other streams or threads, and a
+ * load for the cancels before it; a load replayed from a caller's graph is ordered by the caller. */
 int hfm_mg_load(hfm_mg *mg, int slot, const float *rhs, const float *phi0, hfm_stream_t stream);
 /* Advance every active slot by `cycles` cycles (CUDA graph; slots that converge, fail or
  * hit max_cycles stop on the device and do no more work). */
@@ -560,8 +562,9 @@ int hfm_mg_query(hfm_mg *mg, hfm_slot_stats *stats_host, hfm_stream_t stream);
 int hfm_mg_query_async(hfm_mg *mg, hfm_slot_stats *stats_host, hfm_stream_t stream);
 /* Copy a slot's current solution into phi_out (device, [Z][Y][X] float32). */
 int hfm_mg_fetch(hfm_mg *mg, int slot, float *phi_out, hfm_stream_t stream);
-/* Stop a slot (request cancelled); its memory can be reloaded at once.  From another stream or
- * thread than the runs', it takes effect after the run in flight. */
+/* Stop a slot (request cancelled); its memory can be reloaded at once.  A later run on the same
+ * stream does no work for it; from another stream or thread it waits for no run and ends the
+ * slot at the next convergence check of the run in flight. */
 int hfm_mg_cancel(hfm_mg *mg, int slot, hfm_stream_t stream);
 /* Convenience: load all slots from rhs/phi ([slots][Z][Y][X]), run to completion, fetch the
  * solutions into phi, fill stats_host (may be NULL).  Synchronises `stream`. */
