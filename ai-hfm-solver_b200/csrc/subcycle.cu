@@ -213,9 +213,10 @@ __device__ void sub_faces_init(const SubLevel<T> &L, int64_t inst, float *Fc) {
   }
 }
 
-// The coarse-end V-cycle of one instance with the block's shared memory `sub_smem`.  COH:
-// the right-hand side was written by other blocks of the same launch (read through L2).
-template <int KIND, class T, bool COH>
+// The coarse-end V-cycle of one instance with the block's shared memory `sub_smem`, for the
+// persistent kernel below: other blocks of the same launch wrote the right-hand side, so it is
+// read through L2.
+template <int KIND, class T>
 __device__ void subcycle_body(const SubArgs<T> &a, int64_t inst, unsigned char *sub_smem) {
   float *F = reinterpret_cast<float *>(sub_smem);
   const int nl = a.nlev;
@@ -227,8 +228,7 @@ __device__ void subcycle_body(const SubArgs<T> &a, int64_t inst, unsigned char *
     if (KIND == HFM_OP_SIGMA7) sub_faces_init<T>(L, inst, F + L.o_face);
   }
   for (int i = threadIdx.x; i < a.lv[0].n; i += blockDim.x) {
-    const T *src = a.rhs + inst * (int64_t)a.lv[0].n + i;
-    F[a.lv[0].o_rhs + i] = St<T>::to(COH ? ld_l2<T>(src) : *src);
+    F[a.lv[0].o_rhs + i] = St<T>::to(ld_l2<T>(a.rhs + inst * (int64_t)a.lv[0].n + i));
   }
   __syncthreads();
 
@@ -1350,7 +1350,7 @@ __global__ void __launch_bounds__(kSubThreads) k_small(const __grid_constant__ S
     }
     __syncthreads();
     if (ok_sh) {
-      if (a.kind[s] == SK_SUB) subcycle_body<KIND, T, true>(a.sub, inst, sub_smem);
+      if (a.kind[s] == SK_SUB) subcycle_body<KIND, T>(a.sub, inst, sub_smem);
       else if (a.kind[s] == SK_RESTRICT) small_restrict<KIND, T>(a, s, inst, tile);
       else small_sweep<KIND, T>(a, s, inst, tile);
     }
