@@ -422,7 +422,7 @@ template <class T> struct SubLevel {
   int o_phi, o_tmp, o_rhs;   // float offsets of the level's fields in shared memory
   int o_face;                // float offset of its face arrays and diagonal (SIGMA7)
   int o_idx;                 // float offset of its cell table (8 or 4 bytes per cell)
-  int bx, by;                // bits of x and of y in a 4-byte table's coordinates
+  int bx, by;                // bits of x and of y in a narrow table's coordinates
 };
 template <class T> struct SubArgs {
   SubLevel<T> lv[kMaxSubLevels];

@@ -347,16 +347,16 @@ __device__ void subcycle_body(const SubArgs<T> &a, int64_t inst, unsigned char *
 // per sweep of 16^3.
 constexpr int kProgThreads = 512;
 
-// Cell i of a level: padded index and coordinates, from a table formed once per launch.  With level
-// l0 in quads (TOP) it takes 8 bytes a cell; without, where the levels may fill the shared memory,
-// 4: 16 bits of padded index (at most 36882, 1 x 1 x 4096) below the coordinates, whose bits add
-// up to 15 at most (a level has 4096 cells at most).  (4 bytes for both: the compiler then keeps
-// fewer of the 27-point weights in registers, and the 16 x 32 x 32 program takes 24 us, not 20.)
+// Cell i of a level: padded index and coordinates, from a table formed once per launch.  It takes 8
+// bytes a cell, or, where these would not fit (NARROW), 4: 16 bits of padded index (at most 36882,
+// 1 x 1 x 4096) below the coordinates, whose bits add up to 15 at most (a level has 4096 cells at
+// most).  (With narrow tables the compiler keeps fewer of the 27-point weights in registers where
+// level l0 is in quads: 16 x 32 x 32 takes 24 us, not 20.)
 struct Cell {
   int ip, z, y, x;
 };
-template <bool TOP, class T> __device__ __forceinline__ Cell cell_of(const SubLevel<T> &L, const float *F, int i) {
-  if constexpr (TOP) {
+template <bool NARROW, class T> __device__ __forceinline__ Cell cell_of(const SubLevel<T> &L, const float *F, int i) {
+  if constexpr (!NARROW) {
     const uint2 u = reinterpret_cast<const uint2 *>(F + L.o_idx)[i];
     return Cell{(int)(u.x & 0xffffu), (int)(u.x >> 16), (int)(u.y >> 16), (int)(u.y & 0xffffu)};
   } else {
@@ -365,10 +365,10 @@ template <bool TOP, class T> __device__ __forceinline__ Cell cell_of(const SubLe
                 (int)(c & ((1u << L.bx) - 1u))};
   }
 }
-template <bool TOP, class T>
+template <bool NARROW, class T>
 __device__ __forceinline__ void set_cell(const SubLevel<T> &L, float *F, int i, int z, int y, int x) {
   const unsigned ip = (unsigned)pix(z, y, x, L.Y, L.X);
-  if constexpr (TOP)
+  if constexpr (!NARROW)
     reinterpret_cast<uint2 *>(F + L.o_idx)[i] = make_uint2(ip | ((unsigned)z << 16), ((unsigned)y << 16) | (unsigned)x);
   else
     reinterpret_cast<unsigned *>(F + L.o_idx)[i] =
@@ -378,12 +378,12 @@ __device__ __forceinline__ void set_cell(const SubLevel<T> &L, float *F, int i, 
 // A thread-strided pass over the cells of level L.
 #define HFM_FOR_CELLS(L, F)                                                              \
   for (int i = threadIdx.x; i < (L).n; i += kProgThreads) {                              \
-    const Cell q = cell_of<TOP>(L, F, i);
+    const Cell q = cell_of<NARROW>(L, F, i);
 
 // Cell i of level L: its table entry and, for SIGMA7, its face coefficients (the low ones,
 // and the high ones at the walls) and 1 / diagonal.  The global loads and the shared-memory
 // stores are apart, so that the loads can be in flight while the block clears its fields.
-template <int KIND, class T, bool TOP> struct CellInit {
+template <int KIND, class T, bool NARROW> struct CellInit {
   int x, y, z, t, i;
   float vx, vy, vz, xl, xh, yl, yh, zl, zh;
   __device__ __forceinline__ void load(const SubLevel<T> &L, int64_t inst, int cell) {
@@ -410,7 +410,7 @@ template <int KIND, class T, bool TOP> struct CellInit {
   }
   __device__ __forceinline__ void store(const SubLevel<T> &L, float *F) const {
     const int X = L.X, Y = L.Y, Z = L.Z, P = X * Y;
-    set_cell<TOP>(L, F, i, z, y, x);
+    set_cell<NARROW>(L, F, i, z, y, x);
     if (KIND == HFM_OP_SIGMA7) {
       const float axm = L.cx * (0.5f * (vx + xl)), axp = L.cx * (0.5f * (vx + xh));
       const float aym = L.cy * (0.5f * (vy + yl)), ayp = L.cy * (0.5f * (vy + yh));
@@ -549,7 +549,7 @@ template <int KIND> struct CellPair {
 };
 
 // One sweep of a level's iterate `in` (null: zero) into `out`.
-template <int KIND, bool TOP, class T>
+template <int KIND, bool NARROW, class T>
 __device__ void prog_sweep(const SubLevel<T> &L, float *F, const float *in, float *out, float om) {
   const float *f = F + L.o_rhs, *Fc = F + L.o_face;
   const float *rd = Fc + sub_faces(L.Z, L.Y, L.X);
@@ -570,7 +570,7 @@ __device__ void prog_sweep(const SubLevel<T> &L, float *F, const float *in, floa
 
 // The second phase of a restriction: each coarse cell's eight fine residuals (padded field,
 // ordered z, y, x), averaged into the coarse level's right-hand side.
-template <bool TOP, class T>
+template <bool NARROW, class T>
 __device__ void prog_sum8(const SubLevel<T> &L, float *F, const float *res, const SubLevel<T> &Lc) {
   __syncthreads();
   const int PX = L.X + 2, PXY = PX * (L.Y + 2);
@@ -586,7 +586,7 @@ __device__ void prog_sum8(const SubLevel<T> &L, float *F, const float *res, cons
 
 // Next level's right-hand side = R(A phi - f) (phi null: zero): every fine residual by its own
 // thread into `res`, then the sums.
-template <int KIND, bool TOP, class T>
+template <int KIND, bool NARROW, class T>
 __device__ void prog_restrict(const SubLevel<T> &L, float *F, const float *ph, float *res,
                               const SubLevel<T> &Lc) {
   const float *f = F + L.o_rhs, *Fc = F + L.o_face;
@@ -595,11 +595,11 @@ __device__ void prog_restrict(const SubLevel<T> &L, float *F, const float *ph, f
     const float ax = ph ? sub_apply<KIND, T>(L, ph, Fc, q.z, q.y, q.x, q.ip, i, &dg) : 0.f;
     res[q.ip] = ax - f[i];
   }
-  prog_sum8<TOP, T>(L, F, res, Lc);
+  prog_sum8<NARROW, T>(L, F, res, Lc);
 }
 
 // Next level's right-hand side = R f
-template <bool TOP, class T>
+template <bool NARROW, class T>
 __device__ void prog_restrict_rhs(const SubLevel<T> &L, float *F, const SubLevel<T> &Lc) {
   const float *f = F + L.o_rhs;
   HFM_FOR_CELLS(Lc, F)
@@ -613,7 +613,7 @@ __device__ void prog_restrict_rhs(const SubLevel<T> &L, float *F, const SubLevel
 }
 
 // phi = [phi] + sign * P(coarse) on the level's interior (both padded)
-template <bool TOP, class T>
+template <bool NARROW, class T>
 __device__ void prog_correct(const SubLevel<T> &L, float *F, float *ph, const SubLevel<T> &Lc,
                              const float *coarse, float sign, bool zero) {
   HFM_FOR_CELLS(L, F)
@@ -626,12 +626,12 @@ __device__ void prog_correct(const SubLevel<T> &L, float *F, float *ph, const Su
 // The coarsest level's sweeps of a 7-point operator, one cell per thread (a warp's chain of
 // dependent instructions sets the time of these sweeps: 218 cycles for 64 cells on two warps,
 // 456 in pairs on one warp).  Unrolled by two, so that each field's addresses are formed once.
-template <int KIND, bool TOP, class T>
+template <int KIND, bool NARROW, class T>
 __device__ __forceinline__ void coarse_cells7(const SubLevel<T> &L, float *F, float om, int sweeps, int nthr) {
   const int X = L.X, Y = L.Y, Z = L.Z, PX = X + 2, PXY = PX * (Y + 2), P = X * Y;
   const bool in = (int)threadIdx.x < L.n;
   const int i = in ? threadIdx.x : L.n - 1;
-  const Cell q = cell_of<TOP>(L, F, i);
+  const Cell q = cell_of<NARROW>(L, F, i);
   float c[6], od;
   if (KIND == HFM_OP_CONST7) {
     c[0] = c[1] = L.k[2];
@@ -670,21 +670,25 @@ __device__ __forceinline__ void coarse_cells7(const SubLevel<T> &L, float *F, fl
 // Where the block has a thread for each cell (K27: for each pair of cells, whose 27 neighbours
 // mostly coincide), coefficients stay in registers and a barrier among the warps that hold
 // cells (a warp barrier when one does) parts the sweeps.
-template <int KIND, bool TOP, class T>
+template <int KIND, bool NARROW, bool TOP, class T>
 __device__ int prog_coarse(const SubLevel<T> &L, float *F, float om, int sweeps) {
   const int np = KIND == HFM_OP_K27 ? cell_pairs(L.Z, L.Y, L.X) : L.n;
   if (np > kProgThreads) {
     for (int k = 0; k < sweeps; ++k)
-      prog_sweep<KIND, TOP, T>(L, F, k == 0 ? nullptr : F + (k & 1 ? L.o_tmp : L.o_phi), F + (k & 1 ? L.o_phi : L.o_tmp), om);
+      prog_sweep<KIND, NARROW, T>(L, F, k == 0 ? nullptr : F + (k & 1 ? L.o_tmp : L.o_phi), F + (k & 1 ? L.o_phi : L.o_tmp), om);
     return sweeps & 1;
   }
   const int nthr = (np + 31) & ~31;
   if ((int)threadIdx.x < nthr) {
     if constexpr (KIND != HFM_OP_K27) {
-      coarse_cells7<KIND, TOP, T>(L, F, om, sweeps, nthr);
+      coarse_cells7<KIND, NARROW, T>(L, F, om, sweeps, nthr);
     } else {
       CellPair<KIND> c;
       c.load(L, F, threadIdx.x);
+      if (!TOP) {  // left alone the compiler reads the weights anew in every sweep (6 x 10 x 14: 33.0, not 36.9 us)
+#pragma unroll
+        for (int j = 0; j < 27; ++j) asm volatile("" : "+f"(c.w[j]));
+      }
       float f[2];
       c.rhs(L, F + L.o_rhs, f);
       c.sweep0(f, om);
@@ -962,7 +966,7 @@ template <int KIND> struct TopPair {
   }
 };
 
-template <int KIND, class T, bool TOP>
+template <int KIND, class T, bool TOP, bool NARROW>
 __global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant__ SubProgram<T> P) {
   const SubArgs<T> &a = P.a;
   const int64_t inst = blockIdx.x;
@@ -975,7 +979,7 @@ __global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant_
   // cell is loaded, then its quads; meanwhile the block clears its shared memory (the ghosts
   // of the fields stay zero)
   constexpr int LB = TOP ? 1 : 0;
-  CellInit<KIND, T, TOP> ci;
+  CellInit<KIND, T, NARROW> ci;
   int l = nl - 1, first = 0;
   int k = threadIdx.x;
   auto find = [&]() {
@@ -1024,7 +1028,7 @@ __global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant_
     float *other = F + (c ? L.o_phi : L.o_tmp);
     float *coarse = F + (((cur >> (l + 1)) & 1) ? Lc.o_tmp : Lc.o_phi);
     if (op == SO_COARSE) {
-      const int r = prog_coarse<KIND, TOP, T>(L, F, a.coarse_omega, cnt);
+      const int r = prog_coarse<KIND, NARROW, TOP, T>(L, F, a.coarse_omega, cnt);
       cur = (cur & ~(1u << l)) | ((unsigned)r << l);
     } else if (op == SO_SWEEP0 || op == SO_SWEEP) {
       for (int n = 0; n < cnt; ++n) {
@@ -1056,7 +1060,7 @@ __global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant_
           }
           __syncthreads();
         } else {
-          prog_sweep<KIND, TOP, T>(L, F, zero ? nullptr : ph, other, a.omega);
+          prog_sweep<KIND, NARROW, T>(L, F, zero ? nullptr : ph, other, a.omega);
         }
         float *t = ph;
         ph = other;
@@ -1098,9 +1102,9 @@ __global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant_
           }
           mc.store(L1, other, r);
         }
-        prog_sum8<TOP, T>(L1, F, other, Lc);
+        prog_sum8<NARROW, T>(L1, F, other, Lc);
       } else {
-        prog_restrict<KIND, TOP, T>(L, F, zero ? nullptr : ph, other, Lc);
+        prog_restrict<KIND, NARROW, T>(L, F, zero ? nullptr : ph, other, Lc);
       }
     } else if (op == SO_RESTRICT_RHS) {
       if (TOP && l == 0) {
@@ -1114,7 +1118,7 @@ __global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant_
         }
         __syncthreads();
       } else {
-        prog_restrict_rhs<TOP, T>(L, F, Lc);
+        prog_restrict_rhs<NARROW, T>(L, F, Lc);
       }
     } else {  // SO_CORRECT0, SO_CORRECT, SO_PROLONG
       const float sign = op == SO_PROLONG ? 1.f : -1.f;
@@ -1134,7 +1138,7 @@ __global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant_
         __syncthreads();
       } else if (mid && l == 1) {
         if (mc.valid) {
-          const Cell q = cell_of<TOP>(L1, F, mc.i);
+          const Cell q = cell_of<NARROW>(L1, F, mc.i);
           const float d = sign * coarse[pix(q.z >> 1, q.y >> 1, q.x >> 1, Lc.Y, Lc.X)];
           mc.v[0] = zero ? d : mc.v[0] + d;
           mc.v[1] = !mc.two ? 0.f : zero ? d : mc.v[1] + d;
@@ -1142,7 +1146,7 @@ __global__ void __launch_bounds__(kProgThreads) k_subprog(const __grid_constant_
         }
         __syncthreads();
       } else {
-        prog_correct<TOP, T>(L, F, ph, Lc, coarse, sign, zero);
+        prog_correct<NARROW, T>(L, F, ph, Lc, coarse, sign, zero);
       }
     }
   }
@@ -1393,12 +1397,12 @@ template int launch_small<float>(int, SmallArgs<float>, int, cudaStream_t);
 template int launch_small<__nv_bfloat16>(int, SmallArgs<__nv_bfloat16>, int, cudaStream_t);
 template int launch_small<__half>(int, SmallArgs<__half>, int, cudaStream_t);
 
-template <int KIND, class T, bool TOP>
+template <int KIND, class T, bool TOP, bool NARROW>
 int go_subprog(const SubProgram<T> &p, int B, size_t smem, cudaStream_t s) {
-  int st = set_max_dynamic_smem((const void *)k_subprog<KIND, T, TOP>, (int)kProgramMaxSmem,
+  int st = set_max_dynamic_smem((const void *)k_subprog<KIND, T, TOP, NARROW>, (int)kProgramMaxSmem,
                                 "cudaFuncSetAttribute(k_subprog)");
   if (st) return st;
-  k_subprog<KIND, T, TOP><<<B, kProgThreads, smem, s>>>(p);
+  k_subprog<KIND, T, TOP, NARROW><<<B, kProgThreads, smem, s>>>(p);
   HFM_CHECK_LAUNCH("k_subprog");
   return HFM_OK;
 }
@@ -1413,7 +1417,7 @@ template <class T> bool program_top(const SubProgram<T> &p) {
 // Shared-memory layout of a program: per level the fields, right-hand side and faces as
 // layout_sub places them, then the cell table; the quad form of level l0 keeps two fields
 // without x ghosts and the pair sums only.  Returns the bytes.
-template <class T> size_t layout_program(int kind, SubProgram<T> &p) {
+template <class T> size_t layout_program(int kind, SubProgram<T> &p, bool narrow) {
   const bool top = program_top(p);
   int64_t off = 0;
   for (int l = 0; l < p.a.nlev; ++l) {
@@ -1440,31 +1444,43 @@ template <class T> size_t layout_program(int kind, SubProgram<T> &p) {
     off = q.o_face + (kind == HFM_OP_SIGMA7 ? sub_faces(q.Z, q.Y, q.X) + q.n : 0);
     off = (off + 1) & ~1;
     q.o_idx = (int)off;
-    off = (off + (top ? 2 : 1) * q.n + 3) & ~3;
+    off = (off + (narrow ? 1 : 2) * q.n + 3) & ~3;
   }
   off = (off + 3) & ~3;
   p.clear = (int)(off / 4);
   return (size_t)off * 4;
 }
 
+// Lays the program out, with narrow cell tables where the wide ones do not fit.  Level l0 in
+// quads always leaves room for wide ones.
+template <class T> size_t place_program(int kind, SubProgram<T> &p, bool &narrow) {
+  size_t smem = layout_program<T>(kind, p, narrow = false);
+  if (smem > kProgramMaxSmem && !program_top(p)) smem = layout_program<T>(kind, p, narrow = true);
+  return smem;
+}
+
 template <class T> bool subprogram_fits(int kind, SubProgram<T> &p) {
-  return layout_program<T>(kind, p) <= kProgramMaxSmem;
+  bool narrow;
+  return place_program<T>(kind, p, narrow) <= kProgramMaxSmem;
 }
 
 template <class T>
 int launch_subprogram(int kind, SubProgram<T> &p, int B, cudaStream_t s) {
-  const bool top = program_top(p);
-  const size_t smem = layout_program<T>(kind, p);
+  bool narrow;
+  const size_t smem = place_program<T>(kind, p, narrow);
   if (smem > kProgramMaxSmem) return fail(HFM_ERR_BAD_ARG, "subcycle: levels exceed shared memory");
+  const bool top = program_top(p);
+#define HFM_SUBPROG(KIND)                                                   \
+  return top      ? go_subprog<KIND, T, true, false>(p, B, smem, s)         \
+         : narrow ? go_subprog<KIND, T, false, true>(p, B, smem, s)         \
+                  : go_subprog<KIND, T, false, false>(p, B, smem, s)
   switch (kind) {
-    case HFM_OP_SIGMA7:
-      return top ? go_subprog<HFM_OP_SIGMA7, T, true>(p, B, smem, s) : go_subprog<HFM_OP_SIGMA7, T, false>(p, B, smem, s);
-    case HFM_OP_CONST7:
-      return top ? go_subprog<HFM_OP_CONST7, T, true>(p, B, smem, s) : go_subprog<HFM_OP_CONST7, T, false>(p, B, smem, s);
-    case HFM_OP_K27:
-      return top ? go_subprog<HFM_OP_K27, T, true>(p, B, smem, s) : go_subprog<HFM_OP_K27, T, false>(p, B, smem, s);
+    case HFM_OP_SIGMA7: HFM_SUBPROG(HFM_OP_SIGMA7);
+    case HFM_OP_CONST7: HFM_SUBPROG(HFM_OP_CONST7);
+    case HFM_OP_K27: HFM_SUBPROG(HFM_OP_K27);
     default: return fail(HFM_ERR_UNSUPPORTED, "subcycle: operator kind");
   }
+#undef HFM_SUBPROG
 }
 
 template bool subprogram_fits<float>(int, SubProgram<float> &);
