@@ -27,8 +27,10 @@ __device__ __forceinline__ float at(const float *f, int z, int y, int x, int Z, 
 // all four cells, and the products run two cells per instruction on the packed float32 pipe
 // (fma.rn.f32x2, each weight stored twice).  Taps are summed in the order (dz, dy, dx) with
 // one fused multiply-add each, zero weights included.  Bound by the packed FMA issue and the
-// L1 loads, about equally: at 64 x 128 x 128 k_momentum takes 13 us and
-// k_divergence 7 us; one cell per thread with a bounds check per tap took 71 and 75 us.
+// L1 loads, about equally: at 64 x 128 x 128 k_momentum takes 22 us, k_divergence 13 us and
+// k_pgrad 11 us; one cell per thread with a bounds check per tap took 68, 73 and 31 us.  Rows
+// that are no multiple of four cells take the same quads with scalar loads (27, 22 and 14 us
+// at 64 x 128 x 130).
 constexpr int kRowThreads = 128;
 
 struct W4 {

@@ -421,7 +421,7 @@ int hfm_update2d(float *p, int dtype, const void *w, float sign, int64_t n, hfm_
  * shared memory (the coarsest level of a cycle). */
 int hfm_coarse_jacobi2d(int dtype, const float *w9_host, const void *rhs, void *out, int B, int Y,
                         int X, float omega, int sweeps, unsigned flags, hfm_stream_t stream);
-/* The V-cycle of the coarse levels in one launch, one 1024-thread block per instance with
+/* The V-cycle of the coarse levels in one launch, one 512-thread block per instance with
  * every field in shared memory (float32 between sweeps): from rhs on a first level of at most
  * 4096 cells (Y x X, each coarser level Y/2 x X/2, extents even above the coarsest), nlev <= 8
  * levels with weights w9_levels[9 l .. 9 l + 8], nu_pre >= 1 weighted-Jacobi sweeps from
