@@ -43,7 +43,7 @@ class SolverConfig:
     cycles_per_launch: int = 4
     inner_tol: float = 1e-6     # "ir": inner CG stops at max(inner_tol ||r0||, 0.3 tol ||b||)
     inner_max_cycles: int = 200
-    fused_coarse: bool = True   # deep V-cycle levels (<= 4096 cells) in one fused kernel
+    fused_coarse: bool = True   # deep levels (<= 4096 cells) of a cycle in one fused kernel
     fused_pre: bool = True      # first two pre-sweeps from zero in one pass (SIGMA7, TMA levels)
     faces: bool = True          # 16-bit SIGMA7: face-coefficient kernels on the TMA levels
     persistent: bool = False    # small end of the V-cycle as one persistent kernel (>= 8 slots)

@@ -488,9 +488,9 @@ typedef struct {
   int options;             /* HFM_OPT_* bits (default 0) */
 } hfm_mg_config;
 
-/* options: run every level of the V-cycle as separate kernel launches, including the deep
- * levels that otherwise run as one fused kernel (one block per instance, fields in shared
- * memory, for SIGMA7 levels of at most 4096 cells) */
+/* options: run every level of a cycle as separate kernel launches, including the deep levels that
+ * otherwise run as one fused kernel (V, F and sawtooth cycles; one block per instance, fields in
+ * shared memory, for SIGMA7, CONST7 and 27-point levels of at most 4096 cells) */
 #define HFM_OPT_NO_FUSED_COARSE 1
 /* options: run the first two pre-smoothing sweeps from zero as two passes instead of one
  * (by default the pointwise first sweep phi1 = omega f / diag is formed inside the second) */
