@@ -977,10 +977,9 @@ struct hfm_mg {
   const int *wait_fail = nullptr;  // the device's TMA wait-failure counters (read by checks)
   hfm_operator fine_desc;
   cudaStream_t cap = nullptr;
-  cudaEvent_t masks_done = nullptr;    // after the last call that reads or writes the activity masks
-  cudaEvent_t loads_done = nullptr;    // after the last load
-  cudaEvent_t cancels_done = nullptr;  // after the last cancel
+  cudaEvent_t runs_done = nullptr, loads_done = nullptr, cancels_done = nullptr;  // after the last of each
   std::mutex masks_mu;
+  bool runs = false, cancels = false;  // there was one since the last load (under masks_mu)
   std::atomic<bool> cancelled{false};  // a cancel since the last run started
   std::map<int, cudaGraphExec_t> graphs;
   std::map<int, int64_t> graph_kernels;
@@ -2131,7 +2130,7 @@ int hfm_mg_create(const hfm_mg_config *cfg, int Z, int Y, int X, int slots, hfm_
   if (!st) st = wait_fail_counters(&m->wait_fail);
   if (!st && cudaStreamCreateWithFlags(&m->cap, cudaStreamNonBlocking) != cudaSuccess)
     st = fail(HFM_ERR_CUDA, "cudaStreamCreate failed");
-  for (cudaEvent_t *e : {&m->masks_done, &m->loads_done, &m->cancels_done})
+  for (cudaEvent_t *e : {&m->runs_done, &m->loads_done, &m->cancels_done})
     if (!st && cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess)
       st = fail(HFM_ERR_CUDA, "cudaEventCreate failed");
   if (!st) {
@@ -2153,7 +2152,7 @@ int hfm_mg_create(const hfm_mg_config *cfg, int Z, int Y, int X, int slots, hfm_
   if (st) {
     for (void *p : m->allocs) cudaFree(p);
     if (m->cap) cudaStreamDestroy(m->cap);
-    for (cudaEvent_t e : {m->masks_done, m->loads_done, m->cancels_done})
+    for (cudaEvent_t e : {m->runs_done, m->loads_done, m->cancels_done})
       if (e) cudaEventDestroy(e);
     return st;
   }
@@ -2170,7 +2169,7 @@ int hfm_mg_destroy(hfm_mg *m) {
     cudaStreamDestroy(m->cap);
   }
   cudaDeviceSynchronize();
-  for (cudaEvent_t e : {m->masks_done, m->loads_done, m->cancels_done})
+  for (cudaEvent_t e : {m->runs_done, m->loads_done, m->cancels_done})
     if (e) cudaEventDestroy(e);
   for (void *p : m->allocs) cudaFree(p);
   delete m;
@@ -2217,13 +2216,15 @@ class MaskOrder {
       on_ = false;
     }
     if (!on_) return;
-    cudaStreamWaitEvent(s_, call == MASK_CANCEL ? m->loads_done : m->masks_done, 0);
-    if (call != MASK_RUN) cudaStreamWaitEvent(s_, m->cancels_done, 0);
+    // a load has waited for the runs and cancels before it, so a wait for it is one for them too
+    cudaStreamWaitEvent(s_, m->loads_done, 0);
+    if (call != MASK_CANCEL && m->runs) cudaStreamWaitEvent(s_, m->runs_done, 0);
+    if (call != MASK_RUN && m->cancels) cudaStreamWaitEvent(s_, m->cancels_done, 0);
+    if (call == MASK_LOAD) m->runs = m->cancels = false;
+    else (call == MASK_RUN ? m->runs : m->cancels) = true;
   }
   ~MaskOrder() {
-    if (!on_) return;
-    cudaEventRecord(call_ == MASK_CANCEL ? m_->cancels_done : m_->masks_done, s_);
-    if (call_ == MASK_LOAD) cudaEventRecord(m_->loads_done, s_);
+    if (on_) cudaEventRecord(call_ == MASK_LOAD ? m_->loads_done : call_ == MASK_RUN ? m_->runs_done : m_->cancels_done, s_);
   }
   MaskOrder(const MaskOrder &) = delete;
   MaskOrder &operator=(const MaskOrder &) = delete;
